@@ -1,33 +1,63 @@
 // batched_local.cu -- many independent dense-Gaussian targets of uneven
 // dimension sampled in ONE persistent launch (MALA or HMC).
 //
-// Work items are tiles of up to 32 chains of one target; CTAs pull items from
-// an atomic counter (a persistent scheduler: long items never leave SMs idle
-// behind short ones) and run all n_steps of their tile before taking the next.
-// A tile keeps its positions, gradients and log-densities in shared memory
-// for the whole run. The gradient of log p = -0.5 dx^T P dx (dx = x - mean,
-// P symmetric) is a [32 x d] x [d x d] product per evaluation: each thread owns
-// 8 chains x 4 coordinates of the output and streams P rows from L2 (one P per
-// target serves all its tiles), dx comes from shared memory.
+// Work items are chain tiles of one target; CTAs pull items from an atomic
+// counter (a persistent scheduler, the largest dimensions first: long items
+// never leave SMs idle behind short ones) and run all n_steps of their tile
+// before taking the next. The gradient of log p = -0.5 dx^T P dx (dx = x -
+// mean, P symmetric) is a [chains x d] x [d x d] FP32 product per evaluation,
+// which is what the kernel spends its time on (FMA issue; 2 d^2 FLOPs per
+// chain and evaluation against 4 d + 8 bytes per chain and step).
+//
+// Tile: 12 warps, each owning a 32-chain x 32-coordinate block of the product
+// (8 chains x 4 coordinates per thread; lanes 4 chains x 8 coordinate groups,
+// so that every 16-byte shared-memory read of a warp is conflict-free). A
+// target of d coordinates takes cb = ceil(d / 32) warps side by side and up
+// to floor(12 / cb) chain blocks above each other, so that narrow targets
+// fill the CTA with more chains instead of leaving threads idle. Positions,
+// momenta and gradients of the trajectory stay in the owner threads'
+// registers; dx goes through shared memory and P, packed once per call into
+// rows of 32 cb values, streams from L2 in 16-row stages (16-byte cp.async,
+// three in flight). Each product element is one FMA chain
+// in k order, and the per-chain sums keep one fixed order whatever the tile
+// shape, so the tile shape never changes a trajectory.
+//
+// Measured (48 targets of 8-256 dimensions, 146,569 chains; before: 32-chain
+// tiles of 8 warps with P read from L2 into registers and all state in shared
+// memory): @@MEASURED@@
 //
 // Step semantics are those of fmc_local_steps (MALA.py:26-89, HMC.py:98-151
 // with an identity mass matrix); the output of target t is written to its own
 // buffers [n_chains_t, buf_len, d_t] at the clamped cursor.
+#include <algorithm>
+#include <string.h>
 #include <vector>
 #include "local_steps.cuh"
 
 namespace fmc {
 
-constexpr int kBT = 32;          // chains per tile
-constexpr int kBThreads = 256;   // 64 column groups x 4 chain groups
+constexpr int kBWarps = 12;
+constexpr int kBThreads = 32 * kBWarps;
 constexpr int kBDMax = 256;
+constexpr int kBRows = 32 * kBWarps;     // most chains of a tile (d <= 32)
+constexpr int kBStage = 16;              // rows of P per stage
+constexpr int kBStages = 3;
+// dx rows are padded by 4 floats (consecutive rows four banks apart); the
+// largest of rows * (32 cb + 4) over the tile shapes is 384 * 36
+constexpr int kBDxFloats = kBRows * 36;
+// P stages, or the second array of the MALA sums between evaluations
+constexpr int kBPFloats = kBDxFloats;
+static_assert(kBStages * kBStage * kBDMax <= kBPFloats, "P stages exceed their area");
+constexpr int kBPartFloats = kBWarps * 32 * 8;
 
 struct BatchTarget {
   const float* precision;   // [d, d]
+  float* packed;            // [round_up(d, 16), round_up(d, 32)] (k_pack_precision)
   const float* mean;        // [d] or NULL
   float const_term;
   int d;
   int n_chains;
+  int tile_rows;            // chains per work item (a multiple of 32)
   int chain_offset;         // first row of this target in x0 / x_last / lp_last ([sum C, 256])
   float* out_pos;           // [n_chains, buf_len, d]
   float* out_logp;          // [n_chains, buf_len]
@@ -43,7 +73,7 @@ struct BatchArgs {
   const int32_t* item_chain0;   // [n_items]
   int n_items;
   int* next_item;               // scheduler counter (zeroed before the launch)
-  int kind, n_leapfrog, S, thin;
+  int n_leapfrog, S, thin;
   int64_t buf_len, start;
   Rng rng;
   const float* x0;              // [sum C, 256] (row stride 256)
@@ -51,268 +81,398 @@ struct BatchArgs {
   float* lp_last;               // [sum C]
 };
 
-// Y[c][j] = sum_k DX[c][k] P[k][j] for the tile; also lp_c = -0.5 sum_j DX Y + const.
-// Thread (cg, jg): chains cg*8..cg*8+7, columns jg*4..jg*4+3. The k loop runs
-// in chunks of 4 rows of P with the next two chunks' P values already in
-// registers (the rows stream from L2 with only 8 warps per SM to hide their
-// latency); the 8 chains' dx for a chunk are one float4 shared-memory load each.
-__device__ __forceinline__ void load_p4(const float* __restrict__ P, int d, int k0, int j0, float (&p)[4][4]) {
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int k = k0 + r;
-    const float* row = P + (int64_t)k * d + j0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) p[r][u] = (k < d && j0 + u < d) ? __ldg(row + u) : 0.f;
-  }
+struct BatchSmem {
+  float4* X;      // [8][kBThreads] positions, owner thread's layout
+  float4* G;      // [8][kBThreads] gradients at X
+  float* DX;      // [rows][32 cb + 4]
+  float* P;       // [kBStages][kBStage][32 cb]
+  float* part;    // [rows][8 cb] per-thread partials of dx . P dx
+  float *lpx, *lpy, *sA, *sB, *lpr, *logu;   // [kBRows] per chain
+  int* acc;
+};
+constexpr size_t kBSmemBytes =
+    sizeof(float) * (2 * 8 * 4 * (size_t)kBThreads + kBDxFloats + kBPFloats + kBPartFloats + 7 * (size_t)kBRows);
+static_assert(kBSmemBytes <= 227 * 1024, "shared memory");
+
+// The precision matrices in the layout the product streams: [16 ns][32 cb]
+// with zeros outside [d, d], so that every stage of 16 rows is one contiguous
+// 16-byte aligned block whatever d is.
+__global__ void k_pack_precision(const BatchTarget* __restrict__ targets) {
+  const BatchTarget T = targets[blockIdx.x];
+  const int w = (T.d + 31) & ~31, kp = (T.d + kBStage - 1) & ~(kBStage - 1);
+  for (int k = blockIdx.y; k < kp; k += gridDim.y)
+    for (int j = threadIdx.x; j < w; j += blockDim.x)
+      T.packed[k * w + j] = (k < T.d && j < T.d) ? __ldg(T.precision + (int64_t)k * T.d + j) : 0.f;
 }
 
-__device__ void dense_eval(const BatchTarget& T, const float* X, float* DX, float* G, float* lp, float* red) {
-  const int tid = threadIdx.x, jg = tid & 63, cg = tid >> 6;
-  const int d = T.d;
-  {
-    // dx = x - mean, zero beyond d up to the next multiple of 4 (read by the float4 loads)
-    const int c = tid >> 3, sub = tid & 7;
-    const int d4 = (d + 3) & ~3;
-    for (int j = sub; j < d4; j += 8)
-      DX[c * kBDMax + j] = (j < d) ? X[c * kBDMax + j] - (T.mean ? __ldg(T.mean + j) : 0.f) : 0.f;
-  }
+// one stage (16 rows of 32 cb packed values) into shared memory
+__device__ __forceinline__ void load_stage(const float* __restrict__ P, int w, int k0, float* dst) {
+  const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(dst);
+  const float* src = P + k0 * w;
+  for (int e = threadIdx.x; e < kBStage / 4 * w; e += kBThreads)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s0 + 16 * e), "l"(src + 4 * e));
+}
+
+// g[c][.] = -(dx P) of this thread's 8 chains x 4 coordinates at positions y;
+// with lp != NULL also lp[row] = -0.5 dx . P dx + const for every chain.
+// Starts with a barrier (shared buffers of earlier phases are free after it);
+// ends with a barrier only when lp is written.
+__device__ __forceinline__ void dense_eval(const BatchTarget& T, const BatchSmem& sm, int cb, bool on, int row0, int j0,
+                                           const float4& mean, const float (&y)[8][4], float (&g)[8][4],
+                                           float* lp, int rows) {
+  const int d = T.d, w = 32 * cb, ldx = w + 4;
+  const int ns = (d + kBStage - 1) / kBStage;
   __syncthreads();
-  float acc[8][4] = {};
-  const int j0 = jg * 4;
-  if (j0 < d) {
-    // three register buffers in fixed roles over an unrolled group of three
-    // chunks, so no buffer is ever copied; rows >= d read as zeros
-    float pa[4][4], pb[4][4], pc[4][4];
-    auto fma_chunk = [&](int k0, const float (&p)[4][4]) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 xv = *reinterpret_cast<const float4*>(DX + (cg * 8 + c) * kBDMax + k0);
+  for (int s = 0; s < kBStages - 1; ++s) {
+    if (s < ns) load_stage(T.packed, w, s * kBStage, sm.P + s * kBStage * w);
+    asm volatile("cp.async.commit_group;");
+  }
+  if (on) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          acc[c][u] = fmaf(xv.x, p[0][u], acc[c][u]);
-          acc[c][u] = fmaf(xv.y, p[1][u], acc[c][u]);
-          acc[c][u] = fmaf(xv.z, p[2][u], acc[c][u]);
-          acc[c][u] = fmaf(xv.w, p[3][u], acc[c][u]);
+    for (int c = 0; c < 8; ++c) {
+      // dx = x - mean, zero on the padding coordinates
+      float4 v;
+      v.x = j0 + 0 < d ? y[c][0] - mean.x : 0.f;
+      v.y = j0 + 1 < d ? y[c][1] - mean.y : 0.f;
+      v.z = j0 + 2 < d ? y[c][2] - mean.z : 0.f;
+      v.w = j0 + 3 < d ? y[c][3] - mean.w : 0.f;
+      *reinterpret_cast<float4*>(sm.DX + (row0 + 4 * c) * ldx + j0) = v;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) g[c][u] = 0.f;
+  int buf = 0;
+  for (int s = 0; s < ns; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kBStages - 2));
+    __syncthreads();
+    {
+      // the buffer read in the previous iteration, which every warp has left
+      const int nx = s + kBStages - 1;
+      const int nb = buf == 0 ? kBStages - 1 : buf - 1;
+      if (nx < ns) load_stage(T.packed, w, nx * kBStage, sm.P + nb * kBStage * w);
+      asm volatile("cp.async.commit_group;");
+    }
+    if (on) {
+      const float* Ps = sm.P + buf * kBStage * w + j0;
+      const float* Xs = sm.DX + row0 * ldx + s * kBStage;
+      // rows of P past d are zero; dx has zeros there too up to the tile's 32 cb columns
+#pragma unroll
+      for (int k = 0; k < kBStage; k += 4) {
+        float4 p[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) p[r] = *reinterpret_cast<const float4*>(Ps + (k + r) * w);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float4 x = *reinterpret_cast<const float4*>(Xs + 4 * c * ldx + k);
+          const float xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            g[c][0] = fmaf(xv[r], p[r].x, g[c][0]);
+            g[c][1] = fmaf(xv[r], p[r].y, g[c][1]);
+            g[c][2] = fmaf(xv[r], p[r].z, g[c][2]);
+            g[c][3] = fmaf(xv[r], p[r].w, g[c][3]);
+          }
         }
       }
-    };
-    load_p4(T.precision, d, 0, j0, pa);
-    load_p4(T.precision, d, 4, j0, pb);
-    for (int k0 = 0; k0 < d; k0 += 12) {
-      load_p4(T.precision, d, k0 + 8, j0, pc);
-      fma_chunk(k0, pa);
-      if (k0 + 4 >= d) break;
-      load_p4(T.precision, d, k0 + 12, j0, pa);
-      fma_chunk(k0 + 4, pb);
-      if (k0 + 8 >= d) break;
-      load_p4(T.precision, d, k0 + 16, j0, pb);
-      fma_chunk(k0 + 8, pc);
     }
+    buf = buf == kBStages - 1 ? 0 : buf + 1;
   }
-  // gradient -P dx and the per-chain partial of dx . P dx
-  float part[8];
+  if (lp != nullptr) {
+    const int nj = 8 * cb;
+    if (on) {
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    part[c] = 0.f;
+      for (int c = 0; c < 8; ++c) {
+        const float4 v = *reinterpret_cast<const float4*>(sm.DX + (row0 + 4 * c) * ldx + j0);
+        const float xv[4] = {v.x, v.y, v.z, v.w};
+        float q = 0.f;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + u;
-      if (j < d) {
-        G[(cg * 8 + c) * kBDMax + j] = -acc[c][u];
-        part[c] += DX[(cg * 8 + c) * kBDMax + j] * acc[c][u];
+        for (int u = 0; u < 4; ++u)
+          if (j0 + u < d) q = fmaf(xv[u], g[c][u], q);
+        sm.part[(row0 + 4 * c) * nj + (j0 >> 2)] = q;
       }
     }
-  }
-  // reduce over the 64 column groups: warp shuffles then shared memory
+    __syncthreads();
+    // per chain: the partials of the 64 coordinate groups (absent ones zero)
+    // as two balanced trees of 32, eight lanes per chain
+    const int sub = threadIdx.x & 7;
+    for (int r = threadIdx.x >> 3; r < ((rows + 3) & ~3); r += kBThreads / 8) {
+      const float* pr = sm.part + r * nj;
+      float h[2];
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    float v = part[c];
+      for (int b = 0; b < 2; ++b) {
+        float v[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((tid & 31) == 0) red[(cg * 8 + c) * 2 + ((tid >> 5) & 1)] = v;
+        for (int q = 0; q < 4; ++q) {
+          const int i = 32 * b + sub + 8 * q;
+          v[q] = (r < rows && i < nj) ? pr[i] : 0.f;
+        }
+        float t = (v[0] + v[2]) + (v[1] + v[3]);
+        t += __shfl_xor_sync(0xffffffffu, t, 4);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        h[b] = t;
+      }
+      if (sub == 0 && r < rows) lp[r] = -0.5f * (h[0] + h[1]) + T.const_term;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  if (tid < kBT) lp[tid] = -0.5f * (red[tid * 2] + red[tid * 2 + 1]) + T.const_term;
-  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) g[c][u] = -g[c][u];
 }
 
-// Elementwise passes over a tile use the same mapping: 8 threads per chain
-// (256 threads = 32 chains), thread tid on chain tid >> 3 and coordinates
-// (tid & 7) + 8i.
-// per-chain sum over j < d of f(c, j) in a fixed order: 8 threads per chain
-// (256 threads = 32 chains), strided over j, then a 3-level shuffle
-template <typename F>
-__device__ __forceinline__ float chain_sum(int d, F f) {
-  const int tid = threadIdx.x, c = tid >> 3, sub = tid & 7;
-  float v = 0.f;
-  for (int j = sub; j < d; j += 8) v += f(c, j);
-  v += __shfl_xor_sync(0xffffffffu, v, 1);
-  v += __shfl_xor_sync(0xffffffffu, v, 2);
-  v += __shfl_xor_sync(0xffffffffu, v, 4);
-  return v;
+// out[r] = sum over j < d of E[r][j]^2, eight lanes per chain (lane sub takes
+// j = sub, sub + 8, ...), then a three-level butterfly
+__device__ __forceinline__ void row_sumsq(const float* E, int ldx, int d, int rows, float* out) {
+  const int sub = threadIdx.x & 7;
+  for (int r = threadIdx.x >> 3; r < ((rows + 3) & ~3); r += kBThreads / 8) {
+    float v = 0.f;
+    if (r < rows)
+      for (int j = sub; j < d; j += 8) v = fmaf(E[r * ldx + j], E[r * ldx + j], v);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    if (sub == 0 && r < rows) out[r] = v;
+  }
 }
 
-// normal for (chain c of T, step s, coordinate j): explicit or Philox
-__device__ __forceinline__ float draw_normal(const BatchArgs& a, const Rng& rng, const BatchTarget& T, int c, int s,
-                                             int j) {
-  if (T.noise) return (c < T.n_chains) ? __ldg(T.noise + ((int64_t)c * a.S + s) * T.d + j) : 0.f;
-  const u32x4 r = rng.draw((uint64_t)(T.chain_offset + c), (uint64_t)s, (uint32_t)(j >> 1), RNG_TAG_LOCAL_NORMAL);
-  float z0, z1;
-  box_muller(r.x, r.y, z0, z1);
-  return (j & 1) ? z1 : z0;
+// normals of chain c of T at step s for coordinates j0 .. j0 + 3 (j0 a
+// multiple of 4): explicit, or component j & 1 of the Box-Muller pair of the
+// Philox block keyed by j >> 1
+__device__ __forceinline__ void draw_normals4(const BatchArgs& a, const Rng& rng, const BatchTarget& T, int c, int s,
+                                              int j0, float (&xi)[4]) {
+  if (T.noise) {
+    const float* row = T.noise + ((int64_t)c * a.S + s) * T.d + j0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) xi[u] = (c < T.n_chains && j0 + u < T.d) ? __ldg(row + u) : 0.f;
+    return;
+  }
+#pragma unroll
+  for (int u = 0; u < 4; u += 2) {
+    const u32x4 r = rng.draw((uint64_t)(T.chain_offset + c), (uint64_t)s, (uint32_t)((j0 + u) >> 1),
+                             RNG_TAG_LOCAL_NORMAL);
+    box_muller(r.x, r.y, xi[u], xi[u + 1]);
+  }
 }
 
-__global__ void __launch_bounds__(kBThreads) k_batched_dense(const BatchArgs a) {
-  extern __shared__ float sm[];
+template <int KIND>
+__global__ void __launch_bounds__(kBThreads, 1) k_batched_dense(const BatchArgs a) {
+  extern __shared__ __align__(16) float smraw[];
   const Rng rng = a.rng.at_epoch();
-  float* X = sm;                      // [32][256] current positions
-  float* Gx = X + kBT * kBDMax;       // gradient at X
-  float* Y = Gx + kBT * kBDMax;       // proposal / leapfrog position
-  float* Gy = Y + kBT * kBDMax;       // gradient at Y
-  float* DX = Gy + kBT * kBDMax;      // scratch dx
-  float* Pm = DX + kBT * kBDMax;      // HMC momentum
-  float* lpx = Pm + kBT * kBDMax;     // [32]
-  float* lpy = lpx + kBT;
-  float* red = lpy + kBT;             // [64]
-  float* sA = red + 2 * kBT;          // [32] per-chain sums
-  float* sB = sA + kBT;
-  float* xr_lp = sB + kBT;            // [32] log-density of the last written row
+  BatchSmem sm;
+  sm.X = reinterpret_cast<float4*>(smraw);
+  sm.G = sm.X + 8 * kBThreads;
+  sm.DX = reinterpret_cast<float*>(sm.G + 8 * kBThreads);
+  sm.P = sm.DX + kBDxFloats;
+  sm.part = sm.P + kBPFloats;
+  sm.lpx = sm.part + kBPartFloats;
+  sm.lpy = sm.lpx + kBRows;
+  sm.sA = sm.lpy + kBRows;
+  sm.sB = sm.sA + kBRows;
+  sm.lpr = sm.sB + kBRows;
+  sm.logu = sm.lpr + kBRows;
+  sm.acc = reinterpret_cast<int*>(sm.logu + kBRows);
   __shared__ int item_s;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int s_rec = (a.S - 1) / a.thin * a.thin;   // the last recorded step
 
   for (;;) {
     if (tid == 0) item_s = atomicAdd(a.next_item, 1);
     __syncthreads();
     const int item = item_s;
-    __syncthreads();
     if (item >= a.n_items) break;
     const BatchTarget T = a.targets[a.item_target[item]];
     const int c0 = a.item_chain0[item];
-    const int nc = min(kBT, T.n_chains - c0);
-    const int d = T.d;
-    const float dt = T.step;
-    for (int e = tid; e < kBT * kBDMax; e += kBThreads) {
-      const int c = e / kBDMax, j = e - c * kBDMax;
-      X[e] = (c < nc && j < d) ? a.x0[(int64_t)(T.chain_offset + c0 + c) * kBDMax + j] : 0.f;
+    const int nc = min(T.tile_rows, T.n_chains - c0);
+    const int d = T.d, cb = (d + 31) >> 5, ldx = 32 * cb + 4;
+    const int rows = (nc + 31) & ~31;
+    const int rblk = wid / cb;
+    const bool on = rblk * 32 < rows;                       // this warp has a block
+    const int row0 = rblk * 32 + (lane >> 3);               // chains row0 + 4 c
+    const int j0 = (wid - rblk * cb) * 32 + (lane & 7) * 4;  // coordinates j0 .. j0 + 3
+    const bool vec_out = (d & 3) == 0 && ((uintptr_t)T.out_pos & 15) == 0;
+    const float dt = T.step, dt2 = dt * dt;
+    float4 mean = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (T.mean != nullptr) {
+      if (j0 + 0 < d) mean.x = __ldg(T.mean + j0);
+      if (j0 + 1 < d) mean.y = __ldg(T.mean + j0 + 1);
+      if (j0 + 2 < d) mean.z = __ldg(T.mean + j0 + 2);
+      if (j0 + 3 < d) mean.w = __ldg(T.mean + j0 + 3);
     }
-    __syncthreads();
-    dense_eval(T, X, DX, Gx, lpx, red);
+    float y[8][4], g[8][4];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int r = row0 + 4 * c;
+      const float* xr = a.x0 + (int64_t)(T.chain_offset + c0 + r) * kBDMax + j0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) y[c][u] = (on && r < nc && j0 + u < d) ? xr[u] : 0.f;
+      sm.X[c * kBThreads + tid] = make_float4(y[c][0], y[c][1], y[c][2], y[c][3]);
+    }
+    dense_eval(T, sm, cb, on, row0, j0, mean, y, g, sm.lpx, rows);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) sm.G[c * kBThreads + tid] = make_float4(g[c][0], g[c][1], g[c][2], g[c][3]);
+
     for (int s = 0; s < a.S; ++s) {
-      // ---- proposal (MALA) or leapfrog trajectory (HMC) into Y / Gy / lpy
-      if (a.kind == FMC_KERNEL_MALA) {
-        const float dt2 = dt * dt;
-        for (int j = tid & 7, c = tid >> 3; j < d; j += 8) {
-          const float xi = draw_normal(a, rng, T, c0 + c, s, j);
-          const int i = c * kBDMax + j;
-          Y[i] = (X[i] + dt2 * Gx[i] / 2.0f) + dt * xi;
+      // log-uniforms of the step, one chain per thread
+      if (tid < nc) {
+        float u;
+        if (T.unif) u = __ldg(T.unif + (int64_t)(c0 + tid) * a.S + s);
+        else u = u32_to_unit(rng.draw((uint64_t)(T.chain_offset + c0 + tid), (uint64_t)s, 0u, RNG_TAG_LOCAL_UNIFORM).x);
+        sm.logu[tid] = logf(u);
+      }
+      // ---- proposal (MALA) or leapfrog trajectory (HMC): y, g, lpy
+      if constexpr (KIND == FMC_KERNEL_MALA) {
+        if (on) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            float xi[4];
+            draw_normals4(a, rng, T, c0 + row0 + 4 * c, s, j0, xi);
+            const float4 x = sm.X[c * kBThreads + tid], gx = sm.G[c * kBThreads + tid];
+            y[c][0] = fmaf(dt, xi[0], x.x + dt2 * gx.x / 2.0f);
+            y[c][1] = fmaf(dt, xi[1], x.y + dt2 * gx.y / 2.0f);
+            y[c][2] = fmaf(dt, xi[2], x.z + dt2 * gx.z / 2.0f);
+            y[c][3] = fmaf(dt, xi[3], x.w + dt2 * gx.w / 2.0f);
+          }
+        }
+        dense_eval(T, sm, cb, on, row0, j0, mean, y, g, sm.lpy, rows);
+        // prop - mean0 into DX, x - mean1 into the P area; squared norms per chain
+        if (on) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const float4 x = sm.X[c * kBThreads + tid], gx = sm.G[c * kBThreads + tid];
+            float4 ea, eb;
+            ea.x = y[c][0] - (x.x + dt2 * gx.x / 2.0f);
+            ea.y = y[c][1] - (x.y + dt2 * gx.y / 2.0f);
+            ea.z = y[c][2] - (x.z + dt2 * gx.z / 2.0f);
+            ea.w = y[c][3] - (x.w + dt2 * gx.w / 2.0f);
+            eb.x = x.x - (y[c][0] + dt2 * g[c][0] / 2.0f);
+            eb.y = x.y - (y[c][1] + dt2 * g[c][1] / 2.0f);
+            eb.z = x.z - (y[c][2] + dt2 * g[c][2] / 2.0f);
+            eb.w = x.w - (y[c][3] + dt2 * g[c][3] / 2.0f);
+            *reinterpret_cast<float4*>(sm.DX + (row0 + 4 * c) * ldx + j0) = ea;
+            *reinterpret_cast<float4*>(sm.P + (row0 + 4 * c) * ldx + j0) = eb;
+          }
         }
         __syncthreads();
-        dense_eval(T, Y, DX, Gy, lpy, red);
-        // |prop - mean0|^2 and |x - mean1|^2 per chain
-        const float va = chain_sum(d, [&](int c, int j) {
-          const int i = c * kBDMax + j;
-          const float ea = Y[i] - (X[i] + dt2 * Gx[i] / 2.0f);
-          return ea * ea;
-        });
-        const float vb = chain_sum(d, [&](int c, int j) {
-          const int i = c * kBDMax + j;
-          const float eb = X[i] - (Y[i] + dt2 * Gy[i] / 2.0f);
-          return eb * eb;
-        });
-        if ((tid & 7) == 0) { sA[tid >> 3] = va; sB[tid >> 3] = vb; }
+        row_sumsq(sm.DX, ldx, d, rows, sm.sA);
+        row_sumsq(sm.P, ldx, d, rows, sm.sB);
         __syncthreads();
       } else {
-        for (int j = tid & 7, c = tid >> 3; j < d; j += 8) {
-          const int i = c * kBDMax + j;
-          Pm[i] = draw_normal(a, rng, T, c0 + c, s, j);
-          Y[i] = X[i];
-          Gy[i] = Gx[i];
+        float p[8][4];
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) p[c][u] = 0.f;
+        __syncthreads();   // the last step's readers of DX are done
+        if (on) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            draw_normals4(a, rng, T, c0 + row0 + 4 * c, s, j0, p[c]);
+            *reinterpret_cast<float4*>(sm.DX + (row0 + 4 * c) * ldx + j0) =
+                make_float4(p[c][0], p[c][1], p[c][2], p[c][3]);
+            const float4 x = sm.X[c * kBThreads + tid], gx = sm.G[c * kBThreads + tid];
+            y[c][0] = x.x; y[c][1] = x.y; y[c][2] = x.z; y[c][3] = x.w;
+            // row 0: half kick with the gradient at x
+            p[c][0] = fmaf(dt * 0.5f, gx.x, p[c][0]);
+            p[c][1] = fmaf(dt * 0.5f, gx.y, p[c][1]);
+            p[c][2] = fmaf(dt * 0.5f, gx.z, p[c][2]);
+            p[c][3] = fmaf(dt * 0.5f, gx.w, p[c][3]);
+          }
         }
         __syncthreads();
-        {
-          const float v0 = chain_sum(d, [&](int c, int j) {
-            const float p = Pm[c * kBDMax + j];
-            return p * p;
-          });
-          if ((tid & 7) == 0) sA[tid >> 3] = v0;
-        }
-        __syncthreads();
-        // row 0: half kick with the gradient at x
-        for (int j = tid & 7, c = tid >> 3; j < d; j += 8) {
-          const int i = c * kBDMax + j;
-          Pm[i] = Pm[i] + (dt * 0.5f) * Gy[i];
-        }
-        __syncthreads();
+        row_sumsq(sm.DX, ldx, d, rows, sm.sA);
         for (int r = 1; r <= a.n_leapfrog + 1; ++r) {
-          const float ek = (r == a.n_leapfrog + 1) ? dt * 0.5f : dt;
-          for (int j = tid & 7, c = tid >> 3; j < d; j += 8) {
-            const int i = c * kBDMax + j;
-            Y[i] = Y[i] + dt * Pm[i];
-          }
-          __syncthreads();
-          dense_eval(T, Y, DX, Gy, lpy, red);
-          for (int j = tid & 7, c = tid >> 3; j < d; j += 8) {
-            const int i = c * kBDMax + j;
-            Pm[i] = Pm[i] + ek * Gy[i];
-          }
-          __syncthreads();
+          const bool end = r == a.n_leapfrog + 1;
+          const float ek = end ? dt * 0.5f : dt;
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) y[c][u] = fmaf(dt, p[c][u], y[c][u]);
+          // only the gradient is used before the end point
+          dense_eval(T, sm, cb, on, row0, j0, mean, y, g, end ? sm.lpy : nullptr, rows);
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) p[c][u] = fmaf(ek, g[c][u], p[c][u]);
         }
-        {
-          const float v1 = chain_sum(d, [&](int c, int j) {
-            const float p = Pm[c * kBDMax + j];
-            return p * p;
-          });
-          if ((tid & 7) == 0) sB[tid >> 3] = v1;
+        if (on) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<float4*>(sm.DX + (row0 + 4 * c) * ldx + j0) =
+                make_float4(p[c][0], p[c][1], p[c][2], p[c][3]);
         }
+        __syncthreads();
+        row_sumsq(sm.DX, ldx, d, rows, sm.sB);
         __syncthreads();
       }
       // ---- accept per chain (float-float log-ratio), then commit
-      __shared__ int acc_s[kBT];
-      if (tid < kBT) {
+      const bool rec = s % a.thin == 0;
+      const int64_t orow = a.start + s / a.thin;
+      if (tid < nc) {
         const int c = tid;
-        const int64_t chain = T.chain_offset + c0 + c;
-        float u;
-        if (T.unif) u = (c < nc) ? __ldg(T.unif + (int64_t)(c0 + c) * a.S + s) : 1.f;
-        else u = u32_to_unit(rng.draw((uint64_t)chain, (uint64_t)s, 0u, RNG_TAG_LOCAL_UNIFORM).x);
-        const float logu = logf(u);
         ff ratio;
-        if (a.kind == FMC_KERNEL_MALA) {
-          const ff q = two_sum(sA[c], -sB[c]);
-          ratio = ff_add(two_sum(lpy[c], -lpx[c]), ff_mul_f(q, 0.5f / (dt * dt)));
+        if constexpr (KIND == FMC_KERNEL_MALA) {
+          const ff q = two_sum(sm.sA[c], -sm.sB[c]);
+          ratio = ff_add(two_sum(sm.lpy[c], -sm.lpx[c]), ff_mul_f(q, 0.5f / (dt * dt)));
         } else {
-          ratio = ff_add(two_sum(-lpx[c], 0.5f * sA[c]), ff_neg(two_sum(-lpy[c], 0.5f * sB[c])));
+          ratio = ff_add(two_sum(-sm.lpx[c], 0.5f * sm.sA[c]), ff_neg(two_sum(-sm.lpy[c], 0.5f * sm.sB[c])));
         }
-        acc_s[c] = (c < nc) && f_lt_ff(logu, ratio) ? 1 : 0;
-      }
-      __syncthreads();
-      for (int j = tid & 7, c = tid >> 3; j < d; j += 8) {
-        if (acc_s[c]) {
-          const int i = c * kBDMax + j;
-          X[i] = Y[i];
-          Gx[i] = Gy[i];
-        }
-      }
-      if (tid < kBT && acc_s[tid]) lpx[tid] = lpy[tid];
-      __syncthreads();
-      if (s % a.thin == 0) {
-        const int64_t row = a.start + s / a.thin;
-        for (int j = tid & 7, c = tid >> 3; c < nc && j < d; j += 8) {
-          __stcs(T.out_pos + ((int64_t)(c0 + c) * a.buf_len + row) * d + j, X[c * kBDMax + j]);
-        }
-        if (tid < nc) {
-          __stcs(T.out_logp + (int64_t)(c0 + tid) * a.buf_len + row, lpx[tid]);
-          __stcs(T.out_acc + (int64_t)(c0 + tid) * a.buf_len + row, acc_s[tid] ? 1.f : 0.f);
-          xr_lp[tid] = lpx[tid];
-        }
-        for (int j = tid & 7, c = tid >> 3; c < nc && j < d; j += 8) {
-          a.x_last[(int64_t)(T.chain_offset + c0 + c) * kBDMax + j] = X[c * kBDMax + j];
+        const bool acc = f_lt_ff(sm.logu[c], ratio);
+        sm.acc[c] = acc ? 1 : 0;
+        const float lp = acc ? sm.lpy[c] : sm.lpx[c];
+        sm.lpx[c] = lp;
+        if (rec) {
+          __stcs(T.out_logp + (int64_t)(c0 + c) * a.buf_len + orow, lp);
+          __stcs(T.out_acc + (int64_t)(c0 + c) * a.buf_len + orow, acc ? 1.f : 0.f);
+          if (s == s_rec) a.lp_last[T.chain_offset + c0 + c] = lp;
         }
       }
       __syncthreads();
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const int r = row0 + 4 * c;
+        if (!on || r >= nc) continue;
+        if (sm.acc[r]) {
+          sm.X[c * kBThreads + tid] = make_float4(y[c][0], y[c][1], y[c][2], y[c][3]);
+          sm.G[c * kBThreads + tid] = make_float4(g[c][0], g[c][1], g[c][2], g[c][3]);
+        }
+        if (rec && j0 < d) {
+          const float4 x = sm.X[c * kBThreads + tid];
+          const float xv[4] = {x.x, x.y, x.z, x.w};
+          float* o = T.out_pos + ((int64_t)(c0 + r) * a.buf_len + orow) * d + j0;
+          if (vec_out) {
+            __stcs(reinterpret_cast<float4*>(o), x);
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (j0 + u < d) __stcs(o + u, xv[u]);
+          }
+          if (s == s_rec) {
+            float* xl = a.x_last + (int64_t)(T.chain_offset + c0 + r) * kBDMax + j0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (j0 + u < d) xl[u] = xv[u];
+          }
+        }
+      }
     }
-    if (tid < nc) a.lp_last[T.chain_offset + c0 + tid] = xr_lp[tid];
-    __syncthreads();
+    __syncthreads();   // item_s and the shared buffers are free
   }
+}
+
+// Chains per work item for each target: up to floor(12 / cb) blocks of 32
+// chains (at most `cap`), where cb = ceil(d / 32) warps stand side by side.
+static int batch_tile_rows(int d, int n_chains, int cap) {
+  const int cb = (d + 31) / 32;
+  int rb = kBWarps / cb;
+  if (rb > cap) rb = cap;
+  const int need = (n_chains + 31) / 32;
+  if (rb > need) rb = need;
+  return 32 * rb;
 }
 
 }  // namespace fmc
@@ -321,8 +481,9 @@ using namespace fmc;
 
 extern "C" int fmc_batched_workspace_size(int32_t n_targets, int64_t total_chains, size_t* bytes) {
   FMC_CHECK_ARG(bytes && n_targets >= 1 && total_chains >= 1, "bad arguments");
-  const int64_t items = total_chains / kBT + n_targets;
-  *bytes = (size_t)(256 + n_targets * sizeof(BatchTarget) + 256 + items * 8 + 256);
+  const int64_t items = total_chains / 32 + n_targets;   // at least 32 chains per work item
+  *bytes = (size_t)(256 + n_targets * sizeof(BatchTarget) + 256 + items * 8 + 256) +
+           (size_t)n_targets * kBDMax * kBDMax * sizeof(float);
   return FMC_OK;
 }
 
@@ -344,7 +505,6 @@ extern "C" int fmc_batched_dense_local_steps(const FmcTarget* targets, int32_t n
                 (long long)buf_len);
   FMC_CHECK_ARG(x0 && x_last && lp_last, "NULL device array");
   std::vector<BatchTarget> bt(n_targets);
-  std::vector<int32_t> it, ic;
   int64_t off = 0;
   for (int t = 0; t < n_targets; ++t) {
     const FmcTarget& g = targets[t];
@@ -353,39 +513,68 @@ extern "C" int fmc_batched_dense_local_steps(const FmcTarget* targets, int32_t n
     FMC_CHECK_ARG(g.precision != nullptr, "target %d: no precision matrix", t);
     FMC_CHECK_ARG(n_chains[t] >= 1, "target %d: no chains", t);
     FMC_CHECK_ARG(out_pos[t] && out_logp[t] && out_acc[t], "target %d: NULL output buffer", t);
-    bt[t] = BatchTarget{g.precision, g.mean, g.scalars[0], g.n_dim, n_chains[t], (int)off,
+    bt[t] = BatchTarget{g.precision, nullptr, g.mean, g.scalars[0], g.n_dim, n_chains[t], 0, (int)off,
                         out_pos[t], out_logp[t], out_acc[t], step_sizes[t],
                         noise ? noise[t] : nullptr, unif ? unif[t] : nullptr};
-    for (int c = 0; c < n_chains[t]; c += kBT) {
-      it.push_back(t);
-      ic.push_back(c);
-    }
     off += n_chains[t];
   }
   size_t need = 0;
   fmc_batched_workspace_size(n_targets, off, &need);
   FMC_CHECK_ARG(ws && ws_bytes >= need, "workspace of %zu bytes < %zu needed", ws_bytes, need);
   cudaStream_t st = (cudaStream_t)stream;
+  // Tile height: the most chain blocks per item that still spread over the
+  // SMs. A tile of w warps takes about ceil(w / 4) * 45 d + 2000 cycles per
+  // evaluation (w / 4 warps per scheduler, 32 FMAs per k at about 0.7 of the
+  // issue rate, and the evaluation's barriers); the launch takes the larger
+  // of the mean load per SM and the longest item.
+  const int sms = sm_count();
+  int best_cap = kBWarps;
+  double best = 0.0;
+  for (int cap : {12, 6, 4, 3, 2, 1}) {
+    double total = 0.0, longest = 0.0;
+    for (int t = 0; t < n_targets; ++t) {
+      const int rows = batch_tile_rows(bt[t].d, n_chains[t], cap);
+      const int w = rows / 32 * ((bt[t].d + 31) / 32);
+      const double cost = (w + 3) / 4 * 45.0 * bt[t].d + 2000.0;
+      total += cost * ((n_chains[t] + rows - 1) / rows);
+      if (cost > longest) longest = cost;
+    }
+    const double est = total / sms > longest ? total / sms : longest;
+    if (cap == kBWarps || est < 0.98 * best) {
+      best = est;
+      best_cap = cap;
+    }
+  }
+  // items, the largest dimensions first
+  std::vector<int> order(n_targets);
+  for (int t = 0; t < n_targets; ++t) order[t] = t;
+  std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return bt[p].d > bt[q].d; });
+  std::vector<int32_t> it, ic;
+  for (int t : order) {
+    bt[t].tile_rows = batch_tile_rows(bt[t].d, n_chains[t], best_cap);
+    for (int c = 0; c < n_chains[t]; c += bt[t].tile_rows) {
+      it.push_back(t);
+      ic.push_back(c);
+    }
+  }
+  // scheduler counter, targets and items go up as one copy; copies from
+  // pageable memory are staged before cudaMemcpyAsync returns, so the host
+  // vector may go out of scope
+  const size_t tb = (n_targets * sizeof(BatchTarget) + 255) / 256 * 256;
+  float* packed = (float*)(((uintptr_t)ws + 256 + tb + it.size() * 8 + 15) & ~(uintptr_t)15);
+  for (int t = 0; t < n_targets; ++t) bt[t].packed = packed + (size_t)t * kBDMax * kBDMax;
+  std::vector<char> up(256 + tb + it.size() * 8, 0);
+  memcpy(up.data() + 256, bt.data(), n_targets * sizeof(BatchTarget));
+  memcpy(up.data() + 256 + tb, it.data(), it.size() * 4);
+  memcpy(up.data() + 256 + tb + it.size() * 4, ic.data(), ic.size() * 4);
   char* p = (char*)ws;
-  int* next = (int*)p;
-  p += 256;
-  BatchTarget* dt = (BatchTarget*)p;
-  p += (n_targets * sizeof(BatchTarget) + 255) / 256 * 256;
-  int32_t* ditem_t = (int32_t*)p;
-  int32_t* ditem_c = ditem_t + it.size();
-  // the tables go up with the stream; copies from pageable memory are staged
-  // before cudaMemcpyAsync returns, so the host vectors may go out of scope
-  FMC_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(int), st));
-  FMC_CUDA_TRY(cudaMemcpyAsync(dt, bt.data(), n_targets * sizeof(BatchTarget), cudaMemcpyHostToDevice, st));
-  FMC_CUDA_TRY(cudaMemcpyAsync(ditem_t, it.data(), it.size() * 4, cudaMemcpyHostToDevice, st));
-  FMC_CUDA_TRY(cudaMemcpyAsync(ditem_c, ic.data(), ic.size() * 4, cudaMemcpyHostToDevice, st));
+  FMC_CUDA_TRY(cudaMemcpyAsync(p, up.data(), up.size(), cudaMemcpyHostToDevice, st));
   BatchArgs a{};
-  a.targets = dt;
-  a.item_target = ditem_t;
-  a.item_chain0 = ditem_c;
+  a.targets = (const BatchTarget*)(p + 256);
+  a.item_target = (const int32_t*)(p + 256 + tb);
+  a.item_chain0 = a.item_target + it.size();
   a.n_items = (int)it.size();
-  a.next_item = next;
-  a.kind = params->kind;
+  a.next_item = (int*)p;
   a.n_leapfrog = params->n_leapfrog;
   a.S = n_steps;
   a.thin = thinning;
@@ -395,14 +584,12 @@ extern "C" int fmc_batched_dense_local_steps(const FmcTarget* targets, int32_t n
   a.x0 = x0;
   a.x_last = x_last;
   a.lp_last = lp_last;
-  const size_t smem = (size_t)(6 * kBT * kBDMax + 6 * kBT + 2 * kBT) * sizeof(float);
-  FMC_CUDA_TRY(cudaFuncSetAttribute(k_batched_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  FMC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched_dense, kBThreads, smem));
-  if (per_sm < 1) per_sm = 1;
-  int64_t grid = (int64_t)sm_count() * per_sm;
-  if (grid > a.n_items) grid = a.n_items;
-  k_batched_dense<<<(int)grid, kBThreads, smem, st>>>(a);
+  k_pack_precision<<<dim3((unsigned)n_targets, 16), 256, 0, st>>>(a.targets);
+  FMC_LAUNCH_CHECK();
+  auto kern = params->kind == FMC_KERNEL_MALA ? k_batched_dense<FMC_KERNEL_MALA> : k_batched_dense<FMC_KERNEL_HMC>;
+  FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBSmemBytes));
+  const int grid = a.n_items < sms ? a.n_items : sms;
+  kern<<<grid, kBThreads, kBSmemBytes, st>>>(a);
   FMC_LAUNCH_CHECK();
   return FMC_OK;
 }
