@@ -12,19 +12,28 @@
 // Tile: 12 warps, each owning a 32-chain x 32-coordinate block of the product
 // (8 chains x 4 coordinates per thread; lanes 4 chains x 8 coordinate groups,
 // so that every 16-byte shared-memory read of a warp is conflict-free). A
-// target of d coordinates takes cb = ceil(d / 32) warps side by side and up
-// to floor(12 / cb) chain blocks above each other, so that narrow targets
-// fill the CTA with more chains instead of leaving threads idle. Positions,
-// momenta and gradients of the trajectory stay in the owner threads'
-// registers; dx goes through shared memory and P, packed once per call into
-// rows of 32 cb values, streams from L2 in 16-row stages (16-byte cp.async,
-// three in flight). Each product element is one FMA chain
-// in k order, and the per-chain sums keep one fixed order whatever the tile
-// shape, so the tile shape never changes a trajectory.
+// target of d coordinates takes cb = ceil(d / 32) warps side by side -- a row
+// block of 32 chains -- and up to floor(12 / cb) row blocks, so that narrow
+// targets fill the CTA with more chains instead of leaving threads idle.
+// Positions, momenta and gradients of the trajectory stay in the owner
+// threads' registers; dx is shared by the warps of a row block through shared
+// memory. P, packed once per call into rows of 32 cb values, streams from L2:
+// every warp copies its own 32 columns (cp.async, 8-row stages, three in
+// flight, running on into the next evaluation), so no barrier is needed for
+// P and the only ones in the product loop are the row block's two per
+// evaluation around dx. With one ring per CTA and a CTA barrier per 16 rows
+// instead, warps spent a quarter of their time at that barrier.
+//
+// Each product element is one FMA chain in k order, and the per-chain sums
+// keep one fixed order whatever the tile shape, so the tile shape never
+// changes a trajectory.
 //
 // Measured (48 targets of 8-256 dimensions, 146,569 chains; before: 32-chain
-// tiles of 8 warps with P read from L2 into registers and all state in shared
-// memory): @@MEASURED@@
+// tiles of 8 warps, P read from L2 into registers, all state in shared
+// memory): MALA 10 steps 7.37 -> 3.28 ms, HMC 3 steps of 11
+// gradients 16.4 -> 6.80 ms per call, about 30 TFLOP/s of useful FP32 (46 % of
+// the FMA pipe with padding; issue slots 58 % busy, bound by the latency of the
+// shared-memory reads with two or three warps per scheduler).
 //
 // Step semantics are those of fmc_local_steps (MALA.py:26-89, HMC.py:98-151
 // with an identity mass matrix); the output of target t is written to its own
@@ -40,14 +49,12 @@ constexpr int kBWarps = 12;
 constexpr int kBThreads = 32 * kBWarps;
 constexpr int kBDMax = 256;
 constexpr int kBRows = 32 * kBWarps;     // most chains of a tile (d <= 32)
-constexpr int kBStage = 16;              // rows of P per stage
-constexpr int kBStages = 3;
+constexpr int kBStage = 8;               // rows of P per stage
+constexpr int kBStages = 4;              // stages of a warp's ring
 // dx rows are padded by 4 floats (consecutive rows four banks apart); the
 // largest of rows * (32 cb + 4) over the tile shapes is 384 * 36
 constexpr int kBDxFloats = kBRows * 36;
-// P stages, or the second array of the MALA sums between evaluations
-constexpr int kBPFloats = kBDxFloats;
-static_assert(kBStages * kBStage * kBDMax <= kBPFloats, "P stages exceed their area");
+constexpr int kBRing = kBStages * kBStage * 32;   // floats of one warp's ring
 constexpr int kBPartFloats = kBWarps * 32 * 8;
 
 struct BatchTarget {
@@ -81,17 +88,8 @@ struct BatchArgs {
   float* lp_last;               // [sum C]
 };
 
-struct BatchSmem {
-  float4* X;      // [8][kBThreads] positions, owner thread's layout
-  float4* G;      // [8][kBThreads] gradients at X
-  float* DX;      // [rows][32 cb + 4]
-  float* P;       // [kBStages][kBStage][32 cb]
-  float* part;    // [rows][8 cb] per-thread partials of dx . P dx
-  float *lpx, *lpy, *sA, *sB, *lpr, *logu;   // [kBRows] per chain
-  int* acc;
-};
 constexpr size_t kBSmemBytes =
-    sizeof(float) * (2 * 8 * 4 * (size_t)kBThreads + kBDxFloats + kBPFloats + kBPartFloats + 7 * (size_t)kBRows);
+    sizeof(float) * (2 * 8 * 4 * (size_t)kBThreads + kBDxFloats + kBWarps * kBRing + kBPartFloats + 7 * (size_t)kBRows);
 static_assert(kBSmemBytes <= 227 * 1024, "shared memory");
 
 // The precision matrices in the layout the product streams: [16 ns][32 cb]
@@ -105,101 +103,105 @@ __global__ void k_pack_precision(const BatchTarget* __restrict__ targets) {
       T.packed[k * w + j] = (k < T.d && j < T.d) ? __ldg(T.precision + (int64_t)k * T.d + j) : 0.f;
 }
 
-// one stage (16 rows of 32 cb packed values) into shared memory
-__device__ __forceinline__ void load_stage(const float* __restrict__ P, int w, int k0, float* dst) {
-  const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(dst);
-  const float* src = P + k0 * w;
-  for (int e = threadIdx.x; e < kBStage / 4 * w; e += kBThreads)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s0 + 16 * e), "l"(src + 4 * e));
-}
+// This thread's place in the tile and its row block's shared memory.
+struct BatchBlock {
+  int cb;         // warps (32-coordinate blocks) of the row block
+  int tb;         // thread index within the row block's 32 cb threads
+  int bar;        // the row block's named barrier
+  int r0;         // this thread's chains: r0 + 4 c of the row block's 32
+  int j0;         // its coordinates: j0 .. j0 + 3
+  int ldx;
+  float* DX;      // [32][ldx]
+  float* part;    // [32][8 cb] per-thread partials of dx . P dx
+  float* ring;    // this warp's P stages
+  const float* src;   // its 16 bytes of the packed P's row (lane / 8), column block first
+  int ns, next, buf;  // stages of P, next stage to copy, ring slot to read
+  float4 mean;
+  __device__ __forceinline__ void sync() const {
+    asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(32 * cb) : "memory");
+  }
+  // copy the next stage (8 rows x this warp's 32 columns) into `slot`
+  __device__ __forceinline__ void issue(int slot) {
+    const int lane = threadIdx.x & 31, w = 32 * cb;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ring + slot * (kBStage * 32)) + 16 * lane;
+    const float* p = src + next * kBStage * w;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(p));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 512), "l"(p + 4 * w));
+    asm volatile("cp.async.commit_group;");
+    next = next + 1 == ns ? 0 : next + 1;
+  }
+};
 
 // g[c][.] = -(dx P) of this thread's 8 chains x 4 coordinates at positions y;
-// with lp != NULL also lp[row] = -0.5 dx . P dx + const for every chain.
-// Starts with a barrier (shared buffers of earlier phases are free after it);
-// ends with a barrier only when lp is written.
-__device__ __forceinline__ void dense_eval(const BatchTarget& T, const BatchSmem& sm, int cb, bool on, int row0, int j0,
-                                           const float4& mean, const float (&y)[8][4], float (&g)[8][4],
-                                           float* lp, int rows) {
-  const int d = T.d, w = 32 * cb, ldx = w + 4;
-  const int ns = (d + kBStage - 1) / kBStage;
-  __syncthreads();
+// with lp != NULL also lp[row] = -0.5 dx . P dx + const for the row block's
+// chains. The caller's row block has passed a barrier since its last use of
+// DX; on return DX may still be read by other warps unless lp is given.
+__device__ __forceinline__ void dense_eval(const BatchTarget& T, BatchBlock& B, const float (&y)[8][4],
+                                           float (&g)[8][4], float* lp) {
+  const int d = T.d, ldx = B.ldx, j0 = B.j0;
 #pragma unroll
-  for (int s = 0; s < kBStages - 1; ++s) {
-    if (s < ns) load_stage(T.packed, w, s * kBStage, sm.P + s * kBStage * w);
-    asm volatile("cp.async.commit_group;");
-  }
-  if (on) {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      // dx = x - mean, zero on the padding coordinates
-      float4 v;
-      v.x = j0 + 0 < d ? y[c][0] - mean.x : 0.f;
-      v.y = j0 + 1 < d ? y[c][1] - mean.y : 0.f;
-      v.z = j0 + 2 < d ? y[c][2] - mean.z : 0.f;
-      v.w = j0 + 3 < d ? y[c][3] - mean.w : 0.f;
-      *reinterpret_cast<float4*>(sm.DX + (row0 + 4 * c) * ldx + j0) = v;
-    }
+  for (int c = 0; c < 8; ++c) {
+    // dx = x - mean, zero on the padding coordinates
+    float4 v;
+    v.x = j0 + 0 < d ? y[c][0] - B.mean.x : 0.f;
+    v.y = j0 + 1 < d ? y[c][1] - B.mean.y : 0.f;
+    v.z = j0 + 2 < d ? y[c][2] - B.mean.z : 0.f;
+    v.w = j0 + 3 < d ? y[c][3] - B.mean.w : 0.f;
+    *reinterpret_cast<float4*>(B.DX + (B.r0 + 4 * c) * ldx + j0) = v;
   }
 #pragma unroll
   for (int c = 0; c < 8; ++c)
 #pragma unroll
     for (int u = 0; u < 4; ++u) g[c][u] = 0.f;
-  int buf = 0;
-  for (int s = 0; s < ns; ++s) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kBStages - 2));
-    __syncthreads();
-    {
-      // the buffer read in the previous iteration, which every warp has left
-      const int nx = s + kBStages - 1;
-      const int nb = buf == 0 ? kBStages - 1 : buf - 1;
-      if (nx < ns) load_stage(T.packed, w, nx * kBStage, sm.P + nb * kBStage * w);
-      asm volatile("cp.async.commit_group;");
-    }
-    if (on) {
-      const float* Ps = sm.P + buf * kBStage * w + j0;
-      const float* Xs = sm.DX + row0 * ldx + s * kBStage;
-      // rows of P past d are zero; dx has zeros there too up to the tile's 32 cb columns
+  B.sync();
+  const float* Xs = B.DX + B.r0 * ldx;
+#pragma unroll 1
+  for (int s = 0; s < B.ns; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kBStages - 2) : "memory");
+    __syncwarp();
+    // the slot read in the previous iteration, which every lane has left
+    B.issue((B.buf + kBStages - 1) % kBStages);
+    const float* Ps = B.ring + B.buf * (kBStage * 32) + (threadIdx.x & 7) * 4;
+    // rows of the packed P past d are zero; dx has zeros there too
 #pragma unroll
-      for (int k = 0; k < kBStage; k += 4) {
-        float4 p[4];
+    for (int k = 0; k < kBStage; k += 4) {
+      float4 p[4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) p[r] = *reinterpret_cast<const float4*>(Ps + (k + r) * w);
+      for (int r = 0; r < 4; ++r) p[r] = *reinterpret_cast<const float4*>(Ps + (k + r) * 32);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const float4 x = *reinterpret_cast<const float4*>(Xs + 4 * c * ldx + k);
-          const float xv[4] = {x.x, x.y, x.z, x.w};
+      for (int c = 0; c < 8; ++c) {
+        const float4 x = *reinterpret_cast<const float4*>(Xs + 4 * c * ldx + k);
+        const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            g[c][0] = fmaf(xv[r], p[r].x, g[c][0]);
-            g[c][1] = fmaf(xv[r], p[r].y, g[c][1]);
-            g[c][2] = fmaf(xv[r], p[r].z, g[c][2]);
-            g[c][3] = fmaf(xv[r], p[r].w, g[c][3]);
-          }
+        for (int r = 0; r < 4; ++r) {
+          g[c][0] = fmaf(xv[r], p[r].x, g[c][0]);
+          g[c][1] = fmaf(xv[r], p[r].y, g[c][1]);
+          g[c][2] = fmaf(xv[r], p[r].z, g[c][2]);
+          g[c][3] = fmaf(xv[r], p[r].w, g[c][3]);
         }
       }
     }
-    buf = buf == kBStages - 1 ? 0 : buf + 1;
+    Xs += kBStage;
+    B.buf = (B.buf + 1) % kBStages;
   }
   if (lp != nullptr) {
-    const int nj = 8 * cb;
-    if (on) {
+    const int nj = 8 * B.cb;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 v = *reinterpret_cast<const float4*>(sm.DX + (row0 + 4 * c) * ldx + j0);
-        const float xv[4] = {v.x, v.y, v.z, v.w};
-        float q = 0.f;
+    for (int c = 0; c < 8; ++c) {
+      const float4 v = *reinterpret_cast<const float4*>(B.DX + (B.r0 + 4 * c) * ldx + j0);
+      const float xv[4] = {v.x, v.y, v.z, v.w};
+      float q = 0.f;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (j0 + u < d) q = fmaf(xv[u], g[c][u], q);
-        sm.part[(row0 + 4 * c) * nj + (j0 >> 2)] = q;
-      }
+      for (int u = 0; u < 4; ++u)
+        if (j0 + u < d) q = fmaf(xv[u], g[c][u], q);
+      B.part[(B.r0 + 4 * c) * nj + (j0 >> 2)] = q;
     }
-    __syncthreads();
+    B.sync();
     // per chain: the partials of the 64 coordinate groups (absent ones zero)
     // as two balanced trees of 32, eight lanes per chain
-    const int sub = threadIdx.x & 7;
-    for (int r = threadIdx.x >> 3; r < ((rows + 3) & ~3); r += kBThreads / 8) {
-      const float* pr = sm.part + r * nj;
+    const int sub = B.tb & 7;
+    for (int r = B.tb >> 3; r < 32; r += 4 * B.cb) {
+      const float* pr = B.part + r * nj;
       float h[2];
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
@@ -207,7 +209,7 @@ __device__ __forceinline__ void dense_eval(const BatchTarget& T, const BatchSmem
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int i = 32 * b + sub + 8 * q;
-          v[q] = (r < rows && i < nj) ? pr[i] : 0.f;
+          v[q] = i < nj ? pr[i] : 0.f;
         }
         float t = (v[0] + v[2]) + (v[1] + v[3]);
         t += __shfl_xor_sync(0xffffffffu, t, 4);
@@ -215,9 +217,9 @@ __device__ __forceinline__ void dense_eval(const BatchTarget& T, const BatchSmem
         t += __shfl_xor_sync(0xffffffffu, t, 1);
         h[b] = t;
       }
-      if (sub == 0 && r < rows) lp[r] = -0.5f * (h[0] + h[1]) + T.const_term;
+      if (sub == 0) lp[r] = -0.5f * (h[0] + h[1]) + T.const_term;
     }
-    __syncthreads();
+    B.sync();
   }
 #pragma unroll
   for (int c = 0; c < 8; ++c)
@@ -225,19 +227,27 @@ __device__ __forceinline__ void dense_eval(const BatchTarget& T, const BatchSmem
     for (int u = 0; u < 4; ++u) g[c][u] = -g[c][u];
 }
 
-// out[r] = sum over j < d of E[r][j]^2, eight lanes per chain (lane sub takes
-// j = sub, sub + 8, ...), then a three-level butterfly
-__device__ __forceinline__ void row_sumsq(const float* E, int ldx, int d, int rows, float* out) {
-  const int sub = threadIdx.x & 7;
-  for (int r = threadIdx.x >> 3; r < ((rows + 3) & ~3); r += kBThreads / 8) {
-    float v = 0.f;
-    if (r < rows)
-      for (int j = sub; j < d; j += 8) v = fmaf(E[r * ldx + j], E[r * ldx + j], v);
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    if (sub == 0 && r < rows) out[r] = v;
+// out[r] = sum over j < d of DX[r][j]^2 for the row block, where DX holds v:
+// eight lanes per chain (lane sub takes j = sub, sub + 8, ...), then a
+// three-level butterfly. Barriers before the write, after it and at the end.
+__device__ __forceinline__ void row_sumsq(const BatchTarget& T, const BatchBlock& B, const float (&v)[8][4],
+                                          float* out) {
+  B.sync();
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    *reinterpret_cast<float4*>(B.DX + (B.r0 + 4 * c) * B.ldx + B.j0) = make_float4(v[c][0], v[c][1], v[c][2], v[c][3]);
+  B.sync();
+  const int sub = B.tb & 7;
+  for (int r = B.tb >> 3; r < 32; r += 4 * B.cb) {
+    const float* e = B.DX + r * B.ldx;
+    float t = 0.f;
+    for (int j = sub; j < T.d; j += 8) t = fmaf(e[j], e[j], t);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 4);
+    if (sub == 0) out[r] = t;
   }
+  B.sync();
 }
 
 // normals of chain c of T at step s for coordinates j0 .. j0 + 3 (j0 a
@@ -259,26 +269,169 @@ __device__ __forceinline__ void draw_normals4(const BatchArgs& a, const Rng& rng
   }
 }
 
+// all steps of one work item for this thread's row block
+template <int KIND>
+__device__ __forceinline__ void run_tile(const BatchArgs& a, const Rng& rng, const BatchTarget& T, BatchBlock& B, int c0,
+                                         int nc, float4* sx, float4* sg, float* chain) {
+  // per-chain values of the row block, kBRows apart
+  float *lpx = chain, *lpy = chain + kBRows, *sA = chain + 2 * kBRows, *sB = chain + 3 * kBRows;
+  float* logu = chain + 4 * kBRows;
+  int* acc_s = reinterpret_cast<int*>(chain + 5 * kBRows);
+  const int d = T.d, j0 = B.j0, s_rec = (a.S - 1) / a.thin * a.thin;   // s_rec: the last recorded step
+  const bool vec_out = (d & 3) == 0 && ((uintptr_t)T.out_pos & 15) == 0;
+  const float dt = T.step, dt2 = dt * dt;
+  float y[8][4], g[8][4];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const int r = B.r0 + 4 * c;
+    const float* xr = a.x0 + (int64_t)(T.chain_offset + c0 + r) * kBDMax + j0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) y[c][u] = (r < nc && j0 + u < d) ? xr[u] : 0.f;
+    sx[c * kBThreads] = make_float4(y[c][0], y[c][1], y[c][2], y[c][3]);
+  }
+  dense_eval(T, B, y, g, lpx);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) sg[c * kBThreads] = make_float4(g[c][0], g[c][1], g[c][2], g[c][3]);
+
+  for (int s = 0; s < a.S; ++s) {
+    // log-uniforms of the step, one chain per thread
+    if (B.tb < nc && B.tb < 32) {
+      const int64_t row = c0 + B.tb;
+      float u;
+      if (T.unif) u = __ldg(T.unif + row * a.S + s);
+      else u = u32_to_unit(rng.draw((uint64_t)(T.chain_offset + row), (uint64_t)s, 0u, RNG_TAG_LOCAL_UNIFORM).x);
+      logu[B.tb] = logf(u);
+    }
+    // ---- proposal (MALA) or leapfrog trajectory (HMC): y, g, lpy
+    if constexpr (KIND == FMC_KERNEL_MALA) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        float xi[4];
+        draw_normals4(a, rng, T, c0 + B.r0 + 4 * c, s, j0, xi);
+        const float4 x = sx[c * kBThreads], gx = sg[c * kBThreads];
+        y[c][0] = fmaf(dt, xi[0], x.x + dt2 * gx.x / 2.0f);
+        y[c][1] = fmaf(dt, xi[1], x.y + dt2 * gx.y / 2.0f);
+        y[c][2] = fmaf(dt, xi[2], x.z + dt2 * gx.z / 2.0f);
+        y[c][3] = fmaf(dt, xi[3], x.w + dt2 * gx.w / 2.0f);
+      }
+      dense_eval(T, B, y, g, lpy);
+      // |prop - mean0|^2 and |x - mean1|^2 per chain
+      float e[8][4];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float4 x = sx[c * kBThreads], gx = sg[c * kBThreads];
+        e[c][0] = y[c][0] - (x.x + dt2 * gx.x / 2.0f);
+        e[c][1] = y[c][1] - (x.y + dt2 * gx.y / 2.0f);
+        e[c][2] = y[c][2] - (x.z + dt2 * gx.z / 2.0f);
+        e[c][3] = y[c][3] - (x.w + dt2 * gx.w / 2.0f);
+      }
+      row_sumsq(T, B, e, sA);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float4 x = sx[c * kBThreads];
+        e[c][0] = x.x - (y[c][0] + dt2 * g[c][0] / 2.0f);
+        e[c][1] = x.y - (y[c][1] + dt2 * g[c][1] / 2.0f);
+        e[c][2] = x.z - (y[c][2] + dt2 * g[c][2] / 2.0f);
+        e[c][3] = x.w - (y[c][3] + dt2 * g[c][3] / 2.0f);
+      }
+      row_sumsq(T, B, e, sB);
+    } else {
+      float p[8][4];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) draw_normals4(a, rng, T, c0 + B.r0 + 4 * c, s, j0, p[c]);
+      row_sumsq(T, B, p, sA);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float4 x = sx[c * kBThreads], gx = sg[c * kBThreads];
+        y[c][0] = x.x; y[c][1] = x.y; y[c][2] = x.z; y[c][3] = x.w;
+        // row 0: half kick with the gradient at x
+        p[c][0] = fmaf(dt * 0.5f, gx.x, p[c][0]);
+        p[c][1] = fmaf(dt * 0.5f, gx.y, p[c][1]);
+        p[c][2] = fmaf(dt * 0.5f, gx.z, p[c][2]);
+        p[c][3] = fmaf(dt * 0.5f, gx.w, p[c][3]);
+      }
+      for (int r = 1; r <= a.n_leapfrog + 1; ++r) {
+        const bool end = r == a.n_leapfrog + 1;
+        const float ek = end ? dt * 0.5f : dt;
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) y[c][u] = fmaf(dt, p[c][u], y[c][u]);
+        if (r > 1) B.sync();   // every warp has left the previous product's dx
+        // only the gradient is used before the end point
+        dense_eval(T, B, y, g, end ? lpy : nullptr);
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) p[c][u] = fmaf(ek, g[c][u], p[c][u]);
+      }
+      row_sumsq(T, B, p, sB);
+    }
+    // ---- accept per chain (float-float log-ratio), then commit
+    const bool rec = s % a.thin == 0;
+    const int64_t orow = a.start + s / a.thin;
+    if (B.tb < nc && B.tb < 32) {
+      const int c = B.tb;
+      ff ratio;
+      if constexpr (KIND == FMC_KERNEL_MALA) {
+        const ff q = two_sum(sA[c], -sB[c]);
+        ratio = ff_add(two_sum(lpy[c], -lpx[c]), ff_mul_f(q, 0.5f / (dt * dt)));
+      } else {
+        ratio = ff_add(two_sum(-lpx[c], 0.5f * sA[c]), ff_neg(two_sum(-lpy[c], 0.5f * sB[c])));
+      }
+      const bool acc = f_lt_ff(logu[c], ratio);
+      acc_s[c] = acc ? 1 : 0;
+      const float lp = acc ? lpy[c] : lpx[c];
+      lpx[c] = lp;
+      if (rec) {
+        __stcs(T.out_logp + (int64_t)(c0 + c) * a.buf_len + orow, lp);
+        __stcs(T.out_acc + (int64_t)(c0 + c) * a.buf_len + orow, acc ? 1.f : 0.f);
+        if (s == s_rec) a.lp_last[T.chain_offset + c0 + c] = lp;
+      }
+    }
+    B.sync();
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int r = B.r0 + 4 * c;
+      if (r >= nc) continue;
+      if (acc_s[r]) {
+        sx[c * kBThreads] = make_float4(y[c][0], y[c][1], y[c][2], y[c][3]);
+        sg[c * kBThreads] = make_float4(g[c][0], g[c][1], g[c][2], g[c][3]);
+      }
+      if (rec && j0 < d) {
+        const float4 x = sx[c * kBThreads];
+        const float xv[4] = {x.x, x.y, x.z, x.w};
+        float* o = T.out_pos + ((int64_t)(c0 + r) * a.buf_len + orow) * d + j0;
+        if (vec_out) {
+          __stcs(reinterpret_cast<float4*>(o), x);
+        } else {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (j0 + u < d) __stcs(o + u, xv[u]);
+        }
+        if (s == s_rec) {
+          float* xl = a.x_last + (int64_t)(T.chain_offset + c0 + r) * kBDMax + j0;
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (j0 + u < d) xl[u] = xv[u];
+        }
+      }
+    }
+  }
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(kBThreads, 1) k_batched_dense(const BatchArgs a) {
   extern __shared__ __align__(16) float smraw[];
   const Rng rng = a.rng.at_epoch();
-  BatchSmem sm;
-  sm.X = reinterpret_cast<float4*>(smraw);
-  sm.G = sm.X + 8 * kBThreads;
-  sm.DX = reinterpret_cast<float*>(sm.G + 8 * kBThreads);
-  sm.P = sm.DX + kBDxFloats;
-  sm.part = sm.P + kBPFloats;
-  sm.lpx = sm.part + kBPartFloats;
-  sm.lpy = sm.lpx + kBRows;
-  sm.sA = sm.lpy + kBRows;
-  sm.sB = sm.sA + kBRows;
-  sm.lpr = sm.sB + kBRows;
-  sm.logu = sm.lpr + kBRows;
-  sm.acc = reinterpret_cast<int*>(sm.logu + kBRows);
-  __shared__ int item_s;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int s_rec = (a.S - 1) / a.thin * a.thin;   // the last recorded step
+  float4* sx = reinterpret_cast<float4*>(smraw) + tid;   // [8][kBThreads] positions, owner thread's layout
+  float4* sg = sx + 8 * kBThreads;                       // gradients at those positions
+  float* DX = smraw + 2 * 8 * 4 * kBThreads;
+  float* ring = DX + kBDxFloats;
+  float* part = ring + kBWarps * kBRing;
+  float* chain = part + kBPartFloats;
+  __shared__ int item_s;
 
   for (;;) {
     if (tid == 0) item_s = atomicAdd(a.next_item, 1);
@@ -288,177 +441,33 @@ __global__ void __launch_bounds__(kBThreads, 1) k_batched_dense(const BatchArgs 
     const BatchTarget T = a.targets[a.item_target[item]];
     const int c0 = a.item_chain0[item];
     const int nc = min(T.tile_rows, T.n_chains - c0);
-    const int d = T.d, cb = (d + 31) >> 5, ldx = 32 * cb + 4;
-    const int rows = (nc + 31) & ~31;
-    const int rblk = wid / cb;
-    const bool on = rblk * 32 < rows;                       // this warp has a block
-    const int row0 = rblk * 32 + (lane >> 3);               // chains row0 + 4 c
-    const int j0 = (wid - rblk * cb) * 32 + (lane & 7) * 4;  // coordinates j0 .. j0 + 3
-    const bool vec_out = (d & 3) == 0 && ((uintptr_t)T.out_pos & 15) == 0;
-    const float dt = T.step, dt2 = dt * dt;
-    float4 mean = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (T.mean != nullptr) {
-      if (j0 + 0 < d) mean.x = __ldg(T.mean + j0);
-      if (j0 + 1 < d) mean.y = __ldg(T.mean + j0 + 1);
-      if (j0 + 2 < d) mean.z = __ldg(T.mean + j0 + 2);
-      if (j0 + 3 < d) mean.w = __ldg(T.mean + j0 + 3);
-    }
-    float y[8][4], g[8][4];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int r = row0 + 4 * c;
-      const float* xr = a.x0 + (int64_t)(T.chain_offset + c0 + r) * kBDMax + j0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) y[c][u] = (on && r < nc && j0 + u < d) ? xr[u] : 0.f;
-      sm.X[c * kBThreads + tid] = make_float4(y[c][0], y[c][1], y[c][2], y[c][3]);
-    }
-    dense_eval(T, sm, cb, on, row0, j0, mean, y, g, sm.lpx, rows);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) sm.G[c * kBThreads + tid] = make_float4(g[c][0], g[c][1], g[c][2], g[c][3]);
-
-    for (int s = 0; s < a.S; ++s) {
-      // log-uniforms of the step, one chain per thread
-      if (tid < nc) {
-        float u;
-        if (T.unif) u = __ldg(T.unif + (int64_t)(c0 + tid) * a.S + s);
-        else u = u32_to_unit(rng.draw((uint64_t)(T.chain_offset + c0 + tid), (uint64_t)s, 0u, RNG_TAG_LOCAL_UNIFORM).x);
-        sm.logu[tid] = logf(u);
+    BatchBlock B;
+    B.cb = (T.d + 31) >> 5;
+    const int rb = wid / B.cb, wb = wid - rb * B.cb;   // row block, coordinate block
+    if (32 * rb < nc) {
+      B.tb = wb * 32 + lane;
+      B.bar = 1 + rb;
+      B.r0 = lane >> 3;
+      B.j0 = wb * 32 + (lane & 7) * 4;
+      B.ldx = 32 * B.cb + 4;
+      B.DX = DX + 32 * rb * B.ldx;
+      B.part = part + 32 * rb * 8 * B.cb;
+      B.ring = ring + wid * kBRing;
+      B.src = T.packed + (lane >> 3) * 32 * B.cb + B.j0;
+      B.ns = (T.d + kBStage - 1) / kBStage;
+      B.next = 0;
+      B.buf = 0;
+      B.mean = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (T.mean != nullptr) {
+        if (B.j0 + 0 < T.d) B.mean.x = __ldg(T.mean + B.j0);
+        if (B.j0 + 1 < T.d) B.mean.y = __ldg(T.mean + B.j0 + 1);
+        if (B.j0 + 2 < T.d) B.mean.z = __ldg(T.mean + B.j0 + 2);
+        if (B.j0 + 3 < T.d) B.mean.w = __ldg(T.mean + B.j0 + 3);
       }
-      // ---- proposal (MALA) or leapfrog trajectory (HMC): y, g, lpy
-      if constexpr (KIND == FMC_KERNEL_MALA) {
-        if (on) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            float xi[4];
-            draw_normals4(a, rng, T, c0 + row0 + 4 * c, s, j0, xi);
-            const float4 x = sm.X[c * kBThreads + tid], gx = sm.G[c * kBThreads + tid];
-            y[c][0] = fmaf(dt, xi[0], x.x + dt2 * gx.x / 2.0f);
-            y[c][1] = fmaf(dt, xi[1], x.y + dt2 * gx.y / 2.0f);
-            y[c][2] = fmaf(dt, xi[2], x.z + dt2 * gx.z / 2.0f);
-            y[c][3] = fmaf(dt, xi[3], x.w + dt2 * gx.w / 2.0f);
-          }
-        }
-        dense_eval(T, sm, cb, on, row0, j0, mean, y, g, sm.lpy, rows);
-        // prop - mean0 into DX, x - mean1 into the P area; squared norms per chain
-        if (on) {
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const float4 x = sm.X[c * kBThreads + tid], gx = sm.G[c * kBThreads + tid];
-            float4 ea, eb;
-            ea.x = y[c][0] - (x.x + dt2 * gx.x / 2.0f);
-            ea.y = y[c][1] - (x.y + dt2 * gx.y / 2.0f);
-            ea.z = y[c][2] - (x.z + dt2 * gx.z / 2.0f);
-            ea.w = y[c][3] - (x.w + dt2 * gx.w / 2.0f);
-            eb.x = x.x - (y[c][0] + dt2 * g[c][0] / 2.0f);
-            eb.y = x.y - (y[c][1] + dt2 * g[c][1] / 2.0f);
-            eb.z = x.z - (y[c][2] + dt2 * g[c][2] / 2.0f);
-            eb.w = x.w - (y[c][3] + dt2 * g[c][3] / 2.0f);
-            *reinterpret_cast<float4*>(sm.DX + (row0 + 4 * c) * ldx + j0) = ea;
-            *reinterpret_cast<float4*>(sm.P + (row0 + 4 * c) * ldx + j0) = eb;
-          }
-        }
-        __syncthreads();
-        row_sumsq(sm.DX, ldx, d, rows, sm.sA);
-        row_sumsq(sm.P, ldx, d, rows, sm.sB);
-        __syncthreads();
-      } else {
-        float p[8][4];
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) p[c][u] = 0.f;
-        __syncthreads();   // the last step's readers of DX are done
-        if (on) {
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            draw_normals4(a, rng, T, c0 + row0 + 4 * c, s, j0, p[c]);
-            *reinterpret_cast<float4*>(sm.DX + (row0 + 4 * c) * ldx + j0) =
-                make_float4(p[c][0], p[c][1], p[c][2], p[c][3]);
-            const float4 x = sm.X[c * kBThreads + tid], gx = sm.G[c * kBThreads + tid];
-            y[c][0] = x.x; y[c][1] = x.y; y[c][2] = x.z; y[c][3] = x.w;
-            // row 0: half kick with the gradient at x
-            p[c][0] = fmaf(dt * 0.5f, gx.x, p[c][0]);
-            p[c][1] = fmaf(dt * 0.5f, gx.y, p[c][1]);
-            p[c][2] = fmaf(dt * 0.5f, gx.z, p[c][2]);
-            p[c][3] = fmaf(dt * 0.5f, gx.w, p[c][3]);
-          }
-        }
-        __syncthreads();
-        row_sumsq(sm.DX, ldx, d, rows, sm.sA);
-        for (int r = 1; r <= a.n_leapfrog + 1; ++r) {
-          const bool end = r == a.n_leapfrog + 1;
-          const float ek = end ? dt * 0.5f : dt;
-#pragma unroll
-          for (int c = 0; c < 8; ++c)
-#pragma unroll
-            for (int u = 0; u < 4; ++u) y[c][u] = fmaf(dt, p[c][u], y[c][u]);
-          // only the gradient is used before the end point
-          dense_eval(T, sm, cb, on, row0, j0, mean, y, g, end ? sm.lpy : nullptr, rows);
-#pragma unroll
-          for (int c = 0; c < 8; ++c)
-#pragma unroll
-            for (int u = 0; u < 4; ++u) p[c][u] = fmaf(ek, g[c][u], p[c][u]);
-        }
-        if (on) {
-#pragma unroll
-          for (int c = 0; c < 8; ++c)
-            *reinterpret_cast<float4*>(sm.DX + (row0 + 4 * c) * ldx + j0) =
-                make_float4(p[c][0], p[c][1], p[c][2], p[c][3]);
-        }
-        __syncthreads();
-        row_sumsq(sm.DX, ldx, d, rows, sm.sB);
-        __syncthreads();
-      }
-      // ---- accept per chain (float-float log-ratio), then commit
-      const bool rec = s % a.thin == 0;
-      const int64_t orow = a.start + s / a.thin;
-      if (tid < nc) {
-        const int c = tid;
-        ff ratio;
-        if constexpr (KIND == FMC_KERNEL_MALA) {
-          const ff q = two_sum(sm.sA[c], -sm.sB[c]);
-          ratio = ff_add(two_sum(sm.lpy[c], -sm.lpx[c]), ff_mul_f(q, 0.5f / (dt * dt)));
-        } else {
-          ratio = ff_add(two_sum(-sm.lpx[c], 0.5f * sm.sA[c]), ff_neg(two_sum(-sm.lpy[c], 0.5f * sm.sB[c])));
-        }
-        const bool acc = f_lt_ff(sm.logu[c], ratio);
-        sm.acc[c] = acc ? 1 : 0;
-        const float lp = acc ? sm.lpy[c] : sm.lpx[c];
-        sm.lpx[c] = lp;
-        if (rec) {
-          __stcs(T.out_logp + (int64_t)(c0 + c) * a.buf_len + orow, lp);
-          __stcs(T.out_acc + (int64_t)(c0 + c) * a.buf_len + orow, acc ? 1.f : 0.f);
-          if (s == s_rec) a.lp_last[T.chain_offset + c0 + c] = lp;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const int r = row0 + 4 * c;
-        if (!on || r >= nc) continue;
-        if (sm.acc[r]) {
-          sm.X[c * kBThreads + tid] = make_float4(y[c][0], y[c][1], y[c][2], y[c][3]);
-          sm.G[c * kBThreads + tid] = make_float4(g[c][0], g[c][1], g[c][2], g[c][3]);
-        }
-        if (rec && j0 < d) {
-          const float4 x = sm.X[c * kBThreads + tid];
-          const float xv[4] = {x.x, x.y, x.z, x.w};
-          float* o = T.out_pos + ((int64_t)(c0 + r) * a.buf_len + orow) * d + j0;
-          if (vec_out) {
-            __stcs(reinterpret_cast<float4*>(o), x);
-          } else {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (j0 + u < d) __stcs(o + u, xv[u]);
-          }
-          if (s == s_rec) {
-            float* xl = a.x_last + (int64_t)(T.chain_offset + c0 + r) * kBDMax + j0;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (j0 + u < d) xl[u] = xv[u];
-          }
-        }
-      }
+      for (int q = 0; q < kBStages - 1; ++q) B.issue(q);
+      run_tile<KIND>(a, rng, T, B, c0 + 32 * rb, nc - 32 * rb, sx, sg, chain + 32 * rb);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");   // the stages copied ahead
     }
     __syncthreads();   // item_s and the shared buffers are free
   }
