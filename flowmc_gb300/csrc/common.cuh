@@ -170,10 +170,15 @@ struct Rng {
     }
     return r;
   }
-  __device__ __forceinline__ u32x4 draw(uint64_t row, uint64_t step, uint32_t slot, uint32_t tag) const {
+  // the draw with the round count fixed at compile time (straight-line code)
+  template <int R>
+  __device__ __forceinline__ u32x4 draw_n(uint64_t row, uint64_t step, uint32_t slot, uint32_t tag) const {
     const uint64_t s = step + (ctr_base << 32);
     u32x4 c{(uint32_t)row, (uint32_t)(row >> 32) ^ (uint32_t)(s >> 32), slot, tag ^ (uint32_t)s};
-    return rounds == 7 ? philox4x32<7>(c, k0, k1) : philox4x32<10>(c, k0, k1);
+    return philox4x32<R>(c, k0, k1);
+  }
+  __device__ __forceinline__ u32x4 draw(uint64_t row, uint64_t step, uint32_t slot, uint32_t tag) const {
+    return rounds == 7 ? draw_n<7>(row, step, slot, tag) : draw_n<10>(row, step, slot, tag);
   }
 };
 
@@ -185,6 +190,16 @@ __device__ __forceinline__ float group_sum(float v) {
   for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, G);
   return v;
 }
+// two sums at once: the shuffles of one hide the latency of the other's
+template <int G>
+__device__ __forceinline__ void group_sum2(float& v, float& w) {
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+    const float a = __shfl_xor_sync(0xffffffffu, v, o, G), b = __shfl_xor_sync(0xffffffffu, w, o, G);
+    v += a;
+    w += b;
+  }
+}
 template <int G>
 __device__ __forceinline__ float group_max(float v) {
 #pragma unroll
@@ -195,6 +210,31 @@ template <int G>
 __device__ __forceinline__ float group_bcast(float v, int src_lane_in_group) {
   return __shfl_sync(0xffffffffu, v, src_lane_in_group, G);
 }
+
+// ---------------------------------------------------------------- exact quotients
+// a / b for one divisor used many times: with y = RN(1 / b), the steps q0 = a y,
+// q1 = q0 + (a - q0 b) y, q = q1 + (a - q1 b) y give the correctly rounded
+// quotient (Markstein, IBM J. Res. Dev. 34(1), 1990: q1 is a faithful
+// rounding, its remainder is exact) as long as nothing leaves the normal range
+// (numerators of 2^-60 .. 2^60 with `in_range` divisors): the bits of the
+// division operator without its reciprocal per quotient and range branch.
+struct ConstDiv {
+  float b, y;
+  bool in_range;   // the divisor allows it; numerators up to the caller
+  __device__ __forceinline__ explicit ConstDiv(float divisor) : b(divisor) {
+    asm("rcp.rn.f32 %0, %1;" : "=f"(y) : "f"(divisor));
+    in_range = fabsf(divisor) >= 0x1p-30f && fabsf(divisor) <= 0x1p30f;
+  }
+  __device__ __forceinline__ float operator()(float a) const {
+    const float q0 = __fmul_rn(a, y);
+    const float q1 = __fmaf_rn(__fmaf_rn(-q0, b, a), y, q0);
+    return __fmaf_rn(__fmaf_rn(-q1, b, a), y, q1);
+  }
+};
+
+// compile-time integer as a value, for generic lambdas
+template <int N>
+struct IntC { static constexpr int value = N; };
 
 // ---------------------------------------------------------------- float-float
 struct ff { float hi, lo; };

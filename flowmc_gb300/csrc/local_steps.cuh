@@ -42,6 +42,7 @@ struct LocalArgs {
   const float* mcol;    // HMC column sums of M
   const float* mchol;   // HMC with a dense M: cholesky(inv(M)) [d, d] row-major, or NULL
   int32_t mstage_off;   // floats of dynamic shared memory before the momentum staging
+  int32_t nstage_off;   // floats of dynamic shared memory before the noise chunks ([groups][4][G V])
   const float* x0;
   const float* lp0;
   int32_t C, d, S, thin;
@@ -94,8 +95,40 @@ __device__ __forceinline__ float temper(const LocalArgs& a, float lp, const floa
   return lp;
 }
 
-template <int V>
-__device__ __forceinline__ void draw_normals(const LocalArgs& a, const Rng& rng, int64_t c, int s, int gl,
+// Normals of four consecutive steps s .. s + 3 (s a multiple of 4) for every
+// chain of the warp, into shared memory `ns` (this group's [4][G * V] floats).
+// Coordinate j takes component (j & 3) of the Philox block keyed by j & ~3:
+// (x, y) -> Box-Muller -> j & 3 = 0, 1 and (z, w) -> j & 3 = 2, 3. The stream
+// depends on (chain, step, coordinate) only, never on the lane-group shape,
+// so every (G, V) choice samples the same chains. The G * V blocks of a chunk
+// are dealt out over the group's lanes: V independent Philox + Box-Muller
+// chains per lane and four steps, whose latencies overlap, where a lane
+// drawing its own coordinates step by step waits for each in turn (and for
+// V < 4 computes every block 4 / V times).
+template <int G, int V>
+__device__ __forceinline__ void draw_chunk(const Rng& rng, int64_t c, int s, int gl, float* ns) {
+  constexpr int NB = G * V / 4;   // blocks per step
+  __syncwarp();                   // the previous chunk has been read
+  auto draw = [&](auto rounds) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int item = gl + G * i, t = item / NB, jb = item % NB;
+      const u32x4 r = rng.draw_n<decltype(rounds)::value>((uint64_t)c, (uint64_t)(s + t), (uint32_t)(4 * jb),
+                                                          RNG_TAG_LOCAL_NORMAL);
+      float4 z;
+      box_muller(r.x, r.y, z.x, z.y);
+      box_muller(r.z, r.w, z.z, z.w);
+      *reinterpret_cast<float4*>(ns + (t * NB + jb) * 4) = z;
+    }
+  };
+  if (rng.rounds == 7) draw(IntC<7>{});
+  else draw(IntC<10>{});
+  __syncwarp();
+}
+
+// this lane's normals of step s: explicit, or from the chunk in shared memory
+template <int G, int V>
+__device__ __forceinline__ void draw_normals(const LocalArgs& a, const Rng& rng, int64_t c, int s, int gl, float* ns,
                                              float (&xi)[V]) {
   const int d = a.d;
   if (a.noise) {
@@ -107,49 +140,44 @@ __device__ __forceinline__ void draw_normals(const LocalArgs& a, const Rng& rng,
     }
     return;
   }
-  // Coordinate j takes component (j & 3) of the Philox block keyed by j & ~3:
-  // (x, y) -> Box-Muller -> j&3 = 0, 1 and (z, w) -> j&3 = 2, 3. The stream
-  // depends on (chain, step, coordinate) only, never on the lane-group shape,
-  // so every (G, V) choice samples the same chains.
-  if constexpr (V >= 4) {
+  if ((s & 3) == 0) draw_chunk<G, V>(rng, c, s, gl, ns);
+  const float* row = ns + (s & 3) * (G * V) + gl * V;
+  if constexpr (V % 4 == 0) {
 #pragma unroll
     for (int q = 0; q < V; q += 4) {
-      const u32x4 r = rng.draw(c, s, (uint32_t)(gl * V + q), RNG_TAG_LOCAL_NORMAL);
-      box_muller(r.x, r.y, xi[q], xi[q + 1]);
-      box_muller(r.z, r.w, xi[q + 2], xi[q + 3]);
+      const float4 z = *reinterpret_cast<const float4*>(row + q);
+      xi[q] = z.x; xi[q + 1] = z.y; xi[q + 2] = z.z; xi[q + 3] = z.w;
     }
   } else {
-    const int j = gl * V;   // V = 2: j is even
-    const u32x4 r = rng.draw(c, s, (uint32_t)(j & ~3), RNG_TAG_LOCAL_NORMAL);
-    const bool hi = (j & 2) != 0;
-    float z0, z1;
-    box_muller(hi ? r.z : r.x, hi ? r.w : r.y, z0, z1);
-    if constexpr (V == 1) {
-      xi[0] = (j & 1) ? z1 : z0;
-    } else {
-      xi[0] = z0;
-      xi[1] = z1;
-    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) xi[v] = row[v];
   }
 #pragma unroll
   for (int v = 0; v < V; ++v)
     if (gl * V + v >= d) xi[v] = 0.f;
 }
 
-// Uniforms: step s takes component s & 3 of the Philox block keyed by s >> 2.
-// The G lanes of a group share the work: on steps s = 0 mod 4G, lane gl
-// computes block (s >> 2) + gl into `ub`, and each step the owner lane
-// ((s >> 2) mod G) hands its component to the whole group with a shuffle,
-// so the group agrees on u. One Philox call per 4G steps per lane instead of
-// one per 4 steps; the stream is the same as one lane drawing every block.
+// log of the step's uniform: step s takes component s & 3 of the Philox block
+// keyed by s >> 2. The G lanes of a group share the work: on steps s = 0 mod
+// 4G, lane gl draws block (s >> 2) + gl and takes the four logarithms into
+// `lu`; each step the owner lane ((s >> 2) mod G) hands its component to the
+// whole group with a shuffle, so the group agrees on it. One Philox call and
+// four logarithms per 4G steps per lane; the stream is the same as one lane
+// drawing every block.
 template <int G>
-__device__ __forceinline__ float draw_uniform(const LocalArgs& a, const Rng& rng, int64_t c, int s, int gl,
-                                              u32x4& ub) {
-  if (a.unif) return __ldcs(a.unif + (int64_t)c * a.S + s);
-  if (s % (4 * G) == 0) ub = rng.draw(c, (uint64_t)((s >> 2) + gl), 0u, RNG_TAG_LOCAL_UNIFORM);
+__device__ __forceinline__ float draw_log_uniform(const LocalArgs& a, const Rng& rng, int64_t c, int s, int gl,
+                                                  float (&lu)[4]) {
+  if (a.unif) return logf(__ldcs(a.unif + (int64_t)c * a.S + s));
+  if (s % (4 * G) == 0) {
+    const u32x4 r = rng.draw(c, (uint64_t)((s >> 2) + gl), 0u, RNG_TAG_LOCAL_UNIFORM);
+    lu[0] = logf(u32_to_unit(r.x));
+    lu[1] = logf(u32_to_unit(r.y));
+    lu[2] = logf(u32_to_unit(r.z));
+    lu[3] = logf(u32_to_unit(r.w));
+  }
   const int r = s & 3;
-  const uint32_t mine = r == 0 ? ub.x : r == 1 ? ub.y : r == 2 ? ub.z : ub.w;
-  return u32_to_unit(__shfl_sync(0xffffffffu, mine, (s >> 2) % G, G));
+  const float mine = r == 0 ? lu[0] : r == 1 ? lu[1] : r == 2 ? lu[2] : lu[3];
+  return __shfl_sync(0xffffffffu, mine, (s >> 2) % G, G);
 }
 
 template <int G, int V>
@@ -210,6 +238,7 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
   }
   const float dt = a.step;
   const Rng rng = a.rng.at_epoch();
+  float* ns = smem + a.nstage_off + gib * (4 * G * V);
 
   for (int64_t c = blockIdx.x * groups_per_block + gib; c < a.C_pad;
        c += (int64_t)gridDim.x * groups_per_block) {
@@ -230,7 +259,7 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
 #pragma unroll
     for (int v = 0; v < V; ++v) xr[v] = x[v];
 
-    u32x4 ub{0u, 0u, 0u, 0u};
+    float lu[4] = {0.f, 0.f, 0.f, 0.f};
     // next stored row (every thin-th step, from row `start`); no rows are
     // stored when out_pos is NULL (the tempered chains keep only their end)
     const bool rec = a.out_pos != nullptr;
@@ -241,8 +270,8 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
     int tcount = 0, n_acc = 0;
     for (int s = 0; s < a.S; ++s) {
       float xi[V];
-      draw_normals<V>(a, rng, cc, s, gl, xi);
-      const float logu = logf(draw_uniform<G>(a, rng, cc, s, gl, ub));
+      draw_normals<G, V>(a, rng, cc, s, gl, ns, xi);
+      const float logu = draw_log_uniform<G>(a, rng, cc, s, gl, lu);
       bool acc;
       if constexpr (KIND == FMC_KERNEL_MALA) {
         const float dt2 = dt * dt;
@@ -262,8 +291,7 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
           sa += ea * ea;
           sb += eb * eb;
         }
-        sa = group_sum<G>(sa);
-        sb = group_sum<G>(sb);
+        group_sum2<G>(sa, sb);
         // ratio = (lp1 - lp0) - log q(prop | x) + log q(x | prop)
         //       = (lp1 - lp0) + (|prop - mean0|^2 - |x - mean1|^2) / (2 dt^2)
         // (the Gaussian normalisers cancel). Decided in float32 when log u
@@ -330,15 +358,20 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
         // so the log-density (and its group reduction) is left to the
         // compiler to drop
         const int nlf = a.n_leapfrog;
-        for (int r = 1; r <= nlf; ++r) {
+        auto leapfrog = [&](auto metric) {
+          for (int r = 1; r <= nlf; ++r) {
+            // identity metric: p * 1 is p, the multiply is left out
 #pragma unroll
-          for (int v = 0; v < V; ++v) xq[v] = xq[v] + dt * (p[v] * mc[v]);
-          float lpi = target_eval<TGT, G, V, true>(a.tgt, xq, gq, gl, stage);
-          if (tempered) lpi = temper<G, V, true>(a, lpi, xq, gq, beta, gl);
-          (void)lpi;
+            for (int v = 0; v < V; ++v) xq[v] = xq[v] + dt * (decltype(metric)::value ? p[v] * mc[v] : p[v]);
+            float lpi = target_eval<TGT, G, V, true>(a.tgt, xq, gq, gl, stage);
+            if (tempered) lpi = temper<G, V, true>(a, lpi, xq, gq, beta, gl);
+            (void)lpi;
 #pragma unroll
-          for (int v = 0; v < V; ++v) p[v] = p[v] + dt * gq[v];
-        }
+            for (int v = 0; v < V; ++v) p[v] = p[v] + dt * gq[v];
+          }
+        };
+        if (a.mcol != nullptr) leapfrog(IntC<1>{});
+        else leapfrog(IntC<0>{});
         // last row: drift, half kick, and the log-density at the end point
 #pragma unroll
         for (int v = 0; v < V; ++v) xq[v] = xq[v] + dt * (p[v] * mc[v]);
@@ -469,9 +502,13 @@ inline Shape default_shape(int d) {
 template <int KIND, int TGT, int G, int V>
 int launch_local_t(const LocalArgs& a0, cudaStream_t st) {
   LocalArgs a = a0;
-  const int threads = 256;
-  const int gpb = threads / G;
   const int gpw = 32 / G;
+  // 256-thread blocks, or 64-thread ones when 256 would give fewer than eight
+  // blocks per SM: with one or two blocks per SM the SMs that get the extra
+  // block set the time (64-D mixture, 4096 chains of 16 lanes: 256 blocks on
+  // 152 SMs, against 1024 small ones)
+  const int threads = ((int64_t)a.C * G + 255) / 256 < 8 * (int64_t)sm_count() ? 64 : 256;
+  const int gpb = threads / G;
   a.C_pad = ((int64_t)a.C + gpw - 1) / gpw * gpw;
   size_t smem = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? (size_t)gpb * a.d * sizeof(float) : 0;
   a.tab_smem = 0;
@@ -485,6 +522,9 @@ int launch_local_t(const LocalArgs& a0, cudaStream_t st) {
   }
   a.mstage_off = (int32_t)(smem / sizeof(float));
   if (KIND == FMC_KERNEL_HMC && a.mchol != nullptr) smem += (size_t)gpb * a.d * sizeof(float);
+  smem = (smem + 15) / 16 * 16;
+  a.nstage_off = (int32_t)(smem / sizeof(float));
+  if (a.noise == nullptr) smem += (size_t)threads * 4 * V * sizeof(float);
   auto kern = k_local_steps<KIND, TGT, G, V>;
   if (smem > 48 * 1024) {
     FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

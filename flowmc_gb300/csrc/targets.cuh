@@ -143,48 +143,71 @@ __device__ __forceinline__ float tg_mixture(const FmcTarget& t, const float (&x)
   float Gr[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) Gr[v] = 0.f;
+  // NC components at a time: their sums over the coordinates are reduced
+  // together (the shuffles of one hide the others' latency), then merged one
+  // after the other
+  constexpr int NC = V <= 4 ? 4 : 2;
 #pragma unroll 1
-  for (int k = 0; k < K; ++k) {
-    float q = 0.f;
-    float gk[V];
-    if (tab != nullptr) {
-      float mu[V], iv[V];
-      tab_row<V>(tab + k * d, gl, d, mu);
-      tab_row<V>(tab + (K + k) * d, gl, d, iv);   // 0 on padding coordinates
+  for (int k0 = 0; k0 < K; k0 += NC) {
+    float q[NC], gk[NC][V];
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        const float dx = x[v] - mu[v];
-        q += dx * dx * iv[v];
-        gk[v] = -dx * iv[v];
-      }
-    } else {
+    for (int n = 0; n < NC; ++n) {
+      const int k = k0 + n;
+      q[n] = 0.f;
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        const int j = gl * V + v;
-        gk[v] = 0.f;
-        if (j < d) {
-          const float dx = x[v] - ldg_or(t.mean, (int64_t)k * d + j, 0.f);
-          const float iv = ldg_or(t.inv_var, (int64_t)k * d + j, 1.f);
-          q += dx * dx * iv;
-          gk[v] = -dx * iv;
+      for (int v = 0; v < V; ++v) gk[n][v] = 0.f;
+      if (k >= K) continue;
+      if (tab != nullptr) {
+        float mu[V], iv[V];
+        tab_row<V>(tab + k * d, gl, d, mu);
+        tab_row<V>(tab + (K + k) * d, gl, d, iv);   // 0 on padding coordinates
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const float dx = x[v] - mu[v];
+          q[n] += dx * dx * iv[v];
+          gk[n][v] = -dx * iv[v];
+        }
+      } else {
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const int j = gl * V + v;
+          if (j < d) {
+            const float dx = x[v] - ldg_or(t.mean, (int64_t)k * d + j, 0.f);
+            const float iv = ldg_or(t.inv_var, (int64_t)k * d + j, 1.f);
+            q[n] += dx * dx * iv;
+            gk[n][v] = -dx * iv;
+          }
         }
       }
     }
-    const float e = ldg_or(t.log_w, k, 0.f) - 0.5f * group_sum<G>(q);
-    if (e > m) {
-      const float r = expf(m - e);   // 0 on the first component (m = -inf)
-      S = S * r + 1.f;
-      if (GRAD) {
 #pragma unroll
-        for (int v = 0; v < V; ++v) Gr[v] = Gr[v] * r + gk[v];
-      }
-      m = e;
-    } else {
-      const float w = expf(e - m);
-      S += w;
-      if (GRAD) {
+    for (int o = G / 2; o > 0; o >>= 1) {
+      float w[NC];
 #pragma unroll
-        for (int v = 0; v < V; ++v) Gr[v] += w * gk[v];
+      for (int n = 0; n < NC; ++n) w[n] = __shfl_xor_sync(0xffffffffu, q[n], o, G);
+#pragma unroll
+      for (int n = 0; n < NC; ++n) q[n] += w[n];
+    }
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+      const int k = k0 + n;
+      if (k >= K) break;
+      const float e = ldg_or(t.log_w, k, 0.f) - 0.5f * q[n];
+      if (e > m) {
+        const float r = expf(m - e);   // 0 on the first component (m = -inf)
+        S = S * r + 1.f;
+        if (GRAD) {
+#pragma unroll
+          for (int v = 0; v < V; ++v) Gr[v] = Gr[v] * r + gk[n][v];
+        }
+        m = e;
+      } else {
+        const float w = expf(e - m);
+        S += w;
+        if (GRAD) {
+#pragma unroll
+          for (int v = 0; v < V; ++v) Gr[v] += w * gk[n][v];
+        }
       }
     }
   }
@@ -206,6 +229,30 @@ __device__ __forceinline__ float tg_rosenbrock(const FmcTarget& t, const float (
   // neighbours across the lane boundary
   const float next_first = __shfl_down_sync(0xffffffffu, x[0], 1, G);   // x_{gl*V+V}
   const float prev_last = __shfl_up_sync(0xffffffffu, x[V - 1], 1, G);  // x_{gl*V-1}
+  float a[V], lo, hi;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    a[v] = s1 - x[v];
+    const float m = fabsf(a[v]);
+    lo = v ? fminf(lo, m) : m;
+    hi = v ? fmaxf(hi, m) : m;
+  }
+  // quotients by s0: 2 a / s0 for the gradient, a^2 / s0 for the value
+  const ConstDiv by_s0(s0);
+  float q1[V], q2[V];
+  if (by_s0.in_range && lo >= 0x1p-29f && hi <= 0x1p29f) {
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      if (GRAD) q1[v] = by_s0(2.f * a[v]);
+      q2[v] = by_s0(a[v] * a[v]);
+    }
+  } else {
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      if (GRAD) q1[v] = 2.f * a[v] / s0;
+      q2[v] = a[v] * a[v] / s0;
+    }
+  }
   float s = 0.f;
 #pragma unroll
   for (int v = 0; v < V; ++v) {
@@ -214,12 +261,11 @@ __device__ __forceinline__ float tg_rosenbrock(const FmcTarget& t, const float (
     const float xp = (v > 0) ? x[v - 1] : prev_last;
     const bool has_next = (j + 1 < d);
     const bool has_prev = (j >= 1) && (j < d);
-    const float a = s1 - x[v];
     const float b = xn - x[v] * x[v];
-    if (has_next) s += a * a / s0 + s2 * b * b;
+    if (has_next) s += q2[v] + s2 * b * b;
     if (GRAD) {
       float gv = 0.f;
-      if (has_next) gv += 2.f * a / s0 + 4.f * s2 * x[v] * b;
+      if (has_next) gv += q1[v] + 4.f * s2 * x[v] * b;
       if (has_prev) gv -= 2.f * s2 * (x[v] - xp * xp);
       g[v] = gv;
     }
