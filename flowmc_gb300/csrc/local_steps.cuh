@@ -26,6 +26,17 @@
 //    ends; H uses the incoming log_prob (HMC.py:137).
 //  * GaussianRandomWalk.kernel (Gaussian_random_walk.py:48-61).
 //
+// What bounds it: issue slots and, for few chains, the latency of a step's
+// dependent chain; the stored rows are far below HBM's rate. Measured on GB300
+// (before -> after exact quotients by constants, the noise drawn four steps at a
+// time, value-free leapfrog gradients, branch-free mixture merging on padded
+// shared-memory tables and 64-thread blocks for small launches; all
+// bit-identical): 128-D Rosenbrock HMC, 16,384 chains x 40 steps x 17 gradients
+// 3.43 -> 1.34 ms (98 warp instructions per gradient, 177 before the value-free
+// ones); 64-D mixture MALA, 4096 chains x 50 steps 130 -> 84 us (567 warp
+// instructions per step and pair of chains, 725 before); 5-D dual moon MALA, 20
+// chains x 30 steps 32 -> 28 us.
+//
 // The MH log-ratio is assembled in float-float arithmetic (about 48
 // significant bits) instead of FP64: this GPU's FP64 rate is too low for a
 // per-chain-step operation, and the inputs (lp, squared norms) are FP32.
@@ -70,7 +81,7 @@ struct LocalArgs {
 
 // Tempered log-density (resource/logPDF.py:106-108): (1 / T) * log L(x) +
 // log prior(x), with the gradient scaled the same way.
-template <int G, int V, bool GRAD>
+template <int G, int V, bool GRAD, bool VALUE = true>
 __device__ __forceinline__ float temper(const LocalArgs& a, float lp, const float (&x)[V], float (&g)[V],
                                         float beta, int gl) {
   lp = beta * lp;
@@ -90,7 +101,7 @@ __device__ __forceinline__ float temper(const LocalArgs& a, float lp, const floa
         if constexpr (GRAD) g[v] -= dx * iv;
       }
     }
-    lp += -0.5f * group_sum<G>(s) + a.prior_const;
+    if (VALUE) lp += -0.5f * group_sum<G>(s) + a.prior_const;
   }
   return lp;
 }
@@ -231,7 +242,7 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
   float* stage = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? smem + gib * d : nullptr;
   if constexpr (TGT == FMC_TARGET_DIAG_GAUSSIAN || TGT == FMC_TARGET_GAUSS_MIXTURE) {
     if (a.tab_smem) {
-      stage_target_table(a.tgt, smem);
+      stage_target_table<G, V>(a.tgt, smem);
       __syncthreads();
       stage = smem;
     }
@@ -239,6 +250,7 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
   const float dt = a.step;
   const Rng rng = a.rng.at_epoch();
   float* ns = smem + a.nstage_off + gib * (4 * G * V);
+  const TargetConst<TGT> tc(a.tgt);
 
   for (int64_t c = blockIdx.x * groups_per_block + gib; c < a.C_pad;
        c += (int64_t)gridDim.x * groups_per_block) {
@@ -252,7 +264,7 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
     }
     const bool tempered = a.temps != nullptr;
     const float beta = tempered ? __fdiv_rn(1.f, __ldg(a.temps + cc % a.n_temps)) : 1.f;
-    float lp = target_eval<TGT, G, V, KIND != FMC_KERNEL_GRW>(a.tgt, x, g, gl, stage);
+    float lp = target_eval<TGT, G, V, KIND != FMC_KERNEL_GRW>(a.tgt, tc, x, g, gl, stage);
     if (tempered) lp = temper<G, V, KIND != FMC_KERNEL_GRW>(a, lp, x, g, beta, gl);
     if (KIND != FMC_KERNEL_MALA && a.lp0 != nullptr) lp = __ldg(a.lp0 + cc);
     float xr[V], lpr = lp;
@@ -281,7 +293,7 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
           mean0[v] = x[v] + dt2 * g[v] / 2.0f;
           prop[v] = mean0[v] + dt * xi[v];
         }
-        float lp1 = target_eval<TGT, G, V, true>(a.tgt, prop, g1, gl, stage);
+        float lp1 = target_eval<TGT, G, V, true>(a.tgt, tc, prop, g1, gl, stage);
         if (tempered) lp1 = temper<G, V, true>(a, lp1, prop, g1, beta, gl);
         float sa = 0.f, sb = 0.f;
 #pragma unroll
@@ -354,28 +366,25 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
         const float e0 = dt * 0.5f;
 #pragma unroll
         for (int v = 0; v < V; ++v) p[v] = p[v] + e0 * g[v];
-        // rows 1..n_leapfrog: drift and full kick; only the gradient is used,
-        // so the log-density (and its group reduction) is left to the
-        // compiler to drop
+        // rows 1..n_leapfrog: drift and full kick; only the gradient is used
         const int nlf = a.n_leapfrog;
-        auto leapfrog = [&](auto metric) {
+        auto leapfrog = [&](auto plain) {
           for (int r = 1; r <= nlf; ++r) {
-            // identity metric: p * 1 is p, the multiply is left out
+            // plain: identity metric (p * 1 is p, the multiply is left out), untempered
 #pragma unroll
-            for (int v = 0; v < V; ++v) xq[v] = xq[v] + dt * (decltype(metric)::value ? p[v] * mc[v] : p[v]);
-            float lpi = target_eval<TGT, G, V, true>(a.tgt, xq, gq, gl, stage);
-            if (tempered) lpi = temper<G, V, true>(a, lpi, xq, gq, beta, gl);
-            (void)lpi;
+            for (int v = 0; v < V; ++v) xq[v] = xq[v] + dt * (decltype(plain)::value ? p[v] : p[v] * mc[v]);
+            target_eval<TGT, G, V, true, false>(a.tgt, tc, xq, gq, gl, stage);
+            if (!decltype(plain)::value && tempered) temper<G, V, true, false>(a, 0.f, xq, gq, beta, gl);
 #pragma unroll
             for (int v = 0; v < V; ++v) p[v] = p[v] + dt * gq[v];
           }
         };
-        if (a.mcol != nullptr) leapfrog(IntC<1>{});
+        if (a.mcol == nullptr && !tempered) leapfrog(IntC<1>{});
         else leapfrog(IntC<0>{});
         // last row: drift, half kick, and the log-density at the end point
 #pragma unroll
         for (int v = 0; v < V; ++v) xq[v] = xq[v] + dt * (p[v] * mc[v]);
-        float lpq = target_eval<TGT, G, V, true>(a.tgt, xq, gq, gl, stage);
+        float lpq = target_eval<TGT, G, V, true>(a.tgt, tc, xq, gq, gl, stage);
         if (tempered) lpq = temper<G, V, true>(a, lpq, xq, gq, beta, gl);
         {
           const float eh = dt * 0.5f;
@@ -407,7 +416,7 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
         float prop[V], gdummy[V];
 #pragma unroll
         for (int v = 0; v < V; ++v) prop[v] = x[v] + xi[v] * dt;
-        float lpp = target_eval<TGT, G, V, false>(a.tgt, prop, gdummy, gl, stage);
+        float lpp = target_eval<TGT, G, V, false>(a.tgt, tc, prop, gdummy, gl, stage);
         if (tempered) lpp = temper<G, V, false>(a, lpp, prop, gdummy, beta, gl);
         acc = f_lt_ff(logu, two_sum(lpp, -lp));
         if (acc) {
@@ -459,6 +468,7 @@ __global__ void __launch_bounds__(256) k_target_eval(const FmcTarget t, const fl
   const int64_t gpb = blockDim.x / G, gib = threadIdx.x / G;
   const int d = t.n_dim;
   float* stage = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? smem + gib * d : nullptr;
+  const TargetConst<TGT> tc(t);
   for (int64_t r = blockIdx.x * gpb + gib; r < n_pad; r += (int64_t)gridDim.x * gpb) {
     const bool active = r < n;
     const int64_t rr = active ? r : 0;
@@ -468,7 +478,7 @@ __global__ void __launch_bounds__(256) k_target_eval(const FmcTarget t, const fl
       const int j = gl * V + v;
       xv[v] = (j < d) ? x[rr * d + j] : 0.f;
     }
-    const float lp = target_eval<TGT, G, V, true>(t, xv, gv, gl, stage);
+    const float lp = target_eval<TGT, G, V, true>(t, tc, xv, gv, gl, stage);
     if (active) {
       if (gl == 0) logp[rr] = lp;
       if (grad) {
@@ -514,8 +524,8 @@ int launch_local_t(const LocalArgs& a0, cudaStream_t st) {
   a.tab_smem = 0;
   if (TGT == FMC_TARGET_DIAG_GAUSSIAN || TGT == FMC_TARGET_GAUSS_MIXTURE) {
     const int K = (TGT == FMC_TARGET_GAUSS_MIXTURE) ? a.tgt.n_comp : 1;
-    const size_t tab = (size_t)2 * K * a.d * sizeof(float);
-    if (tab <= 32 * 1024) {   // small tables only: keeps several blocks per SM
+    const size_t tab = (size_t)target_table_floats(K, G * V) * sizeof(float);
+    if (tab <= 33 * 1024) {   // small tables only: keeps several blocks per SM
       smem = tab;
       a.tab_smem = 1;
     }

@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
   const int64_t gpb = blockDim.x / G, gib = threadIdx.x / G;
   const int d = a.d;
   float* stage = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? smem + gib * d : nullptr;
+  const TargetConst<TGT> tc(a.tgt);
   const Rng rng = a.rng.at_epoch();
   for (int64_t c = blockIdx.x * gpb + gib; c < a.C_pad; c += (int64_t)gridDim.x * gpb) {
     const bool active = c < a.C;
@@ -52,7 +53,7 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
       const int j = gl * V + v;
       x[v] = (j < d) ? __ldg(a.x0 + cc * d + j) : 0.f;
     }
-    float lp = target_eval<TGT, G, V, false>(a.tgt, x, g, gl, stage);   // take_steps.py:201-203
+    float lp = target_eval<TGT, G, V, false>(a.tgt, tc, x, g, gl, stage);   // take_steps.py:201-203
     float lnf = __ldg(a.lnf + (int64_t)a.C * a.S + cc);
     float xr[V], lpr = lp;
 #pragma unroll
@@ -65,7 +66,7 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
         const int j = gl * V + v;
         p[v] = (j < d) ? __ldg(a.props + row * d + j) : 0.f;
       }
-      const float lpp = target_eval<TGT, G, V, false>(a.tgt, p, g, gl, stage);
+      const float lpp = target_eval<TGT, G, V, false>(a.tgt, tc, p, g, gl, stage);
       const float lnfp = __ldg(a.lnf + row);
       const float u = a.unif ? __ldg(a.unif + row) : u32_to_unit(rng.draw(cc, s, 0u, RNG_TAG_NF_UNIFORM).x);
       // ratio = (lp_p - lp_c) - (lnf_p - lnf_c)   (NF_proposal.py:102-104)

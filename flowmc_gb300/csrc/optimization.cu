@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(256) k_adam_optimize(const AdamOptArgs a) {
   const int gpb = blockDim.x / G, gib = threadIdx.x / G;
   const int d = a.d;
   float* stage = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? smem + gib * d : nullptr;
+  const TargetConst<TGT> tc(a.tgt);
   const Rng rng = a.rng.at_epoch();
   float lo[V], hi[V];
 #pragma unroll
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(256) k_adam_optimize(const AdamOptArgs a) {
       s2[v] = 0.f;
     }
     for (int s = 0; s < a.S; ++s) {
-      target_eval<TGT, G, V, true>(a.tgt, x, g, gl, stage);
+      target_eval<TGT, G, V, true>(a.tgt, tc, x, g, gl, stage);
       float xi;
       if (a.noise) {
         xi = __ldg(a.noise + cc * a.S + s);
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(256) k_adam_optimize(const AdamOptArgs a) {
         x[v] = xn < lo[v] ? lo[v] : (xn > hi[v] ? hi[v] : xn);
       }
     }
-    const float lp = target_eval<TGT, G, V, false>(a.tgt, x, g, gl, stage);
+    const float lp = target_eval<TGT, G, V, false>(a.tgt, tc, x, g, gl, stage);
     if (active) {
 #pragma unroll
       for (int v = 0; v < V; ++v) {

@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(256) k_pt_exchange(const ExchangeArgs a) {
   const int gpb = blockDim.x / G, gib = threadIdx.x / G;
   const int T = a.T, d = a.d;
   float* stage = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? smem + gib * d : nullptr;
+  const TargetConst<TGT> tc(a.tgt);
   float* tail = smem + ((TGT == FMC_TARGET_DENSE_GAUSSIAN) ? gpb * d : 0);
   int* cnt = reinterpret_cast<int*>(tail);                  // [kMaxTemps]
   float* Ls = tail + kMaxTemps + gib * T;                    // this group's log-densities
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(256) k_pt_exchange(const ExchangeArgs a) {
     for (int t = 0; t < T; ++t) {
       float xv[V], gv[V];
       load_row<G, V>(xc + (int64_t)t * d, xv, gl, d);
-      const float l = target_eval<TGT, G, V, false>(a.tgt, xv, gv, gl, stage);
+      const float l = target_eval<TGT, G, V, false>(a.tgt, tc, xv, gv, gl, stage);
       if (gl == 0) {
         Ls[t] = l;
         perm[t] = t;
