@@ -216,29 +216,34 @@ __device__ __forceinline__ float group_bcast(float v, int src_lane_in_group) {
 // division operator without its reciprocal per quotient and range branch, for
 // divisors of magnitude 2^-30 .. 2^30 (`in_range`) and numerators that are 0 or
 // of magnitude 2^-60 .. 2^60 (the caller's check).
-//  * operator(): with y = RN(1 / b), q0 = a y, q1 = q0 + (a - q0 b) y,
+//  * MarkDiv: with y = RN(1 / b), q0 = a y, q1 = q0 + (a - q0 b) y,
 //    q = q1 + (a - q1 b) y (Markstein, IBM J. Res. Dev. 34(1), 1990: q1 is a
 //    faithful rounding and its remainder exact). Any divisor.
-//  * two(): with yl = RN(1 / b - y), q = RN(a y + RN(a yl)) (Brisebarre, Muller
+//  * ConstDiv::two(): with yl = RN(1 / b - y), q = RN(a y + RN(a yl)) (Brisebarre, Muller
 //    and Raina, IEEE Trans. Comput. 53(8), 2004). The sum before the last
 //    rounding is within 2^-48 of a / b for significands A, B in [1, 2), so the
 //    rounding goes wrong only with a midpoint m between them: for A >= B that
 //    needs |2^24 A' - (2 M + 1) B'| < 1 in integers A', B' of 24 bits, for A <
 //    B it needs |2^25 A' - (2 M + 1) B'| <= 1; the difference is never 0, and
 //    it is even for even B'. So two() is exact where B' is even (`even`).
-struct ConstDiv {
-  float b, y, yl;
-  bool in_range, even;
-  __device__ __forceinline__ explicit ConstDiv(float divisor) : b(divisor) {
+struct MarkDiv {
+  float b, y;
+  __device__ __forceinline__ explicit MarkDiv(float divisor) : b(divisor) {
     asm("rcp.rn.f32 %0, %1;" : "=f"(y) : "f"(divisor));
-    in_range = fabsf(divisor) >= 0x1p-30f && fabsf(divisor) <= 0x1p30f;
-    even = (__float_as_uint(divisor) & 1u) == 0;
-    yl = __fdiv_rn(__fmaf_rn(-y, divisor, 1.f), divisor);
   }
   __device__ __forceinline__ float operator()(float a) const {
     const float q0 = __fmul_rn(a, y);
     const float q1 = __fmaf_rn(__fmaf_rn(-q0, b, a), y, q0);
     return __fmaf_rn(__fmaf_rn(-q1, b, a), y, q1);
+  }
+};
+struct ConstDiv : MarkDiv {
+  float yl;
+  bool in_range, even;
+  __device__ __forceinline__ explicit ConstDiv(float divisor) : MarkDiv(divisor) {
+    in_range = fabsf(divisor) >= 0x1p-30f && fabsf(divisor) <= 0x1p30f;
+    even = (__float_as_uint(divisor) & 1u) == 0;
+    yl = __fdiv_rn(__fmaf_rn(-y, divisor, 1.f), divisor);
   }
   __device__ __forceinline__ float two(float a) const { return __fmaf_rn(a, y, __fmul_rn(a, yl)); }
 };

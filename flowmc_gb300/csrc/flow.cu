@@ -12,6 +12,7 @@
 // Rows are processed in chunks sized to keep the conditioner outputs
 // (n_t * (3K+1) floats per row) within a bounded workspace.
 #include "flow.cuh"
+#include "flow_f32.h"
 #include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
 
@@ -432,6 +433,24 @@ int flow_apply(const FmcFlow* f, const float* x, int64_t n, float* out, float* o
   int64_t rows;
   const bool bf16 = f->precision == FMC_PREC_BF16;
   if ((rc = check_ws(g, n, bf16, ws, ws_bytes, rows))) return rc;
+  if (!bf16 && flow_f32_fused(g)) {
+    // FP32 flows whose row tile fits in shared memory: one launch, no scratch
+    FlowF32Call c{};
+    c.theta = f->theta;
+    c.aux = f->aux;
+    c.x = x;
+    c.n = n;
+    c.inverse = kind == PASS_INVERSE;
+    c.in_mode = kind == PASS_LOGPROB ? FLOW_IN_DATA : FLOW_IN_ROWS;
+    c.out_mode = kind == PASS_LOGPROB ? FLOW_OUT_LOGP : FLOW_OUT_ROWS;
+    if (kind == PASS_LOGPROB) {
+      c.logp = out;
+    } else {
+      c.y = out;
+      c.ld = out_ld;
+    }
+    return flow_f32_pass(c, g, st);
+  }
   InferWs w;
   carve_infer(g, rows, bf16, ws, w);
   for (int64_t r0 = 0; r0 < n; r0 += rows) {
@@ -464,9 +483,22 @@ int flow_sample(const FmcFlow* f, uint64_t seed, uint64_t counter, const float* 
   int64_t rows;
   const bool bf16 = f->precision == FMC_PREC_BF16;
   if ((rc = check_ws(g, n, bf16, ws, ws_bytes, rows))) return rc;
+  const Rng rng{(uint32_t)seed, (uint32_t)(seed >> 32), counter, rng_epoch()};
+  if (!bf16 && flow_f32_fused(g)) {
+    FlowF32Call c{};
+    c.theta = f->theta;
+    c.aux = f->aux;
+    c.z = z;
+    c.rng = rng;
+    c.n = n;
+    c.inverse = true;
+    c.in_mode = FLOW_IN_BASE;
+    c.out_mode = FLOW_OUT_DATA;
+    c.y = x;
+    return flow_f32_pass(c, g, st);
+  }
   InferWs w;
   carve_infer(g, rows, bf16, ws, w);
-  const Rng rng{(uint32_t)seed, (uint32_t)(seed >> 32), counter, rng_epoch()};
   k_base_sample<<<ew_grid(n * g.d), 256, 0, st>>>(z, rng, n, g.d, f->aux, x);
   FMC_LAUNCH_CHECK();
   for (int64_t r0 = 0; r0 < n; r0 += rows) {

@@ -12,6 +12,7 @@
 // All reductions (bias columns, scale/shift, loss) are two-stage with a fixed
 // order, so gradients are bitwise reproducible.
 #include "flow.cuh"
+#include "flow_f32.h"
 #include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
 
@@ -443,10 +444,25 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     rb = (int)(b < 1 ? 1 : b);
   }
 
-  // ---- forward, saving layer inputs
-  k_standardize<<<eb, 256, 0, st>>>(x, n, d, f->aux, w.xs);
-  FMC_LAUNCH_CHECK();
-  for (int l = 0; l < g.L; ++l) {
+  // ---- forward, saving layer inputs (FP32 flows whose row tile fits in shared
+  // memory: one launch)
+  const bool fused = !bf16 && flow_f32_fused(g);
+  if (fused) {
+    FlowF32Call c{};
+    c.theta = f->theta;
+    c.aux = f->aux;
+    c.x = x;
+    c.n = n;
+    c.in_mode = FLOW_IN_DATA;
+    c.out_mode = FLOW_OUT_LOGP;
+    c.logp = w.logp;
+    c.save = w.xs;
+    if ((rc = flow_f32_pass(c, g, st))) return rc;
+  } else {
+    k_standardize<<<eb, 256, 0, st>>>(x, n, d, f->aux, w.xs);
+    FMC_LAUNCH_CHECK();
+  }
+  for (int l = 0; l < g.L && !fused; ++l) {
     float* xin = w.xs + (int64_t)l * nd;
     float* xout = w.xs + (int64_t)(l + 1) * nd;
     k_affine<<<rb, 256, 0, st>>>(xin, xout, bf16 ? nullptr : w.cond, bf16 ? w.cond16 : nullptr, g.w16_cols(l, 0),
@@ -463,7 +479,7 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     }
   }
   const float* y = w.xs + (int64_t)g.L * nd;
-  {
+  if (!fused) {
     int64_t blocks = (n + 7) / 8;
     if (blocks > (int64_t)sm_count() * 16) blocks = (int64_t)sm_count() * 16;
     k_base_logprob<<<(int)blocks, 256, 0, st>>>(y, w.ld, n, d, f->aux, w.logp);

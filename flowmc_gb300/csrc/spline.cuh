@@ -138,6 +138,109 @@ __device__ __forceinline__ void rqs_inv(float y, const Knots<K>& kn, float& x, f
   if (above) { x = (y - kn.yp[K]) / kn.sl[K] + kn.xp[K]; ld = -logf(kn.sl[K]); }
 }
 
+// softmax numerators e^(r - max) and their sum
+template <int K>
+__device__ __forceinline__ float softmax_num(const float* r, float (&p)[K]) {
+  float m = r[0];
+#pragma unroll
+  for (int k = 1; k < K; ++k) m = fmaxf(m, r[k]);
+  float s = 0.f;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    p[k] = expf(r[k] - m);
+    s += p[k];
+  }
+  return s;
+}
+
+// p[k] / s for every k, correctly rounded: one reciprocal and five FMA-pipe
+// steps each where the smallest numerator allows (s is 1 .. K), else the
+// division operator
+template <int K>
+__device__ __forceinline__ void softmax_div(float (&p)[K], float s) {
+  float lo = p[0];
+#pragma unroll
+  for (int k = 1; k < K; ++k) lo = fminf(lo, p[k]);
+  if (lo >= 0x1p-60f) {
+    const MarkDiv by(s);
+#pragma unroll
+    for (int k = 0; k < K; ++k) p[k] = by(p[k]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k) p[k] = p[k] / s;
+  }
+}
+
+// rqs_fwd / rqs_inv of make_knots(raw) without the knot arrays, the same bits:
+// the knots run on while the bin that holds v is carried along, and only the
+// bin's two slopes (in the tails the end slope) go through the softplus.
+template <int K, bool INV>
+__device__ __forceinline__ void rqs_apply(const float (&raw)[3 * K + 1], float v, const SplineCfg& c, float& out,
+                                          float& ld) {
+  const float scale = (c.rmax - c.rmin) - (float)K * c.min_bin;
+  float pw[K], ph[K];
+  softmax_div<K>(pw, softmax_num<K>(raw, pw));
+  softmax_div<K>(ph, softmax_num<K>(raw + K, ph));
+  const bool below = v <= c.rmin, above = v >= c.rmax;
+  // bin 0 also covers "no bin" (rqSpline.py:70-72)
+  float cw = 0.f, ch = 0.f, xk = c.rmin, yk = c.rmin;   // running left knot
+  float x0 = c.rmin, y0 = c.rmin, x1 = c.rmax, y1 = c.rmax, r0 = raw[2 * K], r1 = raw[2 * K + 1];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    float xn = c.rmax, yn = c.rmax;   // right knot of bin k
+    if (k < K - 1) {
+      cw += pw[k] * scale + c.min_bin;
+      ch += ph[k] * scale + c.min_bin;
+      xn = c.rmin + cw;
+      yn = c.rmin + ch;
+    }
+    const bool in = k == 0 || (INV ? v >= yk && v < yn : v >= xk && v < xn);
+    if (in) {
+      x0 = xk; x1 = xn; y0 = yk; y1 = yn;
+      r0 = raw[2 * K + k];
+      r1 = raw[2 * K + k + 1];
+    }
+    xk = xn;
+    yk = yn;
+  }
+  if (above) r1 = raw[3 * K];
+  const float d0 = softplus_f(r0 + c.slope_offset) + c.min_slope;
+  const float d1 = softplus_f(r1 + c.slope_offset) + c.min_slope;
+  const float w = x1 - x0, h = y1 - y0;
+  const float s = h / w;
+  const float st = d1 + d0 - 2.f * s;
+  float z;
+  if (!INV) {
+    z = fminf(fmaxf((v - x0) / w, 0.f), 1.f);
+  } else {
+    const float ww = fminf(fmaxf((v - y0) / h, 0.f), 1.f);
+    const float cq = -s * ww;
+    const float bq = d0 - st * ww;
+    const float aq = s - bq;
+    // _safe_quadratic_root (rqSpline.py:131-155)
+    const float disc = bq * bq - 4.f * aq * cq;
+    float sqd = sqrtf(fmaxf(disc, 1.17549435e-38f));
+    if (!(disc > 0.f)) sqd = 0.f;
+    const float num = (bq >= 0.f) ? 2.f * cq : -bq + sqd;
+    const float dnm = (bq >= 0.f) ? -bq - sqd : 2.f * aq;
+    z = fminf(fmaxf(num / dnm, 0.f), 1.f);
+  }
+  const float sq = z * z, q = z - sq, om = 1.f - z, sq1 = om * om;
+  const float den = s + st * q;
+  if (!INV) {
+    const float num = h * (s * sq + d0 * q);
+    out = y0 + num / den;
+    ld = 2.f * logf(s) + logf(d1 * sq + 2.f * s * q + d0 * sq1) - 2.f * logf(den);
+    if (below) { out = (v - c.rmin) * d0 + c.rmin; ld = logf(d0); }
+    if (above) { out = (v - c.rmax) * d1 + c.rmax; ld = logf(d1); }
+  } else {
+    out = w * z + x0;
+    ld = -2.f * logf(s) - logf(d1 * sq + 2.f * s * q + d0 * sq1) + 2.f * logf(den);
+    if (below) { out = (v - c.rmin) / d0 + c.rmin; ld = -logf(d0); }
+    if (above) { out = (v - c.rmax) / d1 + c.rmax; ld = -logf(d1); }
+  }
+}
+
 // Adjoint of (y, ld) = rqs_fwd(x; raw): given gy = dL/dy and gl = dL/dld,
 // returns dL/dx and accumulates dL/draw[0..3K] into graw.
 template <int K>
