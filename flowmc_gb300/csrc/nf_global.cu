@@ -6,10 +6,9 @@
 //   2. flow log_prob of the proposals and of the current positions in one
 //      pass (NF_proposal.py:44, 165-166: the proposals' flow density is
 //      recomputed by the forward pass, not taken from the inverse)
-//   3. k_nf_accept: per chain (a lane group, as in the local-step kernel),
-//      the target log-density of each proposal, the sequential
-//      independent-MH scan (NF_proposal.py:91-126) and the thinned buffer
-//      writes, fused in one kernel.
+//   3. k_nf_accept: the target log-density of each proposal, each chain's
+//      sequential independent-MH scan (NF_proposal.py:91-126) and the thinned
+//      buffer writes, fused in one kernel.
 #include "flow.cuh"
 #include "targets.cuh"
 
@@ -32,77 +31,149 @@ struct NfArgs {
   float *out_pos, *out_logp, *out_acc;
   int64_t buf_len, start;
   float *x_last, *lp_last;
-  int64_t C_pad;
+  int32_t chains_per_block;
+  int32_t tab_smem;   // diag Gaussian / mixture: tables staged in shared memory
+  int32_t scan_off;   // floats of dynamic shared memory before the scan's arrays
+  int32_t vec;        // rows are whole 16-byte chunks everywhere
 };
+
+// The accept scan. Only the scan itself is sequential, and it needs three
+// numbers per proposal, so a block takes CB chains and, for up to kNfSteps steps
+// at a time: (1) its lane groups evaluate the proposals' target log-densities in
+// parallel, (2) one thread per chain runs the accepts over shared memory and
+// notes which proposal each step holds, (3) the groups copy those rows to the
+// buffers. A group walking its chain's steps one after the other (before) waited
+// for a proposal's row and a full evaluation at every step: 4096 chains x 50
+// steps of the 64-D mixture 160 -> 78 us, 20 chains x 30 steps of the 5-D dual moon
+// 30 -> 8 us (GB300). Bound by HBM for many chains, by one evaluation and the scan's
+// dependent chain for few.
+constexpr int kNfSteps = 64;
 
 template <int TGT, int G, int V>
 __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
-  extern __shared__ float smem[];
-  const int gl = threadIdx.x % G;
-  const int64_t gpb = blockDim.x / G, gib = threadIdx.x / G;
-  const int d = a.d;
-  float* stage = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? smem + gib * d : nullptr;
+  extern __shared__ __align__(16) float smem[];
+  const int tid = threadIdx.x, gl = tid % G, gib = tid / G, gpb = blockDim.x / G;
+  const int d = a.d, CB = a.chains_per_block;
+  float* stage = nullptr;
   const TargetConst<TGT> tc(a.tgt);
-  const Rng rng = a.rng.at_epoch();
-  for (int64_t c = blockIdx.x * gpb + gib; c < a.C_pad; c += (int64_t)gridDim.x * gpb) {
-    const bool active = c < a.C;
-    const int64_t cc = active ? c : 0;
-    float x[V], g[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      const int j = gl * V + v;
-      x[v] = (j < d) ? __ldg(a.x0 + cc * d + j) : 0.f;
+  if constexpr (TGT == FMC_TARGET_DENSE_GAUSSIAN) {
+    stage = smem + gib * d;
+  } else if constexpr (TGT == FMC_TARGET_DIAG_GAUSSIAN || TGT == FMC_TARGET_GAUSS_MIXTURE) {
+    if (a.tab_smem) {
+      stage_target_table<G, V>(a.tgt, smem);
+      stage = smem;
     }
-    float lp = target_eval<TGT, G, V, false>(a.tgt, tc, x, g, gl, stage);   // take_steps.py:201-203
-    float lnf = __ldg(a.lnf + (int64_t)a.C * a.S + cc);
-    float xr[V], lpr = lp;
-#pragma unroll
-    for (int v = 0; v < V; ++v) xr[v] = x[v];
-    for (int s = 0; s < a.S; ++s) {
-      const int64_t row = cc * a.S + s;
-      float p[V];
+  }
+  const int n = CB * kNfSteps;
+  float* lp_s = smem + a.scan_off;          // [CB][kNfSteps] per proposal
+  float* lnf_s = lp_s + n;
+  float* logu_s = lnf_s + n;
+  int* held_s = reinterpret_cast<int*>(logu_s + n);   // step whose proposal is held (-1: the start), * 2 + accepted
+  float* cur_lp = reinterpret_cast<float*>(held_s + n);   // [CB] state of the scan
+  float* cur_lnf = cur_lp + CB;
+  float* rec_lp = cur_lnf + CB;             // at the last recorded step
+  int* cur = reinterpret_cast<int*>(rec_lp + CB);
+  int* rec = cur + CB;
+  const Rng rng = a.rng.at_epoch();
+
+  for (int64_t c0 = (int64_t)blockIdx.x * CB; c0 < a.C; c0 += (int64_t)gridDim.x * CB) {
+    const int nb = (int)(a.C - c0 < CB ? a.C - c0 : CB);
+    __syncthreads();
+    // log-density at the current positions (take_steps.py:201-203); the loops
+    // below run whole warps (the evaluations shuffle within a group)
+    for (int i0 = 0; i0 < nb; i0 += gpb) {
+      const bool act = i0 + gib < nb;
+      const int i = act ? i0 + gib : 0;
+      float x[V], g[V];
 #pragma unroll
       for (int v = 0; v < V; ++v) {
         const int j = gl * V + v;
-        p[v] = (j < d) ? __ldg(a.props + row * d + j) : 0.f;
+        x[v] = (j < d) ? __ldg(a.x0 + (c0 + i) * d + j) : 0.f;
       }
-      const float lpp = target_eval<TGT, G, V, false>(a.tgt, tc, p, g, gl, stage);
-      const float lnfp = __ldg(a.lnf + row);
-      const float u = a.unif ? __ldg(a.unif + row) : u32_to_unit(rng.draw(cc, s, 0u, RNG_TAG_NF_UNIFORM).x);
-      // ratio = (lp_p - lp_c) - (lnf_p - lnf_c)   (NF_proposal.py:102-104)
-      const ff ratio = ff_add(two_sum(lpp, -lp), ff_neg(two_sum(lnfp, -lnf)));
-      const bool acc = f_lt_ff(logf(u), ratio);
-      if (acc) {
-#pragma unroll
-        for (int v = 0; v < V; ++v) x[v] = p[v];
-        lp = lpp;
-        lnf = lnfp;
+      const float lp = target_eval<TGT, G, V, false>(a.tgt, tc, x, g, gl, stage);
+      if (act && gl == 0) {
+        cur_lp[i] = lp;
+        rec_lp[i] = lp;
+        cur_lnf[i] = __ldg(a.lnf + (int64_t)a.C * a.S + c0 + i);
+        cur[i] = -1;
+        rec[i] = -1;
       }
-      if (s % a.thin == 0) {
-        if (active) {
-          const int64_t orow = cc * a.buf_len + a.start + s / a.thin;
+    }
+    for (int s0 = 0; s0 < a.S; s0 += kNfSteps) {
+      const int ns = min(kNfSteps, a.S - s0);
+      const int items = nb * ns;
+      for (int i0 = 0; i0 < items; i0 += gpb) {
+        const bool act = i0 + gib < items;
+        const int i = act ? i0 + gib : 0;
+        const int ci = i / ns, si = i - ci * ns;
+        const int64_t c = c0 + ci, row = c * a.S + s0 + si;
+        float p[V], g[V];
 #pragma unroll
-          for (int v = 0; v < V; ++v) {
-            const int j = gl * V + v;
-            if (j < d) __stcs(a.out_pos + orow * d + j, x[v]);
+        for (int v = 0; v < V; ++v) {
+          const int j = gl * V + v;
+          p[v] = (j < d) ? __ldg(a.props + row * d + j) : 0.f;
+        }
+        const float lpp = target_eval<TGT, G, V, false>(a.tgt, tc, p, g, gl, stage);
+        if (act && gl == 0) {
+          const int q = ci * kNfSteps + si;
+          lp_s[q] = lpp;
+          lnf_s[q] = __ldg(a.lnf + row);
+          logu_s[q] = logf(a.unif ? __ldg(a.unif + row)
+                                  : u32_to_unit(rng.draw(c, s0 + si, 0u, RNG_TAG_NF_UNIFORM).x));
+        }
+      }
+      __syncthreads();
+      if (tid < nb) {
+        float lp = cur_lp[tid], lnf = cur_lnf[tid];
+        int held = cur[tid];
+        for (int si = 0; si < ns; ++si) {
+          const int q = tid * kNfSteps + si;
+          const float lpp = lp_s[q], lnfp = lnf_s[q];
+          // ratio = (lp_p - lp_c) - (lnf_p - lnf_c)   (NF_proposal.py:102-104)
+          const ff ratio = ff_add(two_sum(lpp, -lp), ff_neg(two_sum(lnfp, -lnf)));
+          const bool acc = f_lt_ff(logu_s[q], ratio);
+          if (acc) {
+            held = s0 + si;
+            lp = lpp;
+            lnf = lnfp;
           }
-          if (gl == 0) {
-            __stcs(a.out_logp + orow, lp);
-            __stcs(a.out_acc + orow, acc ? 1.f : 0.f);
+          held_s[q] = held * 2 + (acc ? 1 : 0);
+          lp_s[q] = lp;
+          if ((s0 + si) % a.thin == 0) {
+            rec[tid] = held;
+            rec_lp[tid] = lp;
           }
         }
-#pragma unroll
-        for (int v = 0; v < V; ++v) xr[v] = x[v];
-        lpr = lp;
+        cur_lp[tid] = lp;
+        cur_lnf[tid] = lnf;
+        cur[tid] = held;
       }
+      __syncthreads();
+      for (int i = gib; i < items; i += gpb) {
+        const int ci = i / ns, si = i - ci * ns, s = s0 + si;
+        if (s % a.thin != 0) continue;
+        const int64_t c = c0 + ci, orow = c * a.buf_len + a.start + s / a.thin;
+        const int h = held_s[ci * kNfSteps + si], held = h >> 1;
+        const float* src = held < 0 ? a.x0 + c * d : a.props + (c * a.S + held) * d;
+        float* dst = a.out_pos + orow * d;
+        if (a.vec) {
+          for (int j = 4 * gl; j < d; j += 4 * G)
+            __stcs(reinterpret_cast<float4*>(dst + j), __ldg(reinterpret_cast<const float4*>(src + j)));
+        } else {
+          for (int j = gl; j < d; j += G) __stcs(dst + j, __ldg(src + j));
+        }
+        if (gl == 0) {
+          __stcs(a.out_logp + orow, lp_s[ci * kNfSteps + si]);
+          __stcs(a.out_acc + orow, (h & 1) ? 1.f : 0.f);
+        }
+      }
+      __syncthreads();
     }
-    if (active) {
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        const int j = gl * V + v;
-        if (j < d) a.x_last[cc * d + j] = xr[v];
-      }
-      if (gl == 0 && a.lp_last) a.lp_last[cc] = lpr;
+    for (int i = gib; i < nb; i += gpb) {
+      const int64_t c = c0 + i;
+      const float* src = rec[i] < 0 ? a.x0 + c * d : a.props + (c * a.S + rec[i]) * d;
+      for (int j = gl; j < d; j += G) a.x_last[c * d + j] = __ldg(src + j);
+      if (gl == 0 && a.lp_last) a.lp_last[c] = rec_lp[i];
     }
   }
 }
@@ -110,17 +181,36 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
 template <int TGT, int G, int V>
 static int launch_nf_t(const NfArgs& a0, cudaStream_t st) {
   NfArgs a = a0;
-  const int threads = 256, gpb = threads / G, gpw = 32 / G;
-  a.C_pad = ((int64_t)a.C + gpw - 1) / gpw * gpw;
-  const size_t smem = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? (size_t)gpb * a.d * sizeof(float) : 0;
-  int64_t blocks = (a.C_pad + gpb - 1) / gpb;
+  const int threads = 256, gpb = threads / G;
+  // one chain per block until they fill the SMs several times over, then four
+  // (fewer idle groups at the end of a chain's steps)
+  a.chains_per_block = a.C <= 8 * sm_count() ? 1 : 4;
+  size_t floats = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? (size_t)gpb * a.d : 0;
+  a.tab_smem = 0;
+  if (TGT == FMC_TARGET_DIAG_GAUSSIAN || TGT == FMC_TARGET_GAUSS_MIXTURE) {
+    const int tab = target_table_floats(TGT == FMC_TARGET_GAUSS_MIXTURE ? a.tgt.n_comp : 1, G * V);
+    if (tab <= 33 * 256) {
+      floats = tab;
+      a.tab_smem = 1;
+    }
+  }
+  floats = (floats + 3) / 4 * 4;
+  a.scan_off = (int)floats;
+  floats += (size_t)a.chains_per_block * (4 * kNfSteps + 5);
+  a.vec = a.d % 4 == 0 && ((uintptr_t)a.out_pos & 15) == 0 && ((uintptr_t)a.props & 15) == 0 &&
+          ((uintptr_t)a.x0 & 15) == 0;
+  int64_t blocks = (a.C + a.chains_per_block - 1) / a.chains_per_block;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
+  auto kern = k_nf_accept<TGT, G, V>;
+  const size_t smem = floats * sizeof(float);
+  if (smem > 48 * 1024)
+    FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // proposals and their flow densities read, thinned rows written
   const double n_rec = (double)((a.S + a.thin - 1) / a.thin);
   KernelTimer kt(FMC_KT_NF_ACCEPT, st, 0.0,
                  (double)a.C * a.S * (4.0 * a.d + 4.0) + (double)a.C * n_rec * (4.0 * a.d + 8.0));
-  k_nf_accept<TGT, G, V><<<(int)blocks, threads, smem, st>>>(a);
+  kern<<<(int)blocks, threads, smem, st>>>(a);
   FMC_LAUNCH_CHECK();
   return FMC_OK;
 }
