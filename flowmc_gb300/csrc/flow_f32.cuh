@@ -46,6 +46,31 @@ struct FlowShape {
     for (int u = 0; u < i; ++u) o += (int64_t)out(l, u) * (in(l, u) + 1);
     return o;
   }
+  // columns of a layer's saved activations: conditioning block, hidden
+  // activations, conditioner outputs (act_col: first column of Linear i's
+  // input; i = nh + 1: its outputs), and of its output gradients
+  __host__ __device__ int act_col(int l, int i) const {
+    int c = 0;
+    for (int u = 0; u < i; ++u) c += in(l, u);
+    return c;
+  }
+  __host__ __device__ int act_cols(int l) const { return act_col(l, nh + 1) + out(l, nh); }
+  __host__ __device__ int64_t act_base(int l) const {   // columns before layer l
+    return (int64_t)(l / 2) * (act_cols(0) + act_cols(1)) + (l & 1) * act_cols(0);
+  }
+  // padded columns of the Linears' output gradients (rows of round_up(out, 4)
+  // floats): those before Linear i of layer l
+  __host__ __device__ int gpad(int l, int i) const { return (out(l, i) + 3) & ~3; }
+  __host__ __device__ int gcols(int l) const {
+    int c = 0;
+    for (int u = 0; u <= nh; ++u) c += gpad(l, u);
+    return c;
+  }
+  __host__ __device__ int64_t gcol(int l, int i) const {
+    int64_t c = (int64_t)(l / 2) * (gcols(0) + gcols(1)) + (l & 1) * gcols(0);
+    for (int u = 0; u < i; ++u) c += gpad(l, u);
+    return c;
+  }
   // outputs per product tile of Linear i
   __host__ __device__ int tile_cols(int i) const { return i == nh ? dg * P : kFlowCols; }
 };
@@ -221,6 +246,147 @@ __device__ __forceinline__ void flow_product(WStream<FlowTile<R>::NT, FlowTile<R
       f2_unpack(acc[q][j][0], out[q][j].x, out[q][j].y);
       f2_unpack(acc[q][j][1], out[q][j].z, out[q][j].w);
     }
+}
+
+// ------------------------------------------------------------------ backward products
+// The stream of weight rows for C[row, n] = sum_k G[row, k] W[k, n] (a Linear's
+// input gradient: k its outputs, n its inputs), layers L-1 .. 0 and Linears
+// nh .. 0, in stages of 16 rows; the last Linear's rows in groups of dg
+// coordinates, each padded to whole stages with zeros.
+template <int NT, int ST>
+struct WtStream {
+  const FlowShape* s;
+  const float* theta;
+  uint32_t ring;
+  int l, i, g0, K, N, slot, k0;   // g0: first row of the group, K: its rows
+  const float* W;                 // row g0 of W
+  bool v2;
+
+  __device__ __forceinline__ void set() {
+    N = s->in(l, i);
+    const int out = s->out(l, i);
+    K = i == s->nh ? min(s->dg * s->P, out - g0) : out;
+    W = theta + s->layer_off(l) + s->w_off(l, i) + (int64_t)g0 * N;
+    v2 = ((uintptr_t)W & 7) == 0 && (N & 1) == 0;
+    k0 = 0;
+  }
+  __device__ __forceinline__ void begin(const FlowShape* shape, const float* th, const float* r) {
+    s = shape;
+    theta = th;
+    ring = (uint32_t)__cvta_generic_to_shared(r);
+    l = s->L - 1;
+    i = s->nh;
+    g0 = slot = 0;
+    set();
+#pragma unroll
+    for (int q = 0; q < ST - 1; ++q) issue();
+  }
+  __device__ __forceinline__ void issue() {
+    if (l >= 0) {
+      const uint32_t dst = ring + slot * (4 * kFlowBK * kFlowCols);
+      if (v2) {
+        constexpr int C2 = kFlowCols / 2, RPT = NT / C2;   // 8-byte chunks per row, rows per pass
+        const int r = threadIdx.x / C2, c = 2 * (threadIdx.x % C2);
+        if (c < N) {
+#pragma unroll
+          for (int q = 0; q < kFlowBK / RPT; ++q) {
+            const int rr = r + RPT * q, k = k0 + rr;
+            const int bytes = k < K ? 8 : 0;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + 4 * (rr * kFlowCols + c)),
+                         "l"(W + (int64_t)(k < K ? k : 0) * N + c), "r"(bytes));
+          }
+        }
+      } else {
+        constexpr int RPT = NT / kFlowCols;
+        const int r = threadIdx.x / kFlowCols, c = threadIdx.x % kFlowCols;
+        if (c < N) {
+#pragma unroll 4
+          for (int q = 0; q < kFlowBK / RPT; ++q) {
+            const int rr = r + RPT * q, k = k0 + rr;
+            const int bytes = k < K ? 4 : 0;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * (rr * kFlowCols + c)),
+                         "l"(W + (int64_t)(k < K ? k : 0) * N + c), "r"(bytes));
+          }
+        }
+      }
+      slot = slot + 1 == ST ? 0 : slot + 1;
+      k0 += kFlowBK;
+      if (k0 >= K) {
+        g0 += K;
+        if (g0 == s->out(l, i)) {
+          g0 = 0;
+          if (--i < 0) {
+            i = s->nh;
+            --l;
+          }
+        }
+        if (l >= 0) set();
+      }
+    }
+    asm volatile("cp.async.commit_group;");
+  }
+};
+
+// columns of a thread in the backward products: pairs or quads of adjacent
+// columns, col(0) .. , groups 32 columns apart
+template <int R>
+struct FlowTileT {
+  using T = FlowTile<R>;
+  static constexpr int E = T::TN >= 4 ? 4 : T::TN;   // adjacent columns
+  static constexpr int NG = T::TN / E;               // groups, 8 E columns apart
+  static __device__ __forceinline__ int col0() {
+    return ((threadIdx.x >> 5) % T::WC) * (8 * T::TN) + (threadIdx.x & 7) * E;
+  }
+};
+
+// acc[q][c][.] += the four rows r0 + 16 q .. of G . W for this thread's TN
+// columns, over K rows of W; G is [k][row] with zeros up to a multiple of 16
+template <int R>
+__device__ __forceinline__ void flow_product_t(WtStream<FlowTile<R>::NT, FlowTile<R>::ST>& w, const float* ring, int& slot,
+                                               const float* G, int N, int K, int r0,
+                                               uint64_t (&acc)[FlowTile<R>::TQ][FlowTile<R>::TN][2]) {
+  using T = FlowTile<R>;
+  using U = FlowTileT<R>;
+  const int c0 = U::col0();
+  const bool on = ((threadIdx.x >> 5) % T::WC) * (8 * T::TN) < N;
+  const float* Gr = G + r0;
+  for (int k0 = 0; k0 < K; k0 += kFlowBK) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(T::ST - 2) : "memory");
+    __syncthreads();
+    w.issue();
+    if (on) {
+      const float* Ws = ring + slot * (kFlowBK * kFlowCols) + c0;
+#pragma unroll
+      for (int k = 0; k < kFlowBK; ++k) {
+        uint64_t b[T::TN];
+#pragma unroll
+        for (int g = 0; g < U::NG; ++g) {
+          if constexpr (U::E == 4) {
+            const float4 v = *reinterpret_cast<const float4*>(Ws + k * kFlowCols + 32 * g);
+            b[4 * g] = f2_pack(v.x, v.x);
+            b[4 * g + 1] = f2_pack(v.y, v.y);
+            b[4 * g + 2] = f2_pack(v.z, v.z);
+            b[4 * g + 3] = f2_pack(v.w, v.w);
+          } else {
+            const float2 v = *reinterpret_cast<const float2*>(Ws + k * kFlowCols);
+            b[0] = f2_pack(v.x, v.x);
+            b[1] = f2_pack(v.y, v.y);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < T::TQ; ++q) {
+          const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(Gr + k * T::LD + 16 * q);
+#pragma unroll
+          for (int j = 0; j < T::TN; ++j) {
+            acc[q][j][0] = f2_fma(a.x, b[j], acc[q][j][0]);
+            acc[q][j][1] = f2_fma(a.y, b[j], acc[q][j][1]);
+          }
+        }
+      }
+    }
+    Gr += kFlowBK * T::LD;
+    slot = slot + 1 == T::ST ? 0 : slot + 1;
+  }
 }
 
 }  // namespace fmc

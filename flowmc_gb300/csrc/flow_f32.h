@@ -19,12 +19,29 @@ struct FlowF32Call {
   float* y;
   float* ld;
   float* logp;
+  // training (forward, FLOW_OUT_LOGP), both or neither: [L + 1, n, d] layer
+  // inputs and the output, and the activations flow_f32_grad reads
   float* save;
+  float* acts;
 };
 
 // whether the flow's row tile fits in shared memory
 bool flow_f32_fused(const FlowGeom& g);
+// rows per CTA (and per tile of the saved activations) for n rows
+int flow_f32_tile(const FlowGeom& g, int64_t n);
 // all layers over c.n rows in one launch
 int flow_f32_pass(const FlowF32Call& c, const FlowGeom& g, cudaStream_t st);
+
+// floats of split-K partials the FP32 weight gradients may use (they bound the
+// number of slices, and with it the order of the sums)
+int64_t kouter_part_floats(const FlowGeom& g);
+// The loss gradient from a forward pass that left `save` and `acts`
+// (flow_f32_bwd.cu): whether the flow's backward tile fits (hidden widths and
+// conditioning block up to 128), floats of its workspace (the activations
+// first), and the gradient itself into grad [n_params].
+bool flow_f32_grad_fits(const FlowGeom& g, int64_t n);
+int64_t flow_f32_grad_floats(const FlowGeom& g, int64_t n);
+int flow_f32_grad(const FlowGeom& g, const float* theta, const float* aux, int64_t n, const float* save, float* ws,
+                  float* grad, cudaStream_t st);
 
 }  // namespace fmc

@@ -15,6 +15,7 @@
 #include "flow_f32.h"
 #include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
+#include "train_sums.cuh"
 
 namespace fmc {
 
@@ -23,6 +24,7 @@ static int64_t a256(int64_t v) { return (v + 255) / 256 * 256; }
 struct TrainWs {
   float *xs, *xa, *cond, *hs, *raw, *graw, *gh0, *gh1, *gcond, *gy, *gxa, *ld, *logp, *part;
   int64_t part_floats;
+  float* f32;          // FP32 flows on the fused path: activations and gradient scratch (flow_f32_bwd.cu)
   // FP32 path: split-K partials of the weight-gradient GEMMs (K = the batch)
   float* spart;
   int64_t spart_floats;
@@ -36,12 +38,6 @@ struct TrainWs {
   uint16_t *cond16, *hs16, *graw16, *gz16[2];
   int64_t n128, n64, hld, ncld, pld;
 };
-
-static int colsum_blocks(int64_t n) {
-  int64_t rb = (n + 511) / 512;
-  if (rb > 128) rb = 128;
-  return (int)(rb < 1 ? 1 : rb);
-}
 
 static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, TrainWs& w, size_t* total) {
   char* p = (char*)ws;
@@ -58,6 +54,13 @@ static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, Train
   };
   const int64_t ntP = (int64_t)g.nt_max() * g.P;
   w.xs = take((int64_t)(g.L + 1) * n * g.d);
+  w.f32 = nullptr;
+  if (!bf16 && flow_f32_grad_fits(g, n)) {
+    w.logp = take(n);
+    w.f32 = take(flow_f32_grad_floats(g, n));
+    if (total) *total = (size_t)used;
+    return;
+  }
   w.xa = take(n * g.d);
   w.cond = take(n * g.nc_max());
   // fp32 conditioner activations and gradients: the FP32 path only
@@ -78,16 +81,7 @@ static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, Train
   w.spart = nullptr;
   w.spart_floats = 0;
   if (!bf16) {
-    int64_t mn = 1;
-    for (int l = 0; l < g.L; ++l)
-      for (int i = 0; i <= g.nh; ++i) {
-        const int64_t f = (int64_t)g.lin_out(l, i) * g.lin_in(l, i);
-        if (f > mn) mn = f;
-      }
-    int64_t s = (int64_t)(16 << 20) / mn;   // about 64 MB of partials at most
-    if (s > kKouterMaxSlices) s = kKouterMaxSlices;
-    if (s < 2) s = 2;
-    w.spart_floats = s * mn;
+    w.spart_floats = kouter_part_floats(g);
     w.spart = take(w.spart_floats);
   }
   w.ldp = w.bpart = w.kpart = w.colpart = nullptr;
@@ -207,23 +201,6 @@ static int colsum_bf16(cudaStream_t st, const uint16_t* gm, int64_t n, int m, in
   return FMC_OK;
 }
 
-template <int NT>
-__device__ __forceinline__ float block_sum(float v, float* sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  float r = 0.f;
-  if (threadIdx.x < 32) {
-    r = (lane < NT / 32) ? sh[lane] : 0.f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-  }
-  return r;  // valid in thread 0
-}
-
 // loss = -mean(logp): one block, fixed order
 __global__ void __launch_bounds__(1024) k_loss(const float* __restrict__ logp, int64_t n, float* __restrict__ loss) {
   __shared__ float sh[32];
@@ -248,51 +225,18 @@ __global__ void __launch_bounds__(256) k_affine_bwd(const float* __restrict__ gx
                                                     const float* __restrict__ xa, int64_t n, int d, int nc, int cpar,
                                                     const float* __restrict__ th_layer, float* __restrict__ gx,
                                                     float* __restrict__ part) {
-  __shared__ float sh[32];
   const float es = expf(th_layer[0]);
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  float st = 0.f, ss = 0.f;
-  for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n; r += warps) {
-    const float* gr = gxa + r * d;
-    const float* xr = xa + r * d;
-    const float* cr = gcond + r * nc;
-    float* out = gx + r * d;
-    for (int j = lane; j < d; j += 32) {
-      float g = gr[j];
-      if ((j & 1) == cpar) g += cr[j >> 1];
-      const float gv = g * es;
-      out[j] = gv;
-      st += gv;
-      ss += g * xr[j];
-    }
-  }
-  st = block_sum<256>(st, sh);
-  ss = block_sum<256>(ss, sh);
-  if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = st;
-    part[2 * blockIdx.x + 1] = ss;
-  }
+  affine_sums(n, d, part, [&](int64_t r, int j, float& g, float& x, float& gv) {
+    g = gxa[r * d + j];
+    if ((j & 1) == cpar) g += gcond[r * nc + (j >> 1)];
+    x = xa[r * d + j];
+    gv = g * es;
+    gx[r * d + j] = gv;
+  });
 }
 
-// the ScalarAffine's two gradients from the nb block partials: one warp,
-// lane i summing partials i, i + 32, ..., then a fixed-order butterfly
 __global__ void k_affine_param_grad(const float* __restrict__ part, int nb, float ld_term, float* __restrict__ g_layer) {
-  const int lane = threadIdx.x & 31;
-  float st = 0.f, ss = 0.f;
-  for (int b = lane; b < nb; b += 32) {
-    st += part[2 * b];
-    ss += part[2 * b + 1];
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    st += __shfl_xor_sync(0xffffffffu, st, o);
-    ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  }
-  if (threadIdx.x == 0) {
-    g_layer[0] = ss + ld_term;  // d/d scale
-    g_layer[1] = st;            // d/d shift
-  }
+  affine_param_grad(part, nb, ld_term, g_layer);
 }
 
 static int ew_blocks(int64_t tot) {
@@ -444,10 +388,8 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     rb = (int)(b < 1 ? 1 : b);
   }
 
-  // ---- forward, saving layer inputs (FP32 flows whose row tile fits in shared
-  // memory: one launch)
-  const bool fused = !bf16 && flow_f32_fused(g);
-  if (fused) {
+  if (w.f32 != nullptr) {
+    // FP32 flows on the fused path: one launch forward, the gradient in a few
     FlowF32Call c{};
     c.theta = f->theta;
     c.aux = f->aux;
@@ -457,12 +399,17 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     c.out_mode = FLOW_OUT_LOGP;
     c.logp = w.logp;
     c.save = w.xs;
+    c.acts = w.f32;
     if ((rc = flow_f32_pass(c, g, st))) return rc;
-  } else {
-    k_standardize<<<eb, 256, 0, st>>>(x, n, d, f->aux, w.xs);
+    k_loss<<<1, 1024, 0, st>>>(w.logp, n, loss);
     FMC_LAUNCH_CHECK();
+    return flow_f32_grad(g, f->theta, f->aux, n, w.xs, w.f32, grad, st);
   }
-  for (int l = 0; l < g.L && !fused; ++l) {
+
+  // ---- forward, saving layer inputs
+  k_standardize<<<eb, 256, 0, st>>>(x, n, d, f->aux, w.xs);
+  FMC_LAUNCH_CHECK();
+  for (int l = 0; l < g.L; ++l) {
     float* xin = w.xs + (int64_t)l * nd;
     float* xout = w.xs + (int64_t)(l + 1) * nd;
     k_affine<<<rb, 256, 0, st>>>(xin, xout, bf16 ? nullptr : w.cond, bf16 ? w.cond16 : nullptr, g.w16_cols(l, 0),
@@ -479,7 +426,7 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     }
   }
   const float* y = w.xs + (int64_t)g.L * nd;
-  if (!fused) {
+  {
     int64_t blocks = (n + 7) / 8;
     if (blocks > (int64_t)sm_count() * 16) blocks = (int64_t)sm_count() * 16;
     k_base_logprob<<<(int)blocks, 256, 0, st>>>(y, w.ld, n, d, f->aux, w.logp);
@@ -553,7 +500,7 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
       }
     }
     // ScalarAffine adjoint -> d(layer input) into gy
-    const int ab = eb < 1024 ? eb : 1024;
+    const int ab = affine_sum_blocks(n, d);
     k_affine_bwd<<<ab, 256, 0, st>>>(w.gxa, w.gcond, w.xa, n, d, g.nc(l), g.cpar(l), th, w.gy, w.part);
     FMC_LAUNCH_CHECK();
     k_affine_param_grad<<<1, 32, 0, st>>>(w.part, ab, gld * (float)d * (float)n, gl);

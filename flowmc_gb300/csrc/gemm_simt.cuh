@@ -190,6 +190,23 @@ __global__ void k_sum_slices(const float* __restrict__ part, int S, int64_t mn, 
   }
 }
 
+// slices of the K rows for an [M, N] output: enough 64 x 64 tiles for two blocks
+// per SM, at least 256 rows each, as many as part_floats floats of partials
+// hold; *kslice: rows per slice (whole 16-row steps)
+inline int64_t kouter_slices(int M, int N, int64_t K, bool has_part, int64_t part_floats, int64_t* kslice) {
+  const int64_t mn = (int64_t)M * N;
+  const int64_t tiles = (int64_t)((N + 63) / 64) * ((M + 63) / 64);
+  int64_t S = (2 * (int64_t)sm_count() + tiles - 1) / tiles;
+  const int64_t by_rows = (K + 255) / 256;   // at least 256 rows per slice
+  if (S > by_rows) S = by_rows;
+  if (S > kKouterMaxSlices) S = kKouterMaxSlices;
+  if (!has_part || S * mn > part_floats) S = has_part ? part_floats / mn : 1;
+  if (S < 1) S = 1;
+  *kslice = (((K + S - 1) / S) + 15) / 16 * 16;
+  S = (K + *kslice - 1) / *kslice;
+  return S < 1 ? 1 : S;
+}
+
 // out [M, N] = A^T B over K rows (A [K, lda], B [K, ldb]); ones: column sums
 // of A. part holds part_floats floats of slice partials; with room for fewer
 // than two slices the single slice is written to out directly.
@@ -197,16 +214,8 @@ inline int kouter(cudaStream_t st, int M, int N, int64_t K, const float* A, int6
                   bool ones, float* part, int64_t part_floats, float* out) {
   if (M <= 0 || N <= 0) return FMC_OK;
   const int64_t mn = (int64_t)M * N;
-  const int64_t tiles = (int64_t)((N + 63) / 64) * ((M + 63) / 64);
-  int64_t S = (2 * (int64_t)sm_count() + tiles - 1) / tiles;
-  const int64_t by_rows = (K + 255) / 256;   // at least 256 rows per slice
-  if (S > by_rows) S = by_rows;
-  if (S > kKouterMaxSlices) S = kKouterMaxSlices;
-  if (part == nullptr || S * mn > part_floats) S = part != nullptr ? part_floats / mn : 1;
-  if (S < 1) S = 1;
-  const int64_t kslice = (((K + S - 1) / S) + 15) / 16 * 16;
-  S = (K + kslice - 1) / kslice;
-  if (S < 1) S = 1;
+  int64_t kslice = 0;
+  const int64_t S = kouter_slices(M, N, K, part != nullptr, part_floats, &kslice);
   float* dst = S > 1 ? part : out;
   dim3 grid((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64), (unsigned)S);
   if (ones)

@@ -53,11 +53,17 @@ __global__ void __launch_bounds__(256) k_sumsq(const float* __restrict__ g, int6
 }
 
 // state[0] = clip factor applied as (g / norm) * max_norm, state[1] = norm; count += 1
-__global__ void k_norm_final(const float* __restrict__ part, int nb, float max_norm, float* __restrict__ state,
-                             int32_t* __restrict__ count) {
+// (the partials are fetched by all threads first: added one after the other
+// straight from memory they took 8-10 us)
+__global__ void __launch_bounds__(kNormBlocks) k_norm_final(const float* __restrict__ part, int nb, float max_norm,
+                                                            float* __restrict__ state, int32_t* __restrict__ count) {
+  __shared__ float sh[kNormBlocks];
+  if (threadIdx.x < nb) sh[threadIdx.x] = part[threadIdx.x];
+  __syncthreads();
   if (threadIdx.x != 0) return;
   float s = 0.f;
-  for (int b = 0; b < nb; ++b) s += part[b];
+#pragma unroll 16
+  for (int b = 0; b < nb; ++b) s += sh[b];
   const float norm = sqrtf(s);
   state[0] = (norm < max_norm) ? 0.f : 1.f;  // 1 -> clip
   state[1] = norm;
@@ -356,7 +362,7 @@ extern "C" int fmc_adamw_step(float* theta, uint16_t* theta_bf16, const float* g
   float* state = part + kNormBlocks;
   k_sumsq<<<kNormBlocks, 256, 0, st>>>(grad, n, part);
   FMC_LAUNCH_CHECK();
-  k_norm_final<<<1, 32, 0, st>>>(part, kNormBlocks, p->max_norm, state, count);
+  k_norm_final<<<1, kNormBlocks, 0, st>>>(part, kNormBlocks, p->max_norm, state, count);
   FMC_LAUNCH_CHECK();
   k_adamw<<<grid_ew(n, 16), 256, 0, st>>>(theta, theta_bf16, grad, m, v, n, state, count, p->lr, p->b1, p->b2, p->eps,
                                           p->weight_decay, p->max_norm, aux, n_aux);
