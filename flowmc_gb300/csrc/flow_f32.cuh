@@ -103,6 +103,25 @@ struct FlowTile {
   static constexpr int ST = R >= 64 ? 2 : 3;
 };
 
+// Tiles of [column][R] go to and from memory as one bulk copy per column (R
+// floats, 16-byte aligned on both sides; smem pitch R + 4). A store is issued by
+// the thread of its column after fence_async + barrier; the tile may be
+// overwritten after the issuing threads' bulk_store_wait and a barrier.
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+template <int R>
+__device__ __forceinline__ void tile_store(const float* tile, float* dst, int cols) {
+  for (int c = threadIdx.x; c < cols; c += FlowTile<R>::NT)
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst + (int64_t)c * R),
+                 "r"((uint32_t)__cvta_generic_to_shared(tile + c * FlowTile<R>::LD)), "r"(4 * R)
+                 : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// all but the `N` newest stores of this thread have read their tile
+template <int N>
+__device__ __forceinline__ void bulk_store_wait() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+
 // lanes: 4 row groups x 8 outputs
 __device__ __forceinline__ int flow_lane_row() { return ((threadIdx.x & 31) >> 3) * 4; }
 __device__ __forceinline__ int flow_lane_col() { return threadIdx.x & 7; }

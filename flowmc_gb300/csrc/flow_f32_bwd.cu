@@ -22,7 +22,11 @@
 // a training trajectory crosses spline knots, and gradients that differ in the
 // last place part from each other there after an optimiser step.
 //
-// @@MEASURED@@
+// Bound by FMA issue and, with eight warps per SM, by the latency of the spline
+// adjoint. Measured on GB300, loss + gradient + AdamW: 16,384 rows of the 32-D
+// flow (8 x [128, 128] x 10 bins) 5.88 -> 2.38 ms (forward 0.79, backward 0.97,
+// weight gradients 0.44 = 48 TFLOP/s, biases 0.07); 10,000 rows of the 5-D flow
+// (4 x [32, 32] x 8 bins) 1.02 -> 0.34 ms.
 #include <algorithm>
 #include "flow_f32.cuh"
 #include "flow_f32.h"
@@ -99,41 +103,55 @@ __global__ void __launch_bounds__(FlowTile<R>::NT, 2) k_flow_f32_bwd(const __gri
     const float* raw = a.acts + ((s.act_base(l) + s.act_col(l, s.nh + 1)) * a.tiles + (int64_t)blockIdx.x * out) * R;
     const int gp = s.gpad(l, s.nh);
     float* graw = a.gout + s.gcol(l, s.nh) * (a.tiles * R) + row_base * gp;
-    for (int n0 = 0, c0t = 0; n0 < out; n0 += tc, c0t += s.dg) {
+    // raw tiles by cp.async, the next group's while this one is worked on; the
+    // copies ride in the weight stream's groups
+    auto fetch = [&](int n0, float* tile) {
       const int N = min(tc, out - n0), Np = (N + 15) & ~15;
-      __syncthreads();   // t0's readers, xs and gy are done
+      const float* src = raw + (int64_t)n0 * R;
       for (int e = tid; e < Np * (R / 4); e += NT) {
         const int c = e / (R / 4), r = (e % (R / 4)) * 4;
-        *reinterpret_cast<float4*>(t0 + c * T::LD + r) =
-            c < N ? *reinterpret_cast<const float4*>(raw + (int64_t)(n0 + c) * R + r) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float* dst = tile + c * T::LD + r;
+        if (c < N)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                       "l"(src + c * R + r));
+        else
+          *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      __syncthreads();
+    };
+    float* tile = t0;
+    float* next = t1;
+    fetch(0, tile);
+    for (int n0 = 0, c0t = 0; n0 < out; n0 += tc, c0t += s.dg) {
+      const int N = min(tc, out - n0);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();   // the tile, xs and gy are complete, the other tile is free
+      if (n0 + tc < out) fetch(n0 + tc, next);
       const int items = (N / P) * R;
       for (int e = tid; e < items; e += NT) {
         const int t = e / R;
-        float prm[P], g[P];
+        float prm[P];
+        float* tp = tile + t * P * T::LD + row;
 #pragma unroll
-        for (int p = 0; p < P; ++p) prm[p] = t0[(t * P + p) * T::LD + row];
-        Knots<K> kn;
-        make_knots<K>(prm, s.cfg, kn);
+        for (int p = 0; p < P; ++p) prm[p] = tp[p * T::LD];
         const int j = row * a.ldx + 2 * (c0t + t) + tpar;
-        gy[j] = rqs_fwd_adjoint<K>(xs[j], prm, s.cfg, kn, gy[j], gld, g);
-#pragma unroll
-        for (int p = 0; p < P; ++p) t0[(t * P + p) * T::LD + row] = g[p];
+        gy[j] = rqs_adjoint<K>(prm, xs[j], s.cfg, gy[j], gld, [&](int p, float v) { tp[p * T::LD] = v; });
       }
       __syncthreads();
       // rows of d raw: eight columns x four rows per warp access (distinct banks,
       // whole sectors)
       for (int e = wid; e < (N + 7) / 8 * (R / 4); e += NW) {
         const int c = e / (R / 4) * 8 + (lane & 7), r = e % (R / 4) * 4 + (lane >> 3);
-        if (c < N) graw[(int64_t)r * gp + n0 + c] = t0[c * T::LD + r];
+        if (c < N) graw[(int64_t)r * gp + n0 + c] = tile[c * T::LD + r];
       }
-      flow_product_t<R>(w, ring, slot, t0, hin, N, r0, acc);
+      flow_product_t<R>(w, ring, slot, tile, hin, N, r0, acc);
+      float* t = tile;
+      tile = next;
+      next = t;
     }
 
     // ---- hidden Linears: dz = (gradient) (1 - h^2), then through the Linear
-    float* cur = t1;
-    float* other = t0;
+    float* cur = tile;   // not the last group's
+    float* other = next;
     for (int i = s.nh - 1; i >= 0; --i) {
       const int H = s.out(l, i), Hp = (H + 15) & ~15;
       const float* h = a.acts + ((s.act_base(l) + s.act_col(l, i + 1)) * a.tiles + (int64_t)blockIdx.x * H) * R;
@@ -374,7 +392,7 @@ __global__ void k_bias_partial(const __grid_constant__ FlowShape s, const float*
   const float* g = gout + col * rows_pad + c;
   const int64_t r0 = blockIdx.y * rows_per, r1 = r0 + rows_per < n ? r0 + rows_per : n;
   float v = 0.f;
-#pragma unroll 8
+#pragma unroll 32   // the adds are one chain, the loads are not
   for (int64_t r = r0; r < r1; ++r) v += g[r * gp];
   part[(col + c) * gridDim.y + blockIdx.y] = v;
 }

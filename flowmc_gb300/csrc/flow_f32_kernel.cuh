@@ -111,11 +111,7 @@ __global__ void __launch_bounds__(FlowTile<R>::NT, 2) k_flow_f32(const __grid_co
           if (SAVE && r < rows) a.save[((int64_t)u * a.n + row_base + r) * d + j] = v0;
           const float v = scalar_affine(v0, es, sh, INV ? 1 : 0);
           xr[j] = v;
-          if ((j & 1) == cpar) {
-            cond[(j >> 1) * T::LD + r] = v;
-            if (SAVE)
-              a.acts[(s.act_base(l) * a.tiles + (int64_t)blockIdx.x * nc + (j >> 1)) * R + r] = v;
-          }
+          if ((j & 1) == cpar) cond[(j >> 1) * T::LD + r] = v;
         }
         for (int k = nc + lane; k < kp; k += 32) cond[k * T::LD + r] = 0.f;
       }
@@ -123,6 +119,17 @@ __global__ void __launch_bounds__(FlowTile<R>::NT, 2) k_flow_f32(const __grid_co
         const float al = scalar_affine_logdet(sc, d, INV ? 1 : 0);
         ld = u == 0 ? al : __fadd_rn(ld, al);
       }
+    }
+    // SAVE: a tile of the layer's array i to the saved activations
+    auto keep = [&](const float* tile, int i, int first, int cols, int of) {
+      fence_async();
+      __syncthreads();
+      tile_store<R>(tile, a.acts + ((s.act_base(l) + s.act_col(l, i)) * a.tiles + (int64_t)blockIdx.x * of + first) * R,
+                    cols);
+    };
+    if (SAVE) {
+      bulk_store_wait<0>();   // the previous layer's last tile
+      keep(cond, 0, 0, nc, nc);
     }
     // ---- hidden Linears
     const float* A = cond;
@@ -135,6 +142,9 @@ __global__ void __launch_bounds__(FlowTile<R>::NT, 2) k_flow_f32(const __grid_co
       for (int n0 = 0; n0 < out; n0 += kFlowCols) {
         const int N = min(kFlowCols, out - n0);
         float4 v[T::TQ][T::TN];
+        // every tile but the newest kept one has been read; the product's
+        // barriers order that before the writes below
+        if (SAVE) bulk_store_wait<1>();
         flow_product<R>(w, ring, slot, A, N, in, r0, c0, v);
         // biased sums to shared memory, then tanh on the thread's own values in a
         // rolled loop (64 inlined tanh would be most of the kernel's code)
@@ -163,12 +173,10 @@ __global__ void __launch_bounds__(FlowTile<R>::NT, 2) k_flow_f32(const __grid_co
             const float4 h = on ? make_float4(tanhf(t.x), tanhf(t.y), tanhf(t.z), tanhf(t.w))
                                 : make_float4(0.f, 0.f, 0.f, 0.f);
             *p = h;
-            if (SAVE && on)
-              *reinterpret_cast<float4*>(a.acts + ((s.act_base(l) + s.act_col(l, i + 1)) * a.tiles +
-                                                   (int64_t)blockIdx.x * out + c) * R + r0 + 16 * q) = h;
           }
         }
       }
+      if (SAVE) keep(cur, i + 1, 0, out, out);
       A = cur;
       float* t = cur;
       cur = other;
@@ -184,28 +192,29 @@ __global__ void __launch_bounds__(FlowTile<R>::NT, 2) k_flow_f32(const __grid_co
       const int N = min(tc, out - n0);
       {
         float4 v[T::TQ][T::TN];
+        if (SAVE) {
+          if (t0 == 0) bulk_store_wait<1>();
+          else bulk_store_wait<0>();   // the previous group's tile
+        }
         flow_product<R>(w, ring, slot, A, N, in, r0, c0, v);
 #pragma unroll
         for (int j = 0; j < T::TN; ++j) {
           const int c = c0 + 8 * j;
           if (c < N) {
             const float b = __ldg(bias + n0 + c);
-            float* sv = SAVE ? a.acts + ((s.act_base(l) + s.act_col(l, s.nh + 1)) * a.tiles +
-                                                      (int64_t)blockIdx.x * out + n0 + c) * R
-                                          : nullptr;
 #pragma unroll
             for (int q = 0; q < T::TQ; ++q) {
               const float4 t = v[q][j];
               const float4 o = make_float4(t.x + b, t.y + b, t.z + b, t.w + b);
               *reinterpret_cast<float4*>(raw + c * T::LD + r0 + 16 * q) = o;
-              if (sv != nullptr) *reinterpret_cast<float4*>(sv + r0 + 16 * q) = o;
             }
           }
         }
       }
       if (t0 == 0)
         for (int e = tid; e < 32 * R; e += NT) lb[e] = 0.f;
-      __syncthreads();
+      if (SAVE) keep(raw, s.nh + 1, n0, N, out);
+      else __syncthreads();
       const int items = (N / P) * R;
       for (int e = tid; e < items; e += NT) {
         const int t = e / R;
@@ -246,6 +255,7 @@ __global__ void __launch_bounds__(FlowTile<R>::NT, 2) k_flow_f32(const __grid_co
       }
     }
   }
+  if (SAVE) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // shared memory outlives the copies
   // ---- results
   if (a.out_mode == FLOW_OUT_LOGP) {
     __syncthreads();   // the sums above have read part

@@ -5,11 +5,10 @@
 //   knots     _normalize_bin_sizes / _normalize_knot_slopes / get_params  (:20-39, :310-338)
 //   forward   _rational_quadratic_spline_fwd (:42-128)
 //   inverse   _safe_quadratic_root + _rational_quadratic_spline_inv (:131-239)
-// The bin is picked with a one-hot predicate loop over compile-time knot
-// indices (as the reference does), so every array stays in registers.
-// The adjoint is written out by hand: through the spline formula, the
-// selected bin's knots, the cumulative sums, the two softmaxes and the
-// softplus slopes.
+// The bin is picked while the knots run by with compile-time indices, so every
+// array stays in registers. The adjoint is written out by hand: through the
+// spline formula, the selected bin's knots, the cumulative sums, the two
+// softmaxes and the softplus slopes.
 #pragma once
 #include <cuda_bf16.h>
 #include "common.cuh"
@@ -20,122 +19,9 @@ struct SplineCfg {
   float rmin, rmax, min_bin, min_slope, slope_offset;
 };
 
-template <int K>
-struct Knots {
-  float xp[K + 1], yp[K + 1], sl[K + 1];
-  float pw[K], ph[K];  // softmax probabilities (kept for the adjoint)
-};
-
 __device__ __forceinline__ float softplus_f(float a) {
   // jax.nn.softplus = logaddexp(a, 0)
   return fmaxf(a, 0.f) + log1pf(expf(-fabsf(a)));
-}
-
-template <int K>
-__device__ __forceinline__ void softmax_k(const float* r, float (&p)[K]) {
-  float m = r[0];
-#pragma unroll
-  for (int k = 1; k < K; ++k) m = fmaxf(m, r[k]);
-  float s = 0.f;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    p[k] = expf(r[k] - m);
-    s += p[k];
-  }
-#pragma unroll
-  for (int k = 0; k < K; ++k) p[k] = p[k] / s;
-}
-
-// raw: the 3K+1 conditioner outputs of one coordinate
-template <int K>
-__device__ __forceinline__ void make_knots(const float* raw, const SplineCfg& c, Knots<K>& kn) {
-  const float R = c.rmax - c.rmin;
-  const float scale = R - (float)K * c.min_bin;
-  softmax_k<K>(raw, kn.pw);
-  softmax_k<K>(raw + K, kn.ph);
-  float cw = 0.f, ch = 0.f;
-  kn.xp[0] = c.rmin;
-  kn.yp[0] = c.rmin;
-#pragma unroll
-  for (int k = 0; k < K - 1; ++k) {
-    cw += kn.pw[k] * scale + c.min_bin;
-    ch += kn.ph[k] * scale + c.min_bin;
-    kn.xp[k + 1] = c.rmin + cw;
-    kn.yp[k + 1] = c.rmin + ch;
-  }
-  kn.xp[K] = c.rmax;
-  kn.yp[K] = c.rmax;
-#pragma unroll
-  for (int k = 0; k <= K; ++k) kn.sl[k] = softplus_f(raw[2 * K + k] + c.slope_offset) + c.min_slope;
-}
-
-struct Bin {
-  float x0, x1, y0, y1, d0, d1;
-  int k;
-};
-
-template <int K>
-__device__ __forceinline__ Bin select_bin(float v, const float (&pos)[K + 1], const Knots<K>& kn) {
-  Bin b{kn.xp[0], kn.xp[1], kn.yp[0], kn.yp[1], kn.sl[0], kn.sl[1], 0};
-#pragma unroll
-  for (int k = 1; k < K; ++k) {
-    if (v >= pos[k] && v < pos[k + 1]) b = Bin{kn.xp[k], kn.xp[k + 1], kn.yp[k], kn.yp[k + 1], kn.sl[k], kn.sl[k + 1], k};
-  }
-  return b;  // bin 0 also covers "no bin" (rqSpline.py:70-72)
-}
-
-template <int K>
-__device__ __forceinline__ void rqs_fwd(float x, const Knots<K>& kn, float& y, float& ld) {
-  const bool below = x <= kn.xp[0];
-  const bool above = x >= kn.xp[K];
-  const Bin b = select_bin<K>(x, kn.xp, kn);
-  const float w = b.x1 - b.x0, h = b.y1 - b.y0;
-  const float s = h / w;
-  float z = (x - b.x0) / w;
-  z = fminf(fmaxf(z, 0.f), 1.f);
-  const float sq = z * z;
-  const float q = z - sq;
-  const float om = 1.f - z;
-  const float sq1 = om * om;
-  const float st = b.d1 + b.d0 - 2.f * s;
-  const float num = h * (s * sq + b.d0 * q);
-  const float den = s + st * q;
-  y = b.y0 + num / den;
-  ld = 2.f * logf(s) + logf(b.d1 * sq + 2.f * s * q + b.d0 * sq1) - 2.f * logf(den);
-  if (below) { y = (x - kn.xp[0]) * kn.sl[0] + kn.yp[0]; ld = logf(kn.sl[0]); }
-  if (above) { y = (x - kn.xp[K]) * kn.sl[K] + kn.yp[K]; ld = logf(kn.sl[K]); }
-}
-
-template <int K>
-__device__ __forceinline__ void rqs_inv(float y, const Knots<K>& kn, float& x, float& ld) {
-  const bool below = y <= kn.yp[0];
-  const bool above = y >= kn.yp[K];
-  const Bin b = select_bin<K>(y, kn.yp, kn);
-  const float w = b.x1 - b.x0, h = b.y1 - b.y0;
-  const float s = h / w;
-  float ww = (y - b.y0) / h;
-  ww = fminf(fmaxf(ww, 0.f), 1.f);
-  const float st = b.d1 + b.d0 - 2.f * s;
-  const float c = -s * ww;
-  const float bb = b.d0 - st * ww;
-  const float a = s - bb;
-  // _safe_quadratic_root (rqSpline.py:131-155)
-  const float disc = bb * bb - 4.f * a * c;
-  float sqd = sqrtf(fmaxf(disc, 1.17549435e-38f));
-  if (!(disc > 0.f)) sqd = 0.f;
-  const float num = (bb >= 0.f) ? 2.f * c : -bb + sqd;
-  const float dnm = (bb >= 0.f) ? -bb - sqd : 2.f * a;
-  float z = num / dnm;
-  z = fminf(fmaxf(z, 0.f), 1.f);
-  x = w * z + b.x0;
-  const float sq = z * z;
-  const float q = z - sq;
-  const float om = 1.f - z;
-  const float sq1 = om * om;
-  const float den = s + st * q;
-  ld = -2.f * logf(s) - logf(b.d1 * sq + 2.f * s * q + b.d0 * sq1) + 2.f * logf(den);
-  if (below) { x = (y - kn.yp[0]) / kn.sl[0] + kn.xp[0]; ld = -logf(kn.sl[0]); }
-  if (above) { x = (y - kn.yp[K]) / kn.sl[K] + kn.xp[K]; ld = -logf(kn.sl[K]); }
 }
 
 // softmax numerators e^(r - max) and their sum
@@ -171,9 +57,10 @@ __device__ __forceinline__ void softmax_div(float (&p)[K], float s) {
   }
 }
 
-// rqs_fwd / rqs_inv of make_knots(raw) without the knot arrays, the same bits:
-// the knots run on while the bin that holds v is carried along, and only the
-// bin's two slopes (in the tails the end slope) go through the softplus.
+// The spline (or its inverse) at v and the log-determinant. raw: the 3K+1
+// conditioner outputs of one coordinate. The knots run on while the bin that
+// holds v is carried along, and only the bin's two slopes (in the tails the end
+// slope) go through the softplus.
 template <int K, bool INV>
 __device__ __forceinline__ void rqs_apply(const float (&raw)[3 * K + 1], float v, const SplineCfg& c, float& out,
                                           float& ld) {
@@ -227,125 +114,136 @@ __device__ __forceinline__ void rqs_apply(const float (&raw)[3 * K + 1], float v
   }
   const float sq = z * z, q = z - sq, om = 1.f - z, sq1 = om * om;
   const float den = s + st * q;
+  const float A = fmaf(d0, sq1, fmaf(d1, sq, __fmul_rn(2.f * s, q)));
   if (!INV) {
     const float num = h * (s * sq + d0 * q);
     out = y0 + num / den;
-    ld = 2.f * logf(s) + logf(d1 * sq + 2.f * s * q + d0 * sq1) - 2.f * logf(den);
+    ld = 2.f * logf(s) + logf(A) - 2.f * logf(den);
     if (below) { out = (v - c.rmin) * d0 + c.rmin; ld = logf(d0); }
     if (above) { out = (v - c.rmax) * d1 + c.rmax; ld = logf(d1); }
   } else {
     out = w * z + x0;
-    ld = -2.f * logf(s) - logf(d1 * sq + 2.f * s * q + d0 * sq1) + 2.f * logf(den);
+    ld = -2.f * logf(s) - logf(A) + 2.f * logf(den);
     if (below) { out = (v - c.rmin) / d0 + c.rmin; ld = -logf(d0); }
     if (above) { out = (v - c.rmax) / d1 + c.rmax; ld = -logf(d1); }
   }
 }
 
-// Adjoint of (y, ld) = rqs_fwd(x; raw): given gy = dL/dy and gl = dL/dld,
-// returns dL/dx and accumulates dL/draw[0..3K] into graw.
-template <int K>
-__device__ __forceinline__ float rqs_fwd_adjoint(float x, const float* raw, const SplineCfg& c, const Knots<K>& kn,
-                                                 float gy, float gl, float* graw) {
-  float gX[K + 1], gY[K + 1], gD[K + 1];
+// Adjoint of (y, ld) = rqs_apply<K, false>(x; raw): given gy = dL/dy and gl =
+// dL/dld, returns dL/dx, and put(p, v) receives dL/draw[p]. Organised around the
+// bin that holds x: only its two knots carry gradient into the cumulative widths
+// and heights, and only its two slopes (in a tail the end slope) through the
+// softplus.
+template <int K, typename F>
+__device__ __forceinline__ float rqs_adjoint(const float (&raw)[3 * K + 1], float x, const SplineCfg& c, float gy,
+                                             float gl, F put) {
+  const float scale = (c.rmax - c.rmin) - (float)K * c.min_bin;
+  float pw[K], ph[K];
+  softmax_div<K>(pw, softmax_num<K>(raw, pw));
+  softmax_div<K>(ph, softmax_num<K>(raw + K, ph));
+  const bool below = x <= c.rmin, above = x >= c.rmax;
+  float cw = 0.f, ch = 0.f, xk = c.rmin, yk = c.rmin;
+  float x0 = c.rmin, y0 = c.rmin, x1 = c.rmax, y1 = c.rmax, r0 = raw[2 * K], r1 = raw[2 * K + 1];
+  int kb = 0;
 #pragma unroll
-  for (int k = 0; k <= K; ++k) { gX[k] = 0.f; gY[k] = 0.f; gD[k] = 0.f; }
-  float gx = 0.f;
-  const bool below = x <= kn.xp[0];
-  const bool above = x >= kn.xp[K];
+  for (int k = 0; k < K; ++k) {
+    float xn = c.rmax, yn = c.rmax;
+    if (k < K - 1) {
+      cw += pw[k] * scale + c.min_bin;
+      ch += ph[k] * scale + c.min_bin;
+      xn = c.rmin + cw;
+      yn = c.rmin + ch;
+    }
+    if (k == 0 || (x >= xk && x < xn)) {
+      x0 = xk; x1 = xn; y0 = yk; y1 = yn;
+      r0 = raw[2 * K + k];
+      r1 = raw[2 * K + k + 1];
+      kb = k;
+    }
+    xk = xn;
+    yk = yn;
+  }
+  int k0 = kb, k1 = kb + 1;   // the slopes with gradients g_d0, g_d1
+  if (above) {
+    r1 = raw[3 * K];
+    k1 = K;
+  }
+  const float d0 = softplus_f(r0 + c.slope_offset) + c.min_slope;
+  const float d1 = softplus_f(r1 + c.slope_offset) + c.min_slope;
+  float gx, g_x0 = 0.f, g_x1 = 0.f, g_y0 = 0.f, g_y1 = 0.f, g_d0 = 0.f, g_d1 = 0.f;
   if (below) {
-    gx = gy * kn.sl[0];
-    gD[0] = gy * (x - kn.xp[0]) + gl / kn.sl[0];
+    gx = gy * d0;
+    g_d0 = gy * (x - c.rmin) + gl / d0;
+    k1 = -1;
   } else if (above) {
-    gx = gy * kn.sl[K];
-    gD[K] = gy * (x - kn.xp[K]) + gl / kn.sl[K];
+    gx = gy * d1;
+    g_d1 = gy * (x - c.rmax) + gl / d1;
+    k0 = -1;
   } else {
-    const Bin b = select_bin<K>(x, kn.xp, kn);
-    const float w = b.x1 - b.x0, h = b.y1 - b.y0;
+    const float w = x1 - x0, h = y1 - y0;
     const float s = h / w;
-    const float zr = (x - b.x0) / w;
+    const float zr = (x - x0) / w;
     const float z = fminf(fmaxf(zr, 0.f), 1.f);
     const float sq = z * z, q = z - sq, om = 1.f - z, sq1 = om * om;
-    const float st = b.d1 + b.d0 - 2.f * s;
-    const float num = h * (s * sq + b.d0 * q);
+    const float st = d1 + d0 - 2.f * s;
+    const float num = h * (s * sq + d0 * q);
     const float den = s + st * q;
-    const float A = b.d1 * sq + 2.f * s * q + b.d0 * sq1;
+    const float A = fmaf(d0, sq1, fmaf(d1, sq, __fmul_rn(2.f * s, q)));
     // y = y0 + num/den ; ld = 2 log s + log A - 2 log den
     const float g_num = gy / den;
     const float g_den = -gy * num / (den * den) - 2.f * gl / den;
     const float g_A = gl / A;
     float g_s = 2.f * gl / s;
-    float g_h = g_num * (s * sq + b.d0 * q);
+    float g_h = g_num * (s * sq + d0 * q);
     g_s += g_num * h * sq;
-    float g_sq = g_num * h * s;
-    float g_d0 = g_num * h * q;
-    float g_q = g_num * h * b.d0;
-    // den = s + (d1 + d0 - 2 s) q
     g_s += g_den * (1.f - 2.f * q);
-    float g_d1 = g_den * q;
-    g_d0 += g_den * q;
-    g_q += g_den * st;
-    // A = d1 sq + 2 s q + d0 (1-z)^2
-    g_d1 += g_A * sq;
-    g_sq += g_A * b.d1;
     g_s += g_A * 2.f * q;
-    g_q += g_A * 2.f * s;
-    g_d0 += g_A * sq1;
-    float g_z = -g_A * b.d0 * 2.f * om;
-    // q = z - z^2, sq = z^2
-    g_z += g_q * (1.f - 2.f * z) + g_sq * 2.f * z;
+    // sums of products with the rounding of each spelled out
+    const float nh = __fmul_rn(g_num, h);
+    g_d0 = fmaf(g_A, sq1, fmaf(nh, q, __fmul_rn(g_den, q)));
+    g_d1 = fmaf(g_A, sq, __fmul_rn(g_den, q));
+    const float g_q = fmaf(g_A * 2.f, s, fmaf(nh, d0, __fmul_rn(g_den, st)));
+    const float g_sq = fmaf(nh, s, __fmul_rn(g_A, d1));
+    const float g_z =
+        fmaf(__fmul_rn(-g_A, d0) * 2.f, om, fmaf(g_sq * 2.f, z, __fmul_rn(g_q, fmaf(-2.f, z, 1.f))));
     const float g_zr = (zr > 0.f && zr < 1.f) ? g_z : 0.f;
-    // zr = (x - x0)/w ; s = h/w
     gx = g_zr / w;
-    float g_x0 = -g_zr / w;
+    g_x0 = -g_zr / w;
     float g_w = -g_zr * zr / w - g_s * s / w;
     g_h += g_s / w;
-    // w = x1 - x0, h = y1 - y0
-    const float g_x1 = g_w;
+    g_x1 = g_w;
     g_x0 -= g_w;
-    const float g_y1 = g_h;
-    const float g_y0 = gy - g_h;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (k == b.k) {
-        gX[k] += g_x0; gX[k + 1] += g_x1;
-        gY[k] += g_y0; gY[k + 1] += g_y1;
-        gD[k] += g_d0; gD[k + 1] += g_d1;
-      }
-    }
+    g_y1 = g_h;
+    g_y0 = gy - g_h;
   }
-  // knots: X_k = rmin + sum_{i<k} w_i for 1 <= k <= K-1 (X_0, X_K constant)
-  const float scale = (c.rmax - c.rmin) - (float)K * c.min_bin;
-  float gpw[K], gph[K];
-  float accx = 0.f, accy = 0.f;
-#pragma unroll
-  for (int i = K - 1; i >= 0; --i) {
-    // g_w[i] = sum_{k=i+1}^{K-1} gX[k]
-    gpw[i] = accx * scale;
-    gph[i] = accy * scale;
-    if (i >= 1) { accx += gX[i]; accy += gY[i]; }
-  }
-  // softmax adjoint
+  // interior knot k (1 <= k <= K-1) is rmin + sum of the bins before it: bin i
+  // collects the gradients of the bin's two knots that lie beyond i
+  const float ax1 = kb + 1 <= K - 1 ? g_x1 : 0.f, ay1 = kb + 1 <= K - 1 ? g_y1 : 0.f;
+  const float axs = kb >= 1 ? ax1 + g_x0 : ax1, ays = kb >= 1 ? ay1 + g_y0 : ay1;
+  const float gw_eq = __fmul_rn(ax1, scale), gh_eq = __fmul_rn(ay1, scale);
+  const float gw_lt = __fmul_rn(axs, scale), gh_lt = __fmul_rn(ays, scale);
   float dw = 0.f, dh = 0.f;
 #pragma unroll
-  for (int i = 0; i < K; ++i) { dw += kn.pw[i] * gpw[i]; dh += kn.ph[i] * gph[i]; }
+  for (int i = 0; i < K; ++i) {
+    dw = fmaf(pw[i], i < kb ? gw_lt : i == kb ? gw_eq : 0.f, dw);
+    dh = fmaf(ph[i], i < kb ? gh_lt : i == kb ? gh_eq : 0.f, dh);
+  }
 #pragma unroll
   for (int i = 0; i < K; ++i) {
-    graw[i] = kn.pw[i] * (gpw[i] - dw);
-    graw[K + i] = kn.ph[i] * (gph[i] - dh);
+    put(i, pw[i] * __fsub_rn(i < kb ? gw_lt : i == kb ? gw_eq : 0.f, dw));
+    put(K + i, ph[i] * __fsub_rn(i < kb ? gh_lt : i == kb ? gh_eq : 0.f, dh));
   }
   // slopes: d_k = softplus(raw + off) + min_slope -> sigmoid
+  const float s0 = g_d0 * (1.f / (1.f + expf(-(r0 + c.slope_offset))));
+  const float s1 = g_d1 * (1.f / (1.f + expf(-(r1 + c.slope_offset))));
 #pragma unroll
-  for (int k = 0; k <= K; ++k) {
-    const float a = raw[2 * K + k] + c.slope_offset;
-    const float sg = 1.f / (1.f + expf(-a));
-    graw[2 * K + k] = gD[k] * sg;
-  }
+  for (int k = 0; k <= K; ++k) put(2 * K + k, k == k0 ? s0 : k == k1 ? s1 : 0.f);
   return gx;
 }
 
 // ---------------------------------------------------------------- inference, one bin
-// Inference-only spline for the BF16 path: the same function as make_knots +
-// rqs_fwd / rqs_inv, but only the bin that holds v is built. Both softmax
+// Inference-only spline for the BF16 path: the same function as rqs_apply, with
+// only the bin that holds v built. Both softmax
 // normalisers are still needed (every knot depends on them), the knot
 // positions are running sums whose last value at or below v picks the bin
 // (identical to the one-hot selection: knots increase, so exactly one k has
@@ -449,7 +347,7 @@ __device__ __forceinline__ void softmax_weights(const float (&raw)[3 * K + 1], f
 }
 
 // The spline of the bin that holds v only, for the fused tensor-core
-// epilogue (same function as rqs_forward/rqs_inverse up to rounding):
+// epilogue (same function as rqs_apply up to rounding):
 // unnormalised softmax weights (softmax_weights), the bin
 // found by comparing v with the running knots while carrying only what the
 // bin needs (cumulative sums before it, its own weights, its two slope
@@ -539,7 +437,7 @@ __device__ __forceinline__ void rqs_apply_fast(const float (&raw)[3 * K + 1], fl
 
 // Adjoint of rqs_apply_fast<K, false> for the BF16 training path: given
 // gy = dL/dy and gl = dL/dlogdet, returns dL/dx and writes dL/draw[0..3K] as
-// bf16 to out. Same derivative as rqs_fwd_adjoint, organised around the one
+// bf16 to out. Same derivative as rqs_adjoint, organised around the one
 // bin that holds x: only its two knots carry gradient into the cumulative
 // widths/heights (so dL/dw_i is a two-term prefix rule) and only its two
 // slopes go through the softplus derivative; the rest of the slope

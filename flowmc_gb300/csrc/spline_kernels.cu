@@ -25,13 +25,10 @@ __global__ void __launch_bounds__(256) k_spline(const float* __restrict__ raw, f
       float prm[P];
 #pragma unroll
       for (int p = 0; p < P; ++p) prm[p] = __ldg(rr + t * P + p);
-      Knots<K> kn;
-      make_knots<K>(prm, cfg, kn);
       const int j = 2 * t + tpar;
       float* xp = xa + r * d + j;
       float out, l;
-      if (INV) rqs_inv<K>(*xp, kn, out, l);
-      else rqs_fwd<K>(*xp, kn, out, l);
+      rqs_apply<K, INV>(prm, *xp, cfg, out, l);
       *xp = out;
       acc += l;
     }
@@ -53,16 +50,12 @@ __global__ void __launch_bounds__(256) k_spline_bwd(const float* __restrict__ ra
     const float* rr = raw + r * (int64_t)nt * P;
     float* gr = graw + r * (int64_t)nt * P;
     for (int t = lane; t < nt; t += 32) {
-      float prm[P], g[P];
+      float prm[P];
 #pragma unroll
       for (int p = 0; p < P; ++p) prm[p] = __ldg(rr + t * P + p);
-      Knots<K> kn;
-      make_knots<K>(prm, cfg, kn);
       const int j = 2 * t + tpar;
-      const float gx = rqs_fwd_adjoint<K>(xa[r * d + j], prm, cfg, kn, gy[r * d + j], gld, g);
-      gxa[r * d + j] = gx;
-#pragma unroll
-      for (int p = 0; p < P; ++p) gr[t * P + p] = g[p];
+      gxa[r * d + j] = rqs_adjoint<K>(prm, xa[r * d + j], cfg, gy[r * d + j], gld,
+                                      [&](int p, float v) { gr[t * P + p] = v; });
     }
     for (int k = lane; k < ncond; k += 32) {
       const int j = 2 * k + cpar;
