@@ -483,7 +483,7 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
         const int out = g.lin_out(l, i), in = g.lin_in(l, i);
         const float* a_in = (i == 0) ? w.cond : w.hs + (int64_t)(i - 1) * n * g.h_max();
         // dW = g^T a_in  [out, in], split along the batch
-        if ((rc = kouter(st, out, in, n, gcur, out, a_in, in, false, w.spart, w.spart_floats, gl + g.lin_w(l, i))))
+        if ((rc = kouter(st, out, in, n, gcur, out, a_in, in, w.spart, w.spart_floats, gl + g.lin_w(l, i))))
           return rc;
         if ((rc = colsum(st, gcur, n, out, w.part, gl + g.lin_b(l, i)))) return rc;
         float* gnext = (i == 0) ? w.gcond : gbufs[i & 1];

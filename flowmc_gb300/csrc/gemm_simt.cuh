@@ -17,8 +17,6 @@ enum GemmEpi : int {
   EPI_BIAS = 1,       // C = AB + bias
   EPI_BIAS_TANH = 2,  // C = tanh(AB + bias)
   EPI_DTANH = 3,      // C = AB * (1 - aux^2)   (aux = tanh output of the forward)
-  EPI_BIAS_RELU = 4,  // C = max(AB + bias, 0)
-  EPI_DRELU = 5,      // C = AB where aux > 0, else 0   (aux = relu output of the forward)
 };
 
 template <bool A_KMAJOR, bool B_KMAJOR, int EPI>
@@ -86,10 +84,6 @@ __global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float*
         v += bias[gj];
       } else if (EPI == EPI_BIAS_TANH) {
         v = tanhf(v + bias[gj]);
-      } else if (EPI == EPI_BIAS_RELU) {
-        v = fmaxf(v + bias[gj], 0.f);
-      } else if (EPI == EPI_DRELU) {
-        v = (aux[gi * ldaux + gj] > 0.f) ? v : 0.f;
       } else {
         const float h = aux[gi * ldaux + gj];
         v = v * (1.f - h * h);
@@ -130,8 +124,8 @@ inline int sgemm(cudaStream_t st, int64_t M, int N, int K, const float* A, int64
 constexpr int kKouterMaxSlices = 64;
 
 // part[z][i][j] = sum over rows k of slice z of A[k*lda + i] * B[k*ldb + j]
-// (ONES: B = 1, N = 1 -- column sums). 64 x 64 tiles, 16 rows per step.
-template <bool ONES>
+// 64 x 64 tiles, 16 rows per step.
+template <int U = 0>
 __global__ void __launch_bounds__(256) k_sgemm_kouter(int M, int N, int64_t K, int64_t kslice,
                                                       const float* __restrict__ A, int64_t lda,
                                                       const float* __restrict__ B, int64_t ldb,
@@ -152,7 +146,7 @@ __global__ void __launch_bounds__(256) k_sgemm_kouter(int M, int N, int64_t K, i
       const int64_t gk = k0 + kk;
       As[kk][ii] = (gk < ke && i0 + ii < M) ? A[gk * lda + i0 + ii] : 0.f;
       float b = 0.f;
-      if (gk < ke && j0 + ii < N) b = ONES ? 1.f : B[gk * ldb + j0 + ii];
+      if (gk < ke && j0 + ii < N) b = B[gk * ldb + j0 + ii];
       Bs[kk][ii] = b;
     }
     __syncthreads();
@@ -207,21 +201,17 @@ inline int64_t kouter_slices(int M, int N, int64_t K, bool has_part, int64_t par
   return S < 1 ? 1 : S;
 }
 
-// out [M, N] = A^T B over K rows (A [K, lda], B [K, ldb]); ones: column sums
-// of A. part holds part_floats floats of slice partials; with room for fewer
+// out [M, N] = A^T B over K rows (A [K, lda], B [K, ldb]). part holds part_floats floats of slice partials; with room for fewer
 // than two slices the single slice is written to out directly.
 inline int kouter(cudaStream_t st, int M, int N, int64_t K, const float* A, int64_t lda, const float* B, int64_t ldb,
-                  bool ones, float* part, int64_t part_floats, float* out) {
+                  float* part, int64_t part_floats, float* out) {
   if (M <= 0 || N <= 0) return FMC_OK;
   const int64_t mn = (int64_t)M * N;
   int64_t kslice = 0;
   const int64_t S = kouter_slices(M, N, K, part != nullptr, part_floats, &kslice);
   float* dst = S > 1 ? part : out;
   dim3 grid((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64), (unsigned)S);
-  if (ones)
-    k_sgemm_kouter<true><<<grid, 256, 0, st>>>(M, N, K, kslice, A, lda, nullptr, 0, dst);
-  else
-    k_sgemm_kouter<false><<<grid, 256, 0, st>>>(M, N, K, kslice, A, lda, B, ldb, dst);
+  k_sgemm_kouter<><<<grid, 256, 0, st>>>(M, N, K, kslice, A, lda, B, ldb, dst);
   FMC_LAUNCH_CHECK();
   if (S > 1) {
     int64_t b = (mn + 255) / 256;

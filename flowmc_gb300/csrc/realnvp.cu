@@ -8,16 +8,23 @@
 // the reference model, so optax's weight decay moves them off 0/1; they live
 // in aux and every kernel uses the general formula.
 //
-// Per layer and row block: the first Linears of both MLPs as one GEMM
-// (W1 = [W1s; W1t], relu epilogue), the two second Linears as GEMMs with
-// bias epilogues, then one warp per row applies the coupling and sums the
-// log-det. The backward recomputes a layer's activations from its stored
-// input, runs the coupling adjoint elementwise, the two relu-masked dH GEMMs
-// and the dc GEMM, and forms the weight and bias gradients as split-K
-// GEMMs over the batch (fixed-order slice sums: deterministic). FP32 SIMT
-// GEMMs throughout: RealNVP's MLPs are narrow [d, H, d].
+// Per layer and row block: the first Linears of both MLPs as one GEMM (W1 =
+// [W1s; W1t], relu epilogue), the two second Linears as one launch of two GEMMs
+// with bias epilogues, then one warp per row applies the coupling, sums the
+// log-det and leaves the next layer's masked input. Training keeps every layer's
+// masked input, hidden activations and conditioner outputs; the backward is,
+// per layer, the coupling adjoint, one launch of the two relu-masked dH GEMMs
+// and the dc GEMM, which adds into the input gradient. The weight and bias
+// gradients of all layers are formed at the end: one grid of split-row outer
+// products with fixed-order slice sums (deterministic), two launches of column
+// sums. FP32 SIMT GEMMs throughout (gemm_f32.cuh): RealNVP's MLPs are narrow
+// [d, H, d].
+//
+// Measured on GB300 (32-D, 8 layers, H = 256): loss + gradient of 16,384 rows
+// 3.64 -> 1.31 ms (212 launches -> 58; the GEMMs 0.89 ms, the weight gradients
+// 0.17 ms = 50 TFLOP/s).
 #include "flow.cuh"
-#include "gemm_simt.cuh"
+#include "gemm_f32.cuh"
 
 namespace fmc {
 
@@ -48,7 +55,7 @@ static int rnvp_geom(const FmcRealNVP* f, RnvpGeom& g) {
 }
 
 constexpr int64_t kRnvpChunk = 65536;   // rows per inference chunk
-constexpr int kMaxSlices = kKouterMaxSlices;   // split-K slices of the weight gradients
+constexpr int kMaxSlices = 64;   // row slices of the weight gradients
 
 static int grid_for(int64_t tot, int per_sm = 8) {
   int64_t b = (tot + 255) / 256;
@@ -72,10 +79,12 @@ __global__ void k_rnvp_cond(const float* __restrict__ x, const float* __restrict
     cond[i] = x[i] * m[i % d];
 }
 
-// one warp per row; y may alias x. first: ld = sum, else ld += sum
+// one warp per row; y may alias x. first: ld = sum, else ld += sum. With m_next
+// also cond_next = y * m_next, the next layer's conditioner input
 __global__ void k_rnvp_couple(const float* x, const float* __restrict__ sraw, const float* __restrict__ tt,
                               const float* __restrict__ m, int64_t n, int d, float dt, int inverse, float* y,
-                              float* __restrict__ ld, int first) {
+                              float* __restrict__ ld, int first, const float* __restrict__ m_next,
+                              float* __restrict__ cond_next) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n; r += warps) {
@@ -86,7 +95,9 @@ __global__ void k_rnvp_couple(const float* x, const float* __restrict__ sraw, co
       const float s = tanhf(sraw[e]) * dt;        // MLPAffine: tanh(scale_MLP(c)) * dt
       const float t = tt[e] * dt;                 //            shift_MLP(c) * dt
       const float ya = inverse ? xv * expf(-s) - t : (xv + t) * expf(s);
-      y[e] = (1.f - mj) * ya + mj * xv;           // MaskedCouplingLayer mix
+      const float yv = (1.f - mj) * ya + mj * xv; // MaskedCouplingLayer mix
+      y[e] = yv;
+      if (m_next != nullptr) cond_next[e] = yv * m_next[j];
       acc += (1.f - mj) * s;
     }
 #pragma unroll
@@ -120,11 +131,62 @@ __global__ void k_rnvp_couple_bwd(const float* __restrict__ x, float* __restrict
   }
 }
 
-__global__ void k_rnvp_add_masked(float* __restrict__ gx, const float* __restrict__ dc, const float* __restrict__ m,
-                                  int64_t n, int d) {
-  const int64_t tot = n * d;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x)
-    gx[e] += dc[e] * m[e % d];
+// per layer W2s^T, W2t^T [H, d] and W1^T [d, 2H]: the K-major operands of the
+// backward GEMMs
+__global__ void k_rnvp_transpose(const float* __restrict__ theta, RnvpGeom g, float* __restrict__ out) {
+  const int64_t hd = (int64_t)g.H * g.d, per = 4 * hd;
+  const float* th = theta + blockIdx.y * g.per_layer;
+  float* o = out + blockIdx.y * per;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < per; e += (int64_t)gridDim.x * blockDim.x) {
+    if (e < 2 * hd) {
+      const int64_t q = e % hd, h = q / g.d, j = q % g.d;
+      o[e] = th[(e < hd ? g.off_W2s : g.off_W2t) + j * g.H + h];
+    } else {
+      const int64_t q = e - 2 * hd, j = q / (2 * g.H), h = q % (2 * g.H);
+      o[e] = th[h * g.d + j];
+    }
+  }
+}
+
+// column sums of dz [n, 2H], d sraw and d t [n, d] of layer blockIdx.z / 3 over
+// row block blockIdx.y into part[parameter][row block]
+__device__ __forceinline__ int rnvp_bias(const RnvpGeom& g, int which, int64_t& off) {
+  off = which == 0 ? g.off_b1 : which == 1 ? g.off_b2s : g.off_b2t;
+  return which == 0 ? 2 * g.H : g.d;
+}
+__global__ void k_rnvp_bias_partial(RnvpGeom g, const float* __restrict__ dz, const float* __restrict__ ds,
+                                    const float* __restrict__ dt, int64_t n, int64_t rows_per, float* __restrict__ part) {
+  const int l = blockIdx.z / 3, which = blockIdx.z % 3;
+  int64_t off;
+  const int cols = rnvp_bias(g, which, off), c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  const float* src = (which == 0 ? dz : which == 1 ? ds : dt) + (int64_t)l * n * cols + c;
+  const int64_t r0 = blockIdx.y * rows_per, r1 = r0 + rows_per < n ? r0 + rows_per : n;
+  float v = 0.f;
+#pragma unroll 16
+  for (int64_t r = r0; r < r1; ++r) v += src[r * cols];
+  const int64_t first = which == 0 ? 0 : which == 1 ? 2 * g.H : 2 * g.H + g.d;
+  part[((int64_t)l * (2 * g.H + 2 * g.d) + first + c) * gridDim.y + blockIdx.y] = v;
+}
+__global__ void k_rnvp_bias_final(RnvpGeom g, const float* __restrict__ part, int rb, float* __restrict__ grad) {
+  const int l = blockIdx.z / 3, which = blockIdx.z % 3;
+  int64_t off;
+  const int cols = rnvp_bias(g, which, off), c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  const int64_t first = which == 0 ? 0 : which == 1 ? 2 * g.H : 2 * g.H + g.d;
+  const float* p = part + ((int64_t)l * (2 * g.H + 2 * g.d) + first + c) * rb;
+  float v = 0.f;
+  for (int b = 0; b < rb; ++b) v += p[b];
+  grad[l * g.per_layer + off + c] = v;
+}
+// grad = sum of the slices (bias entries are overwritten by k_rnvp_bias_final)
+__global__ void k_rnvp_sum_slices(const float* __restrict__ part, int S, int64_t n, float* __restrict__ grad) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    float v = 0.f;
+#pragma unroll 4
+    for (int z = 0; z < S; ++z) v += part[z * n + e];
+    grad[e] = v;
+  }
 }
 
 // log N(y; 0, I) + ld (realNVP.py:218-221: the standard normal, not the base distribution)
@@ -176,40 +238,47 @@ struct RnvpScratch {
 
 static const float* layer_mask(const RnvpGeom& g, const float* aux, int l) { return aux + 2 * g.d + 2 + (int64_t)l * g.d; }
 
-// the layer's conditioner: cond = x * m, h = relu(cond W1^T + b1), sraw, tt
-static int rnvp_conditioner(cudaStream_t st, const RnvpGeom& g, const float* th, const float* m, const float* x,
-                            int64_t rows, const RnvpScratch& s) {
+// the layer's conditioner on cond = x * m: h = relu(cond W1^T + b1), sraw, tt
+static int rnvp_conditioner(cudaStream_t st, const RnvpGeom& g, const float* th, int64_t rows, const RnvpScratch& s) {
   const int d = g.d, H = g.H;
-  k_rnvp_cond<<<grid_for(rows * d), 256, 0, st>>>(x, m, rows, d, s.cond);
-  FMC_LAUNCH_CHECK();
-  int rc = sgemm<true, true, EPI_BIAS_RELU>(st, rows, 2 * H, d, s.cond, d, th, d, th + g.off_b1, nullptr, 0, s.h,
-                                            2 * H, 0.f);
+  G32Args a{};
+  a.M = rows;
+  a.p[0] = G32Problem{s.cond, th, th + g.off_b1, nullptr, s.h};
+  a.lda = a.ldb = d;
+  a.ldc = 2 * H;
+  a.N = 2 * H;
+  a.K = d;
+  int rc = gemm_f32<G32_BIAS_RELU>(st, a, 1);
   if (rc) return rc;
-  rc = sgemm<true, true, EPI_BIAS>(st, rows, d, H, s.h, 2 * H, th + g.off_W2s, H, th + g.off_b2s, nullptr, 0, s.sraw,
-                                   d, 0.f);
-  if (rc) return rc;
-  return sgemm<true, true, EPI_BIAS>(st, rows, d, H, s.h + H, 2 * H, th + g.off_W2t, H, th + g.off_b2t, nullptr, 0,
-                                     s.tt, d, 0.f);
+  a.p[0] = G32Problem{s.h, th + g.off_W2s, th + g.off_b2s, nullptr, s.sraw};
+  a.p[1] = G32Problem{s.h + H, th + g.off_W2t, th + g.off_b2t, nullptr, s.tt};
+  a.lda = 2 * H;
+  a.ldb = H;
+  a.ldc = d;
+  a.N = d;
+  a.K = H;
+  return gemm_f32<G32_BIAS>(st, a, 2);
 }
 
 // all layers, in place on x [rows, d] (forward: 0..L-1, inverse: L-1..0); ld = the summed log-det
 static int rnvp_pass(cudaStream_t st, const RnvpGeom& g, const FmcRealNVP* f, float* x, int64_t rows, float* ld,
                      bool inverse, const RnvpScratch& s) {
+  k_rnvp_cond<<<grid_for(rows * g.d), 256, 0, st>>>(x, layer_mask(g, f->aux, inverse ? g.L - 1 : 0), rows, g.d, s.cond);
+  FMC_LAUNCH_CHECK();
   for (int i = 0; i < g.L; ++i) {
     const int l = inverse ? g.L - 1 - i : i;
-    const float* th = f->theta + (int64_t)l * g.per_layer;
-    const float* m = layer_mask(g, f->aux, l);
-    int rc = rnvp_conditioner(st, g, th, m, x, rows, s);
+    int rc = rnvp_conditioner(st, g, f->theta + (int64_t)l * g.per_layer, rows, s);
     if (rc) return rc;
-    k_rnvp_couple<<<warp_grid(rows), 256, 0, st>>>(x, s.sraw, s.tt, m, rows, g.d, g.dt, inverse ? 1 : 0, x, ld,
-                                                   i == 0 ? 1 : 0);
+    const float* next = i + 1 < g.L ? layer_mask(g, f->aux, inverse ? l - 1 : l + 1) : nullptr;
+    k_rnvp_couple<<<warp_grid(rows), 256, 0, st>>>(x, s.sraw, s.tt, layer_mask(g, f->aux, l), rows, g.d, g.dt,
+                                                   inverse ? 1 : 0, x, ld, i == 0 ? 1 : 0, next, s.cond);
     FMC_LAUNCH_CHECK();
   }
   return FMC_OK;
 }
 
 static size_t infer_floats(const RnvpGeom& g, int64_t rows) {
-  return (size_t)rows * (4 * (size_t)g.d + 2 * (size_t)g.H) + (size_t)rows + 64;
+  return (size_t)rows * (4 * (size_t)g.d + 2 * (size_t)g.H) + (size_t)rows + 64 * 8;
 }
 
 static int carve_infer(const RnvpGeom& g, int64_t rows, void* ws, size_t ws_bytes, RnvpScratch& s, float** xa,
@@ -217,22 +286,46 @@ static int carve_infer(const RnvpGeom& g, int64_t rows, void* ws, size_t ws_byte
   FMC_CHECK_ARG(ws != nullptr && ws_bytes >= infer_floats(g, rows) * sizeof(float),
                 "workspace of %zu bytes is smaller than fmc_rnvp_workspace_size", ws_bytes);
   float* p = (float*)ws;
-  s.cond = p; p += rows * g.d;
-  s.h = p; p += rows * 2 * (int64_t)g.H;
-  s.sraw = p; p += rows * g.d;
-  s.tt = p; p += rows * g.d;
-  *xa = p; p += rows * g.d;
+  auto take = [&](int64_t floats) {
+    float* r = p;
+    p += (floats + 63) / 64 * 64;   // 256-byte pieces: 16-byte copies where the shapes allow them
+    return r;
+  };
+  s.cond = take(rows * g.d);
+  s.h = take(rows * 2 * (int64_t)g.H);
+  s.sraw = take(rows * g.d);
+  s.tt = take(rows * g.d);
+  *xa = take(rows * g.d);
   *ld = p;
   return FMC_OK;
 }
 
-static int64_t train_part_floats(const RnvpGeom& g) {
-  return (int64_t)kMaxSlices * 2 * g.H * (int64_t)g.d;
+// row slices of the weight gradients: enough 256 x 32 tiles for two CTAs per SM,
+// at least 256 rows each
+static int wgrad_slices(const RnvpGeom& g, int64_t n, int64_t* rows_per) {
+  auto tiles = [](int64_t M, int64_t N) { return ((M + kK32M - 1) / kK32M) * ((N + kK32N - 1) / kK32N); };
+  const int64_t per = g.L * (tiles(2 * g.H, g.d) + 2 * tiles(g.H, g.d));
+  int64_t S = (4 * (int64_t)sm_count() + per - 1) / per;
+  const int64_t by_rows = (n + 255) / 256;
+  if (S > by_rows) S = by_rows;
+  if (S > kMaxSlices) S = kMaxSlices;
+  if (S < 1) S = 1;
+  *rows_per = ((n + S - 1) / S + kG32BK - 1) / kG32BK * kG32BK;
+  return (int)((n + *rows_per - 1) / *rows_per);
 }
 
+static int bias_blocks(int64_t n) {
+  const int64_t b = (n + 511) / 512;
+  return (int)(b < 1 ? 1 : b > 128 ? 128 : b);
+}
+
+// every layer's input, masked input, hidden activations, conditioner outputs
+// (later their gradients) and hidden gradients; two input gradients
 static size_t train_floats(const RnvpGeom& g, int64_t n) {
-  const size_t d = g.d, H = g.H;
-  return (size_t)n * ((g.L + 1) * d + 6 * d + 4 * H + 2) + (size_t)train_part_floats(g) + 64;
+  const size_t d = g.d, H = g.H, L = g.L;
+  int64_t rp;
+  return (size_t)n * ((L + 1) * d + L * (3 * d + 4 * H) + 2 * d + 2) + (size_t)wgrad_slices(g, n, &rp) * g.n_params +
+         L * 4 * H * d + L * (2 * H + 2 * d) * bias_blocks(n) + 64 * 12;
 }
 
 }  // namespace fmc
@@ -356,36 +449,47 @@ extern "C" int fmc_rnvp_loss_grad(const FmcRealNVP* flow, const float* x, int64_
                 "workspace of %zu bytes is smaller than fmc_rnvp_workspace_size", ws_bytes);
   cudaStream_t st = (cudaStream_t)stream;
   const int d = g.d, H = g.H;
+  const int64_t nd = n * d, nh = n * 2 * (int64_t)H;
   float* p = (float*)ws;
-  float* X = p; p += (int64_t)(g.L + 1) * n * d;   // layer inputs, X[L] = y
-  RnvpScratch s;
-  s.cond = p; p += n * d;
-  s.h = p; p += n * 2 * (int64_t)H;
-  s.sraw = p; p += n * d;
-  s.tt = p; p += n * d;
-  float* gy = p; p += n * d;
-  float* gx = p; p += n * d;
-  float* dh = p; p += n * 2 * (int64_t)H;
-  float* dc = p; p += n * d;
-  float* ld = p; p += n;
-  float* logp = p; p += n;
+  auto take = [&](int64_t floats) {
+    float* r = p;
+    p += (floats + 63) / 64 * 64;   // 256-byte pieces: 16-byte copies where the shapes allow them
+    return r;
+  };
+  float* X = take((g.L + 1) * nd);   // layer inputs, X[L] = y
+  float* cond = take(g.L * nd);
+  float* sraw = take(g.L * nd);
+  float* tt = take(g.L * nd);
+  float* h = take(g.L * nh);
+  float* dz = take(g.L * nh);
+  float* gy = take(nd);
+  float* gx = take(nd);
+  float* ld = take(n);
+  float* logp = take(n);
+  float* wt = take((int64_t)g.L * 4 * H * d);
+  const int rb = bias_blocks(n);
+  float* bpart = take((int64_t)g.L * (2 * H + 2 * d) * rb);
   float* part = p;
-  const int64_t part_floats = train_part_floats(g);
+  int64_t rows_per = 0;
+  const int slices = wgrad_slices(g, n, &rows_per);
 
-  // forward, keeping every layer's input
+  // forward, keeping every layer's activations
   k_standardize<<<grid_for(n * d), 256, 0, st>>>(x, n, d, flow->aux, X);
   FMC_LAUNCH_CHECK();
+  k_rnvp_cond<<<grid_for(n * d), 256, 0, st>>>(X, layer_mask(g, flow->aux, 0), n, d, cond);
+  FMC_LAUNCH_CHECK();
   for (int l = 0; l < g.L; ++l) {
-    const float* th = flow->theta + (int64_t)l * g.per_layer;
-    const float* m = layer_mask(g, flow->aux, l);
-    const float* xl = X + (int64_t)l * n * d;
-    float* xn = X + (int64_t)(l + 1) * n * d;
-    rc = rnvp_conditioner(st, g, th, m, xl, n, s);
+    const RnvpScratch s{cond + l * nd, h + l * nh, sraw + l * nd, tt + l * nd};
+    rc = rnvp_conditioner(st, g, flow->theta + (int64_t)l * g.per_layer, n, s);
     if (rc) return rc;
-    k_rnvp_couple<<<warp_grid(n), 256, 0, st>>>(xl, s.sraw, s.tt, m, n, d, g.dt, 0, xn, ld, l == 0 ? 1 : 0);
+    const bool last = l + 1 == g.L;
+    k_rnvp_couple<<<warp_grid(n), 256, 0, st>>>(X + l * nd, s.sraw, s.tt, layer_mask(g, flow->aux, l), n, d, g.dt, 0,
+                                                X + (l + 1) * nd, ld, l == 0 ? 1 : 0,
+                                                last ? nullptr : layer_mask(g, flow->aux, l + 1),
+                                                last ? nullptr : cond + (l + 1) * nd);
     FMC_LAUNCH_CHECK();
   }
-  float* y = X + (int64_t)g.L * n * d;
+  float* y = X + (int64_t)g.L * nd;
   k_rnvp_logprob<<<warp_grid(n), 256, 0, st>>>(y, ld, n, d, logp);
   FMC_LAUNCH_CHECK();
   k_rnvp_loss<<<1, 1024, 0, st>>>(logp, n, loss);
@@ -394,43 +498,62 @@ extern "C" int fmc_rnvp_loss_grad(const FmcRealNVP* flow, const float* x, int64_
   // backward: loss = -mean(ld + log N(y)) -> dL/dy = y / n, dL/d ld = -1 / n
   k_rnvp_scale<<<grid_for(n * d), 256, 0, st>>>(y, n * d, 1.f / (float)n, gy);
   FMC_LAUNCH_CHECK();
+  k_rnvp_transpose<<<dim3((unsigned)grid_for(4ll * H * d, 1), (unsigned)g.L), 256, 0, st>>>(flow->theta, g, wt);
+  FMC_LAUNCH_CHECK();
   const float gld = -1.f / (float)n;
   for (int l = g.L - 1; l >= 0; --l) {
-    const float* th = flow->theta + (int64_t)l * g.per_layer;
-    float* gth = grad + (int64_t)l * g.per_layer;
     const float* m = layer_mask(g, flow->aux, l);
-    const float* xl = X + (int64_t)l * n * d;
-    rc = rnvp_conditioner(st, g, th, m, xl, n, s);
-    if (rc) return rc;
-    k_rnvp_couple_bwd<<<grid_for(n * d), 256, 0, st>>>(xl, s.sraw, s.tt, m, gy, n, d, g.dt, gld, gx);
+    const float* wl = wt + (int64_t)l * 4 * H * d;
+    k_rnvp_couple_bwd<<<grid_for(n * d), 256, 0, st>>>(X + l * nd, sraw + l * nd, tt + l * nd, m, gy, n, d, g.dt, gld, gx);
     FMC_LAUNCH_CHECK();
-    // dH = [dsraw W2s, dtt W2t] masked by relu'
-    rc = sgemm<true, false, EPI_DRELU>(st, n, H, d, s.sraw, d, th + g.off_W2s, H, nullptr, s.h, 2 * H, dh, 2 * H, 0.f);
+    // dz = [dsraw W2s, dtt W2t] masked by relu'
+    G32Args a{};
+    a.M = n;
+    a.p[0] = G32Problem{sraw + l * nd, wl, nullptr, h + l * nh, dz + l * nh};
+    a.p[1] = G32Problem{tt + l * nd, wl + (int64_t)H * d, nullptr, h + l * nh + H, dz + l * nh + H};
+    a.lda = a.ldb = d;
+    a.ldaux = a.ldc = 2 * H;
+    a.N = H;
+    a.K = d;
+    rc = gemm_f32<G32_DRELU>(st, a, 2);
     if (rc) return rc;
-    rc = sgemm<true, false, EPI_DRELU>(st, n, H, d, s.tt, d, th + g.off_W2t, H, nullptr, s.h + H, 2 * H, dh + H,
-                                       2 * H, 0.f);
-    if (rc) return rc;
-    // dc = dH W1; gx += dc * m
-    rc = sgemm<true, false, EPI_NONE>(st, n, d, 2 * H, dh, 2 * H, th, d, nullptr, nullptr, 0, dc, d, 0.f);
-    if (rc) return rc;
-    k_rnvp_add_masked<<<grid_for(n * d), 256, 0, st>>>(gx, dc, m, n, d);
-    FMC_LAUNCH_CHECK();
-    // weight and bias gradients over the batch
-    rc = kouter(st, d, H, n, s.sraw, d, s.h, 2 * H, false, part, part_floats, gth + g.off_W2s);
-    if (rc) return rc;
-    rc = kouter(st, d, 1, n, s.sraw, d, nullptr, 0, true, part, part_floats, gth + g.off_b2s);
-    if (rc) return rc;
-    rc = kouter(st, d, H, n, s.tt, d, s.h + H, 2 * H, false, part, part_floats, gth + g.off_W2t);
-    if (rc) return rc;
-    rc = kouter(st, d, 1, n, s.tt, d, nullptr, 0, true, part, part_floats, gth + g.off_b2t);
-    if (rc) return rc;
-    rc = kouter(st, 2 * H, d, n, dh, 2 * H, s.cond, d, false, part, part_floats, gth);
-    if (rc) return rc;
-    rc = kouter(st, 2 * H, 1, n, dh, 2 * H, nullptr, 0, true, part, part_floats, gth + g.off_b1);
+    // gx += (dz W1) * m
+    a.p[0] = G32Problem{dz + l * nh, wl + 2ll * H * d, m, nullptr, gx};
+    a.lda = a.ldb = 2 * H;
+    a.ldc = d;
+    a.N = d;
+    a.K = 2 * H;
+    rc = gemm_f32<G32_ADD_MASKED>(st, a, 1);
     if (rc) return rc;
     float* t = gy;
     gy = gx;
     gx = t;
   }
+  // weight and bias gradients of all layers over the batch. The second
+  // Linears' as h^T d(output), stored transposed: the wide side is the tall
+  // operand of the 256 x 32 tiles
+  K32Args k{};
+  k.p[0] = K32Problem{dz, cond, nh, nd, 2 * H, d, 2 * H, d, 0, d, 1};
+  k.p[1] = K32Problem{h, sraw, nh, nd, 2 * H, d, H, d, g.off_W2s, 1, H};
+  k.p[2] = K32Problem{h + H, tt, nh, nd, 2 * H, d, H, d, g.off_W2t, 1, H};
+  k.n_problems = 3;
+  k.rows = n;
+  k.rows_per_slice = rows_per;
+  k.per_layer = g.per_layer;
+  k.n_params = g.n_params;
+  k.part = part;
+  const unsigned tiles = (unsigned)(((2 * H + kK32M - 1) / kK32M) * ((d + kK32N - 1) / kK32N));
+  constexpr int ksmem = kG32Stages * kK32StageFloats * 4;
+  FMC_CUDA_TRY(cudaFuncSetAttribute(k_kouter_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, ksmem));
+  k_kouter_f32<<<dim3(tiles, (unsigned)slices, (unsigned)(3 * g.L)), kK32Threads, ksmem, st>>>(k);
+  FMC_LAUNCH_CHECK();
+  k_rnvp_sum_slices<<<grid_for(g.n_params), 256, 0, st>>>(part, slices, g.n_params, grad);
+  FMC_LAUNCH_CHECK();
+  const unsigned cb = (unsigned)((2 * H > d ? 2 * H : d) + 127) / 128;
+  k_rnvp_bias_partial<<<dim3(cb, (unsigned)rb, (unsigned)(3 * g.L)), 128, 0, st>>>(g, dz, sraw, tt, n, (n + rb - 1) / rb,
+                                                                                  bpart);
+  FMC_LAUNCH_CHECK();
+  k_rnvp_bias_final<<<dim3(cb, 1, (unsigned)(3 * g.L)), 128, 0, st>>>(g, bpart, rb, grad);
+  FMC_LAUNCH_CHECK();
   return FMC_OK;
 }
