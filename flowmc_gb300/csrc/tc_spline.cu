@@ -27,7 +27,8 @@
 //
 // Both kernels are persistent (tile t = blockIdx.x, +gridDim.x, ...): warp 0
 // issues the TMA loads of a STAGES-deep ring (stages of one or, for the
-// forward/inverse kernel where K allows, two 64-wide K chunks), warp 1 owns
+// forward/inverse kernel where K allows, two 64-wide K chunks), the last warp
+// moves the x tiles, warp 1 owns
 // the TMEM and issues tcgen05.mma into two accumulators (the epilogue of one tile overlaps the
 // MMAs of the next), and kSplineEpiPerQuarter warps per TMEM lane quarter run
 // the epilogue, warp h of a quarter taking coordinates h, h + E, ... of the
@@ -42,7 +43,9 @@ namespace tc {
 
 constexpr int kSplEpiWarps = 4 * kSplineEpiPerQuarter;
 constexpr int kSplEpiThreads = 32 * kSplEpiWarps;
-constexpr int kSplThreads = 64 + kSplEpiThreads;
+constexpr int kSplPairThreads = 64 + kSplEpiThreads;    // the CTA-pair kernel
+constexpr int kSplThreads = kSplPairThreads + 32;        // and the box warp of the one-CTA kernels
+constexpr int kBoxWarp = 2 + kSplEpiWarps;
 
 template <int K>
 struct SplineTile {
@@ -154,12 +157,11 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
-template <int BN, int STAGES, int CH>
-__device__ __forceinline__ Pipe pipe_setup(uint8_t* base, int warp) {
-  using S = SplSmem<BN, STAGES, CH>;
+template <int STAGES>
+__device__ __forceinline__ Pipe pipe_setup(uint8_t* base, uint8_t* bars, int warp) {
   Pipe p;
   p.base = base;
-  p.full = (uint64_t*)(base + STAGES * S::STAGE_BYTES);
+  p.full = (uint64_t*)bars;
   p.empty = p.full + STAGES;
   p.acc_full = p.empty + STAGES;
   p.acc_empty = p.acc_full + 2;
@@ -291,19 +293,19 @@ __device__ __forceinline__ void release_acc(const Pipe& p, int b, int lane) {
   if (lane == 0) mbar_arrive(&p.acc_empty[b]);
 }
 
-// named barrier over the epilogue warps only (id 0 is __syncthreads)
-__device__ __forceinline__ void epi_sync(int id) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(kSplEpiThreads) : "memory");
+// barrier over the four warps (one per TMEM lane quarter) that share h
+__device__ __forceinline__ void quarters_sync(int h) {
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + h) : "memory");
 }
 
-// OR of v over the epilogue warps (barrier 3 with a predicate reduction), so
-// that every epilogue warp takes the same branch before a named barrier
-__device__ __forceinline__ bool epi_any(bool v) {
+// OR of v over those four warps, so that they take the same branch before
+// a named barrier
+__device__ __forceinline__ bool quarters_any(int h, bool v) {
   uint32_t r;
   asm volatile(
-      "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n barrier.red.or.pred p, 3, %2, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+      "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n barrier.red.or.pred p, %2, 128, q;\n selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(r)
-      : "r"((uint32_t)v), "r"(kSplEpiThreads)
+      : "r"((uint32_t)v), "r"(1 + kSplineEpiPerQuarter + h)
       : "memory");
   return r != 0;
 }
@@ -315,16 +317,47 @@ struct BiasRows {
   static constexpr int PP = (3 * K + 1 + 3) / 4 * 4;
 };
 
+// Position of 16-byte chunk j of row r in a box of CH16 chunks per row: the
+// chunk order the box's TMA swizzle writes, so that the 32 rows of a warp
+// spread over the banks -- none for an odd number of chunks per row, 32-byte
+// swizzle for two, 64-byte swizzle for four.
+template <int CH16>
+__device__ __forceinline__ int box_chunk(int r, int j) {
+  if constexpr (CH16 == 2) return j ^ ((r >> 2) & 1);
+  if constexpr (CH16 == 4) return j ^ ((r >> 1) & 3);
+  return j;
+}
+
+// fp32 boxes of DG coordinate pairs per row (x, dL/dy)
+template <int DG>
+struct XBox {
+  static constexpr int XS = 2 * DG;                 // floats per row
+  static constexpr int CH16 = XS / 4;               // 16-byte chunks per row
+  // the wider groups (K <= 5) leave no shared memory for boxes
+  static constexpr bool kOk = CH16 == 2 || CH16 == 4 || (CH16 % 2 == 1 && CH16 <= 5);
+  static constexpr int SWIZZLE = CH16 == 2 ? 32 : CH16 == 4 ? 64 : 0;
+  static constexpr int FLOATS = BM * XS;
+  static constexpr int BYTES = FLOATS * 4;
+  static_assert(!kOk || BYTES % 1024 == 0, "boxes stay on the swizzle pattern's period");
+  // float offset of column c of row r
+  __device__ static __forceinline__ int at(int r, int c) {
+    return r * XS + 4 * box_chunk<CH16>(r, c >> 2) + (c & 3);
+  }
+};
+
 // x tiles staged through shared memory (x_tma): the group's column span of
 // a 128-row tile -- 2 DG floats per row, the transformed coordinates and the
 // conditioning ones between them -- is one TMA box of the fp32 tensor map
-// tmX over x [M, d]. The first epilogue warp's lane 0 loads the next tile's
-// box while the current tile is computed (two buffers) and, after the
-// epilogue warps have written y into the buffer, stores the box back. Every
-// tile owns its rows' column span alone, so the write-back (which also
-// rewrites the untouched conditioning columns with their own values) races
-// with nothing. Without x_tma (row stride not a multiple of 16 bytes) each
-// thread reads and writes its coordinates of x directly.
+// tmX over x [M, d]. The box warp (the CTA's last) keeps kXBufs boxes in
+// turn: it loads tile i + 2's box while tile i + 1 is computed, and once the
+// epilogue warps have written y into tile i's box it stores the box back,
+// adds the rows' log-det partials and writes the next layer's operand. So no
+// epilogue warp waits for a store, a load it could have had earlier, or the
+// other epilogue warps. Every tile owns its rows' column span alone, so the
+// write-back (which also rewrites the untouched conditioning columns with
+// their own values) races with nothing. Without x_tma (row stride not a
+// multiple of 16 bytes, or no shared memory left) each thread reads and
+// writes its coordinates of x directly.
 //
 // Next-layer fold (fold_th != nullptr, x boxes only, even n_dim): the box
 // leaves with the next coupling layer's ScalarAffine applied to every
@@ -332,6 +365,15 @@ struct BiasRows {
 // direction), and the next layer's bf16 conditioning block -- the affined
 // transformed coordinates of this layer, conditioning index t -- is written
 // to cond16 [M, ldc16]; that layer then needs no separate affine launch.
+//
+// The tile's work without its arithmetic, copies and MMAs used to be two
+// thirds of the time: x was read and written at a 64-byte row pitch (all 32
+// rows of a warp in two banks, four accesses per coordinate), and one
+// epilogue lane waited for the last tile's store before the others could go
+// on. Measured at 69,632 rows, 64 dims, 256 units, 8 bins: 61 -> 43 us forward,
+// 64 -> 45 us inverse; at 65,536 rows, 128 dims, 512 units, 12 bins, where the
+// operands' way into the SM (64 B/clock) bounds it: 132 -> 128 us.
+constexpr int kXBufs = 3;
 template <int KB, bool INV, int STAGES, int CH>
 __global__ void __launch_bounds__(kSplThreads, 1)
     k_tc_spline(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -341,15 +383,19 @@ __global__ void __launch_bounds__(kSplThreads, 1)
                 uint16_t* __restrict__ cond16, int ldc16, int* err) {
   using T = SplineTile<KB>;
   constexpr int P = T::P, DG = T::DG, BN = T::BN, E = kSplineEpiPerQuarter, PP = BiasRows<KB>::PP;
-  constexpr int XS = 2 * DG;   // floats per row of an x box
+  using X = XBox<DG>;
   using S = SplSmem<BN, STAGES, CH>;
   if (tc_skip(err)) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  float* sbias = (float*)(base + STAGES * S::STAGE_BYTES + 256);   // after the ring and its barriers
-  uint64_t* xfull = (uint64_t*)(base + STAGES * S::STAGE_BYTES + 192);   // [2], in the barrier block
-  float* xbuf = (float*)((((uintptr_t)(sbias + (bias_smem ? nt * PP : 0))) + 127) & ~(uintptr_t)127);
-  float* lred = xbuf + 2 * BM * XS;   // [2][E][BM] log-det partials of a tile (x boxes only)
+  const bool xt = X::kOk && x_tma != 0;
+  // ring | x boxes | barriers | log-det partials [2][E][BM] | bias rows
+  float* xbuf = (float*)(base + STAGES * S::STAGE_BYTES);
+  uint8_t* bars = base + STAGES * S::STAGE_BYTES + (xt ? kXBufs * X::BYTES : 0);
+  uint64_t* xfull = (uint64_t*)(bars + 128);   // [kXBufs] box loaded
+  uint64_t* xdone = xfull + kXBufs;            // [kXBufs] box rewritten by the epilogue warps
+  float* lred = (float*)(bars + 256);
+  float* sbias = lred + (xt ? 2 * E * BM : 0);
   if (bias_smem) {
     for (int i = threadIdx.x; i < nt * PP; i += blockDim.x) {
       const int t = i / PP, pp = i - t * PP;
@@ -357,59 +403,116 @@ __global__ void __launch_bounds__(kSplThreads, 1)
     }   // visible after pipe_setup's __syncthreads
   }
   if (threadIdx.x == 0) {
-    mbar_init(&xfull[0], 1);
-    mbar_init(&xfull[1], 1);   // pipe_setup's fence and barrier publish these
+    for (int j = 0; j < kXBufs; ++j) {
+      mbar_init(&xfull[j], 1);
+      mbar_init(&xdone[j], kSplEpiWarps);
+    }   // pipe_setup's fence and barrier publish these
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nk = (K + BK * CH - 1) / (BK * CH);   // stages per tile (K a multiple of BK * CH when CH > 1)
   const int tiles = (M + BM - 1) / BM * n_groups;
-  const Pipe p = pipe_setup<BN, STAGES, CH>(base, warp);
+  const Pipe p = pipe_setup<STAGES>(base, bars, warp);
+  const bool fold = fold_th != nullptr;
 
   if (warp == 0) {
     if (lane == 0) producer<BN, STAGES, CH>(p, &tmA, &tmB, tiles, n_groups, nk);
   } else if (warp == 1) {
     if (lane == 0) mma_issuer<BN, STAGES, CH>(p, tiles, nk);
+  } else if (warp == kBoxWarp) {
+    if (xt) {
+      const int step = (int)gridDim.x;
+      int issued = 0;   // boxes loaded so far (lane 0)
+      auto load_box = [&](int t) {   // tile t is this CTA's tile number `issued`
+        const int j = issued % kXBufs;
+        mbar_expect_tx(&xfull[j], X::BYTES);
+        tma_load_2d(xbuf + j * X::FLOATS, &tmX, &xfull[j], 2 * (t % n_groups) * DG, (t / n_groups) * BM);
+        ++issued;
+      };
+      if (lane == 0)
+        for (int k = 0; k < 2; ++k)
+          if ((int)blockIdx.x + k * step < tiles) load_box(blockIdx.x + k * step);
+      int local = 0;
+      for (int t = blockIdx.x; t < tiles; t += step, ++local) {
+        const int j = local % kXBufs, b = local & 1;
+        const int m0 = (t / n_groups) * BM, g = t % n_groups;
+        const float* xb = xbuf + j * X::FLOATS;
+        const bool bad = *p.abort_flag || !mbar_wait(&xdone[j], (uint32_t)(local / kXBufs) & 1u);
+        if (__any_sync(0xffffffffu, bad)) {
+          *p.abort_flag = 1;
+          break;
+        }
+        if (lane == 0) {
+          tma_store_2d_f32(&tmX, smem_u32(xb), 2 * g * DG, m0);   // rows past M are clipped
+          bulk_commit();
+        }
+        // the quarter's E log-det partials of a row, in order: one partial
+        // per group and row is written
+#pragma unroll
+        for (int r = lane; r < BM; r += 32) {
+          if (m0 + r < M) {
+            float sl = 0.f;
+#pragma unroll
+            for (int k = 0; k < E; ++k) sl += lred[(b * E + k) * BM + r];
+            ldp[(int64_t)g * M + m0 + r] = sl;
+          }
+        }
+        if (fold) {
+          // the rows' next-layer conditioning values, bf16, two per chunk
+          // (x_tma: n_dim is a multiple of 4, so nt and DG are even)
+          const int t0 = g * DG, tn = nt - t0 < DG ? nt - t0 : DG;
+#pragma unroll
+          for (int r = lane; r < BM; r += 32) {
+            if (m0 + r < M) {
+              uint32_t* cr = reinterpret_cast<uint32_t*>(cond16 + (int64_t)(m0 + r) * ldc16 + t0);
+              uint32_t w[X::CH16];
+#pragma unroll
+              for (int c = 0; c < X::CH16; ++c) {
+                const float4 v = *reinterpret_cast<const float4*>(xb + X::at(r, 4 * c));
+                w[c] = (uint32_t)f32_to_bf16_rn(tpar ? v.y : v.x) | ((uint32_t)f32_to_bf16_rn(tpar ? v.w : v.z) << 16);
+              }
+              if constexpr (X::CH16 == 4) {
+                if (tn == DG) {   // 16-byte aligned: t0 and ldc16 are multiples of 8
+                  *reinterpret_cast<uint4*>(cr) = make_uint4(w[0], w[1], w[2], w[3]);
+                  continue;
+                }
+              }
+#pragma unroll
+              for (int c = 0; c < X::CH16; ++c)
+                if (2 * c < tn) cr[c] = w[c];
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0 && t + 2 * step < tiles) {
+          // into the box of tile local - 1, whose store has been read once at
+          // most one (this tile's) is outstanding
+          bulk_wait_read_1();
+          load_box(t + 2 * step);
+        }
+      }
+      if (lane == 0) {
+        bulk_wait_all();   // the stores have completed before the CTA exits
+        // boxes loaded for tiles the loop did not finish (after an abort) land first (bounded)
+        for (int k = local; k < issued; ++k) mbar_wait(&xfull[k % kXBufs], (uint32_t)(k / kXBufs) & 1u);
+      }
+    }
   } else {
     const int q = warp & 3;          // TMEM lane quarter
     const int h = (warp - 2) >> 2;   // coordinates h, h + E, ... of the group
     const int row = q * 32 + lane;
-    const bool xt = x_tma != 0;
-    const bool elect = warp == 2 && lane == 0;   // issues the x boxes' copies
     // the next layer's affine (common.py:229, 238), as its own launch would apply it
-    const bool fold = fold_th != nullptr;
     const float fs = fold ? fold_th[0] : 0.f, ft = fold ? fold_th[1] : 0.f;
     const float fes = expf(INV ? -fs : fs);
     auto next_affine = [&](float v) { return scalar_affine(v, fes, ft, INV ? 1 : 0); };
-    constexpr uint32_t kXBytes = BM * XS * 4;
-    int issued = 0;   // x boxes loaded so far (by the elected lane)
-    if (xt && elect && (int)blockIdx.x < tiles) {
-      const int t0 = blockIdx.x;
-      mbar_expect_tx(&xfull[0], kXBytes);
-      tma_load_2d(xbuf, &tmX, &xfull[0], 2 * (t0 % n_groups) * DG, (t0 / n_groups) * BM);
-      issued = 1;
-    }
     int local = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++local) {
-      const int b = local & 1, use = local >> 1;
+      const int b = local & 1, use = local >> 1, j = local % kXBufs;
       const int m0 = (t / n_groups) * BM, g = t % n_groups;
       const int gm = m0 + row;
-      float* xb = xbuf + b * (BM * XS);
-      if (xt && elect) {
-        // the next tile's box goes into the other buffer once the previous
-        // tile's store has finished reading it
-        bulk_wait_read_0();
-        const int tn = t + (int)gridDim.x;
-        if (tn < tiles) {
-          mbar_expect_tx(&xfull[b ^ 1], kXBytes);
-          tma_load_2d(xbuf + (b ^ 1) * (BM * XS), &tmX, &xfull[b ^ 1], 2 * (tn % n_groups) * DG,
-                      (tn / n_groups) * BM);
-          ++issued;
-        }
-      }
-      // every epilogue warp leaves the loop at the same tile (named barriers follow)
+      float* xb = xbuf + j * X::FLOATS;
       bool bad = *p.abort_flag || !mbar_wait(&p.acc_full[b], (uint32_t)use & 1u);
-      if (xt && !bad) bad = !mbar_wait(&xfull[b], (uint32_t)use & 1u);
-      if (epi_any(bad)) {
+      if (xt && !bad) bad = !mbar_wait(&xfull[j], (uint32_t)(local / kXBufs) & 1u);
+      if (__any_sync(0xffffffffu, bad)) {
         *p.abort_flag = 1;
         break;
       }
@@ -423,8 +526,15 @@ __global__ void __launch_bounds__(kSplThreads, 1)
         float raw[P];
         tmem_ld_coord<P, T::PPC>(tb + (uint32_t)(u * T::PPC), raw);   // warp-collective: every lane loads
         if (gm < M) {
-          float* xp = xt ? xb + row * XS + 2 * u + tpar : xa + (int64_t)gm * d + 2 * tcoord + tpar;
-          const float xv = *xp;
+          // the coordinate and its conditioning partner, adjacent in the box
+          float2 xc;
+          float2* bp = reinterpret_cast<float2*>(xb + X::at(row, 2 * u));
+          float* xp = xa + (int64_t)gm * d + 2 * tcoord + tpar;
+          if (xt)
+            xc = *bp;
+          else
+            xc = make_float2(*xp, 0.f);
+          const float xv = xt && tpar ? xc.y : xc.x;
           if (bias_smem) {
             const float4* bb = reinterpret_cast<const float4*>(sbias + tcoord * PP);
             float bl[PP];
@@ -444,60 +554,34 @@ __global__ void __launch_bounds__(kSplThreads, 1)
           }
           float y, l;
           rqs_apply_fast<KB, INV>(raw, xv, cfg, y, l);
-          if (fold) {
-            // this coordinate and its conditioning partner in the box (the
-            // partner is conditioning here, transformed by the next layer)
-            y = next_affine(y);
-            float* cp = xb + row * XS + 2 * u + (1 - tpar);
-            *cp = next_affine(*cp);
+          if (xt) {
+            float c = tpar ? xc.x : xc.y;
+            if (fold) {
+              // the partner is conditioning here, transformed by the next layer
+              y = next_affine(y);
+              c = next_affine(c);
+            }
+            *bp = tpar ? make_float2(c, y) : make_float2(y, c);
+          } else {
+            *xp = y;
           }
-          *xp = y;
           ldsum += l;
         }
       }
-      // log-det partials: with the x boxes the quarter's E warps add theirs
-      // in shared memory (two tile-parity buffers: a warp may start the next
-      // tile while warp 0 of its quarter still reads this one) and one
-      // partial per group and row is written; otherwise one per warp.
-      // Partial-major: a warp writes 128 contiguous bytes.
-      if (xt)
-        lred[(b * E + h) * BM + row] = ldsum;
-      else if (gm < M)
-        ldp[(int64_t)(E * g + h) * M + gm] = ldsum;
-      release_acc(p, b, lane);
+      // log-det partials: with the x boxes the box warp adds the quarter's E
+      // (two tile-parity buffers: tile i + 2's box, which this warp has waited
+      // for by then, is loaded after tile i's partials are read); otherwise
+      // one per warp. Partial-major: a warp writes 128 contiguous bytes.
       if (xt) {
-        // y is in the buffer: make the writes visible to the copy engine, then
-        // one lane stores the box (rows past M are clipped by the store)
+        lred[(b * E + h) * BM + row] = ldsum;
+        // y is in the box: visible to the copy engine before the box warp stores it
         fence_proxy_async_smem();
-        epi_sync(1);
-        if (elect) {
-          tma_store_2d_f32(&tmX, smem_u32(xb), 2 * g * DG, m0);
-          bulk_commit();
-        }
-        if (h == 0 && gm < M) {
-          float sl = 0.f;
-#pragma unroll
-          for (int k = 0; k < E; ++k) sl += lred[(b * E + k) * BM + row];
-          ldp[(int64_t)g * M + gm] = sl;
-          if (fold) {
-            // the row's next-layer conditioning values, bf16, two per 4-byte
-            // store (DG is even; the group's last coordinate may be alone)
-            const int t0 = g * DG, tn = nt - t0 < DG ? nt - t0 : DG;
-            const float* yr = xb + row * XS + tpar;
-            uint16_t* cr = cond16 + (int64_t)gm * ldc16 + t0;
-            int u = 0;
-            for (; u + 1 < tn; u += 2)
-              *reinterpret_cast<uint32_t*>(cr + u) =
-                  (uint32_t)f32_to_bf16_rn(yr[2 * u]) | ((uint32_t)f32_to_bf16_rn(yr[2 * u + 2]) << 16);
-            if (u < tn) cr[u] = f32_to_bf16_rn(yr[2 * u]);
-          }
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&xdone[j]);
+      } else if (gm < M) {
+        ldp[(int64_t)(E * g + h) * M + gm] = ldsum;
       }
-    }
-    if (xt && elect) {
-      bulk_wait_all();   // the stores have completed before the CTA exits
-      // boxes loaded for tiles the loop did not finish (after an abort) land first (bounded)
-      for (int k = local; k < issued; ++k) mbar_wait(&xfull[k & 1], (uint32_t)(k >> 1) & 1u);
+      release_acc(p, b, lane);
     }
   }
   pipe_teardown(p, warp, lane, err);
@@ -514,24 +598,23 @@ struct SplineBwdArgs {
   int d, nt, tpar, cpar;
 };
 
-// Shared-memory position of 16-byte chunk j of row r in a d-raw staging box
-// (OPC bf16 per row): the chunk order the box's TMA swizzle expects, so the
-// 32 rows of a warp land in distinct banks -- none for an odd number of
-// chunks per row, 32-byte swizzle for two, 64-byte swizzle for four.
-template <int OCH>
-__device__ __forceinline__ int draw_chunk(int r, int j) {
-  if constexpr (OCH == 2) return j ^ ((r >> 2) & 1);
-  if constexpr (OCH == 4) return j ^ ((r >> 1) & 3);
-  return j;
-}
-
 // With x_tma the group's column span of x and of dL/dy for a 128-row tile
-// arrive as two TMA boxes (loaded one tile ahead, two buffers each), the
-// adjoint is written into the dL/dy box in place -- its conditioning columns
-// keep dL/dy, which is their dL/dx -- and the box is stored to gxa. Each tile
-// owns its rows' column span, as in the forward kernel. d raw of coordinate t
-// is staged as a [128 rows][OPC] box (its P values, zeros up to OPC) and
-// stored by TMA to columns [t * OPC, (t + 1) * OPC) of graw (tmR).
+// arrive as two TMA boxes (two buffers each, loaded by the box warp one to
+// two tiles ahead together with the group's bias rows); the adjoint is
+// written into the dL/dy box in place -- its conditioning columns keep dL/dy,
+// which is their dL/dx -- and the box warp stores the box to gxa. Each tile
+// owns its rows' column span, as in the forward kernel.
+//
+// d raw of coordinate t is staged as a [128 rows][OPC] box (its P values,
+// zeros up to OPC), one staging box per coordinate of the group, and stored
+// by TMA to columns [t * OPC, (t + 1) * OPC) of graw (tmR). The four warps
+// that share h handle the same coordinates h, h + E, ...; they alone meet
+// once per coordinate: when its box is written, one of them stores it, all
+// of them add its columns, and by then the box of their next coordinate,
+// stored one coordinate earlier, has been read. Nothing waits for the other
+// coordinates' warps. One barrier over all twelve and a wait for the tile's
+// stores at its end, and the bias as global loads, took 242 us at 65,536 rows,
+// 128 dims, 512 units, 12 bins; now 197 us.
 template <int KB, int STAGES>
 __global__ void __launch_bounds__(kSplThreads, 1)
     k_tc_spline_bwd(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -539,54 +622,89 @@ __global__ void __launch_bounds__(kSplThreads, 1)
                     const __grid_constant__ CUtensorMap tmGx, const __grid_constant__ CUtensorMap tmR, int x_tma,
                     int M, int n_groups, int K, const SplineBwdArgs a, SplineCfg cfg, int* err) {
   using T = SplineTile<KB>;
-  constexpr int P = T::P, DG = T::DG, BN = T::BN, E = kSplineEpiPerQuarter;
+  constexpr int P = T::P, DG = T::DG, BN = T::BN, E = kSplineEpiPerQuarter, PP = BiasRows<KB>::PP;
   constexpr int OPC = T::OPC, OCH = OPC / 8, OBOX = BM * OPC * 2;
-  constexpr int CP = DG * OPC / 2;                 // column pairs of a group's staged boxes
   constexpr int RP = kSplineBwdRowParts;
   constexpr int RROWS = (BM + RP - 1) / RP;        // rows per column-sum part
-  static_assert(RP * CP <= kSplEpiThreads, "one thread per column pair and row part");
-  constexpr int XS = 2 * DG;   // floats per row of a box
+  using X = XBox<DG>;
   using S = SplSmem<BN, STAGES, 1>;
   if (tc_skip(err)) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  // staging boxes 1024 bytes after the ring (the barrier block between), then the x / dL/dy boxes
-  uint8_t* stg = base + STAGES * S::STAGE_BYTES + 1024;
-  uint64_t* xfull = (uint64_t*)(base + STAGES * S::STAGE_BYTES + 192);   // [2], in the barrier block
-  float* boxes = (float*)(stg + DG * OBOX);                                 // [2][x | dL/dy]
+  const bool xt = X::kOk && x_tma != 0;
+  // ring | staging boxes | [2][x | dL/dy] boxes | barriers | [2] the group's bias rows
+  uint8_t* stg = base + STAGES * S::STAGE_BYTES;
+  float* boxes = (float*)(stg + DG * OBOX);
+  uint8_t* bars = stg + DG * OBOX + (xt ? 4 * X::BYTES : 0);
+  uint64_t* xfull = (uint64_t*)(bars + 128);   // [2] boxes and bias rows loaded
+  uint64_t* xdone = xfull + 2;                 // [2] dL/dy box rewritten by the epilogue warps
+  float* sbias = (float*)(bars + 256);         // [2][DG * PP], x boxes only
   if (threadIdx.x == 0) {
-    mbar_init(&xfull[0], 1);
-    mbar_init(&xfull[1], 1);   // pipe_setup's fence and barrier publish these
+    for (int j = 0; j < 2; ++j) {
+      mbar_init(&xfull[j], 1);
+      mbar_init(&xdone[j], kSplEpiWarps);
+    }   // pipe_setup's fence and barrier publish these
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nk = (K + BK - 1) / BK;
   const int tiles = (M + BM - 1) / BM * n_groups;
   const int ntP = a.nt * P;
-  const Pipe p = pipe_setup<BN, STAGES, 1>(base, warp);
+  const Pipe p = pipe_setup<STAGES>(base, bars, warp);
 
   if (warp == 0) {
     if (lane == 0) producer<BN, STAGES, 1>(p, &tmA, &tmB, tiles, n_groups, nk);
   } else if (warp == 1) {
     if (lane == 0) mma_issuer<BN, STAGES, 1>(p, tiles, nk);
+  } else if (warp == kBoxWarp) {
+    if (xt) {
+      const int step = (int)gridDim.x;
+      int issued = 0;   // tiles loaded so far
+      auto load = [&](int t) {
+        const int j = issued & 1, g = t % n_groups;
+        const int n = (a.nt - g * DG < DG ? a.nt - g * DG : DG) * P;
+        const float* bb = a.bias + (int64_t)g * DG * P;
+        for (int i = lane; i < n; i += 32) sbias[j * (DG * PP) + (i / P) * PP + i % P] = __ldg(bb + i);
+        __syncwarp();   // the rows are written before lane 0's arrival publishes them
+        if (lane == 0) {
+          float* xb = boxes + (2 * j) * X::FLOATS;
+          mbar_expect_tx(&xfull[j], 2 * X::BYTES);
+          tma_load_2d(xb, &tmX, &xfull[j], 2 * g * DG, (t / n_groups) * BM);
+          tma_load_2d(xb + X::FLOATS, &tmGy, &xfull[j], 2 * g * DG, (t / n_groups) * BM);
+        }
+        ++issued;
+      };
+      for (int k = 0; k < 2; ++k)
+        if ((int)blockIdx.x + k * step < tiles) load(blockIdx.x + k * step);
+      int local = 0;
+      for (int t = blockIdx.x; t < tiles; t += step, ++local) {
+        const int b = local & 1;
+        const bool bad = *p.abort_flag || !mbar_wait(&xdone[b], (uint32_t)(local >> 1) & 1u);
+        if (__any_sync(0xffffffffu, bad)) {
+          *p.abort_flag = 1;
+          break;
+        }
+        if (lane == 0) {
+          const float* gb = boxes + (2 * b + 1) * X::FLOATS;
+          tma_store_2d_f32(&tmGx, smem_u32(gb), 2 * (t % n_groups) * DG, (t / n_groups) * BM);
+          bulk_commit();
+        }
+        if (t + 2 * step < tiles) {
+          if (lane == 0) bulk_wait_read_0();   // the box is free once its store has read it
+          __syncwarp();
+          load(t + 2 * step);
+        }
+      }
+      if (lane == 0) {
+        bulk_wait_all();   // the stores have completed before the CTA exits
+        // boxes loaded for tiles the loop did not finish (after an abort) land first (bounded)
+        for (int k = local; k < issued; ++k) mbar_wait(&xfull[k & 1], (uint32_t)(k >> 1) & 1u);
+      }
+    }
   } else {
     const int q = warp & 3;
     const int h = (warp - 2) >> 2;
     const int row = q * 32 + lane;
-    const int et = threadIdx.x - 64;   // 0 .. kSplEpiThreads-1
-    const bool xt = x_tma != 0;
-    const bool elect = warp == 2 && lane == 0;   // issues the boxes' copies
-    constexpr uint32_t kBox = BM * XS;           // floats per box
-    auto load_boxes = [&](int tt, int buf) {
-      float* xb = boxes + (2 * buf) * kBox;
-      mbar_expect_tx(&xfull[buf], 2 * kBox * 4);
-      tma_load_2d(xb, &tmX, &xfull[buf], 2 * (tt % n_groups) * DG, (tt / n_groups) * BM);
-      tma_load_2d(xb + kBox, &tmGy, &xfull[buf], 2 * (tt % n_groups) * DG, (tt / n_groups) * BM);
-    };
-    int issued = 0;
-    if (xt && elect && (int)blockIdx.x < tiles) {
-      load_boxes(blockIdx.x, 0);
-      issued = 1;
-    }
+    const bool elect = ((warp - 2) & 3) == 0 && lane == 0;   // stores the boxes of the coordinates of h
     int local = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++local) {
       const int b = local & 1, use = local >> 1;
@@ -594,21 +712,12 @@ __global__ void __launch_bounds__(kSplThreads, 1)
       const int m0 = mt * BM;
       const int gm = m0 + row;
       const bool row_ok = gm < M;
-      float* xb = boxes + (2 * b) * kBox;
-      float* gb = xb + kBox;
-      if (xt && elect) {
-        // the next tile's boxes go into the other buffers (every earlier
-        // store finished reading shared memory at the end of the last tile)
-        const int tn = t + (int)gridDim.x;
-        if (tn < tiles) {
-          load_boxes(tn, b ^ 1);
-          ++issued;
-        }
-      }
-      // the tile loop has named barriers: all epilogue warps leave it together
+      float* xb = boxes + (2 * b) * X::FLOATS;
+      float* gb = xb + X::FLOATS;
       bool bad = *p.abort_flag || !mbar_wait(&p.acc_full[b], (uint32_t)use & 1u);
       if (xt && !bad) bad = !mbar_wait(&xfull[b], (uint32_t)use & 1u);
-      if (epi_any(bad)) {
+      // the tile loop has named barriers: the four warps of h leave it together
+      if (quarters_any(h, bad)) {
         *p.abort_flag = 1;
         break;
       }
@@ -624,13 +733,22 @@ __global__ void __launch_bounds__(kSplThreads, 1)
 #pragma unroll
         for (int i = 0; i < OPC; ++i) ov[i] = 0;
         if (row_ok) {
-          const float* bb = a.bias + (int64_t)tcoord * P;
-#pragma unroll
-          for (int i = 0; i < P; ++i) raw[i] += __ldg(bb + i);
           if (xt) {
-            const int jb = row * XS + 2 * u + a.tpar;
+            const float4* bb = reinterpret_cast<const float4*>(sbias + b * (DG * PP) + u * PP);
+#pragma unroll
+            for (int i = 0; i < PP / 4; ++i) {
+              const float4 bv = bb[i];
+              raw[4 * i] += bv.x;
+              if (4 * i + 1 < P) raw[4 * i + 1] += bv.y;
+              if (4 * i + 2 < P) raw[4 * i + 2] += bv.z;
+              if (4 * i + 3 < P) raw[4 * i + 3] += bv.w;
+            }
+            const int jb = X::at(row, 2 * u + a.tpar);
             gb[jb] = rqs_fwd_adjoint_fast<KB>(raw, xb[jb], gb[jb], a.gld, cfg, ov);
           } else {
+            const float* bb = a.bias + (int64_t)tcoord * P;
+#pragma unroll
+            for (int i = 0; i < P; ++i) raw[i] += __ldg(bb + i);
             const int64_t j = (int64_t)gm * a.d + 2 * tcoord + a.tpar;
             a.gxa[j] = rqs_fwd_adjoint_fast<KB>(raw, a.xa[j], a.gy[j], a.gld, cfg, ov);
           }
@@ -642,58 +760,53 @@ __global__ void __launch_bounds__(kSplThreads, 1)
           uint32_t w4[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) w4[k] = (uint32_t)ov[8 * j + 2 * k] | ((uint32_t)ov[8 * j + 2 * k + 1] << 16);
-          st_shared_v4(rb + (uint32_t)(draw_chunk<OCH>(row, j) * 16), w4[0], w4[1], w4[2], w4[3]);
+          st_shared_v4(rb + (uint32_t)(box_chunk<OCH>(row, j) * 16), w4[0], w4[1], w4[2], w4[3]);
+        }
+        // the staged box's generic writes, before the copy engine reads them;
+        // the box written next was stored at least one coordinate ago
+        fence_proxy_async_smem();
+        if (elect) bulk_wait_read_0();
+        quarters_sync(h);
+        if (elect) {
+          tma_store_2d(&tmR, smem_u32(stg + u * OBOX), tcoord * OPC, m0);
+          bulk_commit();
+        }
+        // column sums of d raw over the tile's rows (rows >= M were staged as
+        // zeros), while the store reads the same box: one column over row
+        // part `part`, in row order
+        for (int e = (q << 5) | lane; e < RP * P; e += 128) {
+          const int part = e / P, c = e - part * P;
+          const uint8_t* box = stg + u * OBOX;
+          const int jc = c >> 3, wofs = (c & 7) * 2;
+          float sum = 0.f;
+          const int r1 = (part + 1) * RROWS < BM ? (part + 1) * RROWS : BM;
+#pragma unroll 4
+          for (int r = part * RROWS; r < r1; ++r)
+            sum += __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t*>(
+                                       box + r * (OPC * 2) + box_chunk<OCH>(r, jc) * 16 + wofs)
+                                   << 16);
+          a.bpart[(int64_t)(mt * RP + part) * ntP + (int64_t)tcoord * P + c] = sum;
+        }
+        if (u == h && u + E >= nu) {
+          // the only coordinate of this tile: the next one is staged in the same box
+          if (elect) bulk_wait_read_0();
+          quarters_sync(h);
         }
       }
       release_acc(p, b, lane);
-      if (!xt && g == 0 && row_ok) {
+      if (xt) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&xdone[b]);
+      } else if (g == 0 && row_ok) {
         const int ncond = a.d - a.nt;
         for (int k = h; k < ncond; k += E) {
           const int64_t j = (int64_t)gm * a.d + 2 * k + a.cpar;
           a.gxa[j] = a.gy[j];
         }
       }
-      // the staged boxes' generic writes, before the copy engine reads them
-      fence_proxy_async_smem();
-      epi_sync(1);
-      if (elect) {
-        if (xt) tma_store_2d_f32(&tmGx, smem_u32(gb), 2 * g * DG, m0);
-        for (int u = 0; u < nu; ++u) tma_store_2d(&tmR, smem_u32(stg + u * OBOX), (g * DG + u) * OPC, m0);
-        bulk_commit();
-      }
-      // column sums of d raw over the tile's rows (rows >= M were staged as
-      // zeros), while the stores read the same boxes: thread e takes column
-      // pair cp = e % CP of the group's boxes over row part e / CP, in row order
-      if (et < RP * CP) {
-        const int cp = et % CP, part = et / CP;
-        const int u = cp / (OPC / 2), p2 = cp - u * (OPC / 2);
-        if (u < nu && 2 * p2 < P) {
-          const uint8_t* box = stg + u * OBOX;
-          const int j = (2 * p2) >> 3, wofs = ((2 * p2) & 7) * 2;
-          float s0 = 0.f, s1 = 0.f;
-          const int r1 = (part + 1) * RROWS < BM ? (part + 1) * RROWS : BM;
-#pragma unroll 4
-          for (int r = part * RROWS; r < r1; ++r) {
-            const uint32_t v =
-                *reinterpret_cast<const uint32_t*>(box + r * (OPC * 2) + draw_chunk<OCH>(r, j) * 16 + wofs);
-            s0 += __uint_as_float(v << 16);
-            s1 += __uint_as_float(v & 0xffff0000u);
-          }
-          float* dst = a.bpart + (int64_t)(mt * RP + part) * ntP + (int64_t)(g * DG + u) * P + 2 * p2;
-          dst[0] = s0;
-          if (2 * p2 + 1 < P) dst[1] = s1;
-        }
-      }
-      // the boxes are free again once the stores have read them
-      if (elect) bulk_wait_read_0();
-      epi_sync(2);
     }
-    if (elect) {
-      bulk_wait_all();   // the stores have completed before the CTA exits
-      // boxes loaded for tiles the loop did not finish (after an abort) land first (bounded)
-      if (xt)
-        for (int k = local; k < issued; ++k) mbar_wait(&xfull[k & 1], (uint32_t)(k >> 1) & 1u);
-    }
+    if (elect) bulk_wait_all();   // the stores have completed before the CTA exits
   }
   pipe_teardown(p, warp, lane, err);
 }
@@ -853,7 +966,7 @@ __device__ __forceinline__ void pipe_teardown_pair(const Pipe& p, int warp, int 
 }
 
 template <int KB, bool INV, int STAGES>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSplThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSplPairThreads, 1)
     k_tc_spline2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
                  int n_groups, int nt, int K, const float* __restrict__ bias, int bias_smem, float* __restrict__ xa,
                  int d, int tpar, float* __restrict__ ldp, SplineCfg cfg, int* err) {
@@ -989,7 +1102,8 @@ int ld_reduce_steps(cudaStream_t st, const float* ldp, const LdSteps& s, int64_t
 
 int tc_error_word(int** out);
 int make_tma_map_bf16(CUtensorMap* m, const void* base, int64_t inner, int64_t outer, int64_t ld, int box_outer);
-int make_tma_map_f32(CUtensorMap* m, const void* base, int64_t inner, int64_t outer, int box_inner, int box_outer);
+int make_tma_map_f32(CUtensorMap* m, const void* base, int64_t inner, int64_t outer, int box_inner, int box_outer,
+                     int swizzle = 0);
 int make_tma_map_bf16_box(CUtensorMap* m, const void* base, int64_t inner, int64_t outer, int64_t ld, int box_inner,
                           int box_outer, int swizzle);
 int make_tma_map_bf16_chunks(CUtensorMap* m, const void* base, int64_t inner, int64_t outer, int64_t ld,
@@ -1014,17 +1128,19 @@ static int launch_spl(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap&
   using T = tc::SplineTile<KB>;
   using S = tc::SplSmem<T::BN, STAGES, CH>;
   auto kern = tc::k_tc_spline<KB, INV, STAGES, CH>;
-  // the ring, its barriers, (when they fit) the layer's bias rows and the two
+  // the ring, its barriers, (when they fit) the layer's bias rows and the
   // x boxes (when x's row stride allows a tensor map)
   const size_t bias_bytes = (size_t)nt * tc::BiasRows<KB>::PP * sizeof(float);
-  // the two x boxes and the per-tile log-det partials of the quarter's warps
-  const size_t x_bytes = 128 + 2 * (size_t)tc::BM * 2 * T::DG * sizeof(float) +
-                         2 * (size_t)kSplineEpiPerQuarter * tc::BM * sizeof(float);
+  // the x boxes and the per-tile log-det partials of the quarter's warps
+  using X = tc::XBox<T::DG>;
+  const size_t x_bytes = tc::kXBufs * (size_t)X::BYTES + 2 * (size_t)kSplineEpiPerQuarter * tc::BM * sizeof(float);
   CUtensorMap mx;
   memset(&mx, 0, sizeof(mx));
-  int x_tma = make_tma_map_f32(&mx, xa, d, M, 2 * T::DG, tc::BM) == FMC_OK ? 1 : 0;
-  if (!x_tma) (void)cudaGetLastError();
-  if (x_tma && S::TOTAL + x_bytes > 227 * 1024) x_tma = 0;
+  int x_tma = 0;
+  if (X::kOk && S::TOTAL + x_bytes <= 227 * 1024) {
+    x_tma = make_tma_map_f32(&mx, xa, d, M, 2 * T::DG, tc::BM, X::SWIZZLE) == FMC_OK ? 1 : 0;
+    if (!x_tma) (void)cudaGetLastError();
+  }
   const size_t base_bytes = (size_t)S::TOTAL + (x_tma ? x_bytes : 0);
   const int bias_smem = base_bytes + bias_bytes <= 227 * 1024 ? 1 : 0;
   const size_t total = base_bytes + (bias_smem ? bias_bytes : 0);
@@ -1074,7 +1190,7 @@ static int launch_spl2(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap
   if (max_pairs == 0) {
     cudaLaunchConfig_t cfg_l = {};
     cfg_l.gridDim = dim3(2 * (unsigned)(sm_count() / 2), 1, 1);
-    cfg_l.blockDim = dim3(tc::kSplThreads, 1, 1);
+    cfg_l.blockDim = dim3(tc::kSplPairThreads, 1, 1);
     cfg_l.dynamicSmemBytes = total;
     int n = 0;
     FMC_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, (void*)kern, &cfg_l));
@@ -1086,7 +1202,7 @@ static int launch_spl2(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap
   const int64_t tiles = (M + 2 * tc::BM - 1) / (2 * tc::BM) * n_groups;
   const int64_t pairs = tiles < max_pairs ? tiles : max_pairs;
   note_grid(INV ? FMC_KT_TC_SPLINE_INV : FMC_KT_TC_SPLINE_FWD, (int)(2 * pairs), 2);
-  kern<<<(unsigned)(2 * pairs), tc::kSplThreads, total, st>>>(ma, mb, (int)M, n_groups, nt, K, bias, bias_smem, xa, d,
+  kern<<<(unsigned)(2 * pairs), tc::kSplPairThreads, total, st>>>(ma, mb, (int)M, n_groups, nt, K, bias, bias_smem, xa, d,
                                                              tpar, ldp, cfg, err);
   FMC_LAUNCH_CHECK();
   return FMC_OK;
@@ -1117,11 +1233,13 @@ static int launch_spl_bwd(cudaStream_t st, const CUtensorMap& ma, const CUtensor
   constexpr int STAGES = 3;
   using T = tc::SplineTile<KB>;
   using S = tc::SplSmem<T::BN, STAGES, 1>;
-  // ring, slack and barrier block (S::TOTAL), the rest of a 1024-byte block, the staging boxes
-  constexpr int TOTAL = S::TOTAL + 768 + T::STG_BYTES;
-  static_assert(TOTAL + 16 <= 227 * 1024, "fused spline adjoint: shared memory over the per-CTA limit");
-  // x and dL/dy boxes (two buffers each) when the row stride allows tensor maps and they fit
-  constexpr int BOXES = 128 + 4 * tc::BM * 2 * T::DG * (int)sizeof(float);
+  // ring, slack and barrier block (S::TOTAL), the staging boxes
+  constexpr int TOTAL = S::TOTAL + T::STG_BYTES;
+  static_assert(TOTAL <= 227 * 1024, "fused spline adjoint: shared memory over the per-CTA limit");
+  // x and dL/dy boxes (two buffers each) and the group's bias rows when the
+  // row stride allows tensor maps and they fit
+  using X = tc::XBox<T::DG>;
+  constexpr int BOXES = 4 * X::BYTES + 2 * T::DG * tc::BiasRows<KB>::PP * (int)sizeof(float);
   CUtensorMap mx, mgy, mgx;
   memset(&mx, 0, sizeof(mx));
   memset(&mgy, 0, sizeof(mgy));
@@ -1132,9 +1250,10 @@ static int launch_spl_bwd(cudaStream_t st, const CUtensorMap& ma, const CUtensor
   const int swz = och == 2 ? 32 : och == 4 ? 64 : 0;
   int rc = make_tma_map_bf16_box(&mr, graw, ldg, M, ldg, T::OPC, tc::BM, swz);
   if (rc) return rc;
-  int x_tma = TOTAL + BOXES + 16 <= 227 * 1024 && make_tma_map_f32(&mx, a.xa, a.d, M, 2 * T::DG, tc::BM) == FMC_OK &&
-              make_tma_map_f32(&mgy, a.gy, a.d, M, 2 * T::DG, tc::BM) == FMC_OK &&
-              make_tma_map_f32(&mgx, a.gxa, a.d, M, 2 * T::DG, tc::BM) == FMC_OK;
+  int x_tma = X::kOk && TOTAL + BOXES <= 227 * 1024 &&
+              make_tma_map_f32(&mx, a.xa, a.d, M, 2 * T::DG, tc::BM, X::SWIZZLE) == FMC_OK &&
+              make_tma_map_f32(&mgy, a.gy, a.d, M, 2 * T::DG, tc::BM, X::SWIZZLE) == FMC_OK &&
+              make_tma_map_f32(&mgx, a.gxa, a.d, M, 2 * T::DG, tc::BM, X::SWIZZLE) == FMC_OK;
   const int total = TOTAL + (x_tma ? BOXES : 0);
   auto kern = tc::k_tc_spline_bwd<KB, STAGES>;
   static int attr = 0;
