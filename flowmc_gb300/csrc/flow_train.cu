@@ -36,8 +36,26 @@ struct TrainWs {
   // BF16 path (tensor-core GEMMs): activations and gradients, row-major (the
   // weight-gradient GEMMs read them MN-major, so no transposed copies)
   uint16_t *cond16, *hs16, *graw16, *gz16[2];
+  bool keep;           // cond16 and hs16 hold every layer's block (layer stride cond_ls, hs_ls)
+  int64_t cond_ls, hs_ls;
   int64_t n128, n64, hld, ncld, pld;
 };
+
+// The BF16 forward's conditioning operands and hidden activations, kept for the
+// backward up to this many bytes of workspace (recomputed layer by layer in
+// one layer's buffers beyond). At 65,536 rows, 128 dims, 12 layers, two hidden
+// layers of 512 they are 1.7 GB and save 24 GEMMs and 12 affine passes.
+// Together with the folded affine of the kept forward: 12.18 -> 11.12 ms a step.
+constexpr int64_t kKeepBytes = (int64_t)16 << 30;
+
+// Input-gradient GEMMs from this depth on run on CTA pairs (half the weight
+// rows per CTA: the operands' way into the SM, 64 B/clock, limits one-CTA
+// tiles of 128 x 256). 65,536 x 512 outputs: 132 -> 121 us at a depth of
+// 2560; at 512 the pair's set-up and its epilogue cost more: 45 -> 52 us.
+// A pair per two SMs at least, or the larger tiles leave SMs idle.
+static bool dgrad_pairs(int64_t n, int in, int depth) {
+  return depth >= 1024 && n * in >= (int64_t)sm_count() * 128 * 256;
+}
 
 static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, TrainWs& w, size_t* total) {
   char* p = (char*)ws;
@@ -86,6 +104,7 @@ static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, Train
   }
   w.ldp = w.bpart = w.kpart = w.colpart = nullptr;
   w.kpart_floats = 0;
+  w.keep = false;
   w.cond16 = w.hs16 = w.graw16 = nullptr;
   w.gz16[0] = w.gz16[1] = nullptr;
   if (bf16) {
@@ -94,8 +113,11 @@ static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, Train
     w.hld = FlowGeom::rup(g.h_max(), 64);
     w.ncld = FlowGeom::rup(g.nc_max(), 64);
     w.pld = FlowGeom::rup((int64_t)g.nt_max() * g.spl_opc, 64);   // padded d-raw rows
-    w.cond16 = take16(w.n128 * w.ncld);
-    w.hs16 = take16((int64_t)g.nh * w.n128 * w.hld);
+    w.cond_ls = w.n128 * w.ncld;
+    w.hs_ls = (int64_t)g.nh * w.n128 * w.hld;
+    w.keep = 2 * g.L * (w.cond_ls + w.hs_ls) <= kKeepBytes;
+    w.cond16 = take16((w.keep ? g.L : 1) * w.cond_ls);
+    w.hs16 = take16((w.keep ? g.L : 1) * w.hs_ls);
     w.graw16 = take16(w.n128 * w.pld);
     for (int k = 0; k < 2; ++k) {
       w.gz16[k] = take16(w.n128 * w.hld);
@@ -264,10 +286,20 @@ static int recompute_mlp(const FmcFlow* f, const FlowGeom& g, int l, int64_t n, 
   return FMC_OK;
 }
 
-// BF16 recompute of layer l's conditioner hidden layers (from the bf16
-// conditioning block k_affine left in w.cond16): tanh activations in bf16;
-// the last Linear is recomputed inside the fused spline adjoint
-static int recompute_hidden_bf16(const FmcFlow* f, const FlowGeom& g, int l, int64_t n, TrainWs& w, cudaStream_t st) {
+// layer l's conditioning operand and hidden activations
+static TrainWs layer_ws(const TrainWs& w, int l) {
+  TrainWs r = w;
+  if (w.keep) {
+    r.cond16 += l * w.cond_ls;
+    r.hs16 += l * w.hs_ls;
+  }
+  return r;
+}
+
+// BF16 conditioner hidden layers of layer l (from the bf16 conditioning block
+// in w.cond16): tanh activations in bf16; the last Linear is inside the fused
+// spline and recomputed inside its adjoint
+static int hidden_bf16(const FmcFlow* f, const FlowGeom& g, int l, int64_t n, TrainWs& w, cudaStream_t st) {
   const float* th = f->theta + g.layer_off[l];
   int rc = FMC_OK;
   const uint16_t* a = w.cond16;
@@ -348,7 +380,7 @@ static int backward_mlp_bf16(const FmcFlow* f, const FlowGeom& g, int l, int64_t
         e1.ldpart = in;
       }
       if ((rc = tc_gemm(st, gcur, n, w.n128, kg, WT, in, g.w16t_rows(l, i), e1, w.gz16[nxt], ldo, ldo,
-                        tc::TC_EPI_DTANH_BF16, 0, false, ldcur)))
+                        tc::TC_EPI_DTANH_BF16, 0, dgrad_pairs(n, in, kg), ldcur)))
         return rc;
       gcur = w.gz16[nxt];
       ldcur = ldo;
@@ -406,19 +438,59 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     return flow_f32_grad(g, f->theta, f->aux, n, w.xs, w.f32, grad, st);
   }
 
-  // ---- forward, saving layer inputs
-  k_standardize<<<eb, 256, 0, st>>>(x, n, d, f->aux, w.xs);
+  // ---- forward, saving layer inputs: with `folded`, each layer's spline input
+  // (its ScalarAffine applied by the layer before) and conditioning operand
+  const bool keep = bf16 && w.keep;
+  const bool folded = keep && 2 * g.nt(0) == d && tc_spline_boxes(g, f);
+  if (keep && n < 64) {
+    // the weight-gradient GEMMs read 64-row blocks of the bf16 operands: rows
+    // [n, 64) stay zero (the kernels below write rows < n only)
+    FMC_CUDA_TRY(cudaMemsetAsync(w.cond16, 0, (size_t)(g.L * w.cond_ls) * 2, st));
+    if (g.nh > 0) FMC_CUDA_TRY(cudaMemsetAsync(w.hs16, 0, (size_t)(g.L * w.hs_ls) * 2, st));
+  } else if (folded && g.nc(0) < w.ncld && g.L > 1) {
+    // padding columns: the splines write the conditioning ones only
+    FMC_CUDA_TRY(cudaMemsetAsync(w.cond16 + w.cond_ls, 0, (size_t)((g.L - 1) * w.cond_ls) * 2, st));
+  }
+  k_standardize<<<eb, 256, 0, st>>>(x, n, d, f->aux, folded ? w.xs + nd : w.xs);
   FMC_LAUNCH_CHECK();
-  for (int l = 0; l < g.L; ++l) {
+  if (folded) {
+    k_affine<<<rb, 256, 0, st>>>(w.xs + nd, w.xs, nullptr, w.cond16, g.w16_cols(0, 0), n, d, g.nc(0), g.cpar(0),
+                                 f->theta + g.layer_off[0], 0, w.ld, 1);
+    FMC_LAUNCH_CHECK();
+    for (int l = 0; l < g.L; ++l) {
+      TrainWs wl = layer_ws(w, l);
+      if ((rc = hidden_bf16(f, g, l, n, wl, st))) return rc;
+      const uint16_t* h_last = g.nh > 0 ? wl.hs16 + (int64_t)(g.nh - 1) * w.n128 * w.hld : wl.cond16;
+      SplineFold fold{};
+      const bool next = l + 1 < g.L;
+      if (next) {
+        fold.th_next = f->theta + g.layer_off[l + 1];
+        fold.cond16 = wl.cond16 + w.cond_ls;
+        fold.ldc16 = g.w16_cols(l + 1, 0);
+      }
+      bool done = false;
+      if ((rc = tc_linear_spline(st, g, f, l, h_last, n, w.n128, false, w.xs + (int64_t)l * nd, w.ld, w.ldp,
+                                 next ? &fold : nullptr, &done, nullptr, w.xs + (int64_t)(l + 1) * nd)))
+        return rc;
+      FMC_CHECK_ARG(done == next, "the spline kernel left out the next layer's affine");
+    }
+  }
+  for (int l = 0; l < g.L && !folded; ++l) {
     float* xin = w.xs + (int64_t)l * nd;
     float* xout = w.xs + (int64_t)(l + 1) * nd;
-    k_affine<<<rb, 256, 0, st>>>(xin, xout, bf16 ? nullptr : w.cond, bf16 ? w.cond16 : nullptr, g.w16_cols(l, 0),
-                                 n, d, g.nc(l), g.cpar(l), f->theta + g.layer_off[l], 0, w.ld, l == 0 ? 1 : 0);
+    k_affine<<<rb, 256, 0, st>>>(xin, xout, bf16 ? nullptr : w.cond,
+                                 bf16 ? layer_ws(w, l).cond16 : nullptr, g.w16_cols(l, 0), n, d, g.nc(l), g.cpar(l), f->theta + g.layer_off[l], 0, w.ld, l == 0 ? 1 : 0);
     FMC_LAUNCH_CHECK();
     if (bf16) {
       // the inference path: hidden layers, then the last Linear fused with the spline
       const uint16_t* h_last = nullptr;
-      if ((rc = conditioner_bf16_hidden(f, g, l, n, nullptr, w.cond16, w.gz16[0], w.gz16[1], &h_last, st))) return rc;
+      if (keep) {
+        TrainWs wl = layer_ws(w, l);
+        if ((rc = hidden_bf16(f, g, l, n, wl, st))) return rc;
+        h_last = g.nh > 0 ? wl.hs16 + (int64_t)(g.nh - 1) * w.n128 * w.hld : wl.cond16;
+      } else if ((rc = conditioner_bf16_hidden(f, g, l, n, nullptr, w.cond16, w.gz16[0], w.gz16[1], &h_last, st))) {
+        return rc;
+      }
       if ((rc = tc_linear_spline(st, g, f, l, h_last, n, w.n128, false, xout, w.ld, w.ldp))) return rc;
     } else {
       if ((rc = recompute_mlp(f, g, l, n, w, st))) return rc;
@@ -439,11 +511,12 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
   const float inv_n = 1.0f / (float)n;
   const float gld = -inv_n;
   if (bf16 && n < 64) {
-    // the weight-gradient GEMMs read 64-row blocks of the bf16 operands: rows
-    // [n, 64) stay zero (the kernels below write rows < n only)
-    FMC_CUDA_TRY(cudaMemsetAsync(w.cond16, 0, (size_t)64 * w.ncld * 2, st));
-    for (int i = 0; i < g.nh; ++i)
-      FMC_CUDA_TRY(cudaMemsetAsync(w.hs16 + (int64_t)i * w.n128 * w.hld, 0, (size_t)64 * w.hld * 2, st));
+    // as above, for the operands that the backward writes
+    if (!keep) {
+      FMC_CUDA_TRY(cudaMemsetAsync(w.cond16, 0, (size_t)64 * w.ncld * 2, st));
+      for (int i = 0; i < g.nh; ++i)
+        FMC_CUDA_TRY(cudaMemsetAsync(w.hs16 + (int64_t)i * w.n128 * w.hld, 0, (size_t)64 * w.hld * 2, st));
+    }
     FMC_CUDA_TRY(cudaMemsetAsync(w.graw16, 0, (size_t)64 * w.pld * 2, st));
     for (int k = 0; k < 2; ++k) FMC_CUDA_TRY(cudaMemsetAsync(w.gz16[k], 0, (size_t)64 * w.hld * 2, st));
   }
@@ -453,24 +526,28 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     const float* th = f->theta + g.layer_off[l];
     float* gl = grad + g.layer_off[l];
     const float* xin = w.xs + (int64_t)l * nd;
-    // the layer's spline input, and its conditioning block as the first
-    // GEMM's operand (bf16, zero padded) or in fp32
-    k_affine<<<rb, 256, 0, st>>>(xin, w.xa, bf16 ? nullptr : w.cond, bf16 ? w.cond16 : nullptr,
-                                 bf16 ? g.w16_cols(l, 0) : 0, n, d, g.nc(l), g.cpar(l), th, 0, nullptr, 0);
-    FMC_LAUNCH_CHECK();
+    const float* xa = folded ? xin : w.xa;
+    if (!folded) {
+      // the layer's spline input, and (unless kept) its conditioning block as
+      // the first GEMM's operand (bf16, zero padded) or in fp32
+      k_affine<<<rb, 256, 0, st>>>(xin, w.xa, bf16 ? nullptr : w.cond, bf16 && !keep ? w.cond16 : nullptr,
+                                   bf16 ? g.w16_cols(l, 0) : 0, n, d, g.nc(l), g.cpar(l), th, 0, nullptr, 0);
+      FMC_LAUNCH_CHECK();
+    }
     if (bf16) {
       // hidden activations, then the last Linear recomputed inside the fused
       // spline adjoint, which leaves d raw in the padded bf16 layout
-      if ((rc = recompute_hidden_bf16(f, g, l, n, w, st))) return rc;
-      const uint16_t* h_last = g.nh > 0 ? w.hs16 + (int64_t)(g.nh - 1) * w.n128 * w.hld : w.cond16;
-      if ((rc = tc_linear_spline_bwd(st, g, f, l, h_last, n, w.n128, w.xa, w.gy, gld, w.gxa, w.graw16, w.pld,
+      TrainWs wl = layer_ws(w, l);
+      if (!keep && (rc = hidden_bf16(f, g, l, n, wl, st))) return rc;
+      const uint16_t* h_last = g.nh > 0 ? wl.hs16 + (int64_t)(g.nh - 1) * w.n128 * w.hld : wl.cond16;
+      if ((rc = tc_linear_spline_bwd(st, g, f, l, h_last, n, w.n128, xa, w.gy, gld, w.gxa, w.graw16, w.pld,
                                      w.bpart)))
         return rc;
       const int ntP = g.lin_out(l, g.nh);
       k_colsum_rows<<<(ntP + 31) / 32, 1024, 0, st>>>(w.bpart, (int)(w.n128 / 128) * kSplineBwdRowParts, ntP,
                                                     gl + g.lin_b(l, g.nh));
       FMC_LAUNCH_CHECK();
-      if ((rc = backward_mlp_bf16(f, g, l, n, w, gl, st))) return rc;
+      if ((rc = backward_mlp_bf16(f, g, l, n, wl, gl, st))) return rc;
     } else {
       if ((rc = recompute_mlp(f, g, l, n, w, st))) return rc;
       if ((rc = launch_spline_bwd(g.K, st, w.raw, w.xa, w.gy, gld, w.graw, w.gxa, n, d, g.nt(l), g.tpar(l), g.cpar(l),
@@ -501,7 +578,7 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     }
     // ScalarAffine adjoint -> d(layer input) into gy
     const int ab = affine_sum_blocks(n, d);
-    k_affine_bwd<<<ab, 256, 0, st>>>(w.gxa, w.gcond, w.xa, n, d, g.nc(l), g.cpar(l), th, w.gy, w.part);
+    k_affine_bwd<<<ab, 256, 0, st>>>(w.gxa, w.gcond, xa, n, d, g.nc(l), g.cpar(l), th, w.gy, w.part);
     FMC_LAUNCH_CHECK();
     k_affine_param_grad<<<1, 32, 0, st>>>(w.part, ab, gld * (float)d * (float)n, gl);
     FMC_LAUNCH_CHECK();

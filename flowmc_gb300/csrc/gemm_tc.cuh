@@ -59,11 +59,15 @@ struct SplineFold {
 // then added to ld. With fold, *folded says whether the kernel applied the
 // next layer's affine (and added its log-determinant to ld after this
 // layer's): only the x-box path does; otherwise the caller applies it.
+// xo: write the spline's output there and leave xa as it is (where
+// tc_spline_boxes says that x moves in boxes).
 // With ld == nullptr the partials stay in ldp for the caller to add later
 // (ld_reduce_steps); *parts_out gets their count.
 int tc_linear_spline(cudaStream_t st, const FlowGeom& g, const FmcFlow* f, int l, const uint16_t* A, int64_t M,
                      int64_t rows_a, bool inverse, float* xa, float* ld, float* ldp,
-                     const SplineFold* fold = nullptr, bool* folded = nullptr, int* parts_out = nullptr);
+                     const SplineFold* fold = nullptr, bool* folded = nullptr, int* parts_out = nullptr,
+                     float* xo = nullptr);
+bool tc_spline_boxes(const FlowGeom& g, const FmcFlow* f);
 
 // The log-det partials of up to kLdMaxSteps consecutive fused spline launches
 // of one flow pass, left in place and added to ld by one launch: step k's

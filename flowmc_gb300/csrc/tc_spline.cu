@@ -350,7 +350,8 @@ struct XBox {
 // conditioning ones between them -- is one TMA box of the fp32 tensor map
 // tmX over x [M, d]. The box warp (the CTA's last) keeps kXBufs boxes in
 // turn: it loads tile i + 2's box while tile i + 1 is computed, and once the
-// epilogue warps have written y into tile i's box it stores the box back,
+// epilogue warps have written y into tile i's box it stores the box back
+// (tmXo: x itself, or another [M, d] buffer where x is to be kept),
 // adds the rows' log-det partials and writes the next layer's operand. So no
 // epilogue warp waits for a store, a load it could have had earlier, or the
 // other epilogue warps. Every tile owns its rows' column span alone, so the
@@ -377,8 +378,8 @@ constexpr int kXBufs = 3;
 template <int KB, bool INV, int STAGES, int CH>
 __global__ void __launch_bounds__(kSplThreads, 1)
     k_tc_spline(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                const __grid_constant__ CUtensorMap tmX, int x_tma, int M, int n_groups, int nt, int K,
-                const float* __restrict__ bias, int bias_smem, float* __restrict__ xa, int d, int tpar,
+                const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmXo, int x_tma, int M,
+                int n_groups, int nt, int K, const float* __restrict__ bias, int bias_smem, float* __restrict__ xa, int d, int tpar,
                 float* __restrict__ ldp, SplineCfg cfg, const float* __restrict__ fold_th,
                 uint16_t* __restrict__ cond16, int ldc16, int* err) {
   using T = SplineTile<KB>;
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(kSplThreads, 1)
           break;
         }
         if (lane == 0) {
-          tma_store_2d_f32(&tmX, smem_u32(xb), 2 * g * DG, m0);   // rows past M are clipped
+          tma_store_2d_f32(&tmXo, smem_u32(xb), 2 * g * DG, m0);   // rows past M are clipped
           bulk_commit();
         }
         // the quarter's E log-det partials of a row, in order: one partial
@@ -1120,10 +1121,22 @@ int spline_groups(int K_bins, int nt, int* dg, int* bn) {
 // CH K chunks per ring stage: 4 one-chunk stages, or 2 two-chunk stages
 // (3-D operand maps; half the TMA operations per tile, measured 3-4 % faster
 // on GB300 at 512 hidden units)
+// shared memory the x boxes and the per-tile log-det partials of the quarter's
+// warps take beside a ring of that kind, and whether there is room for them
+template <int KB, int CH>
+struct SplBoxes {
+  static constexpr int STAGES = CH == 1 ? 4 : 2;
+  using T = tc::SplineTile<KB>;
+  using X = tc::XBox<T::DG>;
+  static constexpr size_t BYTES =
+      tc::kXBufs * (size_t)X::BYTES + 2 * (size_t)kSplineEpiPerQuarter * tc::BM * sizeof(float);
+  static constexpr bool kOk = X::kOk && tc::SplSmem<T::BN, STAGES, CH>::TOTAL + BYTES <= 227 * 1024;
+};
+
 template <int KB, bool INV, int CH>
 static int launch_spl(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb, int64_t M, int n_groups, int nt,
-                      int K, const float* bias, float* xa, int d, int tpar, float* ldp, SplineCfg cfg, int* parts,
-                      const SplineFold* fold, bool* folded) {
+                      int K, const float* bias, float* xa, float* xo, int d, int tpar, float* ldp, SplineCfg cfg,
+                      int* parts, const SplineFold* fold, bool* folded) {
   constexpr int STAGES = CH == 1 ? 4 : 2;
   using T = tc::SplineTile<KB>;
   using S = tc::SplSmem<T::BN, STAGES, CH>;
@@ -1131,15 +1144,20 @@ static int launch_spl(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap&
   // the ring, its barriers, (when they fit) the layer's bias rows and the
   // x boxes (when x's row stride allows a tensor map)
   const size_t bias_bytes = (size_t)nt * tc::BiasRows<KB>::PP * sizeof(float);
-  // the x boxes and the per-tile log-det partials of the quarter's warps
-  using X = tc::XBox<T::DG>;
-  const size_t x_bytes = tc::kXBufs * (size_t)X::BYTES + 2 * (size_t)kSplineEpiPerQuarter * tc::BM * sizeof(float);
-  CUtensorMap mx;
+  using B = SplBoxes<KB, CH>;
+  constexpr size_t x_bytes = B::BYTES;
+  CUtensorMap mx, mxo;
   memset(&mx, 0, sizeof(mx));
   int x_tma = 0;
-  if (X::kOk && S::TOTAL + x_bytes <= 227 * 1024) {
-    x_tma = make_tma_map_f32(&mx, xa, d, M, 2 * T::DG, tc::BM, X::SWIZZLE) == FMC_OK ? 1 : 0;
+  if (B::kOk) {
+    x_tma = make_tma_map_f32(&mx, xa, d, M, 2 * T::DG, tc::BM, B::X::SWIZZLE) == FMC_OK ? 1 : 0;
     if (!x_tma) (void)cudaGetLastError();
+  }
+  mxo = mx;
+  if (xo != nullptr) {
+    FMC_CHECK_ARG(x_tma, "spline output apart from its input needs the x boxes");
+    const int rc = make_tma_map_f32(&mxo, xo, d, M, 2 * T::DG, tc::BM, B::X::SWIZZLE);
+    if (rc) return rc;
   }
   const size_t base_bytes = (size_t)S::TOTAL + (x_tma ? x_bytes : 0);
   const int bias_smem = base_bytes + bias_bytes <= 227 * 1024 ? 1 : 0;
@@ -1157,8 +1175,8 @@ static int launch_spl(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap&
   note_grid(INV ? FMC_KT_TC_SPLINE_INV : FMC_KT_TC_SPLINE_FWD, (int)grid, 1);
   // the next layer's affine rides on the x boxes only
   const bool fo = fold != nullptr && x_tma;
-  kern<<<(unsigned)grid, tc::kSplThreads, total, st>>>(ma, mb, mx, x_tma, (int)M, n_groups, nt, K, bias, bias_smem,
-                                                       xa, d, tpar, ldp, cfg, fo ? fold->th_next : nullptr,
+  kern<<<(unsigned)grid, tc::kSplThreads, total, st>>>(ma, mb, mx, mxo, x_tma, (int)M, n_groups, nt, K, bias,
+                                                       bias_smem, xa, d, tpar, ldp, cfg, fo ? fold->th_next : nullptr,
                                                        fo ? fold->cond16 : nullptr, fo ? fold->ldc16 : 0, err);
   FMC_LAUNCH_CHECK();
   *parts = x_tma ? n_groups : kSplineEpiPerQuarter * n_groups;
@@ -1213,18 +1231,21 @@ static int launch_spl2(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap
 // pair kernel exists only for those widths)
 template <int KB, bool INV>
 static int launch_spl_tiles(bool pair, bool wide, cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb,
-                            int64_t M, int n_groups, int nt, int K, const float* bias, float* xa, int d, int tpar,
-                            float* ldp, SplineCfg cfg, int* parts, const SplineFold* fold, bool* folded) {
+                            int64_t M, int n_groups, int nt, int K, const float* bias, float* xa, float* xo, int d,
+                            int tpar, float* ldp, SplineCfg cfg, int* parts, const SplineFold* fold, bool* folded) {
   *folded = false;
   if constexpr (tc::SplineTile<KB>::BN % 32 == 0) {
     if (pair) {
+      FMC_CHECK_ARG(xo == nullptr, "spline output apart from its input needs the x boxes");
       *parts = kSplineEpiPerQuarter * n_groups;
       return launch_spl2<KB, INV>(st, ma, mb, M, n_groups, nt, K, bias, xa, d, tpar, ldp, cfg);
     }
   }
   if (wide)
-    return launch_spl<KB, INV, 2>(st, ma, mb, M, n_groups, nt, K, bias, xa, d, tpar, ldp, cfg, parts, fold, folded);
-  return launch_spl<KB, INV, 1>(st, ma, mb, M, n_groups, nt, K, bias, xa, d, tpar, ldp, cfg, parts, fold, folded);
+    return launch_spl<KB, INV, 2>(st, ma, mb, M, n_groups, nt, K, bias, xa, xo, d, tpar, ldp, cfg, parts, fold,
+                                 folded);
+  return launch_spl<KB, INV, 1>(st, ma, mb, M, n_groups, nt, K, bias, xa, xo, d, tpar, ldp, cfg, parts, fold,
+                                 folded);
 }
 
 template <int KB>
@@ -1274,12 +1295,26 @@ static int launch_spl_bwd(cudaStream_t st, const CUtensorMap& ma, const CUtensor
 
 #define FMC_SPLINE_BINS(X) X(2) X(3) X(4) X(5) X(6) X(8) X(10) X(12) X(16)
 
+// Whether tc_linear_spline moves x in boxes (every layer: n_dim even), and so
+// takes SplineFold and an output buffer apart from its input
+bool tc_spline_boxes(const FlowGeom& g, const FmcFlow* f) {
+  int dg, bn;
+  spline_groups(g.K, g.nt_max(), &dg, &bn);
+  if (g.d % 4 != 0 || g.d < 2 * dg || (f->tile_rows == 256 && bn % 32 == 0)) return false;
+  const bool wide = g.w16_cols(0, g.nh) % (2 * tc::BK) == 0;
+#define SPL_CASE(k) \
+  if (g.K == k) return wide ? SplBoxes<k, 2>::kOk : SplBoxes<k, 1>::kOk;
+  FMC_SPLINE_BINS(SPL_CASE)
+#undef SPL_CASE
+  return false;
+}
+
 // The last Linear of layer l fused with its spline: A = the last tanh
 // activation (bf16 [rows_a, K]), Bg = the grouped weights, xa updated in place,
 // ld[r] accumulated.
 int tc_linear_spline(cudaStream_t st, const FlowGeom& g, const FmcFlow* f, int l, const uint16_t* A, int64_t M,
                      int64_t rows_a, bool inverse, float* xa, float* ld, float* ldp, const SplineFold* fold,
-                     bool* folded, int* parts_out) {
+                     bool* folded, int* parts_out, float* xo) {
   bool fo = false;
   if (folded) *folded = false;
   // the fold pairs every conditioning coordinate with a transformed one
@@ -1317,9 +1352,9 @@ int tc_linear_spline(cudaStream_t st, const FlowGeom& g, const FmcFlow* f, int l
 #define SPL_CASE(k)                                                                                          \
   if (g.K == k) {                                                                                            \
     rc = inverse                                                                                             \
-             ? launch_spl_tiles<k, true>(pair, wide, st, ma, mb, M, n_groups, nt, Kd, bias, xa, g.d, g.tpar(l),  \
+             ? launch_spl_tiles<k, true>(pair, wide, st, ma, mb, M, n_groups, nt, Kd, bias, xa, xo, g.d, g.tpar(l),  \
                                          ldp, g.cfg, &parts, fold, &fo)                                            \
-             : launch_spl_tiles<k, false>(pair, wide, st, ma, mb, M, n_groups, nt, Kd, bias, xa, g.d, g.tpar(l), \
+             : launch_spl_tiles<k, false>(pair, wide, st, ma, mb, M, n_groups, nt, Kd, bias, xa, xo, g.d, g.tpar(l), \
                                           ldp, g.cfg, &parts, fold, &fo);                                          \
   } else
     FMC_SPLINE_BINS(SPL_CASE) {
