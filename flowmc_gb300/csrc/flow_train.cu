@@ -168,25 +168,44 @@ __global__ void k_colsum_final(const float* __restrict__ part, int rb, int m, fl
 }
 
 // out[j] = sum over rows of part[r * m + j] for a tall partial matrix: a
-// block takes 32 columns, its 32 warps rows w, w + 32, ... (coalesced
-// 128-byte loads), then the 32 per-warp sums are added in warp order
-__global__ void __launch_bounds__(1024) k_colsum_rows(const float* __restrict__ part, int rows, int m,
-                                                      float* __restrict__ out) {
-  __shared__ float sh[32][33];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int j = blockIdx.x * 32 + lane;
+// block takes kRowsCols columns, thread (w, column) of it rows w, w + 32, ...,
+// then the 32 sums of a column are added in order of w. Few rows per thread
+// and few columns altogether: what counts is loads in flight, so eight columns
+// (one 32-byte sector) to a block, four times the blocks of whole 128-byte
+// lines, and sixteen loads ahead. Three sums of a
+// layer, 2 x (2048 x 512) and 1536 x 2368: 31 -> 19 us.
+constexpr int kRowsCols = 8;
+__global__ void __launch_bounds__(32 * kRowsCols) k_colsum_rows(const float* __restrict__ part, int rows, int m,
+                                                                float* __restrict__ out) {
+  __shared__ float sh[32][kRowsCols + 1];
+  const int c = threadIdx.x % kRowsCols, w = threadIdx.x / kRowsCols;
+  const int j = blockIdx.x * kRowsCols + c;
   float s = 0.f;
-  if (j < m)
-#pragma unroll 4
-    for (int r = w; r < rows; r += 32) s += part[(int64_t)r * m + j];
-  sh[w][lane] = s;
+  if (j < m) {
+    int r = w;
+    for (; r + 15 * 32 < rows; r += 16 * 32) {
+      float v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = part[(int64_t)(r + 32 * k) * m + j];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) s += v[k];
+    }
+    for (; r < rows; r += 32) s += part[(int64_t)r * m + j];
+  }
+  sh[w][c] = s;
   __syncthreads();
-  if (w == 0 && j < m) {
+  if (threadIdx.x < kRowsCols && j < m) {
     float t = 0.f;
 #pragma unroll
-    for (int k = 0; k < 32; ++k) t += sh[k][lane];
+    for (int k = 0; k < 32; ++k) t += sh[k][c];
     out[j] = t;
   }
+}
+
+static int colsum_rows(cudaStream_t st, const float* part, int64_t rows, int m, float* out) {
+  k_colsum_rows<<<(m + kRowsCols - 1) / kRowsCols, 32 * kRowsCols, 0, st>>>(part, (int)rows, m, out);
+  FMC_LAUNCH_CHECK();
+  return FMC_OK;
 }
 
 static int colsum(cudaStream_t st, const float* gm, int64_t n, int m, float* part, float* out) {
@@ -242,19 +261,26 @@ __global__ void k_init_gy(const float* __restrict__ y, int64_t tot, int d, const
 
 // adjoint of xa = (x + t) e^s and of the conditioning gather;
 // writes d x and per-block partial sums of d t and (sum gxa * xa). One warp
-// per row (lanes over the coordinates), rows strided over the grid.
+// per row (lanes over the coordinates), rows strided over the grid; a
+// row's 128 coordinates are loaded before any is used. Memory bound, 117 MB
+// at 65,536 x 128: 34 -> 26 us (two rows ahead: 41 us, too few warps).
 __global__ void __launch_bounds__(256) k_affine_bwd(const float* __restrict__ gxa, const float* __restrict__ gcond,
                                                     const float* __restrict__ xa, int64_t n, int d, int nc, int cpar,
                                                     const float* __restrict__ th_layer, float* __restrict__ gx,
                                                     float* __restrict__ part) {
   const float es = expf(th_layer[0]);
-  affine_sums(n, d, part, [&](int64_t r, int j, float& g, float& x, float& gv) {
-    g = gxa[r * d + j];
-    if ((j & 1) == cpar) g += gcond[r * nc + (j >> 1)];
-    x = xa[r * d + j];
-    gv = g * es;
-    gx[r * d + j] = gv;
-  });
+  affine_sums_ahead(
+      n, d, part,
+      [&](int64_t r, int j, float& g, float& x) {
+        g = gxa[r * d + j];
+        if ((j & 1) == cpar) g += gcond[r * nc + (j >> 1)];
+        x = xa[r * d + j];
+      },
+      [&](int64_t r, int j, float g) {
+        const float gv = g * es;
+        gx[r * d + j] = gv;
+        return gv;
+      });
 }
 
 __global__ void k_affine_param_grad(const float* __restrict__ part, int nb, float ld_term, float* __restrict__ g_layer) {
@@ -361,8 +387,7 @@ static int backward_mlp_bf16(const FmcFlow* f, const FlowGeom& g, int l, int64_t
     if (i < g.nh) {
       if (have_cp) {
         // fixed-order reduction of the per-32-row partials the DTANH GEMM left
-        k_colsum_rows<<<(out + 31) / 32, 1024, 0, st>>>(w.colpart, (int)(w.n128 / 32), out, gl + g.lin_b(l, i));
-        FMC_LAUNCH_CHECK();
+        if ((rc = colsum_rows(st, w.colpart, w.n128 / 32, out, gl + g.lin_b(l, i)))) return rc;
       } else if ((rc = colsum_bf16(st, gcur, n, out, FlowGeom::rup(out, 64), w.part, gl + g.lin_b(l, i)))) {
         return rc;
       }
@@ -544,9 +569,7 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
                                      w.bpart)))
         return rc;
       const int ntP = g.lin_out(l, g.nh);
-      k_colsum_rows<<<(ntP + 31) / 32, 1024, 0, st>>>(w.bpart, (int)(w.n128 / 128) * kSplineBwdRowParts, ntP,
-                                                    gl + g.lin_b(l, g.nh));
-      FMC_LAUNCH_CHECK();
+      if ((rc = colsum_rows(st, w.bpart, w.n128 / 128 * kSplineBwdRowParts, ntP, gl + g.lin_b(l, g.nh)))) return rc;
       if ((rc = backward_mlp_bf16(f, g, l, n, wl, gl, st))) return rc;
     } else {
       if ((rc = recompute_mlp(f, g, l, n, w, st))) return rc;

@@ -61,6 +61,37 @@ __device__ __forceinline__ void affine_sums(int64_t n, int d, float* part, F get
   }
 }
 
+// affine_sums with the loads of a row's four coordinates per lane issued
+// ahead of their use: load(r, j, g, x), then gv = use(r, j, g), in the same order
+template <typename L, typename U>
+__device__ __forceinline__ void affine_sums_ahead(int64_t n, int d, float* part, L load, U use) {
+  __shared__ float sh[32];
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  float st = 0.f, ss = 0.f;
+  auto add = [&](int64_t r, int j, float g, float x) {
+    st += use(r, j, g);
+    ss += g * x;
+  };
+  int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  for (; r < n; r += warps)
+    for (int j0 = lane; j0 < d; j0 += 128) {
+      float g[4], x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (j0 + 32 * k < d) load(r, j0 + 32 * k, g[k], x[k]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (j0 + 32 * k < d) add(r, j0 + 32 * k, g[k], x[k]);
+    }
+  st = block_sum<256>(st, sh);
+  ss = block_sum<256>(ss, sh);
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = st;
+    part[2 * blockIdx.x + 1] = ss;
+  }
+}
+
 // the ScalarAffine's two gradients from the nb block partials: one warp,
 // lane i summing partials i, i + 32, ..., then a fixed-order butterfly
 __device__ __forceinline__ void affine_param_grad(const float* __restrict__ part, int nb, float ld_term,
