@@ -192,6 +192,24 @@ size_t splitk_scratch_floats(int64_t M, int N, int K, int kslices) {
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N : 0;
 }
 
+// K slices of an M x n_store product (fp32 output with scratch for them only)
+template <int BN, int EPI>
+static int gemm_splits(int64_t M, int K, const tc::EpiArgs& ep, int64_t ldc, int n_store) {
+  if (EPI != tc::TC_EPI_F32 || ep.kpart == nullptr) return 1;
+  const int splits = splitk_count((M + tc::BM - 1) / tc::BM * ((n_store + BN - 1) / BN), K, ep.kslices);
+  return (int64_t)splits * M * ldc > ep.kpart_floats ? 1 : splits;
+}
+
+static int splitk_finish(cudaStream_t st, int splits, int64_t M, const tc::EpiArgs& ep, void* C, int64_t ldc,
+                         int n_store) {
+  int64_t blocks = (M * n_store + 255) / 256;
+  if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
+  k_splitk_reduce<<<(int)blocks, 256, 0, st>>>(ep.kpart, splits, M * ldc, M, n_store, ldc, (float*)C, ep.rmap_grp,
+                                              ep.rmap_keep);
+  FMC_LAUNCH_CHECK();
+  return FMC_OK;
+}
+
 template <int BN, int STAGES, int EPI, bool TSTORE, int NSTG = 2, int OPM = 0>
 static int launch_tc(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, int64_t M,
                      int N, int K, const tc::EpiArgs& ep, void* C, int64_t ldc, int n_store) {
@@ -211,11 +229,7 @@ static int launch_tc(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& 
   const int64_t mt = (M + tc::BM - 1) / tc::BM;
   const int64_t tiles = mt * ((n_store + BN - 1) / BN);
   FMC_CHECK_SUPPORTED(tiles < (1ll << 26) && M < (1ll << 31), "GEMM too large (%lld tiles)", (long long)tiles);
-  int splits = 1;
-  if (EPI == tc::TC_EPI_F32 && ep.kpart != nullptr) {
-    splits = splitk_count(tiles, K, ep.kslices);
-    if ((int64_t)splits * M * ldc > ep.kpart_floats) splits = 1;
-  }
+  const int splits = gemm_splits<BN, EPI>(M, K, ep, ldc, n_store);
   const int64_t items = tiles * splits;
   const int64_t grid = items < sm_count() ? items : sm_count();   // persistent: one CTA per SM
   void* out = splits > 1 ? (void*)ep.kpart : C;
@@ -233,25 +247,20 @@ static int launch_tc(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& 
                                                      M * ldc, err);
     FMC_LAUNCH_CHECK();
   }
-  if (splits > 1) {
-    int64_t blocks = (M * n_store + 255) / 256;
-    if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-    k_splitk_reduce<<<(int)blocks, 256, 0, st>>>(ep.kpart, splits, M * ldc, M, n_store, ldc, (float*)C, ep.rmap_grp,
-                                                ep.rmap_keep);
-    FMC_LAUNCH_CHECK();
-  }
-  return FMC_OK;
+  return splits > 1 ? splitk_finish(st, splits, M, ep, C, ldc, n_store) : FMC_OK;
 }
 
-// the CTA-pair form (bf16 outputs through TMA stores): 256-row tiles, a
-// persistent grid of as many clusters of 2 as can be resident
-template <int BN, int STAGES, int EPI, int NSTG = 2>
+// the CTA-pair form (bf16 outputs through TMA stores, or fp32 ones): 256-row
+// tiles, a persistent grid of as many clusters of 2 as can be resident; the
+// K slices are those of the one-CTA form (the same partial sums)
+template <int BN, int STAGES, int EPI, int NSTG = 2, int OPM = 0>
 static int launch_tc_pair(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc,
                           int64_t M, int N, int K, const tc::EpiArgs& ep, void* C, int64_t ldc, int n_store) {
   using S = tc::Smem<BN / 2, STAGES>;
-  constexpr int TOTAL = S::TOTAL + 768 + tc::staging_bytes(NSTG);
+  constexpr bool TSTORE = EPI == tc::TC_EPI_TANH_BF16 || EPI == tc::TC_EPI_DTANH_BF16;
+  constexpr int TOTAL = TSTORE ? S::TOTAL + 768 + tc::staging_bytes(NSTG) : S::TOTAL;
   static_assert(TOTAL + (NSTG == 2 ? 1024 : 0) + 16 <= 227 * 1024, "tcgen05 GEMM: shared memory over the per-CTA limit");
-  auto kern = tc::k_tc_gemm<BN, STAGES, EPI, true, true, NSTG>;
+  auto kern = tc::k_tc_gemm<BN, STAGES, EPI, TSTORE, true, NSTG, OPM>;
   static bool attr_set = false;
   if (!attr_set) {
     FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TOTAL));
@@ -279,18 +288,25 @@ static int launch_tc_pair(cudaStream_t st, const CUtensorMap& ma, const CUtensor
   FMC_CUDA_TRY(cudaGetSymbolAddress((void**)&err, g_tc_error));
   const int64_t tiles = (M + 2 * tc::BM - 1) / (2 * tc::BM) * ((n_store + BN - 1) / BN);
   FMC_CHECK_SUPPORTED(tiles < (1ll << 26) && M < (1ll << 31), "GEMM too large (%lld tiles)", (long long)tiles);
-  const int64_t pairs = tiles < max_pairs ? tiles : max_pairs;
+  int splits = gemm_splits<BN, EPI>(M, K, ep, ldc, n_store);
+  const int64_t items = tiles * splits;
+  const int64_t pairs = items < max_pairs ? items : max_pairs;
   cfg.gridDim = dim3(2 * (unsigned)pairs, 1, 1);
-  const int kid = EPI == tc::TC_EPI_TANH_BF16 ? FMC_KT_TC_GEMM_TANH : FMC_KT_TC_GEMM_DTANH;
-  const double bytes = (double)M * K * 2 + (double)N * K * 2 + (double)M * N * 2 +
-                       (EPI == tc::TC_EPI_DTANH_BF16 ? (double)M * N * 2 : 0.0);
-  KernelTimer kt(kid, st, 2.0 * (double)M * N * K, bytes);
-  note_grid(kid, (int)(2 * pairs), 2);
-  int Mi = (int)M, one = 1;
-  int64_t stride = M * ldc;
-  FMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ma, mb, mc, Mi, N, K, ep, C, ldc, n_store, one, stride, err));
-  FMC_LAUNCH_CHECK();
-  return FMC_OK;
+  void* out = splits > 1 ? (void*)ep.kpart : C;
+  {
+    const int kid = EPI == tc::TC_EPI_TANH_BF16 ? FMC_KT_TC_GEMM_TANH
+                    : EPI == tc::TC_EPI_DTANH_BF16 ? FMC_KT_TC_GEMM_DTANH
+                                                   : FMC_KT_TC_GEMM_F32;
+    const double bytes = (double)M * K * 2 + (double)N * K * 2 + (double)M * N * (TSTORE ? 2 : 4) +
+                         (EPI == tc::TC_EPI_DTANH_BF16 ? (double)M * N * 2 : 0.0);
+    KernelTimer kt(kid, st, 2.0 * (double)M * N * K, bytes);
+    note_grid(kid, (int)(2 * pairs), 2);
+    int Mi = (int)M;
+    int64_t stride = M * ldc;
+    FMC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ma, mb, mc, Mi, N, K, ep, out, ldc, n_store, splits, stride, err));
+    FMC_LAUNCH_CHECK();
+  }
+  return splits > 1 ? splitk_finish(st, splits, M, ep, C, ldc, n_store) : FMC_OK;
 }
 
 // Weight gradient C[out, in] = sum over the n batch rows of G[r, out] * X[r, in]
@@ -313,6 +329,11 @@ int tc_gemm_wgrad(cudaStream_t st, const uint16_t* G, int64_t ldg, int out, cons
   memset(&mc, 0, sizeof(mc));
   const int K = (int)FlowGeom::rup(n, 64);
   FMC_CHECK_SUPPORTED(n < (1ll << 31), "batch too large");
+  // CTA pairs where the output's 128-row tiles pair up: half of X's columns per
+  // CTA (one-CTA tiles of 128 x 256 are limited by the operands' way into the
+  // SM). 65,536 rows, 512 x 512 and 2560 x 512 outputs together: 170 -> 148 us.
+  if (BN == 256 && (out + tc::BM - 1) / tc::BM % 2 == 0)
+    return launch_tc_pair<256, 6, tc::TC_EPI_F32, 2, 3>(st, ma, mb, mc, out, in, K, ep, C, ldc, in);
   if (BN == 256) return launch_tc<256, 4, tc::TC_EPI_F32, false, 2, 3>(st, ma, mb, mc, out, in, K, ep, C, ldc, in);
   return launch_tc<128, 4, tc::TC_EPI_F32, false, 2, 3>(st, ma, mb, mc, out, in, K, ep, C, ldc, in);
 }

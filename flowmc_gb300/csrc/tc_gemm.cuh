@@ -341,7 +341,7 @@ __device__ __forceinline__ bool tc_skip_pair(const int* err) {
 // NSTG = 2 also stages each chunk's 32 bias values in shared memory (one
 // 128-byte slot per epilogue warp, broadcast reads); with NSTG = 1 the bias
 // reaches the lanes by shuffles.
-// PAIR (launched as clusters of 2, no split-K): a tile is 256 rows x BN
+// PAIR (launched as clusters of 2): a tile is 256 rows x BN
 // columns computed by a CTA pair with tcgen05 cta_group::2 -- each CTA loads
 // its 128 rows of A and BN / 2 rows of B (tmB's box is BN / 2 rows), the
 // even CTA issues the MMAs, each CTA runs the epilogue of its own rows.
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   static_assert(!TSTORE || EPI == TC_EPI_TANH_BF16 || EPI == TC_EPI_DTANH_BF16, "TMA store: bf16 epilogues only");
   static_assert(!PAIR || BN % 32 == 0, "a CTA pair splits B into two multiples of 16 rows");
   static_assert(NSTG == 1 || NSTG == 2, "one or two staging buffers per warp");
-  static_assert(OPM == 0 || (!PAIR && BN % 64 == 0), "MN-major operands: one-CTA tiles of whole 64-wide blocks");
+  static_assert(OPM == 0 || (PAIR ? BN / 2 : BN) % 64 == 0, "MN-major operands: whole 64-wide blocks per CTA");
   constexpr bool kBiasSmem = NSTG == 2;
   if (PAIR ? tc_skip_pair(err) : tc_skip(err)) return;
   extern __shared__ uint8_t smem_raw[];
@@ -438,8 +438,20 @@ __global__ void __launch_bounds__(kThreads, 1)
             // both CTAs' copies count on the even CTA's barrier
             const uint32_t full_cl = mapa_shared(smem_u32(&full[s]), 0);
             if (rank == 0) mbar_expect_tx(&full[s], 2 * (S::A_BYTES + S::B_BYTES));
-            tma_load_2d_pair(sa, &tmA, full_cl, k * BK, m0);
-            tma_load_2d_pair(sb, &tmB, full_cl, k * BK, n0);
+            if constexpr ((OPM & 1) != 0) {
+#pragma unroll
+              for (int j = 0; j < BM / 64; ++j)
+                tma_load_2d_pair(sa + j * kMnBlockBytes, &tmA, full_cl, m0 + 64 * j, k * BK);
+            } else {
+              tma_load_2d_pair(sa, &tmA, full_cl, k * BK, m0);
+            }
+            if constexpr ((OPM & 2) != 0) {
+#pragma unroll
+              for (int j = 0; j < BNL / 64; ++j)
+                tma_load_2d_pair(sb + j * kMnBlockBytes, &tmB, full_cl, n0 + 64 * j, k * BK);
+            } else {
+              tma_load_2d_pair(sb, &tmB, full_cl, k * BK, n0);
+            }
           } else {
             mbar_expect_tx(&full[s], S::STAGE_BYTES);
             if constexpr ((OPM & 1) != 0) {
@@ -507,7 +519,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int kk = 0; kk < BK / 16; ++kk) {
             // advance along K inside the swizzle atom: 16 bf16 = 32 bytes
             if constexpr (PAIR)
-              mma_bf16_pair(d, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (k > kb || kk > 0) ? 1u : 0u);
+              mma_bf16_pair(d, da + kStepA * kk, db + kStepB * kk, idesc, (k > kb || kk > 0) ? 1u : 0u);
             else
               mma_bf16(d, da + kStepA * kk, db + kStepB * kk, idesc, (k > kb || kk > 0) ? 1u : 0u);
           }
