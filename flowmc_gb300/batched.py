@@ -25,6 +25,10 @@ _lib.register_extra("fmc_batched_dense_local_steps", ctypes.c_int, [
     ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
     ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p])
 
+_lib.register_extra("fmc_batched_pack_rows", ctypes.c_int, [
+    ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p,
+    ctypes.c_void_p])
+
 D_MAX = 256
 
 
@@ -55,6 +59,24 @@ class BatchedDenseLocalSteps:
             out[self.offsets[t]:self.offsets[t + 1], :x.shape[1]] = x
         return out
 
+    def _packed_rows(self, xs: list, dev) -> torch.Tensor:
+        """The layout of `pack` in one launch, padding columns left unset (the
+        step kernel reads no target's columns past its n_dim), where every
+        position block is as declared; `pack` otherwise (it converts, broadcasts
+        and zero-fills)."""
+        n = len(self.targets)
+        plain = len(xs) == n and dev.type == "cuda" and all(
+            x.dtype == torch.float32 and x.device == dev and x.dim() == 2 and x.shape[0] == c and x.shape[1] == t.n_dim
+            and x.stride(1) == 1 for x, t, c in zip(xs, self.targets, self.n_chains))
+        if not plain:
+            return self.pack(xs)
+        out = torch.empty(self.offsets[-1], D_MAX, device=dev)
+        _lib.check(_lib.lib().fmc_batched_pack_rows(
+            (ctypes.c_void_p * n)(*[x.data_ptr() for x in xs]), (ctypes.c_int64 * n)(*[x.stride(0) for x in xs]),
+            (ctypes.c_int32 * n)(*[t.n_dim for t in self.targets]), (ctypes.c_int32 * n)(*self.n_chains), n,
+            out.data_ptr(), _lib.stream_handle(dev)))
+        return out
+
     def unpack(self, packed: torch.Tensor) -> list:
         return [packed[self.offsets[t]:self.offsets[t + 1], :tg.n_dim] for t, tg in enumerate(self.targets)]
 
@@ -69,8 +91,8 @@ class BatchedDenseLocalSteps:
                         torch.full((c, buf_len), -float("inf"), device=dev),
                         torch.full((c, buf_len), -float("inf"), device=dev))
                        for t, c in zip(self.targets, self.n_chains)]
-        x0 = self.pack(xs)
-        x_last = torch.zeros_like(x0)
+        x0 = self._packed_rows(xs, dev)
+        x_last = torch.empty_like(x0)   # every chain's row up to its n_dim is written, and returned
         lp_last = torch.empty(self.offsets[-1], device=dev)
         tg = (_lib.FmcTarget * n)(*[t.c_struct() for t in self.targets])
         nc = (ctypes.c_int32 * n)(*self.n_chains)

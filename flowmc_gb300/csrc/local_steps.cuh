@@ -41,6 +41,7 @@
 // significant bits) instead of FP64: this GPU's FP64 rate is too low for a
 // per-chain-step operation, and the inputs (lp, squared norms) are FP32.
 #pragma once
+#include <atomic>
 #include "targets.cuh"
 
 namespace fmc {
@@ -539,9 +540,18 @@ int launch_local_t(const LocalArgs& a0, cudaStream_t st) {
   if (smem > 48 * 1024) {
     FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
-  int per_sm = 0;
-  FMC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
-  if (per_sm < 1) per_sm = 1;
+  // blocks per SM, asked for once per launch shape (the last one is kept, in
+  // one word so that threads see a whole entry)
+  static std::atomic<uint64_t> last{0};
+  const uint64_t shape = ((uint64_t)smem << 24) | ((uint64_t)threads << 8);
+  uint64_t known = last.load(std::memory_order_relaxed);
+  if ((known & ~0xffull) != shape) {
+    int q = 0;
+    FMC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, kern, threads, smem));
+    known = shape | (uint64_t)(q < 1 ? 1 : q);
+    last.store(known, std::memory_order_relaxed);
+  }
+  const int per_sm = (int)(known & 0xff);
   const int64_t need = (a.C_pad + gpb - 1) / gpb;
   const int64_t cap = (int64_t)sm_count() * per_sm;
   const int blocks = (int)(need < cap ? need : cap);

@@ -62,8 +62,17 @@ class Profiler:
         return {k: len(v) for k, v in self.events.items()}
 
 
-@contextlib.contextmanager
+_off = contextlib.nullcontext()
+
+
 def region(name: str, units: float = 0.0):
+    if _active is None and not _nvtx:
+        return _off   # nothing to record: no generator, no frame
+    return _region(name, units)
+
+
+@contextlib.contextmanager
+def _region(name: str, units: float):
     if _nvtx:
         with nvtx_range(name), _timed(name, units):
             yield

@@ -77,7 +77,9 @@ class TakeSteps(Strategy):
         bufs = self._buffers(resources)
         kernel = resources[self.kernel_name]
         target = as_target(resources[self.logpdf_name])
-        x0 = torch.atleast_2d(initial_position).to(torch.float32).contiguous()
+        x0 = initial_position
+        if not (type(x0) is torch.Tensor and x0.dim() == 2 and x0.dtype == torch.float32 and x0.is_contiguous()):
+            x0 = torch.atleast_2d(x0).to(torch.float32).contiguous()
         last = self.sample(kernel, subkey.value, x0, target, bufs, self.current_position, data,
                            noise=noise, uniform=uniform)
         self.current_position += self.n_steps // self.thinning   # take_steps.py:143

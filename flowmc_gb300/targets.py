@@ -21,6 +21,9 @@ import torch
 from . import _lib
 
 
+_POINTER_FIELDS = frozenset(("mean", "inv_var", "log_w", "precision"))
+
+
 class Target:
     """Base class: owns the device arrays referenced by the C descriptor."""
 
@@ -52,11 +55,10 @@ class Target:
         s.kind = self.kind
         s.n_dim = self.n_dim
         s.n_comp = self.n_comp
-        for field in ("mean", "inv_var", "log_w", "precision"):
-            t = self._tensors.get(field)
-            setattr(s, field, _lib.ptr(t) if t is not None else None)
-        for i, v in enumerate(self._scalars):
-            s.scalars[i] = float(v)
+        for field, t in self._tensors.items():
+            if field in _POINTER_FIELDS:
+                setattr(s, field, _lib.ptr(t))
+        s.scalars[:] = self._scalars
         return s
 
     # -- the reference's logpdf call signature

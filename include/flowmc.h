@@ -230,7 +230,12 @@ FMC_API int fmc_adam_optimize(const FmcTarget* target, const float* x0, int32_t 
  * for Philox), out_pos/out_logp/out_acc (device pointers to each target's
  * buffers [n_chains_t, buf_len, d_t] / [n_chains_t, buf_len]).
  * x0, x_last: [sum_t n_chains_t, 256] (row stride 256, target t's chains
- * from row sum_{u<t} n_chains_u); lp_last [sum_t n_chains_t]. */
+ * from row sum_{u<t} n_chains_u); lp_last [sum_t n_chains_t].
+ * fmc_batched_pack_rows copies per-target positions (host arrays: device
+ * pointers to [n_chains_t, n_dim_t] rows of stride row_stride_t floats) into
+ * the layout of x0; the columns past n_dim_t are left as they are. */
+FMC_API int fmc_batched_pack_rows(const float* const* x, const int64_t* row_stride, const int32_t* n_dim,
+                                  const int32_t* n_chains, int32_t n_targets, float* packed, void* stream);
 FMC_API int fmc_batched_workspace_size(int32_t n_targets, int64_t total_chains, size_t* bytes);
 FMC_API int fmc_batched_dense_local_steps(const FmcTarget* targets, int32_t n_targets, const int32_t* n_chains,
                                           const FmcLocalParams* params, const float* step_sizes, const float* x0,
