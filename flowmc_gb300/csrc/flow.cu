@@ -80,21 +80,65 @@ int make_geom(const FmcFlow* f, FlowGeom& g) {
 }
 
 // ------------------------------------------------------------------ kernels
-// one warp per row (lanes over the coordinates, rows strided over the grid):
-// no per-element index division
-__global__ void k_standardize(const float* __restrict__ x, int64_t n, int d, const float* __restrict__ aux,
-                              float* __restrict__ out) {
+// One warp per row, lanes over the coordinates: out[r, j] = f(in[r, j], u_j, v_j)
+// with (u_j, v_j) = col(j). Up to 128 coordinates a lane's columns are the same
+// in every row, so their values are worked out once, and two rows are loaded
+// ahead (in may be out: a thread writes the elements that it read).
+template <typename C, typename F>
+__device__ __forceinline__ void map_columns(const float* in, float* out, int64_t n, int d, C col, F f) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n; r += warps)
-    for (int j = lane; j < d; j += 32) out[r * d + j] = (x[r * d + j] - aux[j]) / sqrtf(aux[d + j]);
+  int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (d <= 128) {
+    float u[4], v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (lane + 32 * k < d) col(lane + 32 * k, u[k], v[k]);
+    for (; r < n; r += 2 * warps) {
+      float a[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (lane + 32 * k < d && r + i * warps < n) a[i][k] = in[(r + i * warps) * d + lane + 32 * k];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (lane + 32 * k < d && r + i * warps < n)
+            out[(r + i * warps) * d + lane + 32 * k] = f(a[i][k], u[k], v[k]);
+    }
+    return;
+  }
+  for (; r < n; r += warps)
+    for (int j = lane; j < d; j += 32) {
+      float u, v;
+      col(j, u, v);
+      out[r * d + j] = f(in[r * d + j], u, v);
+    }
 }
 
+// memory bound, 69,632 x 64: 14.3 -> 12.5 us
+__global__ void k_standardize(const float* __restrict__ x, int64_t n, int d, const float* __restrict__ aux,
+                              float* __restrict__ out) {
+  map_columns(
+      x, out, n, d,
+      [&](int j, float& u, float& v) {
+        u = aux[j];
+        v = sqrtf(aux[d + j]);
+      },
+      [](float a, float u, float v) { return (a - u) / v; });
+}
+
+// 204,800 x 64: 34.3 -> 17.7 us
 __global__ void k_destandardize(float* __restrict__ x, int64_t n, int d, const float* __restrict__ aux) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n; r += warps)
-    for (int j = lane; j < d; j += 32) x[r * d + j] = x[r * d + j] * sqrtf(aux[d + j]) + aux[j];
+  map_columns(
+      x, x, n, d,
+      [&](int j, float& u, float& v) {
+        u = aux[j];
+        v = sqrtf(aux[d + j]);
+      },
+      [](float a, float u, float v) { return __fmaf_rn(a, v, u); });
 }
 
 // one warp per row: ScalarAffine of every coordinate, the conditioning
@@ -197,25 +241,34 @@ __global__ void k_base_logprob(const float* __restrict__ y, const float* __restr
   }
 }
 
+// 204,800 x 64: 59.7 us with a Philox block per coordinate, 28.9 us with one per pair
 __global__ void k_base_sample(const float* __restrict__ z, Rng rng0, int64_t n, int d, const float* __restrict__ aux,
                               float* __restrict__ out) {
   const Rng rng = rng0.at_epoch();
   // jax.random.multivariate_normal(0, c I): mean + z @ cholesky(c I).T = sqrt(c) z
   const float sc = sqrtf(aux[2 * d]);
-  const int64_t tot = n * d;
+  if (z) {
+    const int64_t tot = n * d;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x)
+      out[i] = z[i] * sc;
+    return;
+  }
+  // one Philox block and one Box-Muller pair for two coordinates
+  const int pairs = (d + 1) / 2;
+  const int64_t tot = n * pairs;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
-    float v;
-    if (z) {
-      v = z[i];
+    const int64_t r = tot < (1ll << 31) ? (int64_t)((uint32_t)i / (uint32_t)pairs) : i / pairs;
+    const int p = (int)(i - r * pairs);
+    const u32x4 b = rng.draw((uint64_t)r, 0, (uint32_t)p, RNG_TAG_NF_NORMAL);
+    float z0, z1;
+    box_muller(b.x, b.y, z0, z1);
+    float* o = out + r * d + 2 * p;
+    if ((d & 1) == 0 && ((uintptr_t)out & 7) == 0) {
+      *reinterpret_cast<float2*>(o) = make_float2(z0 * sc, z1 * sc);
     } else {
-      const int64_t r = i / d;
-      const int j = (int)(i - r * d);
-      const u32x4 b = rng.draw((uint64_t)r, 0, (uint32_t)(j >> 1), RNG_TAG_NF_NORMAL);
-      float z0, z1;
-      box_muller(b.x, b.y, z0, z1);
-      v = (j & 1) ? z1 : z0;
+      o[0] = z0 * sc;
+      if (2 * p + 1 < d) o[1] = z1 * sc;
     }
-    out[i] = v * sc;
   }
 }
 
