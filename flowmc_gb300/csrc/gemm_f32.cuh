@@ -13,6 +13,7 @@
 // quarters of a warp share: 8 x 8 outputs per thread keep the loads at three
 // quarters of the FMA time, 8 x 4 (outputs of at most 32) at its whole.
 #pragma once
+#include <type_traits>
 #include "flow.cuh"
 
 namespace fmc {
@@ -44,7 +45,7 @@ struct G32Args {
 // per thread, times WK groups of warps that take every WK-th 16-input chunk
 // (outputs too few to fill the SMs: the groups' sums are added through shared
 // memory in order). The tile leaves through shared memory as whole rows.
-template <int WR, int TN, int WK, int EPI>
+template <int WR, int TN, int WK, int EPI, bool SEQ>
 __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_gemm_f32(const __grid_constant__ G32Args a) {
   constexpr int NT = 32 * WR * WK, BM = 32 * WR, BN = 8 * TN, ROWS = BM + BN;
   constexpr int STAGE = WK * ROWS * kG32Pitch, LDT = BN + 8, BKS = WK * kG32BK;
@@ -94,11 +95,12 @@ __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_
     asm volatile("cp.async.commit_group;");
   };
   const int r0 = wid * 32 + (lane >> 3), c0 = lane & 7;   // rows r0 + 4 i, columns c0 + 8 j
-  uint64_t acc[8][TN];
+  using Acc = std::conditional_t<SEQ, float, uint64_t>;
+  Acc acc[8][TN];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < TN; ++j) acc[i][j] = Acc(0);
 #pragma unroll
   for (int q = 0; q < kG32Stages - 1; ++q) issue(q * BKS, q);
   int slot = 0;
@@ -112,16 +114,34 @@ __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_
 #pragma unroll
       for (int k = 0; k < kG32BK; k += 4) {
         if (k0 + grp * kG32BK + k >= a.K) break;
-        ulonglong2 b[TN];
+        if constexpr (SEQ) {
+          float4 b[TN];
 #pragma unroll
-        for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(Bs + 8 * j * kG32Pitch + k);
+          for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(Bs + 8 * j * kG32Pitch + k);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(As + 4 * i * kG32Pitch + k);
+          for (int i = 0; i < 8; ++i) {
+            const float4 v = *reinterpret_cast<const float4*>(As + 4 * i * kG32Pitch + k);
 #pragma unroll
-          for (int j = 0; j < TN; ++j) {
-            acc[i][j] = f2_fma(v.x, b[j].x, acc[i][j]);
-            acc[i][j] = f2_fma(v.y, b[j].y, acc[i][j]);
+            for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(v.x, b[j].x, acc[i][j]);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(v.y, b[j].y, acc[i][j]);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(v.z, b[j].z, acc[i][j]);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(v.w, b[j].w, acc[i][j]);
+          }
+        } else {
+          ulonglong2 b[TN];
+#pragma unroll
+          for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(Bs + 8 * j * kG32Pitch + k);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(As + 4 * i * kG32Pitch + k);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+              acc[i][j] = f2_fma(v.x, b[j].x, acc[i][j]);
+              acc[i][j] = f2_fma(v.y, b[j].y, acc[i][j]);
+            }
           }
         }
       }
@@ -134,9 +154,15 @@ __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      float lo, hi;
-      f2_unpack(acc[i][j], lo, hi);
-      sm[(grp * BM + r0 + 4 * i) * LDT + c0 + 8 * j] = lo + hi;
+      float v;
+      if constexpr (SEQ) {
+        v = acc[i][j];
+      } else {
+        float lo, hi;
+        f2_unpack(acc[i][j], lo, hi);
+        v = lo + hi;
+      }
+      sm[(grp * BM + r0 + 4 * i) * LDT + c0 + 8 * j] = v;
     }
   __syncthreads();
   const bool vout = (a.ldc & 3) == 0 && (a.N & 3) == 0 && ((uintptr_t)p.C & 15) == 0 &&
@@ -186,7 +212,14 @@ __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_
 // two with relu masks, 51 -> 37 us); for outputs of at most 32 columns, and where
 // the wide tiles would leave SMs idle, 64 x 32 of two warps times four input
 // groups ([16384 x 512] x [512 x 32] 32 -> 25 us)
-template <int EPI>
+//
+// SEQ: an output's products added one by one in the order of the inputs, for
+// the forward that a gradient keeps. A relu's derivative jumps where its
+// input is 0, so a last bit there shows in the gradient (1e-6 of it for one
+// row of 16,384); in this order the bits do not depend on the tile. Packed
+// sums of even and odd inputs, and of input groups, otherwise. Loss
+// and gradient of 16,384 rows (32-D, 8 layers, H = 256): 1.30 ms packed, 1.29 in order.
+template <int EPI, bool SEQ = false>
 inline int gemm_f32(cudaStream_t st, const G32Args& a, int count) {
   if (a.M <= 0 || a.N <= 0) return FMC_OK;
   auto go = [&](auto kern, int bm, int bn, int wk, int threads) -> int {
@@ -208,9 +241,12 @@ inline int gemm_f32(cudaStream_t st, const G32Args& a, int count) {
     return FMC_OK;
   };
   const int64_t wide = (a.M + 127) / 128 * ((a.N + 63) / 64) * count;
-  if (a.N <= 32 || wide < sm_count()) return go(k_gemm_f32<2, 4, 4, EPI>, 64, 32, 4, 256);
-  if (a.K <= 64) return go(k_gemm_f32<4, 4, 1, EPI>, 128, 32, 1, 128);
-  return go(k_gemm_f32<4, 8, 1, EPI>, 128, 64, 1, 128);
+  if (a.N <= 32 || wide < sm_count()) {
+    if constexpr (SEQ) return go(k_gemm_f32<2, 4, 1, EPI, SEQ>, 64, 32, 1, 64);
+    else return go(k_gemm_f32<2, 4, 4, EPI, SEQ>, 64, 32, 4, 256);
+  }
+  if (a.K <= 64) return go(k_gemm_f32<4, 4, 1, EPI, SEQ>, 128, 32, 1, 128);
+  return go(k_gemm_f32<4, 8, 1, EPI, SEQ>, 128, 64, 1, 128);
 }
 
 // ------------------------------------------------------------------ weight gradients
