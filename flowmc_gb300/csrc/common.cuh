@@ -8,6 +8,7 @@
 //  * float-float ("double-single") sums after Knuth's TwoSum (TAOCP vol. 2,
 //    4.2.2) for the Metropolis-Hastings log-ratio
 #pragma once
+#include <utility>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -47,6 +48,36 @@ void set_error(const char* fmt, ...);
       return FMC_ERR_CUDA;                                                   \
     }                                                                        \
   } while (0)
+
+// Launches in a chain (programmatic dependent launch): a kernel started by
+// launch_chained may be placed on SMs as the kernel before it on the stream
+// leaves them, instead of after its last block and a launch latency. Every
+// thread of it calls chain_release (the next chained kernel may start in turn)
+// and, before it reads what an earlier kernel wrote or writes anything, and
+// also on a path that does neither, chain_wait (every earlier kernel has
+// completed and its writes are visible).
+// Started the ordinary way such a kernel behaves as any other. The tensor-core
+// kernels (one CTA per SM, the next one's waits for its place) are chained:
+// 4.14 -> 3.74 ms for 96 of them in a global phase, 10.37 -> 10.24 ms a BF16
+// training step. With the small kernels between them chained as well the step
+// took 10.60 ms: their blocks settle beside a running tensor-core CTA.
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                                  A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(block, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
 
 #define FMC_LAUNCH_CHECK()                                                   \
   do {                                                                       \

@@ -243,8 +243,8 @@ static int launch_tc(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& 
                          (EPI == tc::TC_EPI_DTANH_BF16 ? (double)M * N * 2 : 0.0);
     KernelTimer kt(kid, st, 2.0 * (double)M * N * K, bytes);
     note_grid(kid, (int)grid, 1);
-    kern<<<(unsigned)grid, tc::kThreads, TOTAL, st>>>(ma, mb, mc, (int)M, N, K, ep, out, ldc, n_store, splits,
-                                                     M * ldc, err);
+    FMC_CUDA_TRY(launch_chained(kern, (unsigned)grid, tc::kThreads, TOTAL, st, ma, mb, mc, (int)M, N, K, ep, out, ldc,
+                                n_store, splits, M * ldc, err));
     FMC_LAUNCH_CHECK();
   }
   return splits > 1 ? splitk_finish(st, splits, M, ep, C, ldc, n_store) : FMC_OK;
@@ -266,7 +266,9 @@ static int launch_tc_pair(cudaStream_t st, const CUtensorMap& ma, const CUtensor
     FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TOTAL));
     attr_set = true;
   }
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -276,7 +278,7 @@ static int launch_tc_pair(cudaStream_t st, const CUtensorMap& ma, const CUtensor
   cfg.dynamicSmemBytes = TOTAL;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   static int max_pairs = 0;
   if (max_pairs == 0) {
     cfg.gridDim = dim3(2 * (unsigned)(sm_count() / 2), 1, 1);

@@ -355,7 +355,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   static_assert(NSTG == 1 || NSTG == 2, "one or two staging buffers per warp");
   static_assert(OPM == 0 || (PAIR ? BN / 2 : BN) % 64 == 0, "MN-major operands: whole 64-wide blocks per CTA");
   constexpr bool kBiasSmem = NSTG == 2;
-  if (PAIR ? tc_skip_pair(err) : tc_skip(err)) return;
+  chain_release();
+  if (PAIR ? tc_skip_pair(err) : tc_skip(err)) {
+    chain_wait();
+    return;
+  }
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(16) float s_bias[kBiasSmem ? kEpiWarps : 1][32];
   constexpr int BNL = PAIR ? BN / 2 : BN;   // B rows this CTA loads per stage
@@ -416,6 +420,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if constexpr (PAIR) cluster_sync_all();   // both CTAs' barriers exist before either signals the other's
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  chain_wait();   // barriers and TMEM are set up while the kernel before ends
 
   if (warp == 0) {
     if (lane == 0) {

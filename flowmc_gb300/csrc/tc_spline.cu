@@ -386,7 +386,11 @@ __global__ void __launch_bounds__(kSplThreads, 1)
   constexpr int P = T::P, DG = T::DG, BN = T::BN, E = kSplineEpiPerQuarter, PP = BiasRows<KB>::PP;
   using X = XBox<DG>;
   using S = SplSmem<BN, STAGES, CH>;
-  if (tc_skip(err)) return;
+  chain_release();
+  if (tc_skip(err)) {
+    chain_wait();
+    return;
+  }
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const bool xt = X::kOk && x_tma != 0;
@@ -397,12 +401,6 @@ __global__ void __launch_bounds__(kSplThreads, 1)
   uint64_t* xdone = xfull + kXBufs;            // [kXBufs] box rewritten by the epilogue warps
   float* lred = (float*)(bars + 256);
   float* sbias = lred + (xt ? 2 * E * BM : 0);
-  if (bias_smem) {
-    for (int i = threadIdx.x; i < nt * PP; i += blockDim.x) {
-      const int t = i / PP, pp = i - t * PP;
-      sbias[i] = pp < P ? __ldg(bias + t * P + pp) : 0.f;
-    }   // visible after pipe_setup's __syncthreads
-  }
   if (threadIdx.x == 0) {
     for (int j = 0; j < kXBufs; ++j) {
       mbar_init(&xfull[j], 1);
@@ -413,6 +411,14 @@ __global__ void __launch_bounds__(kSplThreads, 1)
   const int nk = (K + BK * CH - 1) / (BK * CH);   // stages per tile (K a multiple of BK * CH when CH > 1)
   const int tiles = (M + BM - 1) / BM * n_groups;
   const Pipe p = pipe_setup<STAGES>(base, bars, warp);
+  chain_wait();   // barriers and TMEM are set up while the kernel before ends
+  if (bias_smem) {
+    for (int i = threadIdx.x; i < nt * PP; i += blockDim.x) {
+      const int t = i / PP, pp = i - t * PP;
+      sbias[i] = pp < P ? __ldg(bias + t * P + pp) : 0.f;
+    }
+    __syncthreads();
+  }
   const bool fold = fold_th != nullptr;
 
   if (warp == 0) {
@@ -629,7 +635,11 @@ __global__ void __launch_bounds__(kSplThreads, 1)
   constexpr int RROWS = (BM + RP - 1) / RP;        // rows per column-sum part
   using X = XBox<DG>;
   using S = SplSmem<BN, STAGES, 1>;
-  if (tc_skip(err)) return;
+  chain_release();
+  if (tc_skip(err)) {
+    chain_wait();
+    return;
+  }
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const bool xt = X::kOk && x_tma != 0;
@@ -651,6 +661,7 @@ __global__ void __launch_bounds__(kSplThreads, 1)
   const int tiles = (M + BM - 1) / BM * n_groups;
   const int ntP = a.nt * P;
   const Pipe p = pipe_setup<STAGES>(base, bars, warp);
+  chain_wait();   // barriers and TMEM are set up while the kernel before ends
 
   if (warp == 0) {
     if (lane == 0) producer<BN, STAGES, 1>(p, &tmA, &tmB, tiles, n_groups, nk);
@@ -1175,9 +1186,9 @@ static int launch_spl(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap&
   note_grid(INV ? FMC_KT_TC_SPLINE_INV : FMC_KT_TC_SPLINE_FWD, (int)grid, 1);
   // the next layer's affine rides on the x boxes only
   const bool fo = fold != nullptr && x_tma;
-  kern<<<(unsigned)grid, tc::kSplThreads, total, st>>>(ma, mb, mx, mxo, x_tma, (int)M, n_groups, nt, K, bias,
-                                                       bias_smem, xa, d, tpar, ldp, cfg, fo ? fold->th_next : nullptr,
-                                                       fo ? fold->cond16 : nullptr, fo ? fold->ldc16 : 0, err);
+  FMC_CUDA_TRY(launch_chained(kern, (unsigned)grid, tc::kSplThreads, total, st, ma, mb, mx, mxo, x_tma, (int)M, n_groups,
+                              nt, K, bias, bias_smem, xa, d, tpar, ldp, cfg, fo ? fold->th_next : nullptr,
+                              fo ? fold->cond16 : nullptr, fo ? fold->ldc16 : 0, err));
   FMC_LAUNCH_CHECK();
   *parts = x_tma ? n_groups : kSplineEpiPerQuarter * n_groups;
   *folded = fo;
@@ -1287,8 +1298,8 @@ static int launch_spl_bwd(cudaStream_t st, const CUtensorMap& ma, const CUtensor
   const int64_t tiles = (M + tc::BM - 1) / tc::BM * n_groups;
   const int64_t grid = tiles < sm_count() ? tiles : sm_count();
   note_grid(FMC_KT_TC_SPLINE_BWD, (int)grid, 1);
-  kern<<<(unsigned)grid, tc::kSplThreads, total, st>>>(ma, mb, mx, mgy, mgx, mr, x_tma, (int)M, n_groups, K, a, cfg,
-                                                       err);
+  FMC_CUDA_TRY(launch_chained(kern, (unsigned)grid, tc::kSplThreads, total, st, ma, mb, mx, mgy, mgx, mr, x_tma, (int)M,
+                              n_groups, K, a, cfg, err));
   FMC_LAUNCH_CHECK();
   return FMC_OK;
 }
