@@ -56,6 +56,9 @@ void set_error(const char* fmt, ...);
 // and, before it reads what an earlier kernel wrote or writes anything, and
 // also on a path that does neither, chain_wait (every earlier kernel has
 // completed and its writes are visible).
+// Read-only loads (__ldg, const __restrict__) are not held back by the wait:
+// they may read theta and other inputs of the whole chain, but not what the
+// kernel before wrote; the chained kernels take that by TMA or plain loads.
 // Started the ordinary way such a kernel behaves as any other. The tensor-core
 // kernels (one CTA per SM, the next one's waits for its place) are chained:
 // 4.14 -> 3.74 ms for 96 of them in a global phase, 10.37 -> 10.24 ms a BF16

@@ -663,17 +663,18 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       };
-      // operands of chunk c0 that come from global memory, loaded ahead
+      // operands of chunk c0 that come from global memory, loaded ahead (plain
+      // loads: the kernel before in the chain may have written them)
       auto prefetch = [&](int c0, float& bl, uint4 (&av)[4]) {
         const int j = n0 + c0 + lane;
-        if (EPI == TC_EPI_TANH_BF16 || EPI == TC_EPI_BIAS_F32) bl = (j < N) ? __ldg(ep.bias + j) : 0.f;
+        if (EPI == TC_EPI_TANH_BF16 || EPI == TC_EPI_BIAS_F32) bl = (j < N) ? ep.bias[j] : 0.f;
         if (EPI == TC_EPI_DTANH_BF16) {
           const int gn0 = n0 + c0;
           const uint16_t* ar = ep.aux + (int64_t)gm * ep.ldaux + gn0;
           if (row_ok && aux_vec && gn0 + 32 <= N) {
             const uint4* a4 = reinterpret_cast<const uint4*>(ar);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) av[i] = __ldg(a4 + i);
+            for (int i = 0; i < 4; ++i) av[i] = a4[i];
           } else {
             uint16_t* hv = reinterpret_cast<uint16_t*>(av);
 #pragma unroll
