@@ -9,5 +9,5 @@ def test_every_included_header_is_watched():
     included = set()
     for src in list(build.CSRC.iterdir()) + list(build.INCLUDE.iterdir()):
         if src.suffix in (".cu", ".cuh", ".h"):
-            included |= set(re.findall(r'#include "([^"]+)"', src.read_text()))
+            included |= {i.rsplit("/", 1)[-1] for i in re.findall(r'#include "([^"]+)"', src.read_text())}
     assert included and included <= watched, included - watched
