@@ -62,13 +62,28 @@ class Profiler:
         return {k: len(v) for k, v in self.events.items()}
 
 
-_off = contextlib.nullcontext()
+class region(contextlib.ContextDecorator):
+    """``with region(name)`` or ``@region(name)``. Whether there is anything to
+    record is asked on entry, so a region made before a Profiler is started
+    records in it; with nothing to record it costs one small object, no generator
+    and no frame."""
 
+    def __init__(self, name: str, units: float = 0.0):
+        self.name = name
+        self.units = units
 
-def region(name: str, units: float = 0.0):
-    if _active is None and not _nvtx:
-        return _off   # nothing to record: no generator, no frame
-    return _region(name, units)
+    def _recreate_cm(self):
+        return region(self.name, self.units)   # a decorated function may call itself
+
+    def __enter__(self):
+        if _active is None and not _nvtx:
+            self._cm = None
+            return
+        self._cm = _region(self.name, self.units)
+        self._cm.__enter__()
+
+    def __exit__(self, *exc):
+        return None if self._cm is None else self._cm.__exit__(*exc)
 
 
 @contextlib.contextmanager
