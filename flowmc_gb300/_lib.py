@@ -256,7 +256,7 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
 
 def stream_handle(device: torch.device | None = None) -> int:
     """cudaStream_t of torch's current stream on `device`."""
-    if device is not None and device.index is not None:
+    if device is not None and device.type == "cuda" and device.index is not None:
         return _raw_stream(device.index)   # the handle alone, without a Stream object
     return torch.cuda.current_stream(device).cuda_stream
 
