@@ -486,8 +486,8 @@ int flow_apply(const FmcFlow* f, const float* x, int64_t n, float* out, float* o
   int64_t rows;
   const bool bf16 = f->precision == FMC_PREC_BF16;
   if ((rc = check_ws(g, n, bf16, ws, ws_bytes, rows))) return rc;
-  if (!bf16 && flow_f32_fused(g)) {
-    // FP32 flows whose row tile fits in shared memory: one launch, no scratch
+  if (const int R = bf16 ? 0 : flow_f32_route(g, n)) {
+    // one launch for all layers, no scratch
     FlowF32Call c{};
     c.theta = f->theta;
     c.aux = f->aux;
@@ -502,7 +502,7 @@ int flow_apply(const FmcFlow* f, const float* x, int64_t n, float* out, float* o
       c.y = out;
       c.ld = out_ld;
     }
-    return flow_f32_pass(c, g, st);
+    return flow_f32_pass(c, g, R, st);
   }
   InferWs w;
   carve_infer(g, rows, bf16, ws, w);
@@ -537,7 +537,7 @@ int flow_sample(const FmcFlow* f, uint64_t seed, uint64_t counter, const float* 
   const bool bf16 = f->precision == FMC_PREC_BF16;
   if ((rc = check_ws(g, n, bf16, ws, ws_bytes, rows))) return rc;
   const Rng rng{(uint32_t)seed, (uint32_t)(seed >> 32), counter, rng_epoch()};
-  if (!bf16 && flow_f32_fused(g)) {
+  if (const int R = bf16 ? 0 : flow_f32_route(g, n)) {
     FlowF32Call c{};
     c.theta = f->theta;
     c.aux = f->aux;
@@ -548,7 +548,7 @@ int flow_sample(const FmcFlow* f, uint64_t seed, uint64_t counter, const float* 
     c.in_mode = FLOW_IN_BASE;
     c.out_mode = FLOW_OUT_DATA;
     c.y = x;
-    return flow_f32_pass(c, g, st);
+    return flow_f32_pass(c, g, R, st);
   }
   InferWs w;
   carve_infer(g, rows, bf16, ws, w);

@@ -22,30 +22,80 @@ static bool flow_f32_smem(const FlowGeom& g, int R, FlowF32Args& a, size_t& byte
   return bytes <= 227 * 1024;
 }
 
-int flow_f32_tile(const FlowGeom& g, int64_t n) {
-  FlowF32Args a{};
-  size_t bytes = 0;
-  return n >= 64 * (int64_t)sm_count() && flow_f32_smem(g, 64, a, bytes) ? 64 : 16;
-}
-
 bool flow_f32_fused(const FlowGeom& g) {
   FlowF32Args a{};
   size_t b;
   return flow_f32_smem(g, 16, a, b);
 }
 
-// rows per CTA: 64 where they fill the SMs and fit in shared memory, else 16
-// (fewer rows per CTA and two more warps per row: latency). Measured on GB300,
-// 5-D flow 4 x [32, 32]: the 620 rows of a 20-chain global step take 39 CTAs of
-// 16 rows; 10,000 rows (157 CTAs of 64) train in 341 us per step, in 16-row tiles
-// 425; a remainder launch of 16-row tiles behind whole waves of 64-row ones
-// did not pay (100,003 rows of the 32-D flow: 3.72 against 3.64 ms).
-int flow_f32_pass(const FlowF32Call& c, const FlowGeom& g, cudaStream_t st) {
+// 64 rows per CTA where they fill the SMs and fit in shared memory, else 16
+// (fewer rows per CTA and two more warps per row: latency). 5-D flow 4 x [32, 32]:
+// 10,000 rows (157 CTAs of 64) train in 341 us per step, in 16-row tiles 425.
+int flow_f32_tile(const FlowGeom& g, int64_t n) {
+  FlowF32Args a{};
+  size_t bytes = 0;
+  return n >= 64 * (int64_t)sm_count() && flow_f32_smem(g, 64, a, bytes) ? 64 : 16;
+}
+
+// The fastest way through a forward or inverse pass: 64 or 16 rows per CTA of
+// the fused kernel, or 0 for the launches per layer (the same bits all three).
+// 16-row tiles win on few rows of narrow conditioners (one launch instead of
+// five per layer), 64-row tiles on many rows where two CTAs share an SM, and the
+// layered 64 x 64 GEMM tiles where a row tile's serial walk over all weights is
+// long (wide layers, many coordinate groups) or a lone CTA per SM leaves its
+// splines uncovered. Where the lines lie depends on all of the sizes, so each way
+// is estimated in microseconds per layer from the counts that drive it:
+//   S   stages (16 inputs x one tile of outputs) of the conditioner
+//   G   coordinate groups of its last Linear (splines between products)
+//   t   row tiles on the fullest SM, r the rounds they run in
+// with coefficients fitted to 630 measured calls (GB300; 5 to 500 dims, 16 to 768
+// units, 4 to 12 bins, 16 to 100,000 rows, 4 layers), which they reproduce
+// within 10 % (16 and 64 rows) and 17 % (layers) for nine calls in ten. The fused
+// kernel has to look a tenth faster; the choice is then within 1 % of the fastest
+// of the three on average, at worst 28 % behind it, and at worst 14 % behind the
+// layers. Taking the fused kernel wherever it fits had cost, against the
+// layers, in us: 32-D, 10 bins, 512 units, 100,000 rows 14,341 -> 24,452; 128-D,
+// 12 bins, 768 units, 16 rows 551 -> 2,873; 128-D, 4 bins, 16 units, 100,000
+// rows 1,409 -> 2,273.
+int flow_f32_route(const FlowGeom& g, int64_t n) {
+  const FlowShape s = flow_shape(g);
+  const double sms = sm_count();
+  double S = 0, G = 0, steps = 0, macs = 0, raw = 0;   // means over the two layer parities
+  for (int l = 0; l < 2; ++l)
+    for (int i = 0; i <= g.nh; ++i) {
+      const int in = s.in(l, i), out = s.out(l, i), tc = s.tile_cols(i);
+      const int tiles = (out + tc - 1) / tc, ks = (in + kFlowBK - 1) / kFlowBK;
+      S += 0.5 * tiles * ks;
+      steps += 0.5 * ks;
+      macs += 0.5e-6 * ((out + 63) / 64 * 64) * (ks * kFlowBK);   // a 64 x 64 GEMM's, padded, in millions
+      if (i == g.nh) {
+        G += 0.5 * tiles;
+        raw += 0.5e-6 * out;
+      }
+    }
+  double best = 0.9 * (28.9 + 0.787 * steps + (double)n * (0.0601 * macs + 1.835 * raw + 0.88e-3));
+  int route = 0;
+  for (int R = 16; R <= 64; R += 48) {
+    FlowF32Args a{};
+    size_t bytes = 0;
+    if (!flow_f32_smem(g, R, a, bytes)) continue;
+    const double t = ceil(ceil((double)n / R) / sms);
+    const double r = ceil(t / (2 * (bytes + 1024) <= 228 * 1024 ? 2 : 1));
+    const double est = R == 16 ? 5.4 + r * (1.5 + 0.256 * S + 1.41 * G) + t * (0.256 * S + 0.05 * G)
+                               : 6.6 + r * (7.6 + 0.578 * S + 1.69 * G) + t * (0.473 * S + 0.101 * g.d);
+    if (est < best) {
+      best = est;
+      route = R;
+    }
+  }
+  return route;
+}
+
+int flow_f32_pass(const FlowF32Call& c, const FlowGeom& g, int R, cudaStream_t st) {
   if (c.n <= 0) return FMC_OK;
   FlowF32Args a{};
   size_t bytes = 0;
-  const bool wide = flow_f32_tile(g, c.n) == 64 && flow_f32_smem(g, 64, a, bytes);
-  if (!wide && !flow_f32_smem(g, 16, a, bytes)) {
+  if (!flow_f32_smem(g, R, a, bytes)) {
     set_error("flow does not fit the fused FP32 kernel");
     return FMC_ERR_UNSUPPORTED;
   }
@@ -62,8 +112,7 @@ int flow_f32_pass(const FlowF32Call& c, const FlowGeom& g, cudaStream_t st) {
   a.logp = c.logp;
   a.save = c.save;
   a.acts = c.acts;
-  a.tiles = (c.n + (wide ? 64 : 16) - 1) / (wide ? 64 : 16);
-  const int R = wide ? 64 : 16;
+  a.tiles = (c.n + R - 1) / R;
   if (c.acts != nullptr) return launch_flow_f32_save(a, R, bytes, st);
   return c.inverse ? launch_flow_f32_inv(a, R, bytes, st) : launch_flow_f32_fwd(a, R, bytes, st);
 }

@@ -27,10 +27,12 @@ struct FlowF32Call {
 
 // whether the flow's row tile fits in shared memory
 bool flow_f32_fused(const FlowGeom& g);
-// rows per CTA (and per tile of the saved activations) for n rows
+// rows per CTA of a forward or inverse pass over n rows; 0: the launches per layer are faster
+int flow_f32_route(const FlowGeom& g, int64_t n);
+// rows per CTA and per tile of the saved activations when training on n rows
 int flow_f32_tile(const FlowGeom& g, int64_t n);
-// all layers over c.n rows in one launch
-int flow_f32_pass(const FlowF32Call& c, const FlowGeom& g, cudaStream_t st);
+// all layers over c.n rows in one launch of R-row tiles
+int flow_f32_pass(const FlowF32Call& c, const FlowGeom& g, int R, cudaStream_t st);
 
 // floats of split-K partials the FP32 weight gradients may use (they bound the
 // number of slices, and with it the order of the sums)

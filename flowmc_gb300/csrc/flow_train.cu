@@ -458,7 +458,7 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     c.logp = w.logp;
     c.save = w.xs;
     c.acts = w.f32;
-    if ((rc = flow_f32_pass(c, g, st))) return rc;
+    if ((rc = flow_f32_pass(c, g, flow_f32_tile(g, n), st))) return rc;
     k_loss<<<1, 1024, 0, st>>>(w.logp, n, loss);
     FMC_LAUNCH_CHECK();
     return flow_f32_grad(g, f->theta, f->aux, n, w.xs, w.f32, grad, st);
