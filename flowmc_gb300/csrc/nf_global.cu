@@ -6,9 +6,10 @@
 //   2. flow log_prob of the proposals and of the current positions in one
 //      pass (NF_proposal.py:44, 165-166: the proposals' flow density is
 //      recomputed by the forward pass, not taken from the inverse)
-//   3. k_nf_accept: the target log-density of each proposal, each chain's
+//   3. k_nf_accept or k_nf_walk: the target log-density of each proposal, each chain's
 //      sequential independent-MH scan (NF_proposal.py:91-126) and the thinned
 //      buffer writes, fused in one kernel.
+#include <algorithm>
 #include "flow.cuh"
 #include "targets.cuh"
 
@@ -32,17 +33,18 @@ struct NfArgs {
   int64_t buf_len, start;
   float *x_last, *lp_last;
   int32_t chains_per_block;
+  int32_t round_steps;   // steps of a round: min(S, kNfSteps)
   int32_t tab_smem;   // diag Gaussian / mixture: tables staged in shared memory
   int32_t scan_off;   // floats of dynamic shared memory before the scan's arrays
   int32_t vec;        // rows are whole 16-byte chunks everywhere
 };
 
 // The accept scan. Only the scan itself is sequential, and it needs three
-// numbers per proposal, so a block takes CB chains and, for up to kNfSteps steps
-// at a time: (1) its lane groups evaluate the proposals' target log-densities in
+// numbers per proposal, so a block takes CB chains and, a round of up to kNfSteps
+// steps at a time: (1) its lane groups evaluate the proposals' target log-densities in
 // parallel, (2) one thread per chain runs the accepts over shared memory and
 // notes which proposal each step holds, (3) the groups copy those rows to the
-// buffers. A group walking its chain's steps one after the other (before) waited
+// buffers. A group walking its chain's steps one after the other (k_nf_walk) waits
 // for a proposal's row and a full evaluation at every step: 4096 chains x 50
 // steps of the 64-D mixture 160 -> 78 us, 20 chains x 30 steps of the 5-D dual moon
 // 30 -> 8 us (GB300). Bound by HBM for many chains, by one evaluation and the scan's
@@ -64,8 +66,8 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
       stage = smem;
     }
   }
-  const int n = CB * kNfSteps;
-  float* lp_s = smem + a.scan_off;          // [CB][kNfSteps] per proposal
+  const int pitch = a.round_steps | 1, n = CB * pitch;   // odd: the scan's threads on different banks
+  float* lp_s = smem + a.scan_off;          // [CB][pitch] per proposal
   float* lnf_s = lp_s + n;
   float* logu_s = lnf_s + n;
   int* held_s = reinterpret_cast<int*>(logu_s + n);   // step whose proposal is held (-1: the start), * 2 + accepted
@@ -99,8 +101,8 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
         rec[i] = -1;
       }
     }
-    for (int s0 = 0; s0 < a.S; s0 += kNfSteps) {
-      const int ns = min(kNfSteps, a.S - s0);
+    for (int s0 = 0; s0 < a.S; s0 += a.round_steps) {
+      const int ns = min(a.round_steps, a.S - s0);
       const int items = nb * ns;
       for (int i0 = 0; i0 < items; i0 += gpb) {
         const bool act = i0 + gib < items;
@@ -115,7 +117,7 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
         }
         const float lpp = target_eval<TGT, G, V, false>(a.tgt, tc, p, g, gl, stage);
         if (act && gl == 0) {
-          const int q = ci * kNfSteps + si;
+          const int q = ci * pitch + si;
           lp_s[q] = lpp;
           lnf_s[q] = __ldg(a.lnf + row);
           logu_s[q] = logf(a.unif ? __ldg(a.unif + row)
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
         float lp = cur_lp[tid], lnf = cur_lnf[tid];
         int held = cur[tid];
         for (int si = 0; si < ns; ++si) {
-          const int q = tid * kNfSteps + si;
+          const int q = tid * pitch + si;
           const float lpp = lp_s[q], lnfp = lnf_s[q];
           // ratio = (lp_p - lp_c) - (lnf_p - lnf_c)   (NF_proposal.py:102-104)
           const ff ratio = ff_add(two_sum(lpp, -lp), ff_neg(two_sum(lnfp, -lnf)));
@@ -153,7 +155,7 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
         const int ci = i / ns, si = i - ci * ns, s = s0 + si;
         if (s % a.thin != 0) continue;
         const int64_t c = c0 + ci, orow = c * a.buf_len + a.start + s / a.thin;
-        const int h = held_s[ci * kNfSteps + si], held = h >> 1;
+        const int h = held_s[ci * pitch + si], held = h >> 1;
         const float* src = held < 0 ? a.x0 + c * d : a.props + (c * a.S + held) * d;
         float* dst = a.out_pos + orow * d;
         if (a.vec) {
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
           for (int j = gl; j < d; j += G) __stcs(dst + j, __ldg(src + j));
         }
         if (gl == 0) {
-          __stcs(a.out_logp + orow, lp_s[ci * kNfSteps + si]);
+          __stcs(a.out_logp + orow, lp_s[ci * pitch + si]);
           __stcs(a.out_acc + orow, (h & 1) ? 1.f : 0.f);
         }
       }
@@ -178,13 +180,106 @@ __global__ void __launch_bounds__(256) k_nf_accept(const NfArgs a) {
   }
 }
 
+// The scan for launches with enough chains to hide its latency: a lane group walks
+// its chain's steps one after the other, evaluating each proposal as it comes and
+// keeping the held position in registers, so that every proposal is read once
+// and nothing is staged. Same bits as k_nf_accept.
+template <int TGT, int G, int V>
+__global__ void __launch_bounds__(256) k_nf_walk(const NfArgs a) {
+  extern __shared__ __align__(16) float smem[];
+  const int gl = threadIdx.x % G, gib = threadIdx.x / G, gpb = blockDim.x / G, gpw = 32 / G;
+  const int d = a.d;
+  float* stage = nullptr;
+  const TargetConst<TGT> tc(a.tgt);
+  if constexpr (TGT == FMC_TARGET_DENSE_GAUSSIAN) {
+    stage = smem + gib * d;
+  } else if constexpr (TGT == FMC_TARGET_DIAG_GAUSSIAN || TGT == FMC_TARGET_GAUSS_MIXTURE) {
+    if (a.tab_smem) {
+      stage_target_table<G, V>(a.tgt, smem);
+      __syncthreads();
+      stage = smem;
+    }
+  }
+  const Rng rng = a.rng.at_epoch();
+  const int64_t c_pad = ((int64_t)a.C + gpw - 1) / gpw * gpw;   // whole warps (the evaluations shuffle)
+  for (int64_t c = (int64_t)blockIdx.x * gpb + gib; c < c_pad; c += (int64_t)gridDim.x * gpb) {
+    const bool active = c < a.C;
+    const int64_t cc = active ? c : 0;
+    float x[V], g[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const int j = gl * V + v;
+      x[v] = (j < d) ? __ldg(a.x0 + cc * d + j) : 0.f;
+    }
+    float lp = target_eval<TGT, G, V, false>(a.tgt, tc, x, g, gl, stage);   // take_steps.py:201-203
+    float lnf = __ldg(a.lnf + (int64_t)a.C * a.S + cc);
+    float xr[V], lpr = lp;
+#pragma unroll
+    for (int v = 0; v < V; ++v) xr[v] = x[v];
+    for (int s = 0; s < a.S; ++s) {
+      const int64_t row = cc * a.S + s;
+      float p[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int j = gl * V + v;
+        p[v] = (j < d) ? __ldg(a.props + row * d + j) : 0.f;
+      }
+      const float lpp = target_eval<TGT, G, V, false>(a.tgt, tc, p, g, gl, stage);
+      const float lnfp = __ldg(a.lnf + row);
+      const float u = a.unif ? __ldg(a.unif + row) : u32_to_unit(rng.draw(cc, s, 0u, RNG_TAG_NF_UNIFORM).x);
+      // ratio = (lp_p - lp_c) - (lnf_p - lnf_c)   (NF_proposal.py:102-104)
+      const ff ratio = ff_add(two_sum(lpp, -lp), ff_neg(two_sum(lnfp, -lnf)));
+      const bool acc = f_lt_ff(logf(u), ratio);
+      if (acc) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) x[v] = p[v];
+        lp = lpp;
+        lnf = lnfp;
+      }
+      if (s % a.thin == 0) {
+        if (active) {
+          const int64_t orow = cc * a.buf_len + a.start + s / a.thin;
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            const int j = gl * V + v;
+            if (j < d) __stcs(a.out_pos + orow * d + j, x[v]);
+          }
+          if (gl == 0) {
+            __stcs(a.out_logp + orow, lp);
+            __stcs(a.out_acc + orow, acc ? 1.f : 0.f);
+          }
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) xr[v] = x[v];
+        lpr = lp;
+      }
+    }
+    if (active) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int j = gl * V + v;
+        if (j < d) a.x_last[cc * d + j] = xr[v];
+      }
+      if (gl == 0 && a.lp_last) a.lp_last[cc] = lpr;
+    }
+  }
+}
+
 template <int TGT, int G, int V>
 static int launch_nf_t(const NfArgs& a0, cudaStream_t st) {
   NfArgs a = a0;
   const int threads = 256, gpb = threads / G;
-  // one chain per block until they fill the SMs several times over, then four
-  // (fewer idle groups at the end of a chain's steps)
-  a.chains_per_block = a.C <= 8 * sm_count() ? 1 : 4;
+  // Chains of a block of k_nf_accept: enough to give every SM eight blocks (four of
+  // the dense Gaussian's, which fill its registers), in whole rounds of them, with at most 512 proposals a round and no more chains than the
+  // scan has threads; where a chain has few steps, at least one proposal per group.
+  a.round_steps = a.S < kNfSteps ? a.S : kNfSteps;
+  {
+    const int64_t slots = (TGT == FMC_TARGET_DENSE_GAUSSIAN ? 4 : 8) * (int64_t)sm_count(), most = std::max(512 / a.round_steps, 1);
+    const int64_t rounds = (a.C + most * slots - 1) / (most * slots);
+    int64_t cb = (a.C + slots * rounds - 1) / (slots * rounds);
+    cb = std::min<int64_t>(std::max<int64_t>(cb, gpb / a.round_steps), threads);
+    a.chains_per_block = (int)std::max<int64_t>(cb, 1);
+  }
   size_t floats = (TGT == FMC_TARGET_DENSE_GAUSSIAN) ? (size_t)gpb * a.d : 0;
   a.tab_smem = 0;
   if (TGT == FMC_TARGET_DIAG_GAUSSIAN || TGT == FMC_TARGET_GAUSS_MIXTURE) {
@@ -196,13 +291,24 @@ static int launch_nf_t(const NfArgs& a0, cudaStream_t st) {
   }
   floats = (floats + 3) / 4 * 4;
   a.scan_off = (int)floats;
-  floats += (size_t)a.chains_per_block * (4 * kNfSteps + 5);
+  // From 20 warps of chains per SM on the walk's latency is hidden, and it reads the
+  // proposals once: over 21 targets of 3 to 200 dims and 1 to 200 steps the staged
+  // scan takes 1.0 to 1.5 of its time at 27 warps, up to 2.0 beyond, and 0.1 to 0.5
+  // of it for 1000 chains of 30 steps. At 13 warps it takes 0.9 to 1.4 of it up to 16
+  // steps or 8 dims, 0.6 to 1.05 otherwise. A single step has nothing to evaluate
+  // ahead. Without the walk, 65,536 chains of the 5-D dual moon took, for 1
+  // and 10 steps, 84 and 172 us, with it 15 and 64; 16,384 chains of a 64-D dense
+  // Gaussian, 1 step: 158, with it 50.
+  const double warps = (double)a.C * G / 32 / sm_count();
+  const bool walk = a.S == 1 || warps >= 20.0 || (warps >= 10.0 && (a.S <= 16 || a.d <= 8));
+  if (!walk) floats += (size_t)a.chains_per_block * (4 * (a.round_steps | 1) + 5);
   a.vec = a.d % 4 == 0 && ((uintptr_t)a.out_pos & 15) == 0 && ((uintptr_t)a.props & 15) == 0 &&
           ((uintptr_t)a.x0 & 15) == 0;
-  int64_t blocks = (a.C + a.chains_per_block - 1) / a.chains_per_block;
+  const int per_block = walk ? gpb : a.chains_per_block;
+  int64_t blocks = (a.C + per_block - 1) / per_block;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  auto kern = k_nf_accept<TGT, G, V>;
+  auto kern = walk ? k_nf_walk<TGT, G, V> : k_nf_accept<TGT, G, V>;
   const size_t smem = floats * sizeof(float);
   if (smem > 48 * 1024)
     FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
