@@ -56,6 +56,11 @@ void set_error(const char* fmt, ...);
 // and, before it reads what an earlier kernel wrote or writes anything, and
 // also on a path that does neither, chain_wait (every earlier kernel has
 // completed and its writes are visible).
+// chain_release stands behind the kernel's tensor-memory allocation: a CTA of
+// the next kernel that found room beside a CTA which had released but not yet
+// allocated could take the SM's tensor memory and hold it while it waits for
+// that very CTA. Behind the allocation no order of arrival can do that,
+// whatever shared memory the two kernels take.
 // Read-only loads (__ldg, const __restrict__) are not held back by the wait:
 // they may read theta and other inputs of the whole chain, but not what the
 // kernel before wrote; the chained kernels take that by TMA or plain loads.

@@ -308,7 +308,10 @@ __device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
 // raised (a bounded wait of an earlier tensor-core launch expired and nobody
 // cleared the word), the CTA does no work at all -- no TMEM allocation, no
 // waits -- so that a run whose tensor-core pipeline broke ends within one
-// wait bound instead of one bound per later launch. The decision is made by
+// wait bound instead of one bound per later launch. A chained launch reads the
+// word before the kernel ahead of it has ended (behind chain_wait the read
+// would lengthen every launch), so the one launch right behind a broken kernel
+// may still do its ordinary work. The decision is made by
 // one thread and shared, so every thread of the CTA takes the same branch.
 __device__ __forceinline__ bool tc_skip(const int* err) {
   __shared__ int s_skip;
@@ -355,7 +358,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   static_assert(NSTG == 1 || NSTG == 2, "one or two staging buffers per warp");
   static_assert(OPM == 0 || (PAIR ? BN / 2 : BN) % 64 == 0, "MN-major operands: whole 64-wide blocks per CTA");
   constexpr bool kBiasSmem = NSTG == 2;
-  chain_release();
   if (PAIR ? tc_skip_pair(err) : tc_skip(err)) {
     chain_wait();
     return;
@@ -420,7 +422,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   if constexpr (PAIR) cluster_sync_all();   // both CTAs' barriers exist before either signals the other's
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  chain_wait();   // barriers and TMEM are set up while the kernel before ends
+  chain_release();   // the next kernel's CTAs come after this one's tensor memory (common.cuh)
+  chain_wait();      // barriers and TMEM are set up while the kernel before ends
 
   if (warp == 0) {
     if (lane == 0) {

@@ -386,7 +386,6 @@ __global__ void __launch_bounds__(kSplThreads, 1)
   constexpr int P = T::P, DG = T::DG, BN = T::BN, E = kSplineEpiPerQuarter, PP = BiasRows<KB>::PP;
   using X = XBox<DG>;
   using S = SplSmem<BN, STAGES, CH>;
-  chain_release();
   if (tc_skip(err)) {
     chain_wait();
     return;
@@ -411,7 +410,8 @@ __global__ void __launch_bounds__(kSplThreads, 1)
   const int nk = (K + BK * CH - 1) / (BK * CH);   // stages per tile (K a multiple of BK * CH when CH > 1)
   const int tiles = (M + BM - 1) / BM * n_groups;
   const Pipe p = pipe_setup<STAGES>(base, bars, warp);
-  chain_wait();   // barriers and TMEM are set up while the kernel before ends
+  chain_release();   // the next kernel's CTAs come after this one's tensor memory (common.cuh)
+  chain_wait();      // barriers and TMEM are set up while the kernel before ends
   if (bias_smem) {
     for (int i = threadIdx.x; i < nt * PP; i += blockDim.x) {
       const int t = i / PP, pp = i - t * PP;
@@ -635,7 +635,6 @@ __global__ void __launch_bounds__(kSplThreads, 1)
   constexpr int RROWS = (BM + RP - 1) / RP;        // rows per column-sum part
   using X = XBox<DG>;
   using S = SplSmem<BN, STAGES, 1>;
-  chain_release();
   if (tc_skip(err)) {
     chain_wait();
     return;
@@ -661,7 +660,8 @@ __global__ void __launch_bounds__(kSplThreads, 1)
   const int tiles = (M + BM - 1) / BM * n_groups;
   const int ntP = a.nt * P;
   const Pipe p = pipe_setup<STAGES>(base, bars, warp);
-  chain_wait();   // barriers and TMEM are set up while the kernel before ends
+  chain_release();   // the next kernel's CTAs come after this one's tensor memory (common.cuh)
+  chain_wait();      // barriers and TMEM are set up while the kernel before ends
 
   if (warp == 0) {
     if (lane == 0) producer<BN, STAGES, 1>(p, &tmA, &tmB, tiles, n_groups, nk);
