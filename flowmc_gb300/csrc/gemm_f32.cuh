@@ -213,14 +213,15 @@ __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_
 // the wide tiles would leave SMs idle, 64 x 32 of two warps times four input
 // groups ([16384 x 512] x [512 x 32] 32 -> 25 us)
 //
-// SEQ: an output's products added one by one in the order of the inputs, for
-// the forward that a gradient keeps. A relu's derivative jumps where its
-// input is 0, so a last bit there shows in the gradient (1e-6 of it for one
-// row of 16,384); in this order the bits do not depend on the tile. Packed
-// sums of even and odd inputs, and of input groups, otherwise. Loss
-// and gradient of 16,384 rows (32-D, 8 layers, H = 256): 1.30 ms packed, 1.29 in order.
-template <int EPI, bool SEQ = false>
+// The forward epilogues (SEQ) add an output's products one by one in the order
+// of the inputs, so that the bits do not depend on the tile: a row's results are the
+// same in a call of one row and of a million, the loss is that of log_prob,
+// and the relu derivative of a kept activation, which jumps where its input is 0,
+// is that of the forward. The gradient's products, summed over the batch anyway,
+// take packed sums of even and odd inputs, and of input groups.
+template <int EPI>
 inline int gemm_f32(cudaStream_t st, const G32Args& a, int count) {
+  constexpr bool SEQ = EPI == G32_BIAS || EPI == G32_BIAS_RELU;
   if (a.M <= 0 || a.N <= 0) return FMC_OK;
   auto go = [&](auto kern, int bm, int bn, int wk, int threads) -> int {
     const int smem = kG32Stages * wk * (bm + bn) * kG32Pitch * 4;

@@ -239,8 +239,7 @@ struct RnvpScratch {
 static const float* layer_mask(const RnvpGeom& g, const float* aux, int l) { return aux + 2 * g.d + 2 + (int64_t)l * g.d; }
 
 // the layer's conditioner on cond = x * m: h = relu(cond W1^T + b1), sraw, tt
-static int rnvp_conditioner(cudaStream_t st, const RnvpGeom& g, const float* th, int64_t rows, const RnvpScratch& s,
-                            bool seq = false) {
+static int rnvp_conditioner(cudaStream_t st, const RnvpGeom& g, const float* th, int64_t rows, const RnvpScratch& s) {
   const int d = g.d, H = g.H;
   G32Args a{};
   a.M = rows;
@@ -249,7 +248,7 @@ static int rnvp_conditioner(cudaStream_t st, const RnvpGeom& g, const float* th,
   a.ldc = 2 * H;
   a.N = 2 * H;
   a.K = d;
-  int rc = seq ? gemm_f32<G32_BIAS_RELU, true>(st, a, 1) : gemm_f32<G32_BIAS_RELU>(st, a, 1);
+  int rc = gemm_f32<G32_BIAS_RELU>(st, a, 1);
   if (rc) return rc;
   a.p[0] = G32Problem{s.h, th + g.off_W2s, th + g.off_b2s, nullptr, s.sraw};
   a.p[1] = G32Problem{s.h + H, th + g.off_W2t, th + g.off_b2t, nullptr, s.tt};
@@ -258,7 +257,7 @@ static int rnvp_conditioner(cudaStream_t st, const RnvpGeom& g, const float* th,
   a.ldc = d;
   a.N = d;
   a.K = H;
-  return seq ? gemm_f32<G32_BIAS, true>(st, a, 2) : gemm_f32<G32_BIAS>(st, a, 2);
+  return gemm_f32<G32_BIAS>(st, a, 2);
 }
 
 // all layers, in place on x [rows, d] (forward: 0..L-1, inverse: L-1..0); ld = the summed log-det
@@ -481,7 +480,7 @@ extern "C" int fmc_rnvp_loss_grad(const FmcRealNVP* flow, const float* x, int64_
   FMC_LAUNCH_CHECK();
   for (int l = 0; l < g.L; ++l) {
     const RnvpScratch s{cond + l * nd, h + l * nh, sraw + l * nd, tt + l * nd};
-    rc = rnvp_conditioner(st, g, flow->theta + (int64_t)l * g.per_layer, n, s, true);
+    rc = rnvp_conditioner(st, g, flow->theta + (int64_t)l * g.per_layer, n, s);
     if (rc) return rc;
     const bool last = l + 1 == g.L;
     k_rnvp_couple<<<warp_grid(n), 256, 0, st>>>(X + l * nd, s.sraw, s.tt, layer_mask(g, flow->aux, l), n, d, g.dt, 0,
