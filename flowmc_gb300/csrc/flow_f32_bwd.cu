@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(256) k_affine_layers(const __grid_constant__ F
   affine_sums(n, d, part + (int64_t)l * gridDim.x * 2, [&](int64_t r, int j, float& g, float& x, float& gv) {
     g = ga[r * d + j];
     x = scalar_affine(xin[r * d + j], es, sh, 0);
-    gv = g * es;
+    gv = __fmul_rn(g, es);
   });
 }
 
@@ -480,10 +480,12 @@ static GradWs grad_ws(const FlowGeom& g, int64_t n) {
   w.gout = al(s.gcol(g.L, 0) * rows);
   w.gaff = al((int64_t)g.L * n * g.d);
   const int64_t pf = kouter_part_floats(g);
+  int64_t most[2] = {0, 0};   // floats of a layer's partials, a bound that grows with n
   for (int l = 0; l < 2; ++l) {
     int64_t off = 0;
     for (int i = 0; i <= g.nh; ++i) {
       w.per_pair += wg_items(s, l, i);
+      most[l] += kouter_most_slices(s.out(l, i), s.in(l, i), n, true, pf) * s.out(l, i) * s.in(l, i);
       w.z.count[l][i] = (int)kouter_slices(s.out(l, i), s.in(l, i), n, true, pf, &w.z.rows[l][i]);
       if (w.z.count[l][i] > w.slices) w.slices = w.z.count[l][i];
       w.z.part_off[l][i] = off;
@@ -491,7 +493,7 @@ static GradWs grad_ws(const FlowGeom& g, int64_t n) {
     }
     w.z.part_layer[l] = off;
   }
-  w.part = al((int64_t)(g.L / 2) * (w.z.part_layer[0] + w.z.part_layer[1]) + (g.L & 1) * w.z.part_layer[0]);
+  w.part = al((int64_t)(g.L / 2) * (most[0] + most[1]) + (g.L & 1) * most[0]);
   w.rb = colsum_blocks(n);
   w.bpart = al(s.gcol(g.L, 0) * w.rb);
   w.ab = affine_sum_blocks(n, g.d);

@@ -41,12 +41,16 @@ struct TrainWs {
   int64_t n128, n64, hld, ncld, pld;
 };
 
-// The BF16 forward's conditioning operands and hidden activations, kept for the
-// backward up to this many bytes of workspace (recomputed layer by layer in
-// one layer's buffers beyond). At 65,536 rows, 128 dims, 12 layers, two hidden
-// layers of 512 they are 1.7 GB and save 24 GEMMs and 12 affine passes.
-// A step there takes 10.2 ms with them kept (and the affine folded into the
-// kept forward) and 11.1 ms recomputed.
+// What the forward keeps for the backward, up to this many bytes of workspace:
+// BF16 the conditioning operands and hidden activations of every layer, FP32 (on
+// the fused path) every layer's activations, beside them the output gradients.
+// Beyond, and where the caller's workspace holds no more, they are recomputed
+// layer by layer in one layer's buffers, so that a batch needs little more
+// than its layers' inputs. BF16, 65,536 rows, 128 dims, 12 layers, two hidden
+// layers of 512: 1.7 GB, which save 24 GEMMs and 12 affine passes, a step 10.2 ms
+// with them kept (and the affine folded into the kept forward) and 11.1 ms
+// recomputed. FP32, 32 dims, 8 layers, two of 128, 10 bins: 0.9 GB for 16,384
+// rows, without the bound 51 GB for a million (7.7 GB layer by layer).
 constexpr int64_t kKeepBytes = (int64_t)16 << 30;
 
 // Input-gradient GEMMs from this depth on run on CTA pairs (half the weight
@@ -58,7 +62,8 @@ static bool dgrad_pairs(int64_t n, int in, int depth) {
   return depth >= 1024 && n * in >= (int64_t)sm_count() * 128 * 256;
 }
 
-static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, TrainWs& w, size_t* total) {
+// keep: the layout that keeps every layer's activations (train_keeps says where there is one)
+static void carve_train(const FlowGeom& g, int64_t n, bool bf16, bool keep, void* ws, TrainWs& w, size_t* total) {
   char* p = (char*)ws;
   int64_t used = 0;
   auto take = [&](int64_t floats) {
@@ -74,7 +79,7 @@ static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, Train
   const int64_t ntP = (int64_t)g.nt_max() * g.P;
   w.xs = take((int64_t)(g.L + 1) * n * g.d);
   w.f32 = nullptr;
-  if (!bf16 && flow_f32_grad_fits(g, n)) {
+  if (!bf16 && keep) {
     w.logp = take(n);
     w.f32 = take(flow_f32_grad_floats(g, n));
     if (total) *total = (size_t)used;
@@ -116,7 +121,7 @@ static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, Train
     w.pld = FlowGeom::rup((int64_t)g.nt_max() * g.spl_opc, 64);   // padded d-raw rows
     w.cond_ls = w.n128 * w.ncld;
     w.hs_ls = (int64_t)g.nh * w.n128 * w.hld;
-    w.keep = 2 * g.L * (w.cond_ls + w.hs_ls) <= kKeepBytes;
+    w.keep = keep;
     w.cond16 = take16((w.keep ? g.L : 1) * w.cond_ls);
     w.hs16 = take16((w.keep ? g.L : 1) * w.hs_ls);
     w.graw16 = take16(w.n128 * w.pld);
@@ -140,11 +145,22 @@ static void carve_train(const FlowGeom& g, int64_t n, bool bf16, void* ws, Train
   if (total) *total = (size_t)used;
 }
 
-size_t train_ws_bytes(const FlowGeom& g, int64_t n, bool bf16) {
+// whether the activations of n rows may be kept
+static bool train_keeps(const FlowGeom& g, int64_t n, bool bf16) {
+  if (!bf16) return flow_f32_grad_fits(g, n) && 4 * flow_f32_grad_floats(g, n) <= kKeepBytes;
+  const int64_t n128 = FlowGeom::rup(n, 128);
+  return 2 * g.L * n128 * (FlowGeom::rup(g.nc_max(), 64) + g.nh * FlowGeom::rup(g.h_max(), 64)) <= kKeepBytes;
+}
+
+static size_t train_ws_bytes(const FlowGeom& g, int64_t n, bool bf16, bool keep) {
   TrainWs w;
   size_t tot = 0;
-  carve_train(g, n, bf16, nullptr, w, &tot);
+  carve_train(g, n, bf16, keep, nullptr, w, &tot);
   return tot;
+}
+
+size_t train_ws_bytes(const FlowGeom& g, int64_t n, bool bf16) {
+  return train_ws_bytes(g, n, bf16, train_keeps(g, n, bf16));
 }
 
 // ------------------------------------------------------------------ kernels
@@ -278,7 +294,7 @@ __global__ void __launch_bounds__(256) k_affine_bwd(const float* __restrict__ gx
         x = xa[r * d + j];
       },
       [&](int64_t r, int j, float g) {
-        const float gv = g * es;
+        const float gv = __fmul_rn(g, es);
         gx[r * d + j] = gv;
         return gv;
       });
@@ -430,12 +446,20 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
   FMC_CHECK_ARG(n >= 1, "n=%lld < 1", (long long)n);
   FMC_CHECK_ARG(x && loss && grad, "NULL array");
   const bool bf16 = f->precision == FMC_PREC_BF16;
-  const size_t need = train_ws_bytes(g, n, bf16);
+  // The activations are kept where the workspace holds them. It may hold less: one
+  // sized for a larger batch, beyond the bound, serves every smaller one.
+  bool keep_all = train_keeps(g, n, bf16);
+  size_t need = train_ws_bytes(g, n, bf16, keep_all);
+  if (keep_all && ws_bytes < need) {
+    const size_t lean = train_ws_bytes(g, n, bf16, false);
+    keep_all = need <= lean;   // a flow of one layer or two may need less with them
+    need = need < lean ? need : lean;
+  }
   FMC_CHECK_ARG(ws && ws_bytes >= need, "workspace of %zu bytes < %zu needed", ws_bytes, need);
   FMC_CHECK_ARG(((uintptr_t)ws & 255) == 0, "workspace must be 256-byte aligned");
   if (bf16) FMC_CHECK_ARG(f->theta_bf16 != nullptr, "BF16 mode needs theta_bf16");
   TrainWs w;
-  carve_train(g, n, bf16, ws, w, nullptr);
+  carve_train(g, n, bf16, keep_all, ws, w, nullptr);
   const int d = g.d;
   const int64_t nd = n * d;
   const int eb = ew_blocks(nd);

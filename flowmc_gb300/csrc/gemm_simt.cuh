@@ -184,10 +184,10 @@ __global__ void k_sum_slices(const float* __restrict__ part, int S, int64_t mn, 
   }
 }
 
-// slices of the K rows for an [M, N] output: enough 64 x 64 tiles for two blocks
-// per SM, at least 256 rows each, as many as part_floats floats of partials
-// hold; *kslice: rows per slice (whole 16-row steps)
-inline int64_t kouter_slices(int M, int N, int64_t K, bool has_part, int64_t part_floats, int64_t* kslice) {
+// most slices of the K rows for an [M, N] output (it only grows with K): enough
+// 64 x 64 tiles for two blocks per SM, at least 256 rows each, as many as
+// part_floats floats of partials hold
+inline int64_t kouter_most_slices(int M, int N, int64_t K, bool has_part, int64_t part_floats) {
   const int64_t mn = (int64_t)M * N;
   const int64_t tiles = (int64_t)((N + 63) / 64) * ((M + 63) / 64);
   int64_t S = (2 * (int64_t)sm_count() + tiles - 1) / tiles;
@@ -195,7 +195,12 @@ inline int64_t kouter_slices(int M, int N, int64_t K, bool has_part, int64_t par
   if (S > by_rows) S = by_rows;
   if (S > kKouterMaxSlices) S = kKouterMaxSlices;
   if (!has_part || S * mn > part_floats) S = has_part ? part_floats / mn : 1;
-  if (S < 1) S = 1;
+  return S < 1 ? 1 : S;
+}
+
+// the slices taken: *kslice rows each (whole 16-row steps), at most the above
+inline int64_t kouter_slices(int M, int N, int64_t K, bool has_part, int64_t part_floats, int64_t* kslice) {
+  int64_t S = kouter_most_slices(M, N, K, has_part, part_floats);
   *kslice = (((K + S - 1) / S) + 15) / 16 * 16;
   S = (K + *kslice - 1) / *kslice;
   return S < 1 ? 1 : S;

@@ -39,7 +39,9 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
 }
 
 // Per-block sums (256 threads) of gv = g * es and g * x over all rows: one warp
-// per row, rows strided over the grid. get(r, j, g, x, gv) gives the values.
+// per row, rows strided over the grid. get(r, j, g, x, gv) gives the values (gv
+// rounded, __fmul_rn: the compiler would fold the product into the sum where it
+// is not stored, and the two paths would differ in the last place).
 template <typename F>
 __device__ __forceinline__ void affine_sums(int64_t n, int d, float* part, F get) {
   __shared__ float sh[32];
@@ -51,7 +53,7 @@ __device__ __forceinline__ void affine_sums(int64_t n, int d, float* part, F get
       float g, x, gv;
       get(r, j, g, x, gv);
       st += gv;
-      ss += g * x;
+      ss = __fmaf_rn(g, x, ss);
     }
   st = block_sum<256>(st, sh);
   ss = block_sum<256>(ss, sh);
@@ -71,7 +73,7 @@ __device__ __forceinline__ void affine_sums_ahead(int64_t n, int d, float* part,
   float st = 0.f, ss = 0.f;
   auto add = [&](int64_t r, int j, float g, float x) {
     st += use(r, j, g);
-    ss += g * x;
+    ss = __fmaf_rn(g, x, ss);
   };
   int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   for (; r < n; r += warps)

@@ -320,7 +320,9 @@ typedef struct FmcFlow {
 FMC_API int fmc_flow_layout(const FmcFlow* flow, int64_t* n_params, int64_t* layer_offsets);
 
 /* Bytes of workspace the flow entry points need for n rows (host call).
- * mode 0: log_prob / forward / inverse / sample;  1: loss + gradient. */
+ * mode 0: log_prob / forward / inverse / sample;  1: loss + gradient (a
+ * workspace of that size serves every smaller n too; the loss and gradient also
+ * run in less, where the forward's activations are recomputed, not kept). */
 FMC_API int fmc_flow_workspace_size(const FmcFlow* flow, int64_t n, int32_t mode, size_t* bytes);
 
 /* BF16 mode: theta_bf16 holds each Linear weight as a zero-padded bf16 block
