@@ -179,6 +179,10 @@ __global__ void k_rnvp_bias_final(RnvpGeom g, const float* __restrict__ part, in
   for (int b = 0; b < rb; ++b) v += p[b];
   grad[l * g.per_layer + off + c] = v;
 }
+__global__ void k_rnvp_add(const float* __restrict__ part, int64_t n, float* __restrict__ grad) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
+    grad[e] += part[e];
+}
 // grad = sum of the slices (bias entries are overwritten by k_rnvp_bias_final)
 __global__ void k_rnvp_sum_slices(const float* __restrict__ part, int S, int64_t n, float* __restrict__ grad) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
@@ -301,8 +305,8 @@ static int carve_infer(const RnvpGeom& g, int64_t rows, void* ws, size_t ws_byte
 }
 
 // row slices of the weight gradients: enough 256 x 32 tiles for two CTAs per SM,
-// at least 256 rows each
-static int wgrad_slices(const RnvpGeom& g, int64_t n, int64_t* rows_per) {
+// at least 256 rows each (*most: a bound that only grows with n)
+static int wgrad_slices(const RnvpGeom& g, int64_t n, int64_t* rows_per, int64_t* most = nullptr) {
   auto tiles = [](int64_t M, int64_t N) { return ((M + kK32M - 1) / kK32M) * ((N + kK32N - 1) / kK32N); };
   const int64_t per = g.L * (tiles(2 * g.H, g.d) + 2 * tiles(g.H, g.d));
   int64_t S = (4 * (int64_t)sm_count() + per - 1) / per;
@@ -310,6 +314,7 @@ static int wgrad_slices(const RnvpGeom& g, int64_t n, int64_t* rows_per) {
   if (S > by_rows) S = by_rows;
   if (S > kMaxSlices) S = kMaxSlices;
   if (S < 1) S = 1;
+  if (most) *most = S;
   *rows_per = ((n + S - 1) / S + kG32BK - 1) / kG32BK * kG32BK;
   return (int)((n + *rows_per - 1) / *rows_per);
 }
@@ -319,13 +324,30 @@ static int bias_blocks(int64_t n) {
   return (int)(b < 1 ? 1 : b > 128 ? 128 : b);
 }
 
-// every layer's input, masked input, hidden activations, conditioner outputs
-// (later their gradients) and hidden gradients; two input gradients
+// Rows of a training chunk. A row keeps every layer's input, masked input, hidden
+// activations, conditioner outputs (later their gradients) and hidden gradients,
+// and two input gradients: 37 KB for 32 dims, 8 layers, H = 256. A batch runs in
+// chunks of as many rows as kRnvpKeepBytes hold (461,000 there), their gradients
+// added in order, so that the workspace grows by four bytes a row from there on: a
+// million rows took 34.7 GiB without the chunks and take 16 with them.
+constexpr size_t kRnvpKeepBytes = (size_t)16 << 30;
+static size_t keep_floats_per_row(const RnvpGeom& g) {
+  const size_t d = g.d, H = g.H, L = g.L;
+  return (L + 1) * d + L * (3 * d + 4 * H) + 2 * d + 1;
+}
+static int64_t train_chunk(const RnvpGeom& g, int64_t n) {
+  const int64_t most = (int64_t)(kRnvpKeepBytes / (4 * keep_floats_per_row(g))) / 256 * 256;
+  const int64_t rows = most < 256 ? 256 : most;
+  return n < rows ? n : rows;
+}
+
 static size_t train_floats(const RnvpGeom& g, int64_t n) {
   const size_t d = g.d, H = g.H, L = g.L;
-  int64_t rp;
-  return (size_t)n * ((L + 1) * d + L * (3 * d + 4 * H) + 2 * d + 2) + (size_t)wgrad_slices(g, n, &rp) * g.n_params +
-         L * 4 * H * d + L * (2 * H + 2 * d) * bias_blocks(n) + 64 * 12;
+  const int64_t m = train_chunk(g, n);
+  int64_t rp, most;
+  wgrad_slices(g, m, &rp, &most);
+  return (size_t)m * keep_floats_per_row(g) + (size_t)n + (size_t)(most + 1) * g.n_params + L * 4 * H * d +
+         L * (2 * H + 2 * d) * bias_blocks(m) + 64 * 14;
 }
 
 }  // namespace fmc
@@ -449,111 +471,122 @@ extern "C" int fmc_rnvp_loss_grad(const FmcRealNVP* flow, const float* x, int64_
                 "workspace of %zu bytes is smaller than fmc_rnvp_workspace_size", ws_bytes);
   cudaStream_t st = (cudaStream_t)stream;
   const int d = g.d, H = g.H;
-  const int64_t nd = n * d, nh = n * 2 * (int64_t)H;
+  const int64_t chunk = train_chunk(g, n);
+  const int64_t cd = chunk * d, ch = chunk * 2 * (int64_t)H;
   float* p = (float*)ws;
   auto take = [&](int64_t floats) {
     float* r = p;
     p += (floats + 63) / 64 * 64;   // 256-byte pieces: 16-byte copies where the shapes allow them
     return r;
   };
-  float* X = take((g.L + 1) * nd);   // layer inputs, X[L] = y
-  float* cond = take(g.L * nd);
-  float* sraw = take(g.L * nd);
-  float* tt = take(g.L * nd);
-  float* h = take(g.L * nh);
-  float* dz = take(g.L * nh);
-  float* gy = take(nd);
-  float* gx = take(nd);
-  float* ld = take(n);
+  float* X = take((g.L + 1) * cd);   // layer inputs, X[L] = y
+  float* cond = take(g.L * cd);
+  float* sraw = take(g.L * cd);
+  float* tt = take(g.L * cd);
+  float* h = take(g.L * ch);
+  float* dz = take(g.L * ch);
+  float* gin[2] = {take(cd), take(cd)};
+  float* ld = take(chunk);
   float* logp = take(n);
   float* wt = take((int64_t)g.L * 4 * H * d);
-  const int rb = bias_blocks(n);
-  float* bpart = take((int64_t)g.L * (2 * H + 2 * d) * rb);
+  float* bpart = take((int64_t)g.L * (2 * H + 2 * d) * bias_blocks(chunk));
+  float* cgrad = take(g.n_params);   // a later chunk's gradient
   float* part = p;
-  int64_t rows_per = 0;
-  const int slices = wgrad_slices(g, n, &rows_per);
-
-  // forward, keeping every layer's activations
-  k_standardize<<<grid_for(n * d), 256, 0, st>>>(x, n, d, flow->aux, X);
-  FMC_LAUNCH_CHECK();
-  k_rnvp_cond<<<grid_for(n * d), 256, 0, st>>>(X, layer_mask(g, flow->aux, 0), n, d, cond);
-  FMC_LAUNCH_CHECK();
-  for (int l = 0; l < g.L; ++l) {
-    const RnvpScratch s{cond + l * nd, h + l * nh, sraw + l * nd, tt + l * nd};
-    rc = rnvp_conditioner(st, g, flow->theta + (int64_t)l * g.per_layer, n, s);
-    if (rc) return rc;
-    const bool last = l + 1 == g.L;
-    k_rnvp_couple<<<warp_grid(n), 256, 0, st>>>(X + l * nd, s.sraw, s.tt, layer_mask(g, flow->aux, l), n, d, g.dt, 0,
-                                                X + (l + 1) * nd, ld, l == 0 ? 1 : 0,
-                                                last ? nullptr : layer_mask(g, flow->aux, l + 1),
-                                                last ? nullptr : cond + (l + 1) * nd);
-    FMC_LAUNCH_CHECK();
-  }
-  float* y = X + (int64_t)g.L * nd;
-  k_rnvp_logprob<<<warp_grid(n), 256, 0, st>>>(y, ld, n, d, logp);
-  FMC_LAUNCH_CHECK();
-  k_rnvp_loss<<<1, 1024, 0, st>>>(logp, n, loss);
-  FMC_LAUNCH_CHECK();
-
-  // backward: loss = -mean(ld + log N(y)) -> dL/dy = y / n, dL/d ld = -1 / n
-  k_rnvp_scale<<<grid_for(n * d), 256, 0, st>>>(y, n * d, 1.f / (float)n, gy);
-  FMC_LAUNCH_CHECK();
   k_rnvp_transpose<<<dim3((unsigned)grid_for(4ll * H * d, 1), (unsigned)g.L), 256, 0, st>>>(flow->theta, g, wt);
   FMC_LAUNCH_CHECK();
   const float gld = -1.f / (float)n;
-  for (int l = g.L - 1; l >= 0; --l) {
-    const float* m = layer_mask(g, flow->aux, l);
-    const float* wl = wt + (int64_t)l * 4 * H * d;
-    k_rnvp_couple_bwd<<<grid_for(n * d), 256, 0, st>>>(X + l * nd, sraw + l * nd, tt + l * nd, m, gy, n, d, g.dt, gld, gx);
-    FMC_LAUNCH_CHECK();
-    // dz = [dsraw W2s, dtt W2t] masked by relu'
-    G32Args a{};
-    a.M = n;
-    a.p[0] = G32Problem{sraw + l * nd, wl, nullptr, h + l * nh, dz + l * nh};
-    a.p[1] = G32Problem{tt + l * nd, wl + (int64_t)H * d, nullptr, h + l * nh + H, dz + l * nh + H};
-    a.lda = a.ldb = d;
-    a.ldaux = a.ldc = 2 * H;
-    a.N = H;
-    a.K = d;
-    rc = gemm_f32<G32_DRELU>(st, a, 2);
-    if (rc) return rc;
-    // gx += (dz W1) * m
-    a.p[0] = G32Problem{dz + l * nh, wl + 2ll * H * d, m, nullptr, gx};
-    a.lda = a.ldb = 2 * H;
-    a.ldc = d;
-    a.N = d;
-    a.K = 2 * H;
-    rc = gemm_f32<G32_ADD_MASKED>(st, a, 1);
-    if (rc) return rc;
-    float* t = gy;
-    gy = gx;
-    gx = t;
-  }
-  // weight and bias gradients of all layers over the batch. The second
-  // Linears' as h^T d(output), stored transposed: the wide side is the tall
-  // operand of the 256 x 32 tiles
-  K32Args k{};
-  k.p[0] = K32Problem{dz, cond, nh, nd, 2 * H, d, 2 * H, d, 0, d, 1};
-  k.p[1] = K32Problem{h, sraw, nh, nd, 2 * H, d, H, d, g.off_W2s, 1, H};
-  k.p[2] = K32Problem{h + H, tt, nh, nd, 2 * H, d, H, d, g.off_W2t, 1, H};
-  k.n_problems = 3;
-  k.rows = n;
-  k.rows_per_slice = rows_per;
-  k.per_layer = g.per_layer;
-  k.n_params = g.n_params;
-  k.part = part;
-  const unsigned tiles = (unsigned)(((2 * H + kK32M - 1) / kK32M) * ((d + kK32N - 1) / kK32N));
   constexpr int ksmem = kG32Stages * kK32StageFloats * 4;
   FMC_CUDA_TRY(cudaFuncSetAttribute(k_kouter_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, ksmem));
-  k_kouter_f32<<<dim3(tiles, (unsigned)slices, (unsigned)(3 * g.L)), kK32Threads, ksmem, st>>>(k);
-  FMC_LAUNCH_CHECK();
-  k_rnvp_sum_slices<<<grid_for(g.n_params), 256, 0, st>>>(part, slices, g.n_params, grad);
-  FMC_LAUNCH_CHECK();
-  const unsigned cb = (unsigned)((2 * H > d ? 2 * H : d) + 127) / 128;
-  k_rnvp_bias_partial<<<dim3(cb, (unsigned)rb, (unsigned)(3 * g.L)), 128, 0, st>>>(g, dz, sraw, tt, n, (n + rb - 1) / rb,
-                                                                                  bpart);
-  FMC_LAUNCH_CHECK();
-  k_rnvp_bias_final<<<dim3(cb, 1, (unsigned)(3 * g.L)), 128, 0, st>>>(g, bpart, rb, grad);
+
+  for (int64_t r0 = 0; r0 < n; r0 += chunk) {
+    const int64_t m = n - r0 < chunk ? n - r0 : chunk;
+    const int64_t nd = m * d, nh = m * 2 * (int64_t)H;
+    // forward, keeping every layer's activations
+    k_standardize<<<grid_for(nd), 256, 0, st>>>(x + r0 * d, m, d, flow->aux, X);
+    FMC_LAUNCH_CHECK();
+    k_rnvp_cond<<<grid_for(nd), 256, 0, st>>>(X, layer_mask(g, flow->aux, 0), m, d, cond);
+    FMC_LAUNCH_CHECK();
+    for (int l = 0; l < g.L; ++l) {
+      const RnvpScratch s{cond + l * nd, h + l * nh, sraw + l * nd, tt + l * nd};
+      rc = rnvp_conditioner(st, g, flow->theta + (int64_t)l * g.per_layer, m, s);
+      if (rc) return rc;
+      const bool last = l + 1 == g.L;
+      k_rnvp_couple<<<warp_grid(m), 256, 0, st>>>(X + l * nd, s.sraw, s.tt, layer_mask(g, flow->aux, l), m, d, g.dt, 0,
+                                                  X + (l + 1) * nd, ld, l == 0 ? 1 : 0,
+                                                  last ? nullptr : layer_mask(g, flow->aux, l + 1),
+                                                  last ? nullptr : cond + (l + 1) * nd);
+      FMC_LAUNCH_CHECK();
+    }
+    float* y = X + (int64_t)g.L * nd;
+    k_rnvp_logprob<<<warp_grid(m), 256, 0, st>>>(y, ld, m, d, logp + r0);
+    FMC_LAUNCH_CHECK();
+
+    // backward: loss = -mean(ld + log N(y)) -> dL/dy = y / n, dL/d ld = -1 / n
+    float *gy = gin[0], *gx = gin[1];
+    k_rnvp_scale<<<grid_for(nd), 256, 0, st>>>(y, nd, 1.f / (float)n, gy);
+    FMC_LAUNCH_CHECK();
+    for (int l = g.L - 1; l >= 0; --l) {
+      const float* mk = layer_mask(g, flow->aux, l);
+      const float* wl = wt + (int64_t)l * 4 * H * d;
+      k_rnvp_couple_bwd<<<grid_for(nd), 256, 0, st>>>(X + l * nd, sraw + l * nd, tt + l * nd, mk, gy, m, d, g.dt, gld,
+                                                      gx);
+      FMC_LAUNCH_CHECK();
+      // dz = [dsraw W2s, dtt W2t] masked by relu'
+      G32Args a{};
+      a.M = m;
+      a.p[0] = G32Problem{sraw + l * nd, wl, nullptr, h + l * nh, dz + l * nh};
+      a.p[1] = G32Problem{tt + l * nd, wl + (int64_t)H * d, nullptr, h + l * nh + H, dz + l * nh + H};
+      a.lda = a.ldb = d;
+      a.ldaux = a.ldc = 2 * H;
+      a.N = H;
+      a.K = d;
+      rc = gemm_f32<G32_DRELU>(st, a, 2);
+      if (rc) return rc;
+      // gx += (dz W1) * mask
+      a.p[0] = G32Problem{dz + l * nh, wl + 2ll * H * d, mk, nullptr, gx};
+      a.lda = a.ldb = 2 * H;
+      a.ldc = d;
+      a.N = d;
+      a.K = 2 * H;
+      rc = gemm_f32<G32_ADD_MASKED>(st, a, 1);
+      if (rc) return rc;
+      float* t = gy;
+      gy = gx;
+      gx = t;
+    }
+    // weight and bias gradients of all layers over the chunk. The second
+    // Linears' as h^T d(output), stored transposed: the wide side is the tall
+    // operand of the 256 x 32 tiles
+    float* out = r0 == 0 ? grad : cgrad;
+    int64_t rows_per = 0;
+    const int slices = wgrad_slices(g, m, &rows_per), rb = bias_blocks(m);
+    K32Args k{};
+    k.p[0] = K32Problem{dz, cond, nh, nd, 2 * H, d, 2 * H, d, 0, d, 1};
+    k.p[1] = K32Problem{h, sraw, nh, nd, 2 * H, d, H, d, g.off_W2s, 1, H};
+    k.p[2] = K32Problem{h + H, tt, nh, nd, 2 * H, d, H, d, g.off_W2t, 1, H};
+    k.n_problems = 3;
+    k.rows = m;
+    k.rows_per_slice = rows_per;
+    k.per_layer = g.per_layer;
+    k.n_params = g.n_params;
+    k.part = part;
+    const unsigned tiles = (unsigned)(((2 * H + kK32M - 1) / kK32M) * ((d + kK32N - 1) / kK32N));
+    k_kouter_f32<<<dim3(tiles, (unsigned)slices, (unsigned)(3 * g.L)), kK32Threads, ksmem, st>>>(k);
+    FMC_LAUNCH_CHECK();
+    k_rnvp_sum_slices<<<grid_for(g.n_params), 256, 0, st>>>(part, slices, g.n_params, out);
+    FMC_LAUNCH_CHECK();
+    const unsigned cb = (unsigned)((2 * H > d ? 2 * H : d) + 127) / 128;
+    k_rnvp_bias_partial<<<dim3(cb, (unsigned)rb, (unsigned)(3 * g.L)), 128, 0, st>>>(g, dz, sraw, tt, m, (m + rb - 1) / rb,
+                                                                                    bpart);
+    FMC_LAUNCH_CHECK();
+    k_rnvp_bias_final<<<dim3(cb, 1, (unsigned)(3 * g.L)), 128, 0, st>>>(g, bpart, rb, out);
+    FMC_LAUNCH_CHECK();
+    if (r0 > 0) {
+      k_rnvp_add<<<grid_for(g.n_params), 256, 0, st>>>(cgrad, g.n_params, grad);
+      FMC_LAUNCH_CHECK();
+    }
+  }
+  k_rnvp_loss<<<1, 1024, 0, st>>>(logp, n, loss);
   FMC_LAUNCH_CHECK();
   return FMC_OK;
 }
