@@ -19,6 +19,8 @@ from .targets import DenseGaussian
 
 _lib.register_extra("fmc_batched_workspace_size", ctypes.c_int,
                     [ctypes.c_int32, ctypes.c_int64, ctypes.POINTER(ctypes.c_size_t)])
+_lib.register_extra("fmc_batched_dense_workspace_size", ctypes.c_int,
+                    [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32, ctypes.POINTER(ctypes.c_size_t)])
 _lib.register_extra("fmc_batched_dense_local_steps", ctypes.c_int, [
     ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.POINTER(_lib.FmcLocalParams), ctypes.c_void_p,
     ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_void_p,
@@ -106,7 +108,9 @@ class BatchedDenseLocalSteps:
         keep = [noise, uniform]
         nb = ctypes.c_size_t()
         L = _lib.lib()
-        _lib.check(L.fmc_batched_workspace_size(n, self.offsets[-1], ctypes.byref(nb)))
+        nd = (ctypes.c_int32 * n)(*[t.n_dim for t in self.targets])
+        _lib.check(L.fmc_batched_dense_workspace_size(ctypes.cast(nd, ctypes.c_void_p), ctypes.cast(nc, ctypes.c_void_p),
+                                                      n, ctypes.byref(nb)))
         wptr, wsize = self._ws.get(nb.value, dev)
         _lib.check(L.fmc_batched_dense_local_steps(
             ctypes.cast(tg, ctypes.c_void_p), n, ctypes.cast(nc, ctypes.c_void_p), ctypes.byref(prm),

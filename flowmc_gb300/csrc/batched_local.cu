@@ -59,7 +59,7 @@ constexpr int kBPartFloats = kBWarps * 32 * 8;
 
 struct BatchTarget {
   const float* precision;   // [d, d]
-  float* packed;            // [round_up(d, 16), round_up(d, 32)] (k_pack_precision)
+  float* packed;            // [round_up(d, 8), round_up(d, 32)] (k_pack_precision)
   const float* mean;        // [d] or NULL
   float const_term;
   int d;
@@ -92,8 +92,8 @@ constexpr size_t kBSmemBytes =
     sizeof(float) * (2 * 8 * 4 * (size_t)kBThreads + kBDxFloats + kBWarps * kBRing + kBPartFloats + 7 * (size_t)kBRows);
 static_assert(kBSmemBytes <= 227 * 1024, "shared memory");
 
-// The precision matrices in the layout the product streams: [16 ns][32 cb]
-// with zeros outside [d, d], so that every stage of 16 rows is one contiguous
+// The precision matrices in the layout the product streams: [8 ns][32 cb]
+// with zeros outside [d, d], so that every stage of 8 rows is one contiguous
 // 16-byte aligned block whatever d is.
 __global__ void k_pack_precision(const BatchTarget* __restrict__ targets) {
   const BatchTarget T = targets[blockIdx.x];
@@ -534,11 +534,33 @@ extern "C" int fmc_batched_pack_rows(const float* const* x, const int64_t* row_s
   return FMC_OK;
 }
 
+// workspace without the packed precision matrices: counter, targets, work items
+static size_t batched_table_bytes(int32_t n_targets, int64_t total_chains) {
+  const int64_t items = total_chains / 32 + n_targets;   // at least 32 chains per work item
+  return (size_t)(256 + n_targets * sizeof(BatchTarget) + 256 + items * 8 + 256);
+}
+
+// floats of a packed precision matrix (k_pack_precision)
+static size_t packed_floats(int d) { return (size_t)((d + kBStage - 1) & ~(kBStage - 1)) * ((d + 31) & ~31); }
+
 extern "C" int fmc_batched_workspace_size(int32_t n_targets, int64_t total_chains, size_t* bytes) {
   FMC_CHECK_ARG(bytes && n_targets >= 1 && total_chains >= 1, "bad arguments");
-  const int64_t items = total_chains / 32 + n_targets;   // at least 32 chains per work item
-  *bytes = (size_t)(256 + n_targets * sizeof(BatchTarget) + 256 + items * 8 + 256) +
-           (size_t)n_targets * kBDMax * kBDMax * sizeof(float);
+  *bytes = batched_table_bytes(n_targets, total_chains) + (size_t)n_targets * packed_floats(kBDMax) * sizeof(float);
+  return FMC_OK;
+}
+
+extern "C" int fmc_batched_dense_workspace_size(const int32_t* n_dim, const int32_t* n_chains, int32_t n_targets,
+                                                size_t* bytes) {
+  FMC_CHECK_ARG(bytes && n_dim && n_chains && n_targets >= 1, "bad arguments");
+  int64_t total = 0;
+  size_t floats = 0;
+  for (int t = 0; t < n_targets; ++t) {
+    FMC_CHECK_ARG(n_dim[t] >= 1 && n_dim[t] <= kBDMax, "target %d: n_dim %d outside [1, %d]", t, n_dim[t], kBDMax);
+    FMC_CHECK_ARG(n_chains[t] >= 1, "target %d: no chains", t);
+    total += n_chains[t];
+    floats += packed_floats(n_dim[t]);
+  }
+  *bytes = batched_table_bytes(n_targets, total) + floats * sizeof(float);
   return FMC_OK;
 }
 
@@ -561,6 +583,7 @@ extern "C" int fmc_batched_dense_local_steps(const FmcTarget* targets, int32_t n
   FMC_CHECK_ARG(x0 && x_last && lp_last, "NULL device array");
   std::vector<BatchTarget> bt(n_targets);
   int64_t off = 0;
+  size_t floats = 0;   // of the packed precision matrices
   for (int t = 0; t < n_targets; ++t) {
     const FmcTarget& g = targets[t];
     FMC_CHECK_ARG(g.kind == FMC_TARGET_DENSE_GAUSSIAN, "target %d is not a dense Gaussian", t);
@@ -572,9 +595,9 @@ extern "C" int fmc_batched_dense_local_steps(const FmcTarget* targets, int32_t n
                         out_pos[t], out_logp[t], out_acc[t], step_sizes[t],
                         noise ? noise[t] : nullptr, unif ? unif[t] : nullptr};
     off += n_chains[t];
+    floats += packed_floats(g.n_dim);
   }
-  size_t need = 0;
-  fmc_batched_workspace_size(n_targets, off, &need);
+  const size_t need = batched_table_bytes(n_targets, off) + floats * sizeof(float);
   FMC_CHECK_ARG(ws && ws_bytes >= need, "workspace of %zu bytes < %zu needed", ws_bytes, need);
   cudaStream_t st = (cudaStream_t)stream;
   // Tile height: the most chain blocks per item that still spread over the
@@ -617,7 +640,10 @@ extern "C" int fmc_batched_dense_local_steps(const FmcTarget* targets, int32_t n
   // vector may go out of scope
   const size_t tb = (n_targets * sizeof(BatchTarget) + 255) / 256 * 256;
   float* packed = (float*)(((uintptr_t)ws + 256 + tb + it.size() * 8 + 15) & ~(uintptr_t)15);
-  for (int t = 0; t < n_targets; ++t) bt[t].packed = packed + (size_t)t * kBDMax * kBDMax;
+  for (int t = 0; t < n_targets; ++t) {
+    bt[t].packed = packed;   // whole 32-float rows: 16-byte aligned
+    packed += packed_floats(bt[t].d);
+  }
   std::vector<char> up(256 + tb + it.size() * 8, 0);
   memcpy(up.data() + 256, bt.data(), n_targets * sizeof(BatchTarget));
   memcpy(up.data() + 256 + tb, it.data(), it.size() * 4);

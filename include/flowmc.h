@@ -236,7 +236,11 @@ FMC_API int fmc_adam_optimize(const FmcTarget* target, const float* x0, int32_t 
  * the layout of x0; the columns past n_dim_t are left as they are. */
 FMC_API int fmc_batched_pack_rows(const float* const* x, const int64_t* row_stride, const int32_t* n_dim,
                                   const int32_t* n_chains, int32_t n_targets, float* packed, void* stream);
+/* workspace bytes: for targets of any dimension, or for those of n_dim and
+ * n_chains (host arrays; 1 KB instead of 256 KB for an 8-D target) */
 FMC_API int fmc_batched_workspace_size(int32_t n_targets, int64_t total_chains, size_t* bytes);
+FMC_API int fmc_batched_dense_workspace_size(const int32_t* n_dim, const int32_t* n_chains, int32_t n_targets,
+                                             size_t* bytes);
 FMC_API int fmc_batched_dense_local_steps(const FmcTarget* targets, int32_t n_targets, const int32_t* n_chains,
                                           const FmcLocalParams* params, const float* step_sizes, const float* x0,
                                           int32_t n_steps, int32_t thinning, uint64_t seed, uint64_t counter,
