@@ -49,6 +49,16 @@ void set_error(const char* fmt, ...);
     }                                                                        \
   } while (0)
 
+// Lets a kernel without static shared memory take `bytes` of dynamic shared memory.
+// The limit belongs to the kernel, not to the launch: every call sets it to the same
+// value, the most there is, so that a thread asking for less cannot pull it from
+// under another's larger launch.
+template <typename... P>
+inline cudaError_t allow_smem(void (*kern)(P...), size_t bytes) {
+  if (bytes <= 48 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
 // Launches in a chain (programmatic dependent launch): a kernel started by
 // launch_chained may be placed on SMs as the kernel before it on the stream
 // leaves them, instead of after its last block and a launch latency. Every

@@ -507,7 +507,7 @@ int64_t flow_f32_grad_floats(const FlowGeom& g, int64_t n) { return grad_ws(g, n
 template <int K, int R>
 static int launch_bwd(const FlowBwdArgs& a, size_t bytes, cudaStream_t st) {
   auto kern = k_flow_f32_bwd<K, R>;
-  FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  FMC_CUDA_TRY(allow_smem(kern, bytes));
   kern<<<(unsigned)a.tiles, FlowTile<R>::NT, bytes, st>>>(a);
   FMC_LAUNCH_CHECK();
   return FMC_OK;

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(FlowTile<R>::NT, 2) k_flow_f32(const __grid_co
 template <int K, int R, bool INV, bool SAVE>
 static int launch_k(const FlowF32Args& a, size_t bytes, cudaStream_t st) {
   auto kern = k_flow_f32<K, R, INV, SAVE>;
-  FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  FMC_CUDA_TRY(allow_smem(kern, bytes));
   kern<<<(unsigned)((a.n + R - 1) / R), FlowTile<R>::NT, bytes, st>>>(a);
   FMC_LAUNCH_CHECK();
   return FMC_OK;

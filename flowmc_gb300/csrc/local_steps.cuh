@@ -537,9 +537,7 @@ int launch_local_t(const LocalArgs& a0, cudaStream_t st) {
   a.nstage_off = (int32_t)(smem / sizeof(float));
   if (a.noise == nullptr) smem += (size_t)threads * 4 * V * sizeof(float);
   auto kern = k_local_steps<KIND, TGT, G, V>;
-  if (smem > 48 * 1024) {
-    FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  }
+  FMC_CUDA_TRY(allow_smem(kern, smem));
   // blocks per SM, asked for once per launch shape (the last one is kept, in
   // one word so that threads see a whole entry)
   static std::atomic<uint64_t> last{0};

@@ -310,8 +310,7 @@ static int launch_nf_t(const NfArgs& a0, cudaStream_t st) {
   if (blocks > cap) blocks = cap;
   auto kern = walk ? k_nf_walk<TGT, G, V> : k_nf_accept<TGT, G, V>;
   const size_t smem = floats * sizeof(float);
-  if (smem > 48 * 1024)
-    FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  FMC_CUDA_TRY(allow_smem(kern, smem));
   // proposals and their flow densities read, thinned rows written
   const double n_rec = (double)((a.S + a.thin - 1) / a.thin);
   KernelTimer kt(FMC_KT_NF_ACCEPT, st, 0.0,

@@ -157,7 +157,7 @@ static int launch_exchange_t(const ExchangeArgs& a0, cudaStream_t st) {
   size_t smem = ((TGT == FMC_TARGET_DENSE_GAUSSIAN) ? (size_t)gpb * a.d : 0) + kMaxTemps + (size_t)2 * gpb * a.T;
   smem *= sizeof(float);
   auto kern = k_pt_exchange<TGT, G, V>;
-  if (smem > 48 * 1024) FMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  FMC_CUDA_TRY(allow_smem(kern, smem));
   int per_sm = 0;
   FMC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
   if (per_sm < 1) per_sm = 1;
