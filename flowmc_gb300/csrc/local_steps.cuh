@@ -138,8 +138,19 @@ __device__ __forceinline__ void draw_chunk(const Rng& rng, int64_t c, int s, int
   __syncwarp();
 }
 
-// this lane's normals of step s: explicit, or from the chunk in shared memory
+// The same normals of one step, drawn by the lane that uses them (whole blocks: V >= 4)
 template <int G, int V>
+__device__ __forceinline__ void draw_own(const Rng& rng, int64_t c, int s, int gl, float (&xi)[V]) {
+#pragma unroll
+  for (int q = 0; q < V; q += 4) {
+    const u32x4 r = rng.draw((uint64_t)c, (uint64_t)s, (uint32_t)(gl * V + q), RNG_TAG_LOCAL_NORMAL);
+    box_muller(r.x, r.y, xi[q], xi[q + 1]);
+    box_muller(r.z, r.w, xi[q + 2], xi[q + 3]);
+  }
+}
+
+// this lane's normals of step s: explicit, its own (SHORT) or from the chunk in shared memory
+template <int G, int V, bool SHORT>
 __device__ __forceinline__ void draw_normals(const LocalArgs& a, const Rng& rng, int64_t c, int s, int gl, float* ns,
                                              float (&xi)[V]) {
   const int d = a.d;
@@ -152,17 +163,21 @@ __device__ __forceinline__ void draw_normals(const LocalArgs& a, const Rng& rng,
     }
     return;
   }
-  if ((s & 3) == 0) draw_chunk<G, V>(rng, c, s, gl, ns);
-  const float* row = ns + (s & 3) * (G * V) + gl * V;
-  if constexpr (V % 4 == 0) {
-#pragma unroll
-    for (int q = 0; q < V; q += 4) {
-      const float4 z = *reinterpret_cast<const float4*>(row + q);
-      xi[q] = z.x; xi[q + 1] = z.y; xi[q + 2] = z.z; xi[q + 3] = z.w;
-    }
+  if constexpr (SHORT) {
+    draw_own<G, V>(rng, c, s, gl, xi);
   } else {
+    if ((s & 3) == 0) draw_chunk<G, V>(rng, c, s, gl, ns);
+    const float* row = ns + (s & 3) * (G * V) + gl * V;
+    if constexpr (V % 4 == 0) {
 #pragma unroll
-    for (int v = 0; v < V; ++v) xi[v] = row[v];
+      for (int q = 0; q < V; q += 4) {
+        const float4 z = *reinterpret_cast<const float4*>(row + q);
+        xi[q] = z.x; xi[q + 1] = z.y; xi[q + 2] = z.z; xi[q + 3] = z.w;
+      }
+    } else {
+#pragma unroll
+      for (int v = 0; v < V; ++v) xi[v] = row[v];
+    }
   }
 #pragma unroll
   for (int v = 0; v < V; ++v)
@@ -233,7 +248,7 @@ constexpr int local_min_blocks() {
              : 0;
 }
 
-template <int KIND, int TGT, int G, int V>
+template <int KIND, int TGT, int G, int V, bool SHORT>
 __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local_steps(const LocalArgs a) {
   extern __shared__ float smem[];
   const int gl = threadIdx.x % G;
@@ -283,7 +298,7 @@ __global__ void __launch_bounds__(256, local_min_blocks<KIND, TGT, V>()) k_local
     int tcount = 0, n_acc = 0;
     for (int s = 0; s < a.S; ++s) {
       float xi[V];
-      draw_normals<G, V>(a, rng, cc, s, gl, ns, xi);
+      draw_normals<G, V, SHORT>(a, rng, cc, s, gl, ns, xi);
       const float logu = draw_log_uniform<G>(a, rng, cc, s, gl, lu);
       bool acc;
       if constexpr (KIND == FMC_KERNEL_MALA) {
@@ -510,6 +525,16 @@ inline Shape default_shape(int d) {
   return {32, 8};
 }
 
+// Shapes with an instance whose lanes draw their own noise step by step (SHORT):
+// those whose lanes' coordinates are whole Philox blocks.
+constexpr bool has_own_noise(int V) { return V % 4 == 0; }
+// It is taken where chunks of four steps would draw a fifth more than S steps use
+// (1, 2, 3, 5, 6, 9, 10 and 13 of them): 100,000 chains of one step, 40-D diagonal
+// Gaussian, random walk 57 us in chunks, 39 so; 100-D mixture 139, 97; 200-D
+// Rosenbrock chain, MALA 237, 158; five steps of these 1.17, 1.15 and 1.22 times. For
+// few chains both take the time of the call.
+inline bool draw_own_noise(int S) { return 5 * ((S + 3) / 4 * 4) >= 6 * S; }
+
 template <int KIND, int TGT, int G, int V>
 int launch_local_t(const LocalArgs& a0, cudaStream_t st) {
   LocalArgs a = a0;
@@ -535,13 +560,18 @@ int launch_local_t(const LocalArgs& a0, cudaStream_t st) {
   if (KIND == FMC_KERNEL_HMC && a.mchol != nullptr) smem += (size_t)gpb * a.d * sizeof(float);
   smem = (smem + 15) / 16 * 16;
   a.nstage_off = (int32_t)(smem / sizeof(float));
-  if (a.noise == nullptr) smem += (size_t)threads * 4 * V * sizeof(float);
-  auto kern = k_local_steps<KIND, TGT, G, V>;
+  auto kern = k_local_steps<KIND, TGT, G, V, false>;
+  bool own = false;
+  if constexpr (has_own_noise(V)) {
+    own = a.noise == nullptr && draw_own_noise(a.S);
+    if (own) kern = k_local_steps<KIND, TGT, G, V, true>;
+  }
+  if (a.noise == nullptr && !own) smem += (size_t)threads * 4 * V * sizeof(float);
   FMC_CUDA_TRY(allow_smem(kern, smem));
   // blocks per SM, asked for once per launch shape (the last one is kept, in
   // one word so that threads see a whole entry)
   static std::atomic<uint64_t> last{0};
-  const uint64_t shape = ((uint64_t)smem << 24) | ((uint64_t)threads << 8);
+  const uint64_t shape = ((uint64_t)smem << 24) | ((uint64_t)threads << 8) | ((uint64_t)own << 8);
   uint64_t known = last.load(std::memory_order_relaxed);
   if ((known & ~0xffull) != shape) {
     int q = 0;
