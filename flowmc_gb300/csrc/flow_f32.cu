@@ -22,19 +22,9 @@ static bool flow_f32_smem(const FlowGeom& g, int R, FlowF32Args& a, size_t& byte
   return bytes <= 227 * 1024;
 }
 
-bool flow_f32_fused(const FlowGeom& g) {
+bool flow_f32_tile_fits(const FlowGeom& g, int R, size_t* bytes) {
   FlowF32Args a{};
-  size_t b;
-  return flow_f32_smem(g, 16, a, b);
-}
-
-// 64 rows per CTA where they fill the SMs and fit in shared memory, else 16
-// (fewer rows per CTA and two more warps per row: latency). 5-D flow 4 x [32, 32]:
-// 10,000 rows (157 CTAs of 64) train in 341 us per step, in 16-row tiles 425.
-int flow_f32_tile(const FlowGeom& g, int64_t n) {
-  FlowF32Args a{};
-  size_t bytes = 0;
-  return n >= 64 * (int64_t)sm_count() && flow_f32_smem(g, 64, a, bytes) ? 64 : 16;
+  return flow_f32_smem(g, R, a, *bytes);
 }
 
 // The fastest way through a forward or inverse pass: 64 or 16 rows per CTA of

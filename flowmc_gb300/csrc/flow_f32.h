@@ -25,12 +25,10 @@ struct FlowF32Call {
   float* acts;
 };
 
-// whether the flow's row tile fits in shared memory
-bool flow_f32_fused(const FlowGeom& g);
+// whether a tile of R rows fits in shared memory, and the bytes it takes
+bool flow_f32_tile_fits(const FlowGeom& g, int R, size_t* bytes);
 // rows per CTA of a forward or inverse pass over n rows; 0: the launches per layer are faster
 int flow_f32_route(const FlowGeom& g, int64_t n);
-// rows per CTA and per tile of the saved activations when training on n rows
-int flow_f32_tile(const FlowGeom& g, int64_t n);
 // all layers over c.n rows in one launch of R-row tiles
 int flow_f32_pass(const FlowF32Call& c, const FlowGeom& g, int R, cudaStream_t st);
 
@@ -38,10 +36,16 @@ int flow_f32_pass(const FlowF32Call& c, const FlowGeom& g, int R, cudaStream_t s
 // number of slices, and with it the order of the sums)
 int64_t kouter_part_floats(const FlowGeom& g);
 // The loss gradient from a forward pass that left `save` and `acts`
-// (flow_f32_bwd.cu): whether the flow's backward tile fits (hidden widths and
-// conditioning block up to 128), floats of its workspace (the activations
-// first), and the gradient itself into grad [n_params].
-bool flow_f32_grad_fits(const FlowGeom& g, int64_t n);
+// (flow_f32_bwd.cu): how n rows train -- `tile` rows per CTA of both passes and per
+// tile of the saved activations (0 where the flow does not fit: hidden widths
+// and conditioning block up to 128), and whether that is faster than the
+// launches per layer --, floats of its workspace (the activations first), and the
+// gradient itself into grad [n_params].
+struct FlowGradRoute {
+  int tile;
+  bool faster;
+};
+FlowGradRoute flow_f32_grad_route(const FlowGeom& g, int64_t n);
 int64_t flow_f32_grad_floats(const FlowGeom& g, int64_t n);
 int flow_f32_grad(const FlowGeom& g, const float* theta, const float* aux, int64_t n, const float* save, float* ws,
                   float* grad, cudaStream_t st);

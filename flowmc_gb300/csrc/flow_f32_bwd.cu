@@ -441,17 +441,68 @@ static size_t bwd_smem(const FlowGeom& g, int R, FlowBwdArgs& a) {
   return sizeof(float) * (2 * (size_t)R * a.ldx + 2 * (size_t)a.act_floats + st * kFlowBK * kFlowCols);
 }
 
-// the forward's tile if the backward fits in the same rows, 0 if it does not
-static int grad_tile(const FlowGeom& g, int64_t n) {
-  if (!flow_f32_fused(g) || g.nc_max() > kFlowCols) return 0;
+// The fastest way to train on n rows, from estimates like flow_f32_route's
+// (microseconds, both passes). What drives them:
+//   S, T   stages of a layer's forward and backward products, G coordinate groups
+//   t      row tiles on the fullest SM, f and b the rounds they run in forward and
+//          backward (two CTAs share an SM where shared memory allows it)
+// and the weight gradients' multiply-adds, which all ways have alike.
+// Coefficients fitted to 750 random calls (GB300; 3 to 250 dims, 8 to 128 units, one
+// to three hidden layers, 2 to 16 bins, 1 to 8 layers, 20 to 60,000 rows), which
+// they reproduce within 15 % (16 and 64 rows) and 21 % (layers) for nine calls in
+// ten. The way taken was on average 0.1 % and at worst 13 % behind the fastest of the
+// three, and at worst 6 % behind the layers. 64 rows wherever they fill the SMs, 16
+// otherwise, was 4 % behind on average and up to 1.7 times the layers' time:
+// 250-D, 2 bins, one hidden layer of 48 units, 2 layers, 12,000 rows 952 us by
+// layers, 1,616 in 64-row tiles, 851 in 16-row ones; 250-D, 16 bins, [48, 48], 4 layers,
+// 1,000 rows 2,739 us by layers, 3,227 in 16-row tiles.
+FlowGradRoute flow_f32_grad_route(const FlowGeom& g, int64_t n) {
+  FlowGradRoute route{0, false};
+  if (g.nc_max() > kFlowCols) return route;
   for (int i = 0; i < g.nh; ++i)
-    if (g.H[i] > kFlowCols) return 0;
-  FlowBwdArgs a{};
-  const int R = flow_f32_tile(g, n);
-  return bwd_smem(g, R, a) <= 227 * 1024 ? R : 0;
+    if (g.H[i] > kFlowCols) return route;
+  const FlowShape s = flow_shape(g);
+  double S = 0, T = 0, G = 0, steps = 0, back = 0, macs = 0, raw = 0;   // means over the two layer parities
+  for (int l = 0; l < 2; ++l)
+    for (int i = 0; i <= g.nh; ++i) {
+      const int in = s.in(l, i), out = s.out(l, i), tc = s.tile_cols(i);
+      const int ks = (in + kFlowBK - 1) / kFlowBK;
+      back += 0.5 * ((out + kFlowBK - 1) / kFlowBK);
+      S += 0.5 * ((out + tc - 1) / tc) * ks;
+      for (int n0 = 0; n0 < out; n0 += tc) T += 0.5 * ((std::min(tc, out - n0) + kFlowBK - 1) / kFlowBK);
+      steps += 0.5 * ks;
+      macs += 0.5e-6 * ((out + 63) / 64 * 64) * (ks * kFlowBK);
+      if (i == g.nh) {
+        G += 0.5 * ((out + tc - 1) / tc);
+        raw += 0.5e-6 * out;
+      }
+    }
+  const double L = g.L, nr = (double)n;
+  // the launches per layer: chains of 16-deep steps forward and back, 32 splines a warp
+  const double layers = 39.8 + L * (93.2 + 7.13 * steps + 0.402 * back + 0.705 * ((g.d + 63) / 64) * g.P +
+                                    nr * (0.166 * macs + 15.9 * raw + 4.29e-3));
+  double fused = 0.0;
+  for (int R = 16; R <= 64; R += 48) {
+    FlowBwdArgs a{};
+    size_t fwd = 0;
+    const size_t bwd = bwd_smem(g, R, a);
+    if (bwd > 227 * 1024 || !flow_f32_tile_fits(g, R, &fwd)) continue;
+    const double t = ceil(ceil((double)n / R) / sm_count());
+    const double f = ceil(t / (2 * (fwd + 1024) <= 228 * 1024 ? 2 : 1));
+    const double b = ceil(t / (2 * (bwd + 1024) <= 228 * 1024 ? 2 : 1));
+    const double est =
+        R == 16 ? 60.1 + L * (f * 0.213 * S + t * (0.481 * S + 0.144 * T + 0.0829 * g.d) +
+                              b * (12.5 + 0.441 * T + 0.268 * G * g.K) + nr * 0.0375 * macs)
+                : 78.9 + L * (f * (19.9 + 1.44 * G) + t * (0.896 * S + 0.157 * T + 0.53 * g.d) + b * 1.59 * T +
+                              nr * (0.0609 * macs + 1.04 * raw + 2.26e-5 * g.d));
+    if (route.tile == 0 || est < fused) {
+      fused = est;
+      route.tile = R;
+    }
+  }
+  route.faster = route.tile != 0 && fused < 0.95 * layers;
+  return route;
 }
-
-bool flow_f32_grad_fits(const FlowGeom& g, int64_t n) { return grad_tile(g, n) != 0; }
 
 int64_t kouter_part_floats(const FlowGeom& g) {
   int64_t mn = 1;
@@ -472,9 +523,9 @@ struct GradWs {
 static GradWs grad_ws(const FlowGeom& g, int64_t n) {
   GradWs w{};
   const FlowShape s = flow_shape(g);
-  w.R = grad_tile(g, n);
+  w.R = flow_f32_grad_route(g, n).tile;
   w.tiles = (n + w.R - 1) / w.R;
-  const int64_t rows = w.tiles * w.R;
+  const int64_t rows = (n + 63) / 64 * 64;   // of the tiles, whatever their height
   auto al = [](int64_t v) { return (v + 63) / 64 * 64; };
   w.acts = al(s.act_base(g.L) * rows);
   w.gout = al(s.gcol(g.L, 0) * rows);

@@ -145,9 +145,9 @@ static void carve_train(const FlowGeom& g, int64_t n, bool bf16, bool keep, void
   if (total) *total = (size_t)used;
 }
 
-// whether the activations of n rows may be kept
+// whether the activations of n rows can be kept
 static bool train_keeps(const FlowGeom& g, int64_t n, bool bf16) {
-  if (!bf16) return flow_f32_grad_fits(g, n) && 4 * flow_f32_grad_floats(g, n) <= kKeepBytes;
+  if (!bf16) return flow_f32_grad_route(g, n).tile != 0 && 4 * flow_f32_grad_floats(g, n) <= kKeepBytes;
   const int64_t n128 = FlowGeom::rup(n, 128);
   return 2 * g.L * n128 * (FlowGeom::rup(g.nc_max(), 64) + g.nh * FlowGeom::rup(g.h_max(), 64)) <= kKeepBytes;
 }
@@ -159,8 +159,13 @@ static size_t train_ws_bytes(const FlowGeom& g, int64_t n, bool bf16, bool keep)
   return tot;
 }
 
+// and whether they are, given the choice
+static bool train_prefers_keeping(const FlowGeom& g, int64_t n, bool bf16) {
+  return train_keeps(g, n, bf16) && (bf16 || flow_f32_grad_route(g, n).faster);
+}
+
 size_t train_ws_bytes(const FlowGeom& g, int64_t n, bool bf16) {
-  return train_ws_bytes(g, n, bf16, train_keeps(g, n, bf16));
+  return train_ws_bytes(g, n, bf16, train_prefers_keeping(g, n, bf16));
 }
 
 // ------------------------------------------------------------------ kernels
@@ -446,14 +451,16 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
   FMC_CHECK_ARG(n >= 1, "n=%lld < 1", (long long)n);
   FMC_CHECK_ARG(x && loss && grad, "NULL array");
   const bool bf16 = f->precision == FMC_PREC_BF16;
-  // The activations are kept where the workspace holds them. It may hold less: one
-  // sized for a larger batch, beyond the bound, serves every smaller one.
-  bool keep_all = train_keeps(g, n, bf16);
+  // The preferred way where the workspace holds it. It may hold less: one sized for
+  // a larger batch, which prefers another way, serves every smaller one.
+  bool keep_all = train_prefers_keeping(g, n, bf16);
   size_t need = train_ws_bytes(g, n, bf16, keep_all);
-  if (keep_all && ws_bytes < need) {
-    const size_t lean = train_ws_bytes(g, n, bf16, false);
-    keep_all = need <= lean;   // a flow of one layer or two may need less with them
-    need = need < lean ? need : lean;
+  if (ws_bytes < need && train_keeps(g, n, bf16)) {
+    const size_t other = train_ws_bytes(g, n, bf16, !keep_all);
+    if (other < need) {
+      need = other;
+      keep_all = !keep_all;
+    }
   }
   FMC_CHECK_ARG(ws && ws_bytes >= need, "workspace of %zu bytes < %zu needed", ws_bytes, need);
   FMC_CHECK_ARG(((uintptr_t)ws & 255) == 0, "workspace must be 256-byte aligned");
@@ -482,7 +489,7 @@ int flow_loss_grad(const FmcFlow* f, const float* x, int64_t n, float* loss, flo
     c.logp = w.logp;
     c.save = w.xs;
     c.acts = w.f32;
-    if ((rc = flow_f32_pass(c, g, flow_f32_tile(g, n), st))) return rc;
+    if ((rc = flow_f32_pass(c, g, flow_f32_grad_route(g, n).tile, st))) return rc;
     k_loss<<<1, 1024, 0, st>>>(w.logp, n, loss);
     FMC_LAUNCH_CHECK();
     return flow_f32_grad(g, f->theta, f->aux, n, w.xs, w.f32, grad, st);
