@@ -15,9 +15,10 @@
 // target of d coordinates takes cb = ceil(d / 32) warps side by side -- a row
 // block of 32 chains -- and up to floor(12 / cb) row blocks, so that narrow
 // targets fill the CTA with more chains instead of leaving threads idle.
-// Positions, momenta and gradients of the trajectory stay in the owner
-// threads' registers; dx is shared by the warps of a row block through shared
-// memory. P, packed once per call into rows of 32 cb values, streams from L2:
+// Positions, momenta and gradients of the trajectory are in the owner threads'
+// registers (168 a thread at 12 warps, of which the HMC instance spills 164 bytes), the
+// position and gradient that the chain holds in shared memory; dx is
+// shared by the warps of a row block through shared memory. P, packed once per call into rows of 32 cb values, streams from L2:
 // every warp copies its own 32 columns (cp.async, 8-row stages, three in
 // flight, running on into the next evaluation), so no barrier is needed for
 // P and the only ones in the product loop are the row block's two per
@@ -30,8 +31,8 @@
 //
 // Measured (48 targets of 8-256 dimensions, 146,569 chains; before: 32-chain
 // tiles of 8 warps, P read from L2 into registers, all state in shared
-// memory): MALA 10 steps 7.37 -> 3.28 ms, HMC 3 steps of 11
-// gradients 16.4 -> 6.80 ms per call, about 30 TFLOP/s of useful FP32 (46 % of
+// memory): MALA 10 steps 7.38 -> 3.03 ms, HMC 3 steps of 11
+// gradients 16.4 -> 6.55 ms per call, about 30 TFLOP/s of useful FP32 (46 % of
 // the FMA pipe with padding; issue slots 58 % busy, bound by the latency of the
 // shared-memory reads with two or three warps per scheduler).
 //

@@ -263,8 +263,8 @@ __device__ __forceinline__ float group_bcast(float v, int src_lane_in_group) {
 // ---------------------------------------------------------------- exact quotients
 // a / b for one divisor used many times, correctly rounded: the bits of the
 // division operator without its reciprocal per quotient and range branch, for
-// divisors of magnitude 2^-30 .. 2^30 (`in_range`) and numerators that are 0 or
-// of magnitude 2^-60 .. 2^60 (the caller's check).
+// divisors of magnitude 2^-30 .. 2^30 (`in_range`) and numerators of magnitude
+// 2^-60 .. 2^60 (the caller's check; a zero would lose its sign).
 //  * MarkDiv: with y = RN(1 / b), q0 = a y, q1 = q0 + (a - q0 b) y,
 //    q = q1 + (a - q1 b) y (Markstein, IBM J. Res. Dev. 34(1), 1990: q1 is a
 //    faithful rounding and its remainder exact). Any divisor.

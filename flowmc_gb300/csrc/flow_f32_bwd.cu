@@ -1,4 +1,4 @@
-// flow_f32_bwd.cu -- gradient of the FP32 flow loss in four launches, from the
+// flow_f32_bwd.cu -- gradient of the FP32 flow loss in seven launches, from the
 // layer inputs and activations the fused forward pass (flow_f32.cu) left behind
 // (NFModel.loss_fn's reverse pass, nf_model/base.py:98-125).
 //

@@ -56,7 +56,8 @@ constexpr int64_t kKeepBytes = (int64_t)16 << 30;
 // Input-gradient GEMMs from this depth on run on CTA pairs (half the weight
 // rows per CTA: the operands' way into the SM, 64 B/clock, limits one-CTA
 // tiles of 128 x 256). 65,536 x 512 outputs: 132 -> 121 us at a depth of
-// 2560; at 512 the pair's set-up and its epilogue cost more: 45 -> 52 us.
+// 2560; at 512 the pair's set-up and its epilogue cost more: 45 -> 52 us. The
+// line lies between these two depths; none between them was measured.
 // A pair per two SMs at least, or the larger tiles leave SMs idle.
 static bool dgrad_pairs(int64_t n, int in, int depth) {
   return depth >= 1024 && n * in >= (int64_t)sm_count() * 128 * 256;

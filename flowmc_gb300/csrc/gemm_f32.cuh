@@ -7,7 +7,8 @@
 // stages in flight) and multiply packed pairs (fma.rn.f32x2), which reach 72
 // TFLOP/s on GB300 where plain FMAs stop at 52 (register ports). The K-major GEMM
 // pairs adjacent inputs -- even and odd inputs summed apart, added at the end --
-// so neither operand has to be duplicated; the outer product pairs adjacent m.
+// so neither operand has to be duplicated (the gradient's products; the forward's
+// are plain FMAs in input order, see gemm_f32); the outer product pairs adjacent m.
 // A 16-byte shared-memory load costs two cycles when each quarter warp reads at
 // most two addresses and four otherwise, so the row operand is the one that
 // quarters of a warp share: 8 x 8 outputs per thread keep the loads at three

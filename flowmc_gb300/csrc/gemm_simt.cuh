@@ -125,8 +125,7 @@ constexpr int kKouterMaxSlices = 64;
 
 // part[z][i][j] = sum over rows k of slice z of A[k*lda + i] * B[k*ldb + j]
 // 64 x 64 tiles, 16 rows per step.
-template <int U = 0>
-__global__ void __launch_bounds__(256) k_sgemm_kouter(int M, int N, int64_t K, int64_t kslice,
+static __global__ void __launch_bounds__(256) k_sgemm_kouter(int M, int N, int64_t K, int64_t kslice,
                                                       const float* __restrict__ A, int64_t lda,
                                                       const float* __restrict__ B, int64_t ldb,
                                                       float* __restrict__ part) {
@@ -216,7 +215,7 @@ inline int kouter(cudaStream_t st, int M, int N, int64_t K, const float* A, int6
   const int64_t S = kouter_slices(M, N, K, part != nullptr, part_floats, &kslice);
   float* dst = S > 1 ? part : out;
   dim3 grid((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64), (unsigned)S);
-  k_sgemm_kouter<><<<grid, 256, 0, st>>>(M, N, K, kslice, A, lda, B, ldb, dst);
+  k_sgemm_kouter<<<grid, 256, 0, st>>>(M, N, K, kslice, A, lda, B, ldb, dst);
   FMC_LAUNCH_CHECK();
   if (S > 1) {
     int64_t b = (mn + 255) / 256;

@@ -21,7 +21,7 @@
 // [d, H, d].
 //
 // Measured on GB300 (32-D, 8 layers, H = 256): loss + gradient of 16,384 rows
-// 3.64 -> 1.31 ms (212 launches -> 58; the GEMMs 0.89 ms, the weight gradients
+// 3.64 -> 1.29 ms (212 launches -> 58; the GEMMs 0.89 ms, the weight gradients
 // 0.17 ms = 50 TFLOP/s).
 #include "flow.cuh"
 #include "gemm_f32.cuh"

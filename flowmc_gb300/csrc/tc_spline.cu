@@ -621,7 +621,10 @@ struct SplineBwdArgs {
 // stored one coordinate earlier, has been read. Nothing waits for the other
 // coordinates' warps. One barrier over all twelve and a wait for the tile's
 // stores at its end, and the bias as global loads, took 242 us at 65,536 rows,
-// 128 dims, 512 units, 12 bins; now 197 us.
+// 128 dims, 512 units, 12 bins; now 197 us. The boxes of x, dL/dy and bias fit beside
+// the ring for 12 and 16 bins only; with 6, 8 and 10 they are 12 to 15 KB too many, and
+// below the groups are too wide for them: x, dL/dy and bias come from global
+// memory there, at a row pitch of d floats.
 template <int KB, int STAGES>
 __global__ void __launch_bounds__(kSplThreads, 1)
     k_tc_spline_bwd(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
