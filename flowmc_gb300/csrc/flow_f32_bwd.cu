@@ -458,7 +458,7 @@ static size_t bwd_smem(const FlowGeom& g, int R, FlowBwdArgs& a) {
 // 1,000 rows 2,739 us by layers, 3,227 in 16-row tiles.
 FlowGradRoute flow_f32_grad_route(const FlowGeom& g, int64_t n) {
   FlowGradRoute route{0, false};
-  if (g.nc_max() > kFlowCols) return route;
+  if (n < 1 || g.nc_max() > kFlowCols) return route;   // (a size may be asked for no rows)
   for (int i = 0; i < g.nh; ++i)
     if (g.H[i] > kFlowCols) return route;
   const FlowShape s = flow_shape(g);
