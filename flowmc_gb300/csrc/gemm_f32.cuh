@@ -42,13 +42,13 @@ struct G32Args {
   int N, K;
 };
 
-// 32 WR rows x 8 TN columns per CTA; WR warps of 4 x 8 lanes with 8 x TN outputs
+// 4 RM WR rows x 8 TN columns per CTA; WR warps of 4 x 8 lanes with RM x TN outputs
 // per thread, times WK groups of warps that take every WK-th 16-input chunk
 // (outputs too few to fill the SMs: the groups' sums are added through shared
 // memory in order). The tile leaves through shared memory as whole rows.
-template <int WR, int TN, int WK, int EPI, bool SEQ>
-__global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_gemm_f32(const __grid_constant__ G32Args a) {
-  constexpr int NT = 32 * WR * WK, BM = 32 * WR, BN = 8 * TN, ROWS = BM + BN;
+template <int WR, int TN, int WK, int EPI, bool SEQ, int RM = 8>
+__global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 2 * RM / (WR * WK) : 1) k_gemm_f32(const __grid_constant__ G32Args a) {
+  constexpr int NT = 32 * WR * WK, BM = 4 * RM * WR, BN = 8 * TN, ROWS = BM + BN;
   constexpr int STAGE = WK * ROWS * kG32Pitch, LDT = BN + 8, BKS = WK * kG32BK;
   extern __shared__ __align__(16) float sm[];
   const G32Problem& p = a.p[blockIdx.z];
@@ -95,11 +95,11 @@ __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_
     }
     asm volatile("cp.async.commit_group;");
   };
-  const int r0 = wid * 32 + (lane >> 3), c0 = lane & 7;   // rows r0 + 4 i, columns c0 + 8 j
+  const int r0 = wid * (4 * RM) + (lane >> 3), c0 = lane & 7;   // rows r0 + 4 i, columns c0 + 8 j
   using Acc = std::conditional_t<SEQ, float, uint64_t>;
-  Acc acc[8][TN];
+  Acc acc[RM][TN];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < RM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = Acc(0);
 #pragma unroll
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_
 #pragma unroll
           for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(Bs + 8 * j * kG32Pitch + k);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < RM; ++i) {
             const float4 v = *reinterpret_cast<const float4*>(As + 4 * i * kG32Pitch + k);
 #pragma unroll
             for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(v.x, b[j].x, acc[i][j]);
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_
 #pragma unroll
           for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(Bs + 8 * j * kG32Pitch + k);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < RM; ++i) {
             const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(As + 4 * i * kG32Pitch + k);
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(32 * WR * WK, TN == 4 ? 16 / (WR * WK) : 1) k_
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < RM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       float v;
@@ -244,8 +244,17 @@ inline int gemm_f32(cudaStream_t st, const G32Args& a, int count) {
   };
   const int64_t wide = (a.M + 127) / 128 * ((a.N + 63) / 64) * count;
   if (a.N <= 32 || wide < sm_count()) {
-    if constexpr (SEQ) return go(k_gemm_f32<2, 4, 1, EPI, SEQ>, 64, 32, 1, 64);
-    else return go(k_gemm_f32<2, 4, 4, EPI, SEQ>, 64, 32, 4, 256);
+    if constexpr (SEQ) {
+      // tiles that leave SMs idle: a quarter of the outputs per thread on four times
+      // the warps, where packed sums would split the inputs (log_prob of 100 rows, 32-D,
+      // 8 layers, H = 256: 226 -> 177 us, 500 rows of 64-D, 4 layers, H = 64: 94 -> 78; up to
+      // two tiles per SM it was 0.9 to 1.07 of the time)
+      if ((a.M + 63) / 64 * ((a.N + 31) / 32) * count <= sm_count())
+        return go(k_gemm_f32<8, 4, 1, EPI, SEQ, 2>, 64, 32, 1, 256);
+      return go(k_gemm_f32<2, 4, 1, EPI, SEQ>, 64, 32, 1, 64);
+    } else {
+      return go(k_gemm_f32<2, 4, 4, EPI, SEQ>, 64, 32, 4, 256);
+    }
   }
   if (a.K <= 64) return go(k_gemm_f32<4, 4, 1, EPI, SEQ>, 128, 32, 1, 128);
   return go(k_gemm_f32<4, 8, 1, EPI, SEQ>, 128, 64, 1, 128);
